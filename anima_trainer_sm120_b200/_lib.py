@@ -101,6 +101,24 @@ def load() -> ctypes.CDLL:
     return lib
 
 
+_host = None
+
+
+def host():
+    """The native host path (``csrc/host``): autograd nodes and launch sequences above the library. Raises if it
+    has not been built."""
+    global _host
+    if _host is None:
+        load()                       # the library first: the module links against it
+        try:
+            from . import _host as module
+        except ImportError as e:
+            raise RuntimeError("anima_trainer_sm120_b200/_host.so cannot be loaded: build it with "
+                               f"`python -m anima_trainer_sm120_b200.build` (there is no fallback path): {e}") from e
+        _host = module
+    return _host
+
+
 def last_error() -> str:
     msg = load().anima_last_error()
     return msg.decode("utf-8", "replace") if msg else ""
@@ -161,7 +179,7 @@ def status_word(device: torch.device) -> torch.Tensor:
     idx = device.index or 0
     w = _status_words.get(idx)
     if w is None:
-        w = torch.zeros(1, dtype=torch.int32, device=device)
+        w = host().status_word(idx)
         _status_words[idx] = w
     return w
 

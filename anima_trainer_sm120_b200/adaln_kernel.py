@@ -12,7 +12,8 @@ from __future__ import annotations
 
 import torch
 
-from . import ops
+from . import fp8_quant, ops
+from ._lib import SCALES_TILED, host
 
 BF16 = torch.bfloat16
 
@@ -34,9 +35,16 @@ def _emits(x: torch.Tensor, rows: int, d: int) -> bool:
     return _EMIT_ROW_OPERAND and x.dtype == BF16 and ops.can_emit_row_codes(rows, d)
 
 
-def _flat(t: torch.Tensor, d: int) -> torch.Tensor:
-    t = t.contiguous().view(-1, d)
-    return t if t.dtype == BF16 else t.to(BF16)
+def _adopt(y: torch.Tensor, codes: torch.Tensor, scales: torch.Tensor) -> None:
+    fp8_quant.adopt_row_operand(y, ops.MXOperand(codes, scales, SCALES_TILED))
+
+
+def _rows_of(x: torch.Tensor, mod: torch.Tensor) -> tuple[int, int]:
+    """(rows, D) of an activation; the modulation tensor must have one row per (batch, time)."""
+    B, T, H, W, D = x.shape
+    N, M = B * T * H * W, mod.numel() // D if D else 0
+    assert N == M * H * W, f"shape mismatch: N={N}, M={M}, HW={H * W}"
+    return N, D
 
 
 def _need_bf16_stream(name: str, *tensors: torch.Tensor) -> None:
@@ -49,75 +57,42 @@ def _need_bf16_stream(name: str, *tensors: torch.Tensor) -> None:
                             "fp32-stream form; use the block's unpatched forward for use_fp32)")
 
 
-class FusedAdaLN(torch.autograd.Function):
-    """``LayerNorm(x, no affine, eps) * (1 + scale) + shift``."""
+class FusedAdaLN:
+    """``LayerNorm(x, no affine, eps) * (1 + scale) + shift`` (native node: ``csrc/host/norm.cpp``)."""
 
     @staticmethod
-    def forward(ctx, x, scale, shift, eps):
+    def apply(x, scale, shift, eps):
         assert x.is_cuda, "FusedAdaLN requires CUDA tensors"
         _need_bf16_stream("FusedAdaLN", x)
-        B, T, H, W, D = x.shape
-        x_flat, scale_flat, shift_flat = _flat(x, D), _flat(scale, D), _flat(shift, D)
-        N, M, HW = x_flat.shape[0], scale_flat.shape[0], H * W
-        assert N == M * HW, f"shape mismatch: N={N}, M={M}, HW={HW}"
-        if _emits(x, N, D):
-            from . import fp8_quant
-            y, mean, rstd, y_row = ops.adaln_fwd(x_flat, scale_flat, shift_flat, eps, HW, quant=True)
-            fp8_quant.adopt_row_operand(y, y_row)
-        else:
-            y, mean, rstd = ops.adaln_fwd(x_flat, scale_flat, shift_flat, eps, HW)
-        ctx.save_for_backward(x_flat, scale_flat, mean, rstd)
-        ctx.x_shape, ctx.scale_shape, ctx.HW = (B, T, H, W, D), scale.shape, HW
-        ctx.dtypes = (x.dtype, scale.dtype, shift.dtype)
-        return y.view(B, T, H, W, D).to(x.dtype)
-
-    @staticmethod
-    def backward(ctx, dy):
-        x_flat, scale_flat, mean, rstd = ctx.saved_tensors
-        B, T, H, W, D = ctx.x_shape
-        dx, dscale, dshift = ops.adaln_bwd(_flat(dy, D), x_flat, scale_flat, mean, rstd, ctx.HW)
-        xd, sd, bd = ctx.dtypes
-        return (dx.view(B, T, H, W, D).to(xd), dscale.view(ctx.scale_shape).to(sd),
-                dshift.view(ctx.scale_shape).to(bd), None)
+        N, D = _rows_of(x, scale)
+        y, codes, scales = host().adaln(x, scale, shift, eps, _emits(x, N, D))
+        if codes is not None:
+            _adopt(y, codes, scales)
+        return y
 
 
 def fused_adaln(x: torch.Tensor, scale: torch.Tensor, shift: torch.Tensor, eps: float) -> torch.Tensor:
     return FusedAdaLN.apply(x, scale, shift, eps)
 
 
-class FusedGatedAdd(torch.autograd.Function):
+class FusedGatedAdd:
     """``out = x + gate * y``; backward ``dx = dout``, ``dy = gate * dout``,
     ``dgate = sum_{h,w}(dout * y)``."""
 
     @staticmethod
-    def forward(ctx, x, gate, y):
+    def apply(x, gate, y):
         assert x.is_cuda, "FusedGatedAdd requires CUDA tensors"
         assert x.shape == y.shape, f"x {x.shape} != y {y.shape}"
         _need_bf16_stream("FusedGatedAdd", x, y)
-        B, T, H, W, D = x.shape
-        x_flat, y_flat, gate_flat = _flat(x, D), _flat(y, D), _flat(gate, D)
-        N, M, HW = x_flat.shape[0], gate_flat.shape[0], H * W
-        assert N == M * HW, f"shape mismatch: N={N}, M={M}, HW={HW}"
-        out = ops.gated_add_fwd(x_flat, gate_flat, y_flat, HW)
-        ctx.save_for_backward(y_flat, gate_flat)
-        ctx.shape, ctx.gate_shape, ctx.HW = (B, T, H, W, D), gate.shape, HW
-        ctx.dtypes = (gate.dtype, y.dtype)
-        return out.view(B, T, H, W, D).to(x.dtype)
-
-    @staticmethod
-    def backward(ctx, dout):
-        y_flat, gate_flat = ctx.saved_tensors
-        B, T, H, W, D = ctx.shape
-        dy, dgate = ops.gated_add_bwd(_flat(dout, D), y_flat, gate_flat, ctx.HW)
-        gd, yd = ctx.dtypes
-        return dout, dgate.view(ctx.gate_shape).to(gd), dy.view(B, T, H, W, D).to(yd)
+        _rows_of(x, gate)
+        return host().gated_add(x, gate, y)
 
 
 def fused_gated_add(x: torch.Tensor, gate: torch.Tensor, y: torch.Tensor) -> torch.Tensor:
     return FusedGatedAdd.apply(x, gate, y)
 
 
-class FusedGatedAddAdaLN(torch.autograd.Function):
+class FusedGatedAddAdaLN:
     """``x_new = x + gate * sub`` followed by ``y = AdaLN(x_new; scale, shift)``: the residual update of one
     sublayer and the modulation of the next, from one read of x and sub. Returns ``(x_new, y)``, each
     bit-identical to ``FusedGatedAdd`` then ``FusedAdaLN``; backward is one kernel too (the AdaLN input
@@ -125,45 +100,16 @@ class FusedGatedAddAdaLN(torch.autograd.Function):
     to the separate kernels."""
 
     @staticmethod
-    def forward(ctx, x, gate, sub, scale, shift, eps):
+    def apply(x, gate, sub, scale, shift, eps):
         assert x.is_cuda, "FusedGatedAddAdaLN requires CUDA tensors"
         assert x.shape == sub.shape, f"x {x.shape} != sub {sub.shape}"
         _need_bf16_stream("FusedGatedAddAdaLN", x, sub)
-        B, T, H, W, D = x.shape
-        x_flat, sub_flat = _flat(x, D), _flat(sub, D)
-        gate_flat, scale_flat, shift_flat = _flat(gate, D), _flat(scale, D), _flat(shift, D)
-        HW = H * W
-        assert x_flat.shape[0] == gate_flat.shape[0] * HW == scale_flat.shape[0] * HW, "modulation shape mismatch"
-        if _emits(x, x_flat.shape[0], D):
-            from . import fp8_quant
-            x_new, y, mean, rstd, y_row = ops.gated_add_adaln_fwd(x_flat, gate_flat, sub_flat, scale_flat, shift_flat,
-                                                                  eps, HW, quant=True)
-            fp8_quant.adopt_row_operand(y, y_row)
-        else:
-            x_new, y, mean, rstd = ops.gated_add_adaln_fwd(x_flat, gate_flat, sub_flat, scale_flat, shift_flat, eps, HW)
-        ctx.save_for_backward(sub_flat, gate_flat, x_new, scale_flat, mean, rstd)
-        ctx.shape, ctx.mod_shape, ctx.HW = (B, T, H, W, D), gate.shape, HW
-        ctx.dtypes = (x.dtype, gate.dtype, sub.dtype, scale.dtype, shift.dtype)
-        return x_new.view(B, T, H, W, D).to(x.dtype), y.view(B, T, H, W, D).to(x.dtype)
-
-    @staticmethod
-    def backward(ctx, d_xnew, d_y):
-        sub_flat, gate_flat, x_new, scale_flat, mean, rstd = ctx.saved_tensors
-        B, T, H, W, D = ctx.shape
-        xd, gd, ud, sd, bd = ctx.dtypes
-        if d_xnew is not None and d_y is not None:      # the usual case: one kernel for both backward ops
-            dout, dsub, dscale, dshift, dgate = ops.gated_add_adaln_bwd(
-                _flat(d_y, D), _flat(d_xnew, D), x_new, scale_flat, mean, rstd, sub_flat, gate_flat, ctx.HW)
-        else:
-            dout = None if d_xnew is None else _flat(d_xnew, D)
-            dscale = dshift = None
-            if d_y is not None:
-                dout, dscale, dshift = ops.adaln_bwd(_flat(d_y, D), x_new, scale_flat, mean, rstd, ctx.HW)
-            dsub, dgate = ops.gated_add_bwd(dout, sub_flat, gate_flat, ctx.HW)
-        if dscale is not None:
-            dscale, dshift = dscale.view(ctx.mod_shape).to(sd), dshift.view(ctx.mod_shape).to(bd)
-        return (dout.view(B, T, H, W, D).to(xd), dgate.view(ctx.mod_shape).to(gd), dsub.view(B, T, H, W, D).to(ud),
-                dscale, dshift, None)
+        N, D = _rows_of(x, gate)
+        _rows_of(x, scale)
+        x_new, y, codes, scales = host().gated_add_adaln(x, gate, sub, scale, shift, eps, _emits(x, N, D))
+        if codes is not None:
+            _adopt(y, codes, scales)
+        return x_new, y
 
 
 def fused_gated_add_adaln(x, gate, sub, scale, shift, eps):

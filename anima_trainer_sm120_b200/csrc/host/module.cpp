@@ -1,0 +1,128 @@
+// Python binding of the native host path (anima_trainer_sm120_b200._host). MXFP8 operands cross the boundary as
+// (codes, scales) tensor pairs; every call runs without the interpreter lock.
+#include <torch/csrc/Exceptions.h>
+#include <torch/csrc/utils/pybind.h>
+
+#include "linear.h"
+#include "norm.h"
+#include "tlokr.h"
+
+namespace py = pybind11;
+using namespace anima_host;
+
+namespace {
+
+using Pair = std::pair<OptTensor, OptTensor>;
+Pair pair_of(const Op& o) { return o.defined() ? Pair{o.codes, o.scales} : Pair{}; }
+
+std::pair<Pair, Pair> py_quantize(const Tensor& x, bool row, bool col, int layout) {
+  TORCH_CHECK_TYPE(x.scalar_type() == BF16, "x must be bfloat16, got ", x.scalar_type());
+  TORCH_CHECK_VALUE(x.dim() == 2, "x must be 2-D, got shape ", x.sizes());
+  const Launch l(x);
+  auto [r, c] = quantize(l, as_matrix(x, x.size(1)), row, col, layout);
+  return {pair_of(r), pair_of(c)};
+}
+
+Tensor py_gemm(const Tensor& ac, const Tensor& as, const Tensor& bc, const Tensor& bs, const OptTensor& bias) {
+  const Launch l(ac);
+  TORCH_CHECK(bc.device() == l.dev && as.device() == l.dev && bs.device() == l.dev, "tensors on different devices");
+  const Op a{ac, as}, b{bc, bs};
+  TORCH_CHECK_VALUE(!bias || (bias->scalar_type() == BF16 && bias->numel() == b.rows() && bias->is_contiguous()),
+                    "bias must be contiguous bfloat16 of length N");
+  Tensor c = empty({a.rows(), b.rows()}, BF16, l.dev);
+  gemm(l, a, b, {c.data_ptr(), b.rows(), false}, ptr(bias));
+  return c;
+}
+
+Tensor py_retile(const Tensor& scales, int64_t rows, int64_t k) {
+  const Launch l(scales);
+  const Tensor s = scales.is_contiguous() ? scales : scales.contiguous();
+  Tensor t = empty({tiled_bytes(rows, k)}, U8, l.dev);
+  check(anima_mx_scales_retile(ptr8(s), rows, k, ptr8(t), l.stream));
+  return t;
+}
+
+Tensor py_lokr(const Tensor& x, const OptTensor& xrc, const OptTensor& xrs, const OptTensor& xcc, const OptTensor& xcs,
+               const Tensor& W, const OptTensor& bias, const Tensor& w1, const Tensor& w2, double alpha, bool first) {
+  return lokr_linear(x, make_op(xrc, xrs), make_op(xcc, xcs), W, bias, w1, w2, alpha, first);
+}
+Tensor py_merged(const Tensor& x, const OptTensor& xrc, const OptTensor& xrs, const OptTensor& xcc, const OptTensor& xcs,
+                 const Tensor& merged, const OptTensor& bias, bool first) {
+  return merged_linear(x, make_op(xrc, xrs), make_op(xcc, xcs), merged, bias, first);
+}
+Tensor py_frozen(const Tensor& x, const Tensor& xrc, const Tensor& xrs, const Tensor& wrc, const Tensor& wrs,
+                 const OptTensor& wcc, const OptTensor& wcs, const OptTensor& w_bf16, const OptTensor& bias) {
+  return frozen_linear(x, {xrc, xrs}, {wrc, wrs}, make_op(wcc, wcs), w_bf16, wrc.size(1), bias);
+}
+Tensor py_lokr_mlp(const Tensor& x, const OptTensor& xrc, const OptTensor& xrs, const OptTensor& xcc, const OptTensor& xcs,
+                   const Tensor& W1, const OptTensor& b1, const Tensor& w1a, const Tensor& w2a, double alpha1,
+                   const Tensor& W2, const OptTensor& b2, const Tensor& w1b, const Tensor& w2b, double alpha2, bool first) {
+  return lokr_mlp(x, make_op(xrc, xrs), make_op(xcc, xcs), W1, b1, w1a, w2a, alpha1, W2, b2, w1b, w2b, alpha2, first);
+}
+
+TLinear py_tlinear(const Tensor& wrc, const Tensor& wrs, const Tensor& wcc, const Tensor& wcs, const OptTensor& bias,
+                   const Tensor& w1, const Tensor& a, const Tensor& b, const OptTensor& mask, double alpha, const Tensor& c,
+                   const std::vector<Tensor>& forms, bool fold, bool fuse_mix) {
+  TORCH_CHECK_VALUE(forms.size() == 8 || forms.size() == 10, "T-LoKr factor forms: 8 or 10 tensors");
+  OptTensor m = mask;
+  if (m) m = bf16_contiguous(*m);
+  TLinear t{{wrc, wrs}, {wcc, wcs}, bias, w1, a, b, m, alpha, c, {forms[0], forms[1]}, {forms[2], forms[3]},
+            {forms[4], forms[5]}, {forms[6], forms[7]}, {}, fold, fuse_mix};
+  if (forms.size() == 10) t.a_scaled = {forms[8], forms[9]};
+  return t;
+}
+Tensor py_tlokr(const Tensor& x, const OptTensor& xrc, const OptTensor& xrs, const TLinear& t, bool first) {
+  return tlokr_linear(x, make_op(xrc, xrs), t, first);
+}
+Tensor py_tlokr_mlp(const Tensor& x, const OptTensor& xrc, const OptTensor& xrs, const TLinear& t1, const TLinear& t2,
+                    bool first) {
+  return tlokr_mlp(x, make_op(xrc, xrs), t1, t2, first);
+}
+Tensor py_tlokr_fwd(const Tensor& xc, const Tensor& xs, const Tensor& gc, const Tensor& gs, const std::vector<int64_t>& lead,
+                    const TLinear& t) {
+  return tlokr_forward_only({xc, xs}, {gc, gs}, lead, t);
+}
+std::vector<Tensor> py_tlokr_bwd(const std::vector<Tensor>& g, const std::vector<Tensor>& x, const std::vector<int64_t>& lead,
+                                 const TLinear& t) {
+  return tlokr_backward_only({g.at(0), g.at(1)}, {g.at(2), g.at(3)}, {x.at(0), x.at(1)}, {x.at(2), x.at(3)}, lead, t);
+}
+
+std::tuple<Tensor, OptTensor, OptTensor> py_adaln(const Tensor& x, const Tensor& scale, const Tensor& shift, double eps,
+                                                  bool quant) {
+  auto [y, op] = adaln(x, scale, shift, eps, quant);
+  const Pair p = pair_of(op);
+  return {y, p.first, p.second};
+}
+std::tuple<Tensor, Tensor, OptTensor, OptTensor> py_gated_add_adaln(const Tensor& x, const Tensor& gate, const Tensor& sub,
+                                                                    const Tensor& scale, const Tensor& shift, double eps,
+                                                                    bool quant) {
+  auto [n, y, op] = gated_add_adaln(x, gate, sub, scale, shift, eps, quant);
+  const Pair p = pair_of(op);
+  return {n, y, p.first, p.second};
+}
+
+}  // namespace
+
+#define ANIMA_DEF(name, fn) m.def(name, torch::wrap_pybind_function_no_gil(fn))
+
+PYBIND11_MODULE(_host, m) {
+  m.doc() = "native autograd nodes and launch sequences above libanima_b200.so";
+  py::class_<TLinear>(m, "TLinear");
+  ANIMA_DEF("status_word", status_word_tensor);
+  ANIMA_DEF("mx_quantize", py_quantize);
+  ANIMA_DEF("mx_gemm", py_gemm);
+  ANIMA_DEF("scales_retile", py_retile);
+  ANIMA_DEF("lokr_linear", py_lokr);
+  ANIMA_DEF("merged_linear", py_merged);
+  ANIMA_DEF("frozen_linear", py_frozen);
+  ANIMA_DEF("lokr_mlp", py_lokr_mlp);
+  ANIMA_DEF("tlinear", py_tlinear);
+  ANIMA_DEF("tlokr_linear", py_tlokr);
+  ANIMA_DEF("tlokr_mlp", py_tlokr_mlp);
+  ANIMA_DEF("tlokr_forward_only", py_tlokr_fwd);
+  ANIMA_DEF("tlokr_backward_only", py_tlokr_bwd);
+  ANIMA_DEF("adaln", py_adaln);
+  ANIMA_DEF("gated_add", gated_add);
+  ANIMA_DEF("gated_add_adaln", py_gated_add_adaln);
+  ANIMA_DEF("rmsnorm_rope", rmsnorm_rope);
+}

@@ -31,7 +31,7 @@ import torch.nn as nn
 import torch.nn.functional as F
 
 from . import ops
-from ._lib import SCALES_TILED
+from ._lib import SCALES_TILED, host
 
 BF16 = torch.bfloat16
 MXFP8_BLOCK = 32
@@ -128,7 +128,7 @@ def quantize_activation(x: torch.Tensor, *, colwise: bool) -> tuple[ops.MXOperan
 # Activation checkpointing (non-reentrant) runs every block twice: a first pass whose saved tensors
 # are discarded, and a recomputation just before the block's backward. Inside ``first_pass()`` the
 # quantised linears therefore skip the operands that only backward reads (column-wise forms) and
-# hand ``save_for_backward`` uninitialised buffers of the same shapes, which the checkpoint drops.
+# hand ``save_for_backward`` stand-ins of the same shapes without memory, which the checkpoint drops.
 _pass = threading.local()
 
 
@@ -147,55 +147,24 @@ def in_first_pass() -> bool:
     return getattr(_pass, "first", False)
 
 
-def _placeholder(rows: int, k: int, device) -> ops.MXOperand:
-    """An operand-shaped pair of uninitialised buffers (no kernel runs)."""
-    return ops.MXOperand(torch.empty((rows, k), dtype=torch.uint8, device=device),
-                         torch.empty(ops.scales_bytes(rows, k, SCALES_TILED), dtype=torch.uint8, device=device),
-                         SCALES_TILED)
+def _wants_grad(*tensors) -> bool:
+    return torch.is_grad_enabled() and any(t is not None and t.requires_grad for t in tensors)
 
 
-def _pack(op: ops.MXOperand | None) -> tuple:
+def _pair(op: ops.MXOperand | None) -> tuple:
     return (None, None) if op is None else (op.codes, op.scales)
 
 
-def _unpack(codes, scales) -> ops.MXOperand | None:
-    return None if codes is None else ops.MXOperand(codes, scales, SCALES_TILED)
-
-
-def _bias_bf16(bias):
-    return None if bias is None else bias.detach().to(BF16).contiguous()
-
-
-class MXFP8FrozenLinear(torch.autograd.Function):
+class MXFP8FrozenLinear:
     """``y = x @ W.T (+ bias)`` for a frozen, pre-quantised W (reference signature
     ``apply(x, W_mx, W_bf16, bias)``). Forward: quantise x, MXFP8 GEMM. Backward: MXFP8 dgrad
     against the column-wise operand when ``W_mx`` carries one, else the reference's bf16
-    ``grad_y @ W_bf16`` (:171)."""
+    ``grad_y @ W_bf16`` (:171). The node itself is native (``csrc/host/linear.cpp``)."""
 
     @staticmethod
-    def forward(ctx, x, W_mx: QuantWeight, W_bf16, bias=None):
+    def apply(x, W_mx: QuantWeight, W_bf16, bias=None):
         x_row, _ = quantize_activation(x, colwise=False)
-        ctx.W_mx, ctx.W_bf16, ctx.has_bias = W_mx, W_bf16, bias is not None
-        n_out = W_bf16.shape[0]
-        if x.dtype == BF16:
-            # allocated in its final shape (not a view of a 2-D result), so a following op may update it in place
-            y = torch.empty(*x.shape[:-1], n_out, dtype=BF16, device=x.device)
-            ops.mx_gemm(x_row, W_mx.row, bias=_bias_bf16(bias), out=y.view(-1, n_out))
-            return y
-        y = ops.mx_gemm(x_row, W_mx.row, bias=_bias_bf16(bias))
-        return y.reshape(*x.shape[:-1], n_out).to(x.dtype)
-
-    @staticmethod
-    def backward(ctx, grad_y):
-        gy2 = _flat2d(grad_y)
-        if ctx.W_mx.col is not None:
-            g_row, _ = ops.mx_quantize(gy2, rowwise=True)
-            gx2 = ops.mx_gemm(g_row, ctx.W_mx.col)
-        else:
-            gx2 = gy2 @ ctx.W_bf16.to(BF16)
-        grad_x = gx2.reshape(*grad_y.shape[:-1], ctx.W_bf16.shape[1]).to(grad_y.dtype)
-        grad_bias = grad_y.reshape(-1, grad_y.shape[-1]).sum(dim=0) if ctx.has_bias else None
-        return grad_x, None, None, grad_bias
+        return host().frozen_linear(x, x_row.codes, x_row.scales, *_pair(W_mx.row), *_pair(W_mx.col), W_bf16, bias)
 
 
 def mxfp8_frozen_linear(x, W_mx, W_bf16, bias=None):
@@ -210,38 +179,16 @@ def fp8_frozen_linear(x, weight_q, weight_bf16, bias):
     return MXFP8FrozenLinear.apply(x, weight_q, weight_bf16, bias)
 
 
-class MXFP8LoKrLinear(torch.autograd.Function):
+class MXFP8LoKrLinear:
     """``y = x @ merged_W.T (+ bias)`` with merged_W quantised just in time (reference
     signature ``apply(x, merged_W, bias)``, :224-264 / :480-511): forward, dgrad and wgrad are
     MXFP8 GEMMs; x and merged_W are each read once to produce both of their operand forms."""
 
     @staticmethod
-    def forward(ctx, x, merged_W, bias=None):
+    def apply(x, merged_W, bias=None):
         first = in_first_pass()
-        need_w = ctx.needs_input_grad[1]
-        x_row, x_col = quantize_activation(x, colwise=need_w and not first)
-        w_row, w_col = ops.mx_quantize(merged_W.detach().to(BF16).contiguous(), rowwise=True, colwise=not first)
-        y = ops.mx_gemm(x_row, w_row, bias=_bias_bf16(bias))
-        if first:
-            n_out, k_in = merged_W.shape
-            w_col = _placeholder(k_in, n_out, x.device)
-            x_col = _placeholder(k_in, x_row.codes.shape[0], x.device) if need_w else None
-        ctx.save_for_backward(*_pack(x_col), *_pack(w_col))
-        ctx.has_bias, ctx.w_dtype, ctx.in_features = bias is not None, merged_W.dtype, merged_W.shape[1]
-        return y.reshape(*x.shape[:-1], merged_W.shape[0]).to(x.dtype)
-
-    @staticmethod
-    def backward(ctx, grad_y):
-        saved = ctx.saved_tensors
-        x_col, w_col = _unpack(*saved[0:2]), _unpack(*saved[2:4])
-        gy2 = _flat2d(grad_y)
-        g_row, g_col = ops.mx_quantize(gy2, rowwise=True, colwise=x_col is not None)
-        grad_x = ops.mx_gemm(g_row, w_col).reshape(*grad_y.shape[:-1], ctx.in_features).to(grad_y.dtype)
-        grad_w = None
-        if x_col is not None:
-            grad_w = ops.mx_gemm(g_col, x_col).to(ctx.w_dtype)          # gy^T @ x
-        grad_bias = grad_y.reshape(-1, grad_y.shape[-1]).sum(dim=0) if ctx.has_bias else None
-        return grad_x, grad_w, grad_bias
+        x_row, x_col = quantize_activation(x, colwise=_wants_grad(merged_W) and not first)
+        return host().merged_linear(x, *_pair(x_row), *_pair(x_col), merged_W, bias, first)
 
 
 def mxfp8_lokr_linear(x, merged_W, bias=None):
@@ -255,7 +202,7 @@ def fp8_lokr_linear(x, merged_W, bias):
     return MXFP8LoKrLinear.apply(x, merged_W, bias)
 
 
-class LoKrLinearFused(torch.autograd.Function):
+class LoKrLinearFused:
     """``y = x @ (W + alpha * kron(w1, w2)).T (+ bias)`` without ever writing the merged weight
     or its gradient's Kronecker expansion to HBM as bf16 tensors of their own:
 
@@ -264,39 +211,15 @@ class LoKrLinearFused(torch.autograd.Function):
     backward  grad_y quantised (both forms) from one read; MXFP8 dgrad; MXFP8 wgrad with fp32
               output; one pass over dW gives dw1 and dw2 (the adjoint of torch.kron that the
               reference obtains through autograd, lokr_patch.py:19-21).
+    What no gradient asks for (the dgrad of an input that needs none, every column form of a
+    no-grad pass) is not computed.
     """
 
     @staticmethod
-    def forward(ctx, x, W, bias, w1, w2, alpha: float):
+    def apply(x, W, bias, w1, w2, alpha: float):
         first = in_first_pass()
-        train = ctx.needs_input_grad[3] or ctx.needs_input_grad[4]
-        x_row, x_col = quantize_activation(x, colwise=train and not first)
-        _, w_row, w_col = ops.lokr_merge_quantize(W.detach(), w1.detach(), w2.detach(), alpha, want_merged=False,
-                                                  rowwise=True, colwise=not first)
-        y = ops.mx_gemm(x_row, w_row, bias=_bias_bf16(bias))
-        if first:
-            n_out, k_in = W.shape
-            w_col = _placeholder(k_in, n_out, x.device)
-            x_col = _placeholder(k_in, x_row.codes.shape[0], x.device) if train else None
-        ctx.save_for_backward(w1, w2, *_pack(x_col), *_pack(w_col))
-        ctx.alpha, ctx.has_bias, ctx.in_features = float(alpha), bias is not None, W.shape[1]
-        return y.reshape(*x.shape[:-1], W.shape[0]).to(x.dtype)
-
-    @staticmethod
-    def backward(ctx, grad_y):
-        saved = ctx.saved_tensors
-        w1, w2 = saved[0:2]
-        x_col, w_col = _unpack(*saved[2:4]), _unpack(*saved[4:6])
-        gy2 = _flat2d(grad_y)
-        g_row, g_col = ops.mx_quantize(gy2, rowwise=True, colwise=x_col is not None)
-        grad_x = ops.mx_gemm(g_row, w_col).reshape(*grad_y.shape[:-1], ctx.in_features).to(grad_y.dtype)
-        g_w1 = g_w2 = None
-        if x_col is not None:
-            dw = ops.mx_gemm(g_col, x_col, out_dtype=torch.float32)
-            d1, d2 = ops.lokr_kron_backward(dw, w1.detach(), w2.detach(), ctx.alpha)
-            g_w1, g_w2 = d1.to(w1.dtype), d2.to(w2.dtype)
-        grad_bias = grad_y.reshape(-1, grad_y.shape[-1]).sum(dim=0) if ctx.has_bias else None
-        return grad_x, None, grad_bias, g_w1, g_w2, None
+        x_row, x_col = quantize_activation(x, colwise=_wants_grad(w1, w2) and not first)
+        return host().lokr_linear(x, *_pair(x_row), *_pair(x_col), W, bias, w1, w2, float(alpha), first)
 
 
 def lokr_linear_fused(x, W, bias, w1, w2, alpha: float = 1.0):

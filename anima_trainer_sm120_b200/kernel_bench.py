@@ -265,11 +265,11 @@ def run(iters: int, only: str | None, small: bool, pick: str | None = None, dire
             g_row = ops.mx_regroup(gbq, rows, d_out)
             y = torch.empty(rows, d_out, dtype=BF16, device="cuda")
             gx = torch.empty(rows, d_in, dtype=BF16, device="cuda")
-            _, fops = tlokr._mx_linear_fwd(x_row, gq, lead, W_mx, None, w1, a, b, mask, 0.5)
-            t_lin = t(lambda: tlokr._mx_linear_fwd(x_row, gq, lead, W_mx, None, w1, a, b, mask, 0.5))
+            tl, host = tlokr._tlinear(W_mx, None, w1, a, b, mask, 0.5), tlokr.host()
+            t_lin = t(lambda: host.tlokr_forward_only(x_row.codes, x_row.scales, gq.codes, gq.scales, lead, tl))
             t_base = t(lambda: ops.mx_gemm(x_row, W_mx.row, out=y))
-            t_bwd = t(lambda: tlokr._mx_linear_bwd(lambda r, k: (gbq, gbq_col), lambda r, k: (gq, gq_col), lead, d_in, W_mx,
-                                                   w1, a, b, mask, 0.5, fops))
+            t_bwd = t(lambda: host.tlokr_backward_only([gbq.codes, gbq.scales, gbq_col.codes, gbq_col.scales],
+                                                       [gq.codes, gq.scales, gq_col.codes, gq_col.scales], lead, tl))
             t_dgrad = t(lambda: ops.mx_gemm(g_row, W_mx.col, out=gx))
             for direction, ms, ms_base, nbytes in (("fwd", t_lin, t_base, 2 * rows * (d_in + d_out)),
                                                    ("bwd", t_bwd, t_dgrad, 2 * rows * (2 * d_in + d_out))):

@@ -5,7 +5,7 @@ anima-trainer runs the block MLP as two independent LoKr linears with an eager G
 ``lokr_patch._patched_forward`` :47-94 and ``FP8LoKrLinear`` ``fp8_quant.py:460-511``). Per MLP that
 writes the activation ``gelu(h)`` [rows, 8192] to HBM and reads it back to quantise it, and in backward
 writes ``grad_act * gelu'(h)`` and reads it back again. Here the two linears and the activation are ONE
-autograd node:
+autograd node (native: ``csrc/host/linear.cpp``):
 
 forward   quantise x; merge+quantise W1; h = x W1^T (bf16, kept for backward);
           ``mx_quantize_gelu(h)`` emits the MXFP8 operands of gelu(h) straight from h;
@@ -27,58 +27,20 @@ from __future__ import annotations
 import torch
 import torch.nn as nn
 
-from . import lokr_patch, ops
-from .fp8_quant import _bias_bf16, _flat2d, _pack, _placeholder, _unpack, in_first_pass, quantize_activation
+from . import lokr_patch
+from ._lib import host
+from .fp8_quant import _pair, _wants_grad, in_first_pass, quantize_activation
 
 _PATCHED: dict[type, object] = {}
 
 
-class LoKrMLPFused(torch.autograd.Function):
+class LoKrMLPFused:
     @staticmethod
-    def forward(ctx, x, W1, b1, w1a, w2a, alpha1: float, W2, b2, w1b, w2b, alpha2: float):
+    def apply(x, W1, b1, w1a, w2a, alpha1: float, W2, b2, w1b, w2b, alpha2: float):
         first = in_first_pass()           # a checkpointed block's first pass keeps nothing for backward
-        train = any(ctx.needs_input_grad[i] for i in (3, 4, 8, 9))
-        both = not first
-        x_row, x_col = quantize_activation(x, colwise=train and both)
-        _, W1_row, W1_col = ops.lokr_merge_quantize(W1.detach(), w1a.detach(), w2a.detach(), alpha1, want_merged=False,
-                                                    rowwise=True, colwise=both)
-        h = ops.mx_gemm(x_row, W1_row, bias=_bias_bf16(b1))
-        a_row, a_col = ops.mx_quantize_gelu(h, rowwise=True, colwise=train and both)
-        _, W2_row, W2_col = ops.lokr_merge_quantize(W2.detach(), w1b.detach(), w2b.detach(), alpha2, want_merged=False,
-                                                    rowwise=True, colwise=both)
-        y = ops.mx_gemm(a_row, W2_row, bias=_bias_bf16(b2))
-        if first:
-            rows, (hid, k_in), n_out = h.shape[0], W1.shape, W2.shape[0]
-            W1_col, W2_col = _placeholder(k_in, hid, x.device), _placeholder(hid, n_out, x.device)
-            if train:
-                x_col, a_col = _placeholder(k_in, rows, x.device), _placeholder(hid, rows, x.device)
-        ctx.save_for_backward(h, w1a, w2a, w1b, w2b, *_pack(x_col), *_pack(a_col), *_pack(W1_col), *_pack(W2_col))
-        ctx.alphas = (float(alpha1), float(alpha2))
-        ctx.in_features = W1.shape[1]
-        return y.reshape(*x.shape[:-1], W2.shape[0]).to(x.dtype)
-
-    @staticmethod
-    def backward(ctx, grad_y):
-        saved = ctx.saved_tensors
-        h, w1a, w2a, w1b, w2b = saved[:5]
-        x_col, a_col, W1_col, W2_col = (_unpack(*saved[i:i + 2]) for i in (5, 7, 9, 11))
-        alpha1, alpha2 = ctx.alphas
-        train = x_col is not None
-        g_row, g_col = ops.mx_quantize(_flat2d(grad_y), rowwise=True, colwise=train)
-        grad_act = ops.mx_gemm(g_row, W2_col)
-        g1a = g2a = g1b = g2b = None
-        if train:
-            d1, d2 = ops.lokr_kron_backward(ops.mx_gemm(g_col, a_col, out_dtype=torch.float32),
-                                            w1b.detach(), w2b.detach(), alpha2)
-            g1b, g2b = d1.to(w1b.dtype), d2.to(w2b.dtype)
-        dh_row, dh_col = ops.mx_quantize_gelu(h, grad_act, rowwise=True, colwise=train)
-        del grad_act
-        grad_x = ops.mx_gemm(dh_row, W1_col).reshape(*grad_y.shape[:-1], ctx.in_features).to(grad_y.dtype)
-        if train:
-            d1, d2 = ops.lokr_kron_backward(ops.mx_gemm(dh_col, x_col, out_dtype=torch.float32),
-                                            w1a.detach(), w2a.detach(), alpha1)
-            g1a, g2a = d1.to(w1a.dtype), d2.to(w2a.dtype)
-        return grad_x, None, None, g1a, g2a, None, None, None, g1b, g2b, None
+        x_row, x_col = quantize_activation(x, colwise=_wants_grad(w1a, w2a, w1b, w2b) and not first)
+        return host().lokr_mlp(x, *_pair(x_row), *_pair(x_col), W1, b1, w1a, w2a, float(alpha1), W2, b2, w1b, w2b,
+                               float(alpha2), first)
 
 
 def _adapter(linear: nn.Module):

@@ -26,7 +26,7 @@ from typing import NamedTuple
 import torch
 
 from . import ops
-from ._lib import SCALES_PLAIN, SCALES_TILED
+from ._lib import SCALES_PLAIN, SCALES_TILED, host
 
 FP8_E4M3_MAX = 448.0
 
@@ -96,46 +96,29 @@ def mxfp8_matmul(A: MXFP8Block, B_data: torch.Tensor, B_scales: torch.Tensor,
             "mxfp8_matmul: the B operand must be contiguous along the contraction axis "
             f"(B_stride_k == 1, B_stride_n == K); got ({B_stride_k}, {B_stride_n})")
     a_op = _as_operand(A.data.reshape(M, K), A.scales, A.tiled)
-    b_codes = torch.as_strided(B_data, (N, K), (K, 1), B_data.storage_offset())
-    b_op = _as_operand(b_codes, B_scales, B_tiled)
-    return ops.mx_gemm(a_op, b_op, bias=bias)
+    if B_data.shape != (N, K) or not B_data.is_contiguous():
+        B_data = torch.as_strided(B_data, (N, K), (K, 1), B_data.storage_offset())
+    b_op = _as_operand(B_data, B_scales, B_tiled)
+    return host().mx_gemm(a_op.codes, a_op.scales, b_op.codes, b_op.scales, bias)
 
 
-class MXFP8FrozenLinearB200(torch.autograd.Function):
+class MXFP8FrozenLinearB200:
     """``y = x @ W.T (+ bias)`` for a frozen, pre-quantised W; forward and dgrad both run
-    as MXFP8 tensor-core GEMMs. Signature of ``MXFP8FrozenLinearTriton.apply``; the saved
-    activation is the quantised one, as in the reference (:384-385)."""
+    as MXFP8 tensor-core GEMMs. Signature of ``MXFP8FrozenLinearTriton.apply``; backward
+    reads no activation, so none is saved (the reference saves the quantised one, :384-385)."""
 
     @staticmethod
-    def forward(ctx, x, W_fwd_data, W_fwd_scales, W_bwd_data, W_bwd_scales, bias=None,
-                W_fwd_tiled=None, W_bwd_tiled=None):
-        D_in = x.shape[-1]
-        D_out = W_fwd_data.shape[0]
-        x_2d = x.reshape(-1, D_in)
-        M = x_2d.shape[0]
-        x_row, _ = ops.mx_quantize(x_2d.to(torch.bfloat16), rowwise=True, layout=SCALES_TILED)
-        w_op = _as_operand(W_fwd_data, W_fwd_scales, W_fwd_tiled)
-        y = ops.mx_gemm(x_row, w_op, bias=bias.to(torch.bfloat16) if bias is not None else None)
-        ctx.save_for_backward(x_row.codes, x_row.scales, W_bwd_data, W_bwd_scales)
-        ctx.W_bwd_tiled = W_bwd_tiled
-        ctx.D_in, ctx.D_out, ctx.M = D_in, D_out, M
-        ctx.has_bias = bias is not None
-        ctx.x_orig_shape = x.shape
-        return y.reshape(*x.shape[:-1], D_out).to(x.dtype)
-
-    @staticmethod
-    def backward(ctx, grad_y):
-        _, _, W_bwd_data, W_bwd_scales = ctx.saved_tensors
-        gy_2d = grad_y.reshape(ctx.M, ctx.D_out)
-        gy_row, _ = ops.mx_quantize(gy_2d.to(torch.bfloat16), rowwise=True, layout=SCALES_TILED)
+    def apply(x, W_fwd_data, W_fwd_scales, W_bwd_data, W_bwd_scales, bias=None, W_fwd_tiled=None, W_bwd_tiled=None):
+        x_2d = x.reshape(-1, x.shape[-1])
+        x_row, _ = ops.mx_quantize(x_2d if x_2d.dtype == torch.bfloat16 else x_2d.to(torch.bfloat16), rowwise=True,
+                                   layout=SCALES_TILED)
+        w = _as_operand(W_fwd_data, W_fwd_scales, W_fwd_tiled)
         # W_bwd_data is the (D_out, D_in) view of a (D_in, D_out) buffer: K-major for dgrad.
         wT = W_bwd_data.t()
         if not wT.is_contiguous():
             raise NotImplementedError("W_bwd must come from quantize_weight_for_dgrad()")
-        w_op = _as_operand(wT, W_bwd_scales, ctx.W_bwd_tiled)
-        grad_x = ops.mx_gemm(gy_row, w_op).reshape(ctx.x_orig_shape).to(grad_y.dtype)
-        grad_bias = grad_y.reshape(-1, ctx.D_out).sum(dim=0) if ctx.has_bias else None
-        return grad_x, None, None, None, None, grad_bias, None, None
+        w_bwd = _as_operand(wT, W_bwd_scales, W_bwd_tiled)
+        return host().frozen_linear(x, x_row.codes, x_row.scales, w.codes, w.scales, w_bwd.codes, w_bwd.scales, None, bias)
 
 
 MXFP8FrozenLinearTriton = MXFP8FrozenLinearB200  # name used by anima-trainer call sites

@@ -85,10 +85,8 @@ def mx_quantize(
     (``[rows, cols]``), ``col_op`` is x quantised along its rows and stored
     transposed (``[cols, rows]``) — i.e. ``quantize_rowwise(x.t().contiguous())``.
     """
-    _bf16_2d(x, "x")
-    if x.stride(1) != 1 and x.shape[1] > 1:
-        x = x.contiguous()
-    return _quantize_call("anima_mx_quantize", x, (), rowwise, colwise, layout)
+    row, col = _lib.host().mx_quantize(x, rowwise, colwise, layout)
+    return MXOperand(*row, layout) if rowwise else None, MXOperand(*col, layout) if colwise else None
 
 
 def mx_quantize_gelu(
@@ -127,12 +125,7 @@ def mx_retile(op: MXOperand) -> MXOperand:
     """PLAIN-scaled operand -> TILED-scaled operand (codes are shared, not copied)."""
     if op.layout == SCALES_TILED:
         return op
-    dev = _lib.require_cuda(op.codes, op.scales)
-    tiled = _alloc_scales(op.rows, op.k, SCALES_TILED, dev)
-    with torch.cuda.device(dev):
-        check(_lib.load().anima_mx_scales_retile(ptr(op.scales.contiguous()), op.rows, op.k, ptr(tiled),
-                                                 _lib.stream_ptr(dev)))
-    return MXOperand(op.codes, tiled, SCALES_TILED)
+    return MXOperand(op.codes, _lib.host().scales_retile(op.scales, op.rows, op.k), SCALES_TILED)
 
 
 def mx_regroup(op: MXOperand, rows: int, k: int) -> MXOperand:

@@ -16,7 +16,7 @@ import weakref
 
 import torch
 
-from . import ops
+from ._lib import host
 
 _PATCHED: dict[type, object] = {}
 _tables: tuple[weakref.ref, torch.Tensor, torch.Tensor] | None = None
@@ -33,23 +33,12 @@ def rope_tables(rope_emb: torch.Tensor) -> tuple[torch.Tensor, torch.Tensor]:
     return cos, sin
 
 
-class FusedRMSNormRoPE(torch.autograd.Function):
-    """out = rope(rmsnorm(x) * weight); x (B, L, H, 128) bf16. Gradient for x only."""
+class FusedRMSNormRoPE:
+    """out = rope(rmsnorm(x) * weight); x (B, L, H, 128) bf16. Gradient for x only (native: ``csrc/host/norm.cpp``)."""
 
     @staticmethod
-    def forward(ctx, x, weight, cos, sin, eps):
-        x = x.contiguous()
-        w = weight.detach().float().contiguous()
-        out, rstd = ops.rmsnorm_rope_fwd(x, w, cos, sin, eps)
-        ctx.save_for_backward(x, w, rstd)
-        ctx.tables = (cos, sin)
-        return out
-
-    @staticmethod
-    def backward(ctx, dout):
-        x, w, rstd = ctx.saved_tensors
-        cos, sin = ctx.tables
-        return ops.rmsnorm_rope_bwd(dout.contiguous(), x, w, cos, sin, rstd), None, None, None, None
+    def apply(x, weight, cos, sin, eps):
+        return host().rmsnorm_rope(x, weight, cos, sin, eps)
 
 
 def _fusable(t: torch.Tensor, norm) -> bool:

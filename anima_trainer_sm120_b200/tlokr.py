@@ -32,6 +32,7 @@ import torch.nn as nn
 import torch.nn.functional as F
 
 from . import ops
+from ._lib import host
 from .tlokr_kernels import rank_mix, rank_mix_wgrad
 
 _FORMAT_VERSION = 1
@@ -281,11 +282,6 @@ FOLD_DELTA = os.environ.get("ANIMA_TLOKR_FOLD_DELTA", "1") != "0"
 FUSE_HIDDEN_MIX = os.environ.get("ANIMA_TLOKR_FUSE_HIDDEN_MIX", "1") != "0"
 
 
-def _can_fold(rows: int, n_cols: int, factor_dim: int, batch: int, rank: int) -> bool:
-    return (FOLD_DELTA and factor_dim == 8 and ops.can_fold_delta(rows, n_cols) and rows % batch == 0
-            and ops.can_mix_to_planes(batch, rows // batch, rank))
-
-
 def _q(t2d: torch.Tensor, *, col: bool = False):
     return ops.mx_quantize(t2d.contiguous() if t2d.dtype == BF16 else t2d.to(BF16).contiguous(),
                            rowwise=True, colwise=col)
@@ -394,218 +390,56 @@ def _structured_delta(module, x: torch.Tensor, *, fp8: bool, base: torch.Tensor 
     return torch.add(base, fn.apply(*args), alpha=alpha)
 
 
-def _mix_operands(hidden, c, mask, transpose: bool, *, row: bool, col: bool):
-    """MXFP8 operands (row form, column form) of ``rank_mix(hidden, c, mask, transpose=...)`` viewed as
-    ``[-1, rank]``. The mix kernel writes them itself where the shape allows, so the mixed tensor never exists in
-    bf16; otherwise the mix is followed by a quantiser launch. Same bits either way."""
-    batch, n, _, rank = hidden.shape
-    # at [8, 4096, 8, 128] the kernel's row form beats mix + quantiser (38.4 against 28.7 + 18.9 us); its column
-    # forms do not (46.6 against 28.7 + 16.9, 62.0 against 28.7 + 30.7), so those keep the two kernels
-    if not col and ops.can_quantise_rank_mix(batch, n, rank):
-        m = None if mask is None else mask.contiguous().to(BF16)
-        r, cl, _ = ops.tlokr_rank_mix_quant(hidden.contiguous(), c.contiguous(), m, transpose, rowwise=row, colwise=col)
-        return r, cl
-    mixed = rank_mix(hidden, c, mask, transpose=transpose)
-    return ops.mx_quantize(mixed.reshape(-1, rank), rowwise=row, colwise=col)
-
-
-def _mx_linear_fwd(x_row, gq, lead_shape, W_mx, bias, w1, w2_a, w2_b, mask, alpha):
-    """``y = x W^T + bias + alpha * delta(x)`` from the row-wise MXFP8 operand of x viewed as ``[rows, K]``
-    (``x_row``) and as the grouped ``[rows * uq, K / uq]`` (``gq``): the same code bytes under two scale tilings.
-    Returns (y, small factor operands kept for backward)."""
-    from .fp8_quant import _bias_bf16
+def _tlinear(W_mx, bias, w1, w2_a, w2_b, mask, alpha: float):
+    """The native description of one quantised T-LoKr linear: base operands, parameters, mask and the factors'
+    forms (kept per parameter version by :func:`_factor_forms`)."""
     c = _factor_forms(w1, quantise=False)
-    uq = c.shape[1]
-    vp, rank = w2_a.shape
-    n_out = W_mx.row.rows
-    aq, aq_col = _factor_forms(w2_a, quantise=True)      # A [vp, r]: row form for out, column form for dgrad
-    bq, bq_col = _factor_forms(w2_b, quantise=True)      # B [r, vq]
-    y = torch.empty(*lead_shape, n_out, dtype=BF16, device=x_row.codes.device)
-    if _can_fold(x_row.rows, n_out, c.shape[0], lead_shape[0], rank) and n_out == c.shape[0] * vp and uq == 8:
-        # Two kernels for the whole linear: (1) hidden = grouped . B^T, the 8x8 mix, the mask and the quantisation
-        # of the mixed tensor, which leaves as eight e4m3 planes (hidden itself stays on the SM); (2) ONE GEMM in
-        # which those planes times alpha * A enter as extra K-blocks of the base projection.
-        m = None if mask is None else mask.contiguous().to(BF16)
-        if FUSE_HIDDEN_MIX:
-            planes, _ = ops.tlokr_hidden_mix_planes(gq, bq, c, m, lead_shape[0], False)
-        else:
-            hidden = ops.mx_gemm(gq, bq).view(lead_shape[0], -1, uq, rank)
-            planes, _ = ops.tlokr_rank_mix_quant_planes(hidden, c, m, False)
-        ops.mx_gemm_delta(x_row, W_mx.row, planes, _scaled_row_form(w2_a, alpha), bias=_bias_bf16(bias),
-                          out=y.view(-1, n_out))
-        return y, (aq_col, bq, bq_col)
-    hidden = ops.mx_gemm(gq, bq).view(lead_shape[0], -1, uq, rank)
-    ops.mx_gemm(x_row, W_mx.row, bias=_bias_bf16(bias), out=y.view(-1, n_out))
-    mq, _ = _mix_operands(hidden, c, mask, False, row=True, col=False)
-    res = y.view(-1, vp)
-    ops.mx_gemm(mq, aq, residual=res, alpha=float(alpha), out=res)       # y += alpha * delta
-    return y, (aq_col, bq, bq_col)
+    forms = []
+    for p in (w2_a, w2_b):                               # A [vp, r], B [r, vq]: row and column operands of each
+        for op in _factor_forms(p, quantise=True):
+            forms += (op.codes, op.scales)
+    if FOLD_DELTA and w2_a.shape[1] == 128:              # alpha * A, the factor a folded delta multiplies by
+        op = _scaled_row_form(w2_a, alpha)
+        forms += (op.codes, op.scales)
+    return host().tlinear(W_mx.row.codes, W_mx.row.scales, W_mx.col.codes, W_mx.col.scales, bias, w1, w2_a, w2_b, mask,
+                          float(alpha), c, forms, FOLD_DELTA, FUSE_HIDDEN_MIX)
 
 
-def _input_operands(quantise, rows: int, K: int, uq: int, keep: bool, device):
-    """MXFP8 operands of a layer input for forward and backward. ``quantise(r, k, col)`` quantises the input viewed
-    as ``[r, k]``. With ``keep`` (a pass whose saved tensors backward will read) the grouped view is quantised in both
-    forms once, so that backward needs neither the bf16 input nor another pass over it; otherwise only the row form
-    is made and uninitialised buffers of the same shapes stand in for what a checkpoint drops anyway.
-    Returns (x_row [rows, K], gq [rows * uq, K / uq], gq_col [K / uq, rows * uq])."""
-    from .fp8_quant import _placeholder
-    if keep:
-        gq, gq_col = quantise(rows * uq, K // uq, True)
-        return ops.mx_regroup(gq, rows, K), gq, gq_col
-    x_row, _ = quantise(rows, K, False)
-    return x_row, ops.mx_regroup(x_row, rows * uq, K // uq), _placeholder(K // uq, rows * uq, device)
+def _row_operand_unless_kept(x, *trainable):
+    """Row-wise operand of x for a pass that backward will not read, else (None, None): the node then quantises the
+    grouped view of x in both forms itself, and its row codes serve the base GEMM too."""
+    from .fp8_quant import _pair, _wants_grad, in_first_pass, quantize_activation
+    first = in_first_pass()
+    if _wants_grad(x, *trainable) and not first:
+        return (None, None), first
+    return _pair(quantize_activation(x, colwise=False)[0]), first
 
 
-def _mx_linear_bwd(quant_grad, quant_grouped, lead_shape, K, W_mx, w1, w2_a, w2_b, mask, alpha, factor_ops):
-    """Backward of :func:`_mx_linear_fwd`. ``quant_grad(rows, k)`` returns the (row, column) MXFP8 operands of the
-    incoming gradient viewed as ``[rows, k]``, so a caller can fold an elementwise op (the derivative of the MLP
-    activation) into that quantisation; ``quant_grouped(rows, k)`` returns the operands of the layer input in its
-    grouped view (saved by the forward pass). Returns (grad_x bf16 [*lead, K], grad_w1, grad_A, grad_B)."""
-    aq_col, bq, bq_col = factor_ops
-    c = _factor_forms(w1, quantise=False)
-    up, uq = c.shape
-    vp, rank = w2_a.shape
-    vq = K // uq
-    rows = 1
-    for d in lead_shape:
-        rows *= d
-    gbq, gbq_col = quant_grad(rows * up, vp)                                        # grad as [rows * up, vp]
-    g_x = torch.empty(*lead_shape, K, dtype=BF16, device=gbq.codes.device)
-    fold = _can_fold(rows, K, uq, lead_shape[0], rank) and K == uq * vq
-    if not fold:
-        ops.mx_gemm(ops.mx_regroup(gbq, rows, up * vp), W_mx.col, out=g_x.view(rows, K))   # base dgrad
-    gq, gq_col = quant_grouped(rows * uq, vq)
-    hidden = ops.mx_gemm(gq, bq).view(lead_shape[0], -1, uq, rank)
-    _, mq_col = _mix_operands(hidden, c, mask, False, row=False, col=True)
-    g_a = ops.mx_gemm(gbq_col, mq_col, out_dtype=torch.float32, alpha=alpha)        # alpha * grad^T @ mixed  [vp, r]
-    g_mixed = ops.mx_gemm(gbq, aq_col, alpha=alpha).view(*hidden.shape)             # alpha * grad @ A        [.., r]
-    g_c = rank_mix_wgrad(g_mixed, hidden, mask)
-    if fold:
-        # grad_hidden leaves as eight planes + its column form; base dgrad and + grad_hidden @ B are one GEMM
-        gh_planes, ghq_col = ops.tlokr_rank_mix_quant_planes(
-            g_mixed, c, None if mask is None else mask.contiguous().to(BF16), True, colwise=True)
-        g_b = ops.mx_gemm(ghq_col, gq_col, out_dtype=torch.float32)                 # grad_hidden^T @ grouped [r, vq]
-        ops.mx_gemm_delta(ops.mx_regroup(gbq, rows, up * vp), W_mx.col, gh_planes, bq_col, out=g_x.view(rows, K))
-        return g_x, g_c.to(w1.dtype), g_a.to(w2_a.dtype), g_b.to(w2_b.dtype)
-    ghq, ghq_col = _mix_operands(g_mixed, c, mask, True, row=True, col=True)        # of grad_hidden
-    g_b = ops.mx_gemm(ghq_col, gq_col, out_dtype=torch.float32)                     # grad_hidden^T @ grouped [r, vq]
-    res = g_x.view(-1, vq)
-    ops.mx_gemm(ghq, bq_col, residual=res, out=res)                                 # g_x += grad_hidden @ B
-    return g_x, g_c.to(w1.dtype), g_a.to(w2_a.dtype), g_b.to(w2_b.dtype)
-
-
-def _bf16c(t: torch.Tensor) -> torch.Tensor:
-    return t.contiguous() if t.dtype == BF16 else t.to(BF16).contiguous()
-
-
-class _MXTLoKrLinear(torch.autograd.Function):
-    """The whole quantised T-LoKr linear, ``x W^T + bias + alpha * delta(x)``, as ONE autograd node.
+class _MXTLoKrLinear:
+    """The whole quantised T-LoKr linear, ``x W^T + bias + alpha * delta(x)``, as ONE autograd node
+    (native: ``csrc/host/tlokr.cpp``).
 
     The reference runs a frozen FP8 base projection (``fp8_frozen_linear``, ``tlokr.py:743``), the
     structured delta (``_FP8StructuredLoKr``, :543-676) and ``torch.add(base, delta, alpha=)`` (:757-759) as
-    three nodes, each quantising its own inputs. As one node:
-
-    * x is quantised row-wise ONCE: the base GEMM contracts it as [rows, K], the delta as the grouped view
-      [rows * uq, K / uq]; the code bytes are the same, only the scales are re-tiled (``ops.mx_regroup``);
-      likewise the incoming gradient serves the base dgrad and the delta chain from one quantisation;
-    * ``+ alpha * delta`` and, in backward, ``+ grad_x(delta)`` are added by the stores of the last GEMM of
-      each chain into the buffer the base GEMM wrote: no separate add kernels, no autograd sum.
-
-    What is saved for backward are the MXFP8 operands of x in its grouped view (both forms, made by one pass
-    over x in the forward that backward will use) and the small factors; the rank-space intermediates are
-    recomputed in backward, as in the reference."""
+    three nodes, each quantising its own inputs. As one node x and the incoming gradient are quantised once each,
+    and the delta enters the base GEMMs (forward and input gradient) as extra K-blocks where the shape allows."""
 
     @staticmethod
-    def forward(ctx, x, W_mx, bias, w1, w2_a, w2_b, mask, alpha: float):
-        from .fp8_quant import _pack, in_first_pass, quantize_activation
-        K, uq = x.shape[-1], w1.shape[1]
-        rows = x.numel() // K
-        train = any(ctx.needs_input_grad[i] for i in (0, 3, 4, 5))
-        keep = train and not in_first_pass()
+    def apply(x, W_mx, bias, w1, w2_a, w2_b, mask, alpha: float):
+        x_row, first = _row_operand_unless_kept(x, w1, w2_a, w2_b, bias)
+        return host().tlokr_linear(x, *x_row, _tlinear(W_mx, bias, w1, w2_a, w2_b, mask, alpha), first)
 
-        def quantise(r, k, col):
-            if not col and (r, k) == (rows, K):
-                return quantize_activation(x, colwise=False)        # shared with other consumers of x
-            return _q(x.reshape(r, k), col=col)
 
-        x_row, gq, gq_col = _input_operands(quantise, rows, K, uq, keep, x.device)
-        y, factor_ops = _mx_linear_fwd(x_row, gq, x.shape[:-1], W_mx, bias, w1, w2_a, w2_b, mask, alpha)
-        ctx.save_for_backward(w1, w2_a, w2_b, *_pack(gq), *_pack(gq_col), *(() if mask is None else (mask,)))
-        ctx.has_mask, ctx.ops, ctx.W_mx = mask is not None, factor_ops, W_mx
-        ctx.alpha, ctx.bias_grad, ctx.x_shape = float(alpha), bias is not None and bias.requires_grad, x.shape
-        return y
+class _MXTLoKrMLP:
+    """``layer2(gelu(layer1(x)))`` with both layers quantised T-LoKr linears, as one native node: the activation and
+    its derivative are evaluated inside the quantiser, so neither ``gelu(h)`` nor ``grad * gelu'(h)`` is ever written
+    as a bf16 tensor."""
 
     @staticmethod
-    def backward(ctx, grad_output):
-        from .fp8_quant import _unpack
-        saved = ctx.saved_tensors        # read once: activation checkpointing unpacks on access
-        w1, w2_a, w2_b = saved[:3]
-        gq, gq_col = _unpack(*saved[3:5]), _unpack(*saved[5:7])
-        mask = saved[7] if ctx.has_mask else None
-        gy = _bf16c(grad_output)
-        g_x, g_c, g_a, g_b = _mx_linear_bwd(
-            lambda r, k: _q(gy.view(r, k), col=True), lambda r, k: (gq, gq_col),
-            ctx.x_shape[:-1], ctx.x_shape[-1], ctx.W_mx, w1, w2_a, w2_b, mask, ctx.alpha, ctx.ops)
-        g_bias = gy.reshape(-1, gy.shape[-1]).sum(dim=0) if ctx.bias_grad else None
-        return g_x, None, g_bias, g_c, g_a, g_b, None, None
-
-
-class _MXTLoKrMLP(torch.autograd.Function):
-    """``layer2(gelu(layer1(x)))`` with both layers quantised T-LoKr linears, as one node: the activation and
-    its derivative are evaluated inside the quantiser (``ops.mx_quantize_gelu``), so neither ``gelu(h)`` nor
-    ``grad * gelu'(h)`` is ever written as a bf16 tensor. Saves the pre-activation h, the grouped MXFP8 operands of
-    both layer inputs and the factors."""
-
-    @staticmethod
-    def forward(ctx, x, W1, b1, w1_1, a_1, b_1, mask1, alpha1: float, W2, b2, w1_2, a_2, b_2, mask2, alpha2: float):
-        from .fp8_quant import _pack, in_first_pass, quantize_activation
-        K, lead = x.shape[-1], x.shape[:-1]
-        rows = x.numel() // K
-        train = any(ctx.needs_input_grad[i] for i in (0, 3, 4, 5, 10, 11, 12))
-        keep = train and not in_first_pass()
-
-        def quantise_x(r, k, col):
-            if not col and (r, k) == (rows, K):
-                return quantize_activation(x, colwise=False)
-            return _q(x.reshape(r, k), col=col)
-
-        x_row, gq1, gq1_col = _input_operands(quantise_x, rows, K, w1_1.shape[1], keep, x.device)
-        h, ops1 = _mx_linear_fwd(x_row, gq1, lead, W1, b1, w1_1, a_1, b_1, mask1, alpha1)
-        hid = h.shape[-1]
-        act_row, gq2, gq2_col = _input_operands(
-            lambda r, k, col: ops.mx_quantize_gelu(h.view(r, k), rowwise=True, colwise=col),
-            rows, hid, w1_2.shape[1], keep, x.device)
-        y, ops2 = _mx_linear_fwd(act_row, gq2, lead, W2, b2, w1_2, a_2, b_2, mask2, alpha2)
-        masks = tuple(m for m in (mask1, mask2) if m is not None)
-        ctx.save_for_backward(h, w1_1, a_1, b_1, w1_2, a_2, b_2, *_pack(gq1), *_pack(gq1_col), *_pack(gq2),
-                              *_pack(gq2_col), *masks)
-        ctx.has_masks = (mask1 is not None, mask2 is not None)
-        ctx.ops, ctx.W = (ops1, ops2), (W1, W2)
-        ctx.alphas, ctx.x_shape = (float(alpha1), float(alpha2)), x.shape
-        return y
-
-    @staticmethod
-    def backward(ctx, grad_output):
-        from .fp8_quant import _unpack
-        saved = ctx.saved_tensors
-        h, w1_1, a_1, b_1, w1_2, a_2, b_2 = saved[:7]
-        gq1, gq1_col, gq2, gq2_col = (_unpack(*saved[i:i + 2]) for i in (7, 9, 11, 13))
-        rest = list(saved[15:])
-        mask1 = rest.pop(0) if ctx.has_masks[0] else None
-        mask2 = rest.pop(0) if ctx.has_masks[1] else None
-        gy = _bf16c(grad_output)
-        lead = ctx.x_shape[:-1]
-        # layer 2: its input gelu(h) was quantised straight from h by the forward pass
-        g_act, g_c2, g_a2, g_b2 = _mx_linear_bwd(
-            lambda r, k: _q(gy.view(r, k), col=True), lambda r, k: (gq2, gq2_col),
-            lead, h.shape[-1], ctx.W[1], w1_2, a_2, b_2, mask2, ctx.alphas[1], ctx.ops[1])
-        # layer 1: its incoming gradient is g_act * gelu'(h), formed inside the quantiser
-        g_x, g_c1, g_a1, g_b1 = _mx_linear_bwd(
-            lambda r, k: ops.mx_quantize_gelu(h.view(r, k), g_act.view(r, k), rowwise=True, colwise=True),
-            lambda r, k: (gq1, gq1_col),
-            lead, ctx.x_shape[-1], ctx.W[0], w1_1, a_1, b_1, mask1, ctx.alphas[0], ctx.ops[0])
-        return (g_x, None, None, g_c1, g_a1, g_b1, None, None,
-                None, None, g_c2, g_a2, g_b2, None, None)
+    def apply(x, W1, b1, w1_1, a_1, b_1, mask1, alpha1: float, W2, b2, w1_2, a_2, b_2, mask2, alpha2: float):
+        x_row, first = _row_operand_unless_kept(x, w1_1, a_1, b_1, w1_2, a_2, b_2)
+        return host().tlokr_mlp(x, *x_row, _tlinear(W1, b1, w1_1, a_1, b_1, mask1, alpha1),
+                                _tlinear(W2, b2, w1_2, a_2, b_2, mask2, alpha2), first)
 
 
 class _ActSpec(NamedTuple):
