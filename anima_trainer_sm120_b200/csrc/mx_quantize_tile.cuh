@@ -53,6 +53,40 @@ __device__ __forceinline__ uint32_t bf16x2_mul(uint32_t a, uint32_t b) {
   return *reinterpret_cast<const uint32_t*>(&r);
 }
 
+// Exponent and conversion of one row block from its packed bf16 bits. `am` is the block's largest |x| in each half
+// of a word (sign bits clear). On the 15 magnitude bits a of a bf16 the rule of mx_exponent is a shift: e + 127 =
+// ((a + 31) >> 7) - 8, because mantissa > 1.75 is exactly what carries; amax below 1e-30 gives 19, inf / nan 254.
+__device__ __forceinline__ uint32_t mx_scale_byte(uint32_t am) {
+  const uint32_t a = max(am & 0xffffu, am >> 16);
+  const int sb = max(19, static_cast<int>((a + 31u) >> 7) - 8);
+  return a >= 0x7f80u ? 254u : static_cast<uint32_t>(sb);
+}
+// 2^-e as a bf16 in both halves
+__device__ __forceinline__ uint32_t mx_inv_bf16x2(uint32_t sb) {
+  const uint32_t one = sb >= 254u ? 0x0040u : (254u - sb) << 7;
+  return one | (one << 16);
+}
+// four values (two words) times 2^-e -> four e4m3 codes; the packed bf16 product is exact for a power of two
+__device__ __forceinline__ uint32_t mx_codes4(uint32_t w0, uint32_t w1, uint32_t inv2) {
+  const uint32_t a = bf16x2_mul(w0, inv2), b = bf16x2_mul(w1, inv2);
+  return e4m3x2(__uint_as_float(a << 16), __uint_as_float(a & 0xffff0000u)) |
+         (e4m3x2(__uint_as_float(b << 16), __uint_as_float(b & 0xffff0000u)) << 16);
+}
+// Scale byte and codes of the 8 values a thread holds of a 32-value row block spread over four adjacent lanes (all
+// lanes of the warp call it). The running maximum starts at 0 and ignores NaN, as fmaxf does.
+__device__ __forceinline__ uint32_t mx_row_block(const uint4& v, uint2& codes) {
+  uint32_t am = bf16x2_max(0u, v.x & 0x7fff7fffu);
+  am = bf16x2_max(am, v.y & 0x7fff7fffu);
+  am = bf16x2_max(am, v.z & 0x7fff7fffu);
+  am = bf16x2_max(am, v.w & 0x7fff7fffu);
+  am = bf16x2_max(am, __shfl_xor_sync(0xffffffffu, am, 1));
+  am = bf16x2_max(am, __shfl_xor_sync(0xffffffffu, am, 2));
+  const uint32_t sb = mx_scale_byte(am), inv2 = mx_inv_bf16x2(sb);
+  codes.x = mx_codes4(v.x, v.y, inv2);
+  codes.y = mx_codes4(v.z, v.w, inv2);
+  return sb;
+}
+
 __device__ __forceinline__ int tiled_offset(int r, int j) {
   return (r & 31) * 16 + (r >> 5) * 4 + j;
 }

@@ -322,6 +322,30 @@ int anima_gated_add_adaln_bwd(const void* d_y, const void* d_xnew, const void* x
                               void* dshift, void* dgate, void* workspace, int64_t workspace_bytes,
                               void* stream);
 
+/* The AdaLN and gated-residual kernels with every option (the entries above are these with dense modulation rows and
+ * all outputs). ld_mod / ld_gate: elements between the modulation rows of consecutive samples (a multiple of 8, >= d),
+ * so that scale, shift and gate may be chunks of one tensor.
+ *   fwd_ex   sub != NULL: x_new = x + gate * sub first; codes_row != NULL: the row-wise operand of y too.
+ *   bwd_ex   d_res != NULL: dx = d_res + the LayerNorm gradient (the other gradient of the same tensor, bf16);
+ *            sub != NULL (needs d_res): also dsub and dgate of the gated residual that made x.
+ *            dscale, dshift and dgate may be NULL: not computed, and with all of them NULL no workspace is used.
+ *   gated_add_bwd_ex   dgate may be NULL (then y may be, and no workspace is used).
+ * Workspaces: anima_adaln_bwd_workspace_bytes (no sub), anima_gated_add_adaln_bwd_workspace_bytes (sub),
+ * anima_gated_add_bwd_workspace_bytes. */
+int anima_adaln_fwd_ex(const void* x, const void* gate, const void* sub, const void* scale, const void* shift,
+                       int64_t ld_mod, float eps, int64_t rows, int64_t hw, int64_t d, void* x_new, void* y,
+                       float* mean, float* rstd, uint8_t* codes_row, uint8_t* scales_row, int scale_layout,
+                       void* stream);
+int anima_adaln_bwd_ex(const void* dy, const void* d_res, const void* x, const void* scale, const void* gate,
+                       const void* sub, int64_t ld_mod, const float* mean, const float* rstd, int64_t rows,
+                       int64_t hw, int64_t d, void* dx, void* dsub, void* dscale, void* dshift, void* dgate,
+                       void* workspace, int64_t workspace_bytes, void* stream);
+int anima_gated_add_fwd_ex(const void* x, const void* gate, int64_t ld_gate, const void* y, int64_t rows,
+                           int64_t hw, int64_t d, void* out, void* stream);
+int anima_gated_add_bwd_ex(const void* dout, const void* y, const void* gate, int64_t ld_gate, int64_t rows,
+                           int64_t hw, int64_t d, void* dy, void* dgate, void* workspace,
+                           int64_t workspace_bytes, void* stream);
+
 /* ---------------------------------------------------------------- T-LoKr rank mix
  * ref: tlokr_kernels.py:15-82, :125-166 (rank_mix).
  * hidden, out bf16 [batch, n, 8, rank]; c bf16 [8,8]; mask bf16 [batch, rank] or NULL.

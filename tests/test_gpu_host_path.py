@@ -85,3 +85,48 @@ def test_every_gradient_subset_and_the_checkpointed_pass_give_the_same_bits(make
 
     y3, again = go(everything, checkpointed)
     assert torch.equal(y3, y) and all(torch.equal(a, b) for a, b in zip(again, grads))
+
+
+def _block_inputs(B, hw, D, mod_grad, chunked):
+    g = torch.Generator(device=DEV).manual_seed(hw + D)
+    x, sub = (_randn(g, B, 1, hw, 1, D).requires_grad_(True) for _ in range(2))
+    if chunked:                               # chunks of one (B, 1, 3 D) tensor, as a modulation MLP returns them
+        mods = [m[:, :, None, None, :] for m in (_randn(g, B, 1, 6 * D, std=0.1)).chunk(6, dim=-1)[:4]]
+    else:
+        mods = [_randn(g, B, 1, 1, 1, D, std=0.1) for _ in range(4)]
+    mods = [m.detach().requires_grad_(mod_grad) for m in mods]
+    return x, sub, mods, [_randn(g, B, 1, hw, 1, D) for _ in range(3)]
+
+
+@pytest.mark.parametrize("B,hw,D", [(2, 24, 256), (1, 7, 2048), (3, 130, 264), (2, 16, 4096)])
+@pytest.mark.parametrize("mod_grad,chunked", [(True, False), (False, True), (True, True)])
+def test_residual_gradient_through_the_modulation_equals_the_separate_sum(B, hw, D, mod_grad, chunked):
+    """x feeds a modulation and the gated residual behind it: its gradient is formed in the modulation's backward
+    kernel. The same graph with the residual reading an unrelated alias of x adds the two gradients in bf16."""
+    from anima_trainer_sm120_b200.adaln_kernel import fused_adaln, fused_gated_add_adaln
+    results = []
+    for routed in (True, False):
+        x, sub, (g0, sc, sh, sc1), (gn, gx, gy) = _block_inputs(B, hw, D, mod_grad, chunked)
+        n = fused_adaln(x, sc, sh, 1e-6)
+        x_new, y = fused_gated_add_adaln(x if routed else x.view_as(x), g0, sub, sc1, sh, 1e-6)
+        mods = [m for m in (g0, sc, sh, sc1) if mod_grad]
+        results.append([n.detach(), x_new.detach(), y.detach(),
+                        *torch.autograd.grad([n, x_new, y], [x, sub, *mods], [gn, gx, gy])])
+    for a, b in zip(*results):
+        assert torch.equal(a, b)
+
+
+def test_modulation_and_residual_can_be_backpropagated_one_after_the_other():
+    from anima_trainer_sm120_b200.adaln_kernel import fused_adaln, fused_gated_add
+    for order in ((0, 1), (1, 0)):
+        grads = []
+        for routed in (True, False):
+            x, sub, (g0, sc, sh, _), (gn, gx, _) = _block_inputs(2, 24, 256, True, False)
+            outs = [fused_adaln(x, sc, sh, 1e-6), fused_gated_add(x if routed else x.view_as(x), g0, sub)]
+            for i in order:
+                outs[i].backward((gn, gx)[i])
+            grads.append([t.grad for t in (x, sub, g0, sc, sh)])
+            with pytest.raises(RuntimeError):
+                outs[0].backward(gn)                       # its saved tensors are gone, as for any node
+        for a, b in zip(*grads):
+            assert torch.equal(a, b)
