@@ -13,7 +13,7 @@ from __future__ import annotations
 import torch
 
 from . import fp8_quant, ops
-from ._lib import SCALES_TILED, host
+from ._lib import host
 
 BF16 = torch.bfloat16
 
@@ -35,8 +35,11 @@ def _emits(x: torch.Tensor, rows: int, d: int) -> bool:
     return _EMIT_ROW_OPERAND and x.dtype == BF16 and ops.can_emit_row_codes(rows, d)
 
 
-def _adopt(y: torch.Tensor, codes: torch.Tensor, scales: torch.Tensor) -> None:
-    fp8_quant.adopt_row_operand(y, ops.MXOperand(codes, scales, SCALES_TILED))
+def _adopt(y: torch.Tensor, made: tuple) -> None:
+    """Hand the row-wise operand the kernel wrote (if it did) to the linears that consume y."""
+    op = ops.operand(made)
+    if op is not None:
+        fp8_quant.adopt_row_operand(y, op)
 
 
 def _rows_of(x: torch.Tensor, mod: torch.Tensor) -> tuple[int, int]:
@@ -65,9 +68,8 @@ class FusedAdaLN:
         assert x.is_cuda, "FusedAdaLN requires CUDA tensors"
         _need_bf16_stream("FusedAdaLN", x)
         N, D = _rows_of(x, scale)
-        y, codes, scales = host().adaln(x, scale, shift, eps, _emits(x, N, D))
-        if codes is not None:
-            _adopt(y, codes, scales)
+        y, made = host().adaln(x, scale, shift, eps, _emits(x, N, D))
+        _adopt(y, made)
         return y
 
 
@@ -106,9 +108,8 @@ class FusedGatedAddAdaLN:
         _need_bf16_stream("FusedGatedAddAdaLN", x, sub)
         N, D = _rows_of(x, gate)
         _rows_of(x, scale)
-        x_new, y, codes, scales = host().gated_add_adaln(x, gate, sub, scale, shift, eps, _emits(x, N, D))
-        if codes is not None:
-            _adopt(y, codes, scales)
+        x_new, y, made = host().gated_add_adaln(x, gate, sub, scale, shift, eps, _emits(x, N, D))
+        _adopt(y, made)
         return x_new, y
 
 

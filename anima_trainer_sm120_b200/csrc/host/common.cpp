@@ -48,13 +48,57 @@ static const Tensor& on_cuda(const Tensor& t) {
 Launch::Launch(const Tensor& t)
     : dev(on_cuda(t).device()), guard(dev), stream(c10::cuda::getCurrentCUDAStream(dev.index()).stream()) {}
 
-Op empty_op(int64_t rows, int64_t k, const at::Device& dev) {
-  return {empty({rows, k}, U8, dev), empty({tiled_bytes(rows, k)}, U8, dev)};
+Op op_in(const Tensor& store, int64_t rows, int64_t k) {
+  uint8_t* p = static_cast<uint8_t*>(store.data_ptr());
+  return {store, Tensor(), p, p + pad256(rows * k), rows, k};
+}
+Op op_of(const Tensor& codes, const Tensor& scales) {
+  TORCH_CHECK_VALUE(codes.dim() == 2 && codes.is_contiguous() && scales.is_contiguous(),
+                    "mx_gemm operands must be contiguous (K-major)");
+  return {codes, scales, static_cast<uint8_t*>(codes.data_ptr()), static_cast<uint8_t*>(scales.data_ptr()), codes.size(0),
+          codes.size(1)};
+}
+Op op_of(const OptTensor& codes, const OptTensor& scales, const OptTensor& store) {
+  if (!codes || !codes->defined()) return {};
+  if (store && store->defined()) return op_in(*store, codes->size(0), codes->size(1));
+  return op_of(*codes, *scales);
+}
+// A contiguous view of `size` bytes-typed elements at byte `offset`, without the dispatcher's view machinery.
+static Tensor bytes_at(const Tensor& store, int64_t offset, at::IntArrayRef size) {
+  auto impl = store.unsafeGetTensorImpl()->shallow_copy_and_detach(c10::VariableVersion(0), true);
+  impl->set_storage_offset(store.storage_offset() + offset);
+  impl->set_sizes_contiguous(size);
+  return Tensor(std::move(impl));
+}
+std::pair<Tensor, Tensor> tensors_of(const Op& o, int layout) {
+  if (o.other.defined()) return {o.store, o.other};
+  const int64_t at = o.scales - o.codes;
+  return {bytes_at(o.store, 0, {o.rows, o.k}), layout == ANIMA_SCALES_PLAIN ? bytes_at(o.store, at, {o.rows, o.k / 32})
+                                                                            : bytes_at(o.store, at, {tiled_bytes(o.rows, o.k)})};
 }
 
+Op empty_op(int64_t rows, int64_t k, const at::Device& dev) { return op_in(empty({store_bytes(rows, k)}, U8, dev), rows, k); }
+
 Op placeholder(int64_t rows, int64_t k, const at::Device& dev) {
-  return {at::detail::empty_strided_cuda({rows, k}, {0, 0}, U8, dev),
-          at::detail::empty_strided_cuda({tiled_bytes(rows, k)}, {0}, U8, dev)};
+  Op o;
+  o.store = at::detail::empty_strided_cuda({store_bytes(rows, k)}, {0}, U8, dev);
+  o.rows = rows;
+  o.k = k;
+  return o;
+}
+
+const Tensor& Kept::get() const {
+  TORCH_CHECK(version == now(),
+              "one of the variables needed for gradient computation has been modified by an inplace operation: a parameter "
+              "of shape ", t.sizes(), " is at version ", now(), "; expected version ", version);
+  return t;
+}
+
+Op HostNode::get_op(size_t& at, const Op& shape) {
+  if (!shape.rows) return {};
+  const Tensor first = get(at++);
+  if (shape.other.defined()) return op_of(first, get(at++));
+  return op_in(first, shape.rows, shape.k);
 }
 
 Mat as_matrix(const Tensor& x, int64_t cols) {
@@ -77,7 +121,7 @@ static void need_blocks(int64_t rows, int64_t cols, bool row, bool col) {
 }
 
 static Op alloc_form(int64_t rows, int64_t k, int layout, const at::Device& dev) {
-  if (layout == ANIMA_SCALES_PLAIN) return {empty({rows, k}, U8, dev), empty({rows, k / 32}, U8, dev)};
+  if (layout == ANIMA_SCALES_PLAIN) return op_in(empty({pad256(rows * k) + rows * (k / 32)}, U8, dev), rows, k);
   return empty_op(rows, k, dev);
 }
 
@@ -87,8 +131,7 @@ std::pair<Op, Op> quantize(const Launch& l, const Mat& x, bool row, bool col, in
   if (row) r = alloc_form(x.rows, x.cols, layout, l.dev);
   if (col) c = alloc_form(x.cols, x.rows, layout, l.dev);
   if (x.rows && x.cols)
-    check(anima_mx_quantize(x.ptr(), x.rows, x.cols, x.ld, ptr8(r.codes), ptr8(r.scales), ptr8(c.codes), ptr8(c.scales),
-                            layout, l.stream));
+    check(anima_mx_quantize(x.ptr(), x.rows, x.cols, x.ld, r.codes, r.scales, c.codes, c.scales, layout, l.stream));
   return {r, c};
 }
 
@@ -99,18 +142,20 @@ std::pair<Op, Op> quantize_gelu(const Launch& l, const Tensor& h, const Tensor& 
   if (row) r = empty_op(rows, cols, l.dev);
   if (col) c = empty_op(cols, rows, l.dev);
   if (rows && cols)
-    check(anima_mx_quantize_gelu(h.data_ptr(), ptr(grad), rows, cols, cols, nullptr, ptr8(r.codes), ptr8(r.scales),
-                                 ptr8(c.codes), ptr8(c.scales), ANIMA_SCALES_TILED, l.stream));
+    check(anima_mx_quantize_gelu(h.data_ptr(), ptr(grad), rows, cols, cols, nullptr, r.codes, r.scales, c.codes, c.scales,
+                                 ANIMA_SCALES_TILED, l.stream));
   return {r, c};
 }
 
 Op regroup(const Launch& l, const Op& a, int64_t rows, int64_t k) {
-  TORCH_CHECK_VALUE(rows * k == a.rows() * a.k() && k % 32 == 0, "cannot view [", a.rows(), ", ", a.k(), "] as [", rows,
-                    ", ", k, "]");
-  Tensor scales = empty({tiled_bytes(rows, k)}, U8, l.dev);
-  if (rows)
-    check(anima_mx_scales_regroup(ptr8(a.scales), a.rows(), a.k(), ptr8(scales), rows, k, l.stream));
-  return {a.codes.view({rows, k}), scales};
+  TORCH_CHECK_VALUE(rows * k == a.rows * a.k && k % 32 == 0, "cannot view [", a.rows, ", ", a.k, "] as [", rows, ", ", k, "]");
+  Op o = a;
+  o.rows = rows;
+  o.k = k;
+  o.other = empty({tiled_bytes(rows, k)}, U8, l.dev);
+  o.scales = static_cast<uint8_t*>(o.other.data_ptr());
+  if (rows) check(anima_mx_scales_regroup(a.scales, a.rows, a.k, o.scales, rows, k, l.stream));
+  return o;
 }
 
 static int factor_flag(const Tensor& w1, const Tensor& w2) {
@@ -133,42 +178,41 @@ std::pair<Op, Op> merge_quantize(const Launch& l, const Tensor& W, const Tensor&
   if (row) r = empty_op(N, K, l.dev);
   if (col) c = empty_op(K, N, l.dev);
   check(anima_lokr_merge_quantize(w.data_ptr(), w1.data_ptr(), w2.data_ptr(), factor_flag(w1, w2),
-                                  static_cast<float>(alpha), N, K, up, uq, nullptr, ptr8(r.codes), ptr8(r.scales),
-                                  ptr8(c.codes), ptr8(c.scales), ANIMA_SCALES_TILED, l.stream));
+                                  static_cast<float>(alpha), N, K, up, uq, nullptr, r.codes, r.scales, c.codes, c.scales,
+                                  ANIMA_SCALES_TILED, l.stream));
   return {r, c};
 }
 
 static void need_same_k(const Op& a, const Op& b) {
-  TORCH_CHECK_VALUE(a.k() == b.k(), "contraction sizes differ: A has K=", a.k(), ", B has K=", b.k());
-  TORCH_CHECK_VALUE(a.codes.is_contiguous() && b.codes.is_contiguous(), "mx_gemm operands must be contiguous (K-major)");
+  TORCH_CHECK_VALUE(a.k == b.k, "contraction sizes differ: A has K=", a.k, ", B has K=", b.k);
 }
 
 void gemm(const Launch& l, const Op& a, const Op& b, const GemmOut& out, const void* bias, const void* residual,
           int64_t ldr, double alpha) {
   need_same_k(a, b);
-  const int64_t M = a.rows(), N = b.rows(), K = a.k();
+  const int64_t M = a.rows, N = b.rows, K = a.k;
   const int64_t bytes = check(anima_mx_gemm_workspace_bytes(M, N, K));
   Tensor ws;
   if (bytes) ws = empty({bytes}, U8, l.dev);
-  check(anima_mx_gemm_ex(ptr8(a.codes), ptr8(a.scales), ptr8(b.codes), ptr8(b.scales), out.c, M, N, K, out.ldc, bias,
+  check(anima_mx_gemm_ex(a.codes, a.scales, b.codes, b.scales, out.c, M, N, K, out.ldc, bias,
                          residual, ldr, static_cast<float>(alpha), out.fp32 ? 1 : 0, ptr(ws), bytes,
                          status_word(l.dev), l.stream));
 }
 
 void gemm_delta(const Launch& l, const Op& a, const Op& b, const Op& planes, const Op& d, void* c, const void* bias) {
   need_same_k(a, b);
-  const int64_t M = a.rows(), N = b.rows(), K = a.k();
+  const int64_t M = a.rows, N = b.rows, K = a.k;
   const int64_t bytes = check(anima_mx_gemm_workspace_bytes(M, N, K));
   Tensor ws;
   if (bytes) ws = empty({bytes}, U8, l.dev);
-  check(anima_mx_gemm_delta(ptr8(a.codes), ptr8(a.scales), ptr8(b.codes), ptr8(b.scales), c, M, N, K, N, bias, 0,
-                            ptr8(planes.codes), ptr8(planes.scales), ptr8(d.codes), ptr8(d.scales), ptr(ws), bytes,
+  check(anima_mx_gemm_delta(a.codes, a.scales, b.codes, b.scales, c, M, N, K, N, bias, 0,
+                            planes.codes, planes.scales, d.codes, d.scales, ptr(ws), bytes,
                             status_word(l.dev), l.stream));
 }
 
 Tensor gemm_f32(const Launch& l, const Op& a, const Op& b, double alpha) {
-  Tensor c = empty({a.rows(), b.rows()}, F32, l.dev);
-  gemm(l, a, b, {c.data_ptr(), b.rows(), true}, nullptr, nullptr, 0, alpha);
+  Tensor c = empty({a.rows, b.rows}, F32, l.dev);
+  gemm(l, a, b, {c.data_ptr(), b.rows, true}, nullptr, nullptr, 0, alpha);
   return c;
 }
 

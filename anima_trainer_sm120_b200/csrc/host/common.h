@@ -11,8 +11,12 @@
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
-#include <torch/csrc/autograd/custom_function.h>
+#include <torch/csrc/autograd/function.h>
+#include <torch/csrc/autograd/functions/utils.h>
+#include <torch/csrc/autograd/saved_variable.h>
+#include <torch/csrc/autograd/variable.h>
 
+#include <mutex>
 #include <optional>
 #include <tuple>
 #include <utility>
@@ -24,23 +28,29 @@ namespace anima_host {
 
 using at::Tensor;
 using OptTensor = std::optional<Tensor>;
-using torch::autograd::AutogradContext;
 using torch::autograd::variable_list;
 
 constexpr auto BF16 = at::kBFloat16;
 constexpr auto F32 = at::kFloat;
 constexpr auto U8 = at::kByte;
 
-// One K-major MXFP8 operand: e4m3 codes [rows, k] and e8m0 scales (TILED unless said otherwise).
+// One K-major MXFP8 operand: e4m3 codes [rows, k] and e8m0 scales (TILED unless said otherwise). Both lie in one
+// allocation (`store`, bytes) when they were made here: one tensor to allocate and one for autograd to save.
 struct Op {
-  Tensor codes, scales;
-  bool defined() const { return codes.defined(); }
-  int64_t rows() const { return codes.size(0); }
-  int64_t k() const { return codes.size(1); }
+  Tensor store, other;      // the memory; `other` only for operands that came as two tensors
+  uint8_t *codes = nullptr, *scales = nullptr;
+  int64_t rows = 0, k = 0;
+  bool defined() const { return store.defined(); }
 };
-inline Op make_op(const OptTensor& codes, const OptTensor& scales) {
-  return codes && codes->defined() ? Op{*codes, *scales} : Op{};
-}
+constexpr int64_t pad256(int64_t n) { return (n + 255) / 256 * 256; }
+inline int64_t tiled_bytes(int64_t rows, int64_t k) { return ((rows + 127) / 128) * ((k + 127) / 128) * 512; }
+inline int64_t store_bytes(int64_t rows, int64_t k) { return pad256(rows * k) + tiled_bytes(rows, k); }
+Op op_in(const Tensor& store, int64_t rows, int64_t k);       // the operand laid out in `store`
+Op op_of(const Tensor& codes, const Tensor& scales);          // [rows, k] codes and their scales
+// what Python passes for an operand: nothing, (codes, scales, None) or (codes, scales, store)
+Op op_of(const OptTensor& codes, const OptTensor& scales, const OptTensor& store);
+// the tensors of an operand, as views of its store
+std::pair<Tensor, Tensor> tensors_of(const Op& o, int layout = ANIMA_SCALES_TILED);
 
 // A bf16 matrix as the kernels take it: pointer, rows, columns, row pitch; `keep` owns the memory.
 struct Mat {
@@ -62,7 +72,6 @@ inline void* ptr(const OptTensor& t) { return t ? ptr(*t) : nullptr; }
 inline Tensor empty(at::IntArrayRef size, at::ScalarType dtype, const at::Device& dev) {
   return at::detail::empty_cuda(size, dtype, dev, std::nullopt);
 }
-inline int64_t tiled_bytes(int64_t rows, int64_t k) { return ((rows + 127) / 128) * ((k + 127) / 128) * 512; }
 
 // Current device and stream for the duration of one call.
 struct Launch {
@@ -76,8 +85,8 @@ int32_t* status_word(const at::Device& dev);      // the GEMM's bounded-wait fla
 Tensor status_word_tensor(int64_t device_index);
 
 Op empty_op(int64_t rows, int64_t k, const at::Device& dev);
-// Stands in for an operand only backward would read, in a pass whose saved tensors a checkpoint drops: its shape and
-// type without its memory.
+// Stands in for the store of an operand only backward would read, in a pass whose saved tensors a checkpoint drops:
+// its shape and type without its memory.
 Op placeholder(int64_t rows, int64_t k, const at::Device& dev);
 
 Mat as_matrix(const Tensor& x, int64_t cols);     // any shape whose elements in order are [-1, cols]; cast to bf16
@@ -113,33 +122,55 @@ inline bool wants(const Tensor& t) { return at::GradMode::is_enabled() && t.defi
 inline bool wants(const OptTensor& t) { return t && wants(*t); }
 inline Tensor cast(const Tensor& t, at::ScalarType dt) { return t.scalar_type() == dt ? t : t.to(dt); }
 
-// Plain values of a node, kept beside its saved tensors.
-template <class T>
-struct Held : torch::CustomClassHolder {
-  T v;
-};
-template <class T>
-void hold(AutogradContext* ctx, T v) {
-  auto h = c10::make_intrusive<Held<T>>();
-  h->v = std::move(v);
-  ctx->saved_data["held"] = c10::IValue::make_capsule(std::move(h));
-}
-template <class T>
-T& held(AutogradContext* ctx) {
-  return static_cast<Held<T>*>(ctx->saved_data["held"].toCapsule().get())->v;
-}
+// ------------------------------------------------------------------------------------------------ autograd nodes
+// A parameter or another small tensor a node reads in backward without handing it to saved-tensor hooks (a
+// checkpointed pass would call them for every tensor); like a saved tensor it may not change in place meanwhile.
+struct Kept {
+  Tensor t;
+  uint32_t version = 0;
+  Kept() = default;
+  Kept(const Tensor& v) : t(v), version(now()) {}
+  const Tensor& get() const;
 
-inline void push(variable_list& v, const Op& a) {
-  if (a.defined()) {
-    v.push_back(a.codes);
-    v.push_back(a.scales);
+ private:
+  uint32_t now() const { return t.defined() && !t.is_inference() ? t.unsafeGetTensorImpl()->version_counter().current_version() : 0; }
+};
+
+// Base of the nodes: saved tensors go through torch's saved-tensor hooks (checkpointing), one output gradient by default.
+struct HostNode : public torch::autograd::Node {
+  std::vector<torch::autograd::SavedVariable> saved;
+
+  void save(const Tensor& t, bool is_output = false) { saved.emplace_back(t, is_output); }
+  void save(const Op& o) {       // an undefined operand saves nothing
+    if (!o.defined()) return;
+    save(o.store);
+    if (o.other.defined()) save(o.other);
   }
+  Tensor get(size_t i) { return saved.at(i).unpack(getptr()); }
+  // the operand saved at position `at` (advanced), of a known shape
+  Op get_op(size_t& at, const Op& shape);
+  void release_variables() override {
+    std::lock_guard<std::mutex> lock(mutex_);
+    for (auto& v : saved) v.reset_data();
+  }
+  // the gradient of output i; zeros where the graph has none
+  Tensor grad_of(variable_list& g, size_t i) { return g[i].defined() ? g[i] : input_metadata(i).zeros_like(); }
+};
+
+inline torch::autograd::Edge edge_of(const Tensor& t) {
+  return wants(t) ? torch::autograd::impl::gradient_edge(t) : torch::autograd::Edge();
 }
-inline Op pop(const variable_list& v, size_t& at, bool there) {
-  if (!there) return {};
-  Op a{v[at], v[at + 1]};
-  at += 2;
-  return a;
+inline torch::autograd::Edge edge_of(const OptTensor& t) { return t ? edge_of(*t) : torch::autograd::Edge(); }
+template <class N, class... Inputs>
+std::shared_ptr<N> make_node(const Inputs&... inputs) {
+  auto node = std::shared_ptr<N>(new N(), torch::autograd::deleteNode);
+  torch::autograd::edge_list edges;
+  edges.reserve(sizeof...(inputs));
+  (edges.push_back(edge_of(inputs)), ...);
+  node->set_next_edges(std::move(edges));
+  return node;
 }
+// Kernels and allocations of a node run below autograd.
+using Below = at::AutoDispatchBelowADInplaceOrView;
 
 }  // namespace anima_host

@@ -2,286 +2,286 @@
 
 namespace anima_host {
 
-using torch::autograd::Function;
-
 namespace {
 
-struct OutBias {           // bias as the GEMM reads it
-  Tensor t;
-  explicit OutBias(const OptTensor& b) : t(b && b->defined() ? bf16_contiguous(*b) : Tensor()) {}
-  const void* ptr() const { return t.defined() ? t.data_ptr() : nullptr; }
-};
+using torch::autograd::set_history;
 
 // [*lead, N] in bf16, then in the dtype of the input
 Tensor project(const Launch& l, const Tensor& x, const Op& x_row, const Op& w_row, const OptTensor& bias) {
-  const int64_t n = w_row.rows();
-  const OutBias b(bias);
-  TORCH_CHECK_VALUE(!b.t.defined() || b.t.numel() == n, "bias must be of length N");
+  const int64_t n = w_row.rows;
+  const Tensor b = bias && bias->defined() ? bf16_contiguous(*bias) : Tensor();
+  TORCH_CHECK_VALUE(!b.defined() || b.numel() == n, "bias must be of length N");
   Tensor y = empty(with_last(x.sizes(), n), BF16, l.dev);
-  if (x_row.rows()) gemm(l, x_row, w_row, {y.data_ptr(), n, false}, b.ptr());
+  if (x_row.rows) gemm(l, x_row, w_row, {y.data_ptr(), n, false}, ptr(b));
   return cast(y, x.scalar_type());
 }
 
 Tensor input_grad(const Launch& l, const Tensor& gy, const Op& g_row, const Op& w_col) {
-  Tensor gx = empty(with_last(gy.sizes(), w_col.rows()), BF16, l.dev);
-  if (g_row.rows()) gemm(l, g_row, w_col, {gx.data_ptr(), w_col.rows(), false});
+  Tensor gx = empty(with_last(gy.sizes(), w_col.rows), BF16, l.dev);
+  if (g_row.rows) gemm(l, g_row, w_col, {gx.data_ptr(), w_col.rows, false});
   return cast(gx, gy.scalar_type());
 }
 
 Tensor bias_grad(const Tensor& gy) { return gy.reshape({-1, gy.size(-1)}).sum(0); }
 
-// ------------------------------------------------------------------------------------------------ LoKr linear
-struct LokrCall {
-  const Tensor* W;
-  Op x_row, x_col;
-  double alpha;
-  bool first, need_x, train, need_bias;
-};
-struct LokrHeld {
-  double alpha;
-  bool need_x, train, need_bias;
-};
-
-Tensor lokr_fwd(const Launch& l, const Tensor& x, const OptTensor& bias, const Tensor& w1, const Tensor& w2, LokrCall& c,
-                Op& w_col) {
-  auto [w_row, col] = merge_quantize(l, *c.W, w1, w2, c.alpha, true, c.need_x && !c.first);
-  w_col = col;
-  return project(l, x, c.x_row, w_row, bias);
+Op shape_of(int64_t rows, int64_t k) {      // of an operand saved as one store
+  Op o;
+  o.rows = rows;
+  o.k = k;
+  return o;
+}
+Op shape_of(const Op& o) {
+  Op s = shape_of(o.rows, o.k);
+  s.other = o.other.defined() ? o.other : Tensor();
+  return s;
 }
 
-struct LokrLinear : Function<LokrLinear> {
-  static Tensor forward(AutogradContext* ctx, const Tensor& x, const OptTensor& bias, const Tensor& w1, const Tensor& w2,
-                        LokrCall* c) {
-    const Launch l(x);
-    Op w_col;
-    Tensor y = lokr_fwd(l, x, bias, w1, w2, *c, w_col);
-    const int64_t n = c->W->size(0), k = c->W->size(1);
-    if (c->first) {
-      if (c->need_x) w_col = placeholder(k, n, l.dev);
-      if (c->train) c->x_col = placeholder(k, c->x_row.rows(), l.dev);
-    }
-    variable_list keep;
-    if (c->train) keep = {w1, w2};
-    push(keep, c->x_col);
-    push(keep, w_col);
-    ctx->save_for_backward(std::move(keep));
-    hold(ctx, LokrHeld{c->alpha, c->need_x, c->train, c->need_bias});
-    return y;
-  }
-  static variable_list backward(AutogradContext* ctx, variable_list grads) {
-    const LokrHeld h = held<LokrHeld>(ctx);
-    const variable_list saved = ctx->get_saved_variables();     // once: checkpointing unpacks on access
-    size_t at = h.train ? 2 : 0;
-    const Op x_col = pop(saved, at, h.train), w_col = pop(saved, at, h.need_x);
-    const Tensor& gy = grads[0];
+// ------------------------------------------------------------------------------------------------ LoKr linear
+struct LokrNode : public HostNode {
+  Kept w1, w2;
+  Op x_col, w_col;      // shapes
+  double alpha;
+  bool need_x, train, need_bias;
+
+  variable_list apply(variable_list&& g) override {
+    std::lock_guard<std::mutex> lock(mutex_);
+    const Tensor gy = grad_of(g, 0);
     const Launch l(gy);
-    auto [g_row, g_col] = quantize(l, as_matrix(gy, gy.size(-1)), h.need_x, h.train);
-    variable_list out(5);
-    if (h.need_x) out[0] = input_grad(l, gy, g_row, w_col);
-    if (h.train) std::tie(out[2], out[3]) = kron_backward(l, gemm_f32(l, g_col, x_col), saved[0], saved[1], h.alpha);
-    if (h.need_bias) out[1] = bias_grad(gy);
+    size_t at = 0;
+    const Op xc = get_op(at, x_col), wc = get_op(at, w_col);
+    auto [g_row, g_col] = quantize(l, as_matrix(gy, gy.size(-1)), need_x, train);
+    variable_list out(4);
+    if (need_x) out[0] = input_grad(l, gy, g_row, wc);
+    if (train) std::tie(out[2], out[3]) = kron_backward(l, gemm_f32(l, g_col, xc), w1.get(), w2.get(), alpha);
+    if (need_bias) out[1] = bias_grad(gy);
     return out;
   }
+  std::string name() const override { return "LoKrLinearFusedBackward"; }
 };
 
 // ------------------------------------------------------------------------------------------------ merged linear
-struct MergedCall {
-  Op x_row, x_col;
-  bool first, need_x, train, need_bias;
-};
-struct MergedHeld {
+struct MergedNode : public HostNode {
+  Op x_col, w_col;
   bool need_x, train, need_bias;
   at::ScalarType w_dtype;
-};
 
-std::pair<Op, Op> quantize_merged(const Launch& l, const Tensor& merged, bool col) {
-  return quantize(l, as_matrix(merged, merged.size(1)), true, col);
-}
-
-struct MergedLinear : Function<MergedLinear> {
-  static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& merged, const OptTensor& bias, MergedCall* c) {
-    const Launch l(x);
-    auto [w_row, w_col] = quantize_merged(l, merged, c->need_x && !c->first);
-    Tensor y = project(l, x, c->x_row, w_row, bias);
-    if (c->first) {
-      if (c->need_x) w_col = placeholder(merged.size(1), merged.size(0), l.dev);
-      if (c->train) c->x_col = placeholder(merged.size(1), c->x_row.rows(), l.dev);
-    }
-    variable_list keep;
-    push(keep, c->x_col);
-    push(keep, w_col);
-    ctx->save_for_backward(std::move(keep));
-    hold(ctx, MergedHeld{c->need_x, c->train, c->need_bias, merged.scalar_type()});
-    return y;
-  }
-  static variable_list backward(AutogradContext* ctx, variable_list grads) {
-    const MergedHeld h = held<MergedHeld>(ctx);
-    const variable_list saved = ctx->get_saved_variables();
-    size_t at = 0;
-    const Op x_col = pop(saved, at, h.train), w_col = pop(saved, at, h.need_x);
-    const Tensor& gy = grads[0];
+  variable_list apply(variable_list&& g) override {
+    std::lock_guard<std::mutex> lock(mutex_);
+    const Tensor gy = grad_of(g, 0);
     const Launch l(gy);
-    auto [g_row, g_col] = quantize(l, as_matrix(gy, gy.size(-1)), h.need_x, h.train);
-    variable_list out(4);
-    if (h.need_x) out[0] = input_grad(l, gy, g_row, w_col);
-    if (h.train) {
-      Tensor gw = empty({g_col.rows(), x_col.rows()}, BF16, l.dev);
-      gemm(l, g_col, x_col, {gw.data_ptr(), x_col.rows(), false});
-      out[1] = cast(gw, h.w_dtype);
+    size_t at = 0;
+    const Op xc = get_op(at, x_col), wc = get_op(at, w_col);
+    auto [g_row, g_col] = quantize(l, as_matrix(gy, gy.size(-1)), need_x, train);
+    variable_list out(3);
+    if (need_x) out[0] = input_grad(l, gy, g_row, wc);
+    if (train) {
+      Tensor gw = empty({g_col.rows, xc.rows}, BF16, l.dev);
+      gemm(l, g_col, xc, {gw.data_ptr(), xc.rows, false});
+      out[1] = cast(gw, w_dtype);
     }
-    if (h.need_bias) out[2] = bias_grad(gy);
+    if (need_bias) out[2] = bias_grad(gy);
     return out;
   }
+  std::string name() const override { return "MXFP8LoKrLinearBackward"; }
 };
 
 // ------------------------------------------------------------------------------------------------ frozen linear
-struct FrozenCall {
-  Op x_row, w_row, w_col;
-  Tensor w_bf16;
-  bool need_x, need_bias;
-};
-struct FrozenHeld {
+struct FrozenNode : public HostNode {
   Op w_col;
   Tensor w_bf16;
   bool need_x, need_bias;
-};
 
-struct FrozenLinear : Function<FrozenLinear> {
-  static Tensor forward(AutogradContext* ctx, const Tensor& x, const OptTensor& bias, FrozenCall* c) {
-    const Launch l(x);
-    hold(ctx, FrozenHeld{c->w_col, c->w_bf16, c->need_x, c->need_bias});
-    return project(l, x, c->x_row, c->w_row, bias);
-  }
-  static variable_list backward(AutogradContext* ctx, variable_list grads) {
-    const FrozenHeld& h = held<FrozenHeld>(ctx);
-    const Tensor& gy = grads[0];
-    variable_list out(3);
-    if (h.need_x) {
+  variable_list apply(variable_list&& g) override {
+    std::lock_guard<std::mutex> lock(mutex_);
+    const Tensor gy = grad_of(g, 0);
+    variable_list out(2);
+    if (need_x) {
       const Launch l(gy);
-      const Mat g = as_matrix(gy, gy.size(-1));
-      if (h.w_col.defined()) {
-        out[0] = input_grad(l, gy, quantize(l, g, true, false).first, h.w_col);
+      const Mat m = as_matrix(gy, gy.size(-1));
+      if (w_col.defined()) {
+        out[0] = input_grad(l, gy, quantize(l, m, true, false).first, w_col);
       } else {
-        Tensor gx = at::matmul(g.keep.reshape({g.rows, g.cols}), h.w_bf16.to(BF16));
-        out[0] = cast(gx.reshape(with_last(gy.sizes(), h.w_bf16.size(1))), gy.scalar_type());
+        Tensor gx = at::matmul(m.keep.reshape({m.rows, m.cols}), w_bf16.to(BF16));
+        out[0] = cast(gx.reshape(with_last(gy.sizes(), w_bf16.size(1))), gy.scalar_type());
       }
     }
-    if (h.need_bias) out[1] = bias_grad(gy);
+    if (need_bias) out[1] = bias_grad(gy);
     return out;
   }
+  std::string name() const override { return "MXFP8FrozenLinearBackward"; }
 };
 
 // ------------------------------------------------------------------------------------------------ LoKr MLP
-struct MlpCall {
-  Op x_row, x_col;
-  const Tensor *W1, *W2;
-  OptTensor b1, b2;
-  double alpha1, alpha2;
-  bool first, need_x, train;
-  bool back() const { return need_x || train; }
-};
-struct MlpHeld {
+struct MlpNode : public HostNode {
+  Kept w1a, w2a, w1b, w2b;
+  Op x_col, a_col, W1_col, W2_col;
   double alpha1, alpha2;
   bool need_x, train;
-};
-struct MlpKept {
-  Tensor h;
-  Op a_col, W1_col, W2_col;
-};
 
-Tensor mlp_fwd(const Launch& l, const Tensor& x, const Tensor& w1a, const Tensor& w2a, const Tensor& w1b,
-               const Tensor& w2b, const MlpCall& c, MlpKept& kept) {
-  const bool back = c.back() && !c.first;
-  const int64_t rows = c.x_row.rows(), hid = c.W1->size(0);
-  Op W1_row, W2_row, a_row;
-  std::tie(W1_row, kept.W1_col) = merge_quantize(l, *c.W1, w1a, w2a, c.alpha1, true, back && c.need_x);
-  const OutBias b1(c.b1);
-  kept.h = empty({rows, hid}, BF16, l.dev);
-  if (rows) gemm(l, c.x_row, W1_row, {kept.h.data_ptr(), hid, false}, b1.ptr());
-  std::tie(a_row, kept.a_col) = quantize_gelu(l, kept.h, Tensor(), rows, hid, true, back && c.train);
-  std::tie(W2_row, kept.W2_col) = merge_quantize(l, *c.W2, w1b, w2b, c.alpha2, true, back);
-  return project(l, x, a_row, W2_row, c.b2);
-}
-
-struct LokrMlp : Function<LokrMlp> {
-  static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& w1a, const Tensor& w2a, const Tensor& w1b,
-                        const Tensor& w2b, MlpCall* c) {
-    const Launch l(x);
-    MlpKept k;
-    Tensor y = mlp_fwd(l, x, w1a, w2a, w1b, w2b, *c, k);
-    if (c->first) {
-      const int64_t rows = c->x_row.rows(), hid = c->W1->size(0), k_in = c->W1->size(1), n_out = c->W2->size(0);
-      if (c->need_x) k.W1_col = placeholder(k_in, hid, l.dev);
-      k.W2_col = placeholder(hid, n_out, l.dev);
-      if (c->train) {
-        c->x_col = placeholder(k_in, rows, l.dev);
-        k.a_col = placeholder(hid, rows, l.dev);
-      }
-    }
-    variable_list keep{k.h, w1a, w2a, w1b, w2b};
-    for (const Op* o : {&c->x_col, &k.a_col, &k.W1_col, &k.W2_col}) push(keep, *o);
-    ctx->save_for_backward(std::move(keep));
-    hold(ctx, MlpHeld{c->alpha1, c->alpha2, c->need_x, c->train});
-    return y;
-  }
-  static variable_list backward(AutogradContext* ctx, variable_list grads) {
-    const MlpHeld m = held<MlpHeld>(ctx);
-    const variable_list saved = ctx->get_saved_variables();
-    size_t at = 5;
-    const Op x_col = pop(saved, at, m.train), a_col = pop(saved, at, m.train), W1_col = pop(saved, at, m.need_x),
-             W2_col = pop(saved, at, true);
-    const Tensor &h = saved[0], &gy = grads[0];
+  variable_list apply(variable_list&& g) override {
+    std::lock_guard<std::mutex> lock(mutex_);
+    const Tensor gy = grad_of(g, 0);
     const Launch l(gy);
+    const Tensor h = get(0);
+    size_t at = 1;
+    const Op xc = get_op(at, x_col), ac = get_op(at, a_col), W1 = get_op(at, W1_col), W2 = get_op(at, W2_col);
     const int64_t rows = h.size(0), hid = h.size(1);
-    auto [g_row, g_col] = quantize(l, as_matrix(gy, gy.size(-1)), true, m.train);
+    auto [g_row, g_col] = quantize(l, as_matrix(gy, gy.size(-1)), true, train);
     Tensor grad_act = empty({rows, hid}, BF16, l.dev);
-    gemm(l, g_row, W2_col, {grad_act.data_ptr(), hid, false});
-    variable_list out(6);
-    if (m.train) std::tie(out[3], out[4]) = kron_backward(l, gemm_f32(l, g_col, a_col), saved[3], saved[4], m.alpha2);
-    auto [dh_row, dh_col] = quantize_gelu(l, h, grad_act, rows, hid, m.need_x, m.train);
+    if (rows) gemm(l, g_row, W2, {grad_act.data_ptr(), hid, false});
+    variable_list out(5);
+    if (train) std::tie(out[3], out[4]) = kron_backward(l, gemm_f32(l, g_col, ac), w1b.get(), w2b.get(), alpha2);
+    auto [dh_row, dh_col] = quantize_gelu(l, h, grad_act, rows, hid, need_x, train);
     grad_act.reset();
-    if (m.need_x) out[0] = input_grad(l, gy, dh_row, W1_col);
-    if (m.train) std::tie(out[1], out[2]) = kron_backward(l, gemm_f32(l, dh_col, x_col), saved[1], saved[2], m.alpha1);
+    if (need_x) out[0] = input_grad(l, gy, dh_row, W1);
+    if (train) std::tie(out[1], out[2]) = kron_backward(l, gemm_f32(l, dh_col, xc), w1a.get(), w2a.get(), alpha1);
     return out;
   }
+  std::string name() const override { return "LoKrMLPFusedBackward"; }
 };
 
 }  // namespace
 
 Tensor lokr_linear(const Tensor& x, Op x_row, Op x_col, const Tensor& W, const OptTensor& bias, const Tensor& w1,
                    const Tensor& w2, double alpha, bool first) {
-  LokrCall c{&W, std::move(x_row), std::move(x_col), alpha, first, wants(x), wants(w1) || wants(w2), wants(bias)};
-  if (c.need_x || c.train || c.need_bias) return LokrLinear::apply(x, bias, w1, w2, &c);
+  const bool need_x = wants(x), train = wants(w1) || wants(w2), need_bias = wants(bias);
   const Launch l(x);
-  Op unused;
-  return lokr_fwd(l, x, bias, w1, w2, c, unused);
+  Tensor y;
+  Op w_col;
+  {
+    Below below;
+    Op w_row;
+    std::tie(w_row, w_col) = merge_quantize(l, W, w1, w2, alpha, true, need_x && !first);
+    y = project(l, x, x_row, w_row, bias);
+    if (first) {
+      if (need_x) w_col = placeholder(W.size(1), W.size(0), l.dev);
+      if (train) x_col = placeholder(W.size(1), x_row.rows, l.dev);
+    }
+  }
+  if (need_x || train || need_bias) {
+    auto n = make_node<LokrNode>(x, bias, w1, w2);
+    if (train) {
+      n->w1 = Kept(w1);
+      n->w2 = Kept(w2);
+      n->save(x_col);
+      n->x_col = shape_of(x_col);
+    }
+    if (need_x) {
+      n->save(w_col);
+      n->w_col = shape_of(w_col);
+    }
+    n->alpha = alpha;
+    n->need_x = need_x;
+    n->train = train;
+    n->need_bias = need_bias;
+    set_history(y, n);
+  }
+  return y;
 }
 
 Tensor merged_linear(const Tensor& x, Op x_row, Op x_col, const Tensor& merged, const OptTensor& bias, bool first) {
-  MergedCall c{std::move(x_row), std::move(x_col), first, wants(x), wants(merged), wants(bias)};
-  if (c.need_x || c.train || c.need_bias) return MergedLinear::apply(x, merged, bias, &c);
+  const bool need_x = wants(x), train = wants(merged), need_bias = wants(bias);
   const Launch l(x);
-  return project(l, x, c.x_row, quantize_merged(l, merged, false).first, bias);
+  Tensor y;
+  Op w_col;
+  {
+    Below below;
+    Op w_row;
+    std::tie(w_row, w_col) = quantize(l, as_matrix(merged, merged.size(1)), true, need_x && !first);
+    y = project(l, x, x_row, w_row, bias);
+    if (first) {
+      if (need_x) w_col = placeholder(merged.size(1), merged.size(0), l.dev);
+      if (train) x_col = placeholder(merged.size(1), x_row.rows, l.dev);
+    }
+  }
+  if (need_x || train || need_bias) {
+    auto n = make_node<MergedNode>(x, merged, bias);
+    if (train) {
+      n->save(x_col);
+      n->x_col = shape_of(x_col);
+    }
+    if (need_x) {
+      n->save(w_col);
+      n->w_col = shape_of(w_col);
+    }
+    n->need_x = need_x;
+    n->train = train;
+    n->need_bias = need_bias;
+    n->w_dtype = merged.scalar_type();
+    set_history(y, n);
+  }
+  return y;
 }
 
-Tensor frozen_linear(const Tensor& x, Op x_row, Op w_row, Op w_col, const OptTensor& w_bf16, int64_t k_in,
-                     const OptTensor& bias) {
-  TORCH_CHECK_VALUE(x.size(-1) == k_in, "input of width ", x.size(-1), " for a weight with ", k_in, " columns");
-  FrozenCall c{std::move(x_row), std::move(w_row), std::move(w_col), w_bf16.value_or(Tensor()), wants(x), wants(bias)};
-  if (c.need_x || c.need_bias) return FrozenLinear::apply(x, bias, &c);
+Tensor frozen_linear(const Tensor& x, Op x_row, Op w_row, Op w_col, const OptTensor& w_bf16, const OptTensor& bias) {
+  TORCH_CHECK_VALUE(x.size(-1) == w_row.k, "input of width ", x.size(-1), " for a weight with ", w_row.k, " columns");
+  const bool need_x = wants(x), need_bias = wants(bias);
   const Launch l(x);
-  return project(l, x, c.x_row, c.w_row, bias);
+  Tensor y;
+  {
+    Below below;
+    y = project(l, x, x_row, w_row, bias);
+  }
+  if (need_x || need_bias) {
+    auto n = make_node<FrozenNode>(x, bias);
+    n->w_col = std::move(w_col);
+    n->w_bf16 = w_bf16.value_or(Tensor());
+    n->need_x = need_x;
+    n->need_bias = need_bias;
+    set_history(y, n);
+  }
+  return y;
 }
 
 Tensor lokr_mlp(const Tensor& x, Op x_row, Op x_col, const Tensor& W1, const OptTensor& b1, const Tensor& w1a,
                 const Tensor& w2a, double alpha1, const Tensor& W2, const OptTensor& b2, const Tensor& w1b,
                 const Tensor& w2b, double alpha2, bool first) {
-  const bool train = wants(w1a) || wants(w2a) || wants(w1b) || wants(w2b);
-  MlpCall c{std::move(x_row), std::move(x_col), &W1, &W2, b1, b2, alpha1, alpha2, first, wants(x), train};
-  if (c.back()) return LokrMlp::apply(x, w1a, w2a, w1b, w2b, &c);
+  const bool train = wants(w1a) || wants(w2a) || wants(w1b) || wants(w2b), need_x = wants(x), back = need_x || train;
+  const bool keep = back && !first;
   const Launch l(x);
-  MlpKept unused;
-  return mlp_fwd(l, x, w1a, w2a, w1b, w2b, c, unused);
+  const int64_t rows = x_row.rows, hid = W1.size(0);
+  Tensor y, h;
+  Op a_col, W1_col, W2_col;
+  {
+    Below below;
+    Op W1_row, W2_row, a_row;
+    std::tie(W1_row, W1_col) = merge_quantize(l, W1, w1a, w2a, alpha1, true, keep && need_x);
+    const Tensor b = b1 && b1->defined() ? bf16_contiguous(*b1) : Tensor();
+    h = empty({rows, hid}, BF16, l.dev);
+    if (rows) gemm(l, x_row, W1_row, {h.data_ptr(), hid, false}, ptr(b));
+    std::tie(a_row, a_col) = quantize_gelu(l, h, Tensor(), rows, hid, true, keep && train);
+    std::tie(W2_row, W2_col) = merge_quantize(l, W2, w1b, w2b, alpha2, true, keep);
+    y = project(l, x, a_row, W2_row, b2);
+    if (back && first) {
+      if (need_x) W1_col = placeholder(W1.size(1), hid, l.dev);
+      W2_col = placeholder(hid, W2.size(0), l.dev);
+      if (train) {
+        x_col = placeholder(W1.size(1), rows, l.dev);
+        a_col = placeholder(hid, rows, l.dev);
+      }
+    }
+  }
+  if (back) {
+    auto n = make_node<MlpNode>(x, w1a, w2a, w1b, w2b);
+    n->save(h);
+    for (auto [op, shape] : {std::pair{&x_col, &n->x_col}, {&a_col, &n->a_col}, {&W1_col, &n->W1_col}, {&W2_col, &n->W2_col}}) {
+      if (op == &x_col && !train) continue;
+      n->save(*op);
+      *shape = shape_of(*op);
+    }
+    if (train) {
+      n->w1a = Kept(w1a);
+      n->w2a = Kept(w2a);
+      n->w1b = Kept(w1b);
+      n->w2b = Kept(w2b);
+    }
+    n->alpha1 = alpha1;
+    n->alpha2 = alpha2;
+    n->need_x = need_x;
+    n->train = train;
+    set_history(y, n);
+  }
+  return y;
 }
 
 }  // namespace anima_host

@@ -12,7 +12,7 @@ Tensor lokr_linear(const Tensor& x, Op x_row, Op x_col, const Tensor& W, const O
 // y = x merged^T + bias with the gradient of merged
 Tensor merged_linear(const Tensor& x, Op x_row, Op x_col, const Tensor& merged, const OptTensor& bias, bool first);
 // y = x W^T + bias, W frozen and quantised; `w_bf16` serves backward when W has no column form
-Tensor frozen_linear(const Tensor& x, Op x_row, Op w_row, Op w_col, const OptTensor& w_bf16, int64_t k_in,
+Tensor frozen_linear(const Tensor& x, Op x_row, Op w_row, Op w_col, const OptTensor& w_bf16,
                      const OptTensor& bias);
 // layer2(gelu(layer1(x))) with both layers LoKr linears
 Tensor lokr_mlp(const Tensor& x, Op x_row, Op x_col, const Tensor& W1, const OptTensor& b1, const Tensor& w1a,

@@ -12,25 +12,31 @@ using namespace anima_host;
 
 namespace {
 
-using Pair = std::pair<OptTensor, OptTensor>;
-Pair pair_of(const Op& o) { return o.defined() ? Pair{o.codes, o.scales} : Pair{}; }
+using O = const OptTensor&;
+// an operand as Python holds it: codes, scales and the allocation both lie in (or nothing)
+using Triple = std::tuple<OptTensor, OptTensor, OptTensor>;
+Triple triple_of(const Op& o, int layout = ANIMA_SCALES_TILED) {
+  if (!o.defined()) return {};
+  auto [codes, scales] = tensors_of(o, layout);
+  return {codes, scales, o.other.defined() ? OptTensor() : OptTensor(o.store)};
+}
 
-std::pair<Pair, Pair> py_quantize(const Tensor& x, bool row, bool col, int layout) {
+std::pair<Triple, Triple> py_quantize(const Tensor& x, bool row, bool col, int layout) {
   TORCH_CHECK_TYPE(x.scalar_type() == BF16, "x must be bfloat16, got ", x.scalar_type());
   TORCH_CHECK_VALUE(x.dim() == 2, "x must be 2-D, got shape ", x.sizes());
   const Launch l(x);
   auto [r, c] = quantize(l, as_matrix(x, x.size(1)), row, col, layout);
-  return {pair_of(r), pair_of(c)};
+  return {triple_of(r, layout), triple_of(c, layout)};
 }
 
 Tensor py_gemm(const Tensor& ac, const Tensor& as, const Tensor& bc, const Tensor& bs, const OptTensor& bias) {
   const Launch l(ac);
   TORCH_CHECK(bc.device() == l.dev && as.device() == l.dev && bs.device() == l.dev, "tensors on different devices");
-  const Op a{ac, as}, b{bc, bs};
-  TORCH_CHECK_VALUE(!bias || (bias->scalar_type() == BF16 && bias->numel() == b.rows() && bias->is_contiguous()),
+  const Op a = op_of(ac, as), b = op_of(bc, bs);
+  TORCH_CHECK_VALUE(!bias || (bias->scalar_type() == BF16 && bias->numel() == b.rows && bias->is_contiguous()),
                     "bias must be contiguous bfloat16 of length N");
-  Tensor c = empty({a.rows(), b.rows()}, BF16, l.dev);
-  gemm(l, a, b, {c.data_ptr(), b.rows(), false}, ptr(bias));
+  Tensor c = empty({a.rows, b.rows}, BF16, l.dev);
+  gemm(l, a, b, {c.data_ptr(), b.rows, false}, ptr(bias));
   return c;
 }
 
@@ -42,63 +48,57 @@ Tensor py_retile(const Tensor& scales, int64_t rows, int64_t k) {
   return t;
 }
 
-Tensor py_lokr(const Tensor& x, const OptTensor& xrc, const OptTensor& xrs, const OptTensor& xcc, const OptTensor& xcs,
-               const Tensor& W, const OptTensor& bias, const Tensor& w1, const Tensor& w2, double alpha, bool first) {
-  return lokr_linear(x, make_op(xrc, xrs), make_op(xcc, xcs), W, bias, w1, w2, alpha, first);
+Tensor py_lokr(const Tensor& x, O xrc, O xrs, O xr, O xcc, O xcs, O xc, const Tensor& W, O bias, const Tensor& w1,
+               const Tensor& w2, double alpha, bool first) {
+  return lokr_linear(x, op_of(xrc, xrs, xr), op_of(xcc, xcs, xc), W, bias, w1, w2, alpha, first);
 }
-Tensor py_merged(const Tensor& x, const OptTensor& xrc, const OptTensor& xrs, const OptTensor& xcc, const OptTensor& xcs,
-                 const Tensor& merged, const OptTensor& bias, bool first) {
-  return merged_linear(x, make_op(xrc, xrs), make_op(xcc, xcs), merged, bias, first);
+Tensor py_merged(const Tensor& x, O xrc, O xrs, O xr, O xcc, O xcs, O xc, const Tensor& merged, O bias, bool first) {
+  return merged_linear(x, op_of(xrc, xrs, xr), op_of(xcc, xcs, xc), merged, bias, first);
 }
-Tensor py_frozen(const Tensor& x, const Tensor& xrc, const Tensor& xrs, const Tensor& wrc, const Tensor& wrs,
-                 const OptTensor& wcc, const OptTensor& wcs, const OptTensor& w_bf16, const OptTensor& bias) {
-  return frozen_linear(x, {xrc, xrs}, {wrc, wrs}, make_op(wcc, wcs), w_bf16, wrc.size(1), bias);
+Tensor py_frozen(const Tensor& x, O xrc, O xrs, O xr, O wrc, O wrs, O wr, O wcc, O wcs, O wc, O w_bf16, O bias) {
+  return frozen_linear(x, op_of(xrc, xrs, xr), op_of(wrc, wrs, wr), op_of(wcc, wcs, wc), w_bf16, bias);
 }
-Tensor py_lokr_mlp(const Tensor& x, const OptTensor& xrc, const OptTensor& xrs, const OptTensor& xcc, const OptTensor& xcs,
-                   const Tensor& W1, const OptTensor& b1, const Tensor& w1a, const Tensor& w2a, double alpha1,
-                   const Tensor& W2, const OptTensor& b2, const Tensor& w1b, const Tensor& w2b, double alpha2, bool first) {
-  return lokr_mlp(x, make_op(xrc, xrs), make_op(xcc, xcs), W1, b1, w1a, w2a, alpha1, W2, b2, w1b, w2b, alpha2, first);
+Tensor py_lokr_mlp(const Tensor& x, O xrc, O xrs, O xr, O xcc, O xcs, O xc, const Tensor& W1, O b1, const Tensor& w1a,
+                   const Tensor& w2a, double alpha1, const Tensor& W2, O b2, const Tensor& w1b, const Tensor& w2b,
+                   double alpha2, bool first) {
+  return lokr_mlp(x, op_of(xrc, xrs, xr), op_of(xcc, xcs, xc), W1, b1, w1a, w2a, alpha1, W2, b2, w1b, w2b, alpha2, first);
 }
 
-TLinear py_tlinear(const Tensor& wrc, const Tensor& wrs, const Tensor& wcc, const Tensor& wcs, const OptTensor& bias,
-                   const Tensor& w1, const Tensor& a, const Tensor& b, const OptTensor& mask, double alpha, const Tensor& c,
-                   const std::vector<Tensor>& forms, bool fold, bool fuse_mix) {
+TLinear py_tlinear(const Tensor& wrc, const Tensor& wrs, const Tensor& wcc, const Tensor& wcs, O bias, const Tensor& w1,
+                   const Tensor& a, const Tensor& b, O mask, double alpha, const Tensor& c, const std::vector<Tensor>& forms,
+                   bool fold, bool fuse_mix) {
   TORCH_CHECK_VALUE(forms.size() == 8 || forms.size() == 10, "T-LoKr factor forms: 8 or 10 tensors");
   OptTensor m = mask;
   if (m) m = bf16_contiguous(*m);
-  TLinear t{{wrc, wrs}, {wcc, wcs}, bias, w1, a, b, m, alpha, c, {forms[0], forms[1]}, {forms[2], forms[3]},
-            {forms[4], forms[5]}, {forms[6], forms[7]}, {}, fold, fuse_mix};
-  if (forms.size() == 10) t.a_scaled = {forms[8], forms[9]};
+  TLinear t{op_of(wrc, wrs), op_of(wcc, wcs), bias, w1, a, b, m, alpha, c, op_of(forms[0], forms[1]),
+            op_of(forms[2], forms[3]), op_of(forms[4], forms[5]), op_of(forms[6], forms[7]), {}, fold, fuse_mix};
+  if (forms.size() == 10) t.a_scaled = op_of(forms[8], forms[9]);
   return t;
 }
-Tensor py_tlokr(const Tensor& x, const OptTensor& xrc, const OptTensor& xrs, const TLinear& t, bool first) {
-  return tlokr_linear(x, make_op(xrc, xrs), t, first);
+Tensor py_tlokr(const Tensor& x, O xrc, O xrs, O xr, const TLinear& t, bool first) {
+  return tlokr_linear(x, op_of(xrc, xrs, xr), t, first);
 }
-Tensor py_tlokr_mlp(const Tensor& x, const OptTensor& xrc, const OptTensor& xrs, const TLinear& t1, const TLinear& t2,
-                    bool first) {
-  return tlokr_mlp(x, make_op(xrc, xrs), t1, t2, first);
+Tensor py_tlokr_mlp(const Tensor& x, O xrc, O xrs, O xr, const TLinear& t1, const TLinear& t2, bool first) {
+  return tlokr_mlp(x, op_of(xrc, xrs, xr), t1, t2, first);
 }
 Tensor py_tlokr_fwd(const Tensor& xc, const Tensor& xs, const Tensor& gc, const Tensor& gs, const std::vector<int64_t>& lead,
                     const TLinear& t) {
-  return tlokr_forward_only({xc, xs}, {gc, gs}, lead, t);
+  return tlokr_forward_only(op_of(xc, xs), op_of(gc, gs), lead, t);
 }
 std::vector<Tensor> py_tlokr_bwd(const std::vector<Tensor>& g, const std::vector<Tensor>& x, const std::vector<int64_t>& lead,
                                  const TLinear& t) {
-  return tlokr_backward_only({g.at(0), g.at(1)}, {g.at(2), g.at(3)}, {x.at(0), x.at(1)}, {x.at(2), x.at(3)}, lead, t);
+  return tlokr_backward_only(op_of(g.at(0), g.at(1)), op_of(g.at(2), g.at(3)), op_of(x.at(0), x.at(1)),
+                             op_of(x.at(2), x.at(3)), lead, t);
 }
 
-std::tuple<Tensor, OptTensor, OptTensor> py_adaln(const Tensor& x, const Tensor& scale, const Tensor& shift, double eps,
-                                                  bool quant) {
+std::tuple<Tensor, Triple> py_adaln(const Tensor& x, const Tensor& scale, const Tensor& shift, double eps, bool quant) {
   auto [y, op] = adaln(x, scale, shift, eps, quant);
-  const Pair p = pair_of(op);
-  return {y, p.first, p.second};
+  return {y, triple_of(op)};
 }
-std::tuple<Tensor, Tensor, OptTensor, OptTensor> py_gated_add_adaln(const Tensor& x, const Tensor& gate, const Tensor& sub,
-                                                                    const Tensor& scale, const Tensor& shift, double eps,
-                                                                    bool quant) {
+std::tuple<Tensor, Tensor, Triple> py_gated_add_adaln(const Tensor& x, const Tensor& gate, const Tensor& sub,
+                                                      const Tensor& scale, const Tensor& shift, double eps, bool quant) {
   auto [n, y, op] = gated_add_adaln(x, gate, sub, scale, shift, eps, quant);
-  const Pair p = pair_of(op);
-  return {n, y, p.first, p.second};
+  return {n, y, triple_of(op)};
 }
 
 }  // namespace

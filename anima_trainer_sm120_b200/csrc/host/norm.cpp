@@ -1,13 +1,8 @@
 #include "norm.h"
 
-#include <torch/csrc/autograd/functions/utils.h>
-#include <torch/csrc/autograd/saved_variable.h>
-
-#include <mutex>
-
 namespace anima_host {
 
-using torch::autograd::Function;
+using torch::autograd::set_history;
 
 namespace {
 
@@ -57,26 +52,26 @@ Tensor scratch(int64_t bytes, const at::Device& dev) { return bytes ? empty({byt
 
 // ------------------------------------------------------------------------------------------------ AdaLN
 struct AdalnOut {
-  Tensor y, x, mean, rstd;      // x as the kernel read it
+  Tensor y, x, stats;           // x as the kernel read it; mean and rstd of its rows
   Mods mods;                    // scale, shift
   Op emitted;
 };
 AdalnOut adaln_fwd(const Launch& l, const Tensor& x, const Tensor& scale, const Tensor& shift, float eps, bool quant) {
   const Rows r = rows_of(x);
-  AdalnOut o{like(x, l.dev), bf16_contiguous(x), empty({r.n}, F32, l.dev), empty({r.n}, F32, l.dev), mods_of({&scale, &shift}), {}};
+  AdalnOut o{like(x, l.dev), bf16_contiguous(x), empty({2, r.n}, F32, l.dev), mods_of({&scale, &shift}), {}};
+  float* stats = o.stats.data_ptr<float>();
   if (quant) o.emitted = empty_op(r.n, r.d, l.dev);
   check(anima_adaln_fwd_ex(o.x.data_ptr(), nullptr, nullptr, o.mods.t[0].data_ptr(), o.mods.t[1].data_ptr(), o.mods.ld, eps, r.n,
-                           r.hw, r.d, nullptr, o.y.data_ptr(), o.mean.data_ptr<float>(), o.rstd.data_ptr<float>(),
-                           ptr8(o.emitted.codes), ptr8(o.emitted.scales), ANIMA_SCALES_TILED, l.stream));
+                           r.hw, r.d, nullptr, o.y.data_ptr(), stats, stats + r.n, o.emitted.codes, o.emitted.scales, ANIMA_SCALES_TILED, l.stream));
   return o;
 }
 
 // dx (+ d_res, another gradient of x), dscale, dshift (undefined unless `mod`)
 std::tuple<Tensor, Tensor, Tensor> adaln_bwd(const Launch& l, const Tensor& dy_, const Tensor& d_res_, const Tensor& x,
-                                             const Tensor& scale, int64_t ld, const Tensor& mean, const Tensor& rstd,
-                                             bool mod) {
+                                             const Tensor& scale, int64_t ld, const Tensor& stats_, bool mod) {
   const Rows r = rows_of(x);
   const Tensor dy = bf16_contiguous(dy_), d_res = d_res_.defined() ? bf16_contiguous(d_res_) : Tensor();
+  const float* stats = stats_.data_ptr<float>();
   Tensor dx = like(x, l.dev), ds, db;
   const int64_t bytes = mod ? check(anima_adaln_bwd_workspace_bytes(r.n, r.hw, r.d)) : 0;
   const Tensor ws = scratch(bytes, l.dev);
@@ -85,8 +80,7 @@ std::tuple<Tensor, Tensor, Tensor> adaln_bwd(const Launch& l, const Tensor& dy_,
     db = dense_like(scale, l.dev);
   }
   check(anima_adaln_bwd_ex(dy.data_ptr(), ptr(d_res), x.data_ptr(), scale.data_ptr(), nullptr, nullptr, ld,
-                           mean.data_ptr<float>(), rstd.data_ptr<float>(), r.n, r.hw, r.d, dx.data_ptr(), nullptr, ptr(ds),
-                           ptr(db), nullptr, ptr(ws), bytes, l.stream));
+                           stats, stats + r.n, r.n, r.hw, r.d, dx.data_ptr(), nullptr, ptr(ds), ptr(db), nullptr, ptr(ws), bytes, l.stream));
   return {dx, ds, db};
 }
 
@@ -106,8 +100,7 @@ std::pair<Tensor, Tensor> gated_bwd(const Launch& l, const Tensor& dout_, const 
 // The node has a second output slot, an alias of x: the gated residual that reads the same x right after its
 // modulation (every sublayer does) takes its x from there, so its gradient arrives here and dx = that + dx_ln is one
 // kernel instead of two and an addition (3 passes over a gradient). Values are those of the separate addition.
-struct AdalnNode : public torch::autograd::Node {
-  torch::autograd::SavedVariable x, scale, mean, rstd;
+struct AdalnNode : public HostNode {      // saves x, scale, statistics
   int64_t ld;
   at::ScalarType dt_x, dt_scale, dt_shift;
   bool used = false;
@@ -120,11 +113,10 @@ struct AdalnNode : public torch::autograd::Node {
       return out;
     }
     used = true;
-    const auto self = getptr();
-    const Tensor xs = x.unpack(self), sc = scale.unpack(self), mu = mean.unpack(self), rs = rstd.unpack(self);
-    const Launch l(xs);
+    const Tensor x = get(0), scale = get(1), stats = get(2);
+    const Launch l(x);
     const bool mod = task_should_compute_output(1) || task_should_compute_output(2);
-    auto [dx, ds, db] = adaln_bwd(l, g[0], g[1], xs, sc, ld, mu, rs, mod);
+    auto [dx, ds, db] = adaln_bwd(l, g[0], g[1], x, scale, ld, stats, mod);
     out[0] = back_to(dx, dt_x);
     out[1] = back_to(ds, dt_scale);
     out[2] = back_to(db, dt_shift);
@@ -132,9 +124,7 @@ struct AdalnNode : public torch::autograd::Node {
   }
   // A pass that only went through the alias leaves the saved tensors for the one that needs them.
   void release_variables() override {
-    std::lock_guard<std::mutex> lock(mutex_);
-    if (!used) return;
-    for (auto* v : {&x, &scale, &mean, &rstd}) v->reset_data();
+    if (used) HostNode::release_variables();
   }
   std::string name() const override { return "FusedAdaLNBackward"; }
 };
@@ -167,11 +157,6 @@ Tensor through_modulation(const Tensor& x) {
 }
 
 // ------------------------------------------------------------------------------------------------ gated residual
-struct GatedHeld {
-  at::ScalarType x, gate, y;
-  int64_t ld;
-  bool mod;
-};
 Tensor gated_fwd(const Launch& l, const Tensor& x_, const Tensor& y, const Mods& gate) {
   const Rows r = rows_of(x_);
   const Tensor x = bf16_contiguous(x_);
@@ -181,152 +166,101 @@ Tensor gated_fwd(const Launch& l, const Tensor& x_, const Tensor& y, const Mods&
   return out;
 }
 
-struct GatedAdd : Function<GatedAdd> {
-  static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& gate, const Tensor& y, bool mod) {
-    const Launch l(x);
-    const Tensor yc = bf16_contiguous(y);
-    const Mods g = mods_of({&gate});
-    ctx->save_for_backward({yc, g.t[0]});
-    hold(ctx, GatedHeld{x.scalar_type(), gate.scalar_type(), y.scalar_type(), g.ld, mod});
-    return gated_fwd(l, x, yc, g);
+struct GatedNode : public HostNode {      // saves y, gate
+  int64_t ld;
+  at::ScalarType dt_gate, dt_y;
+
+  variable_list apply(variable_list&& g) override {
+    std::lock_guard<std::mutex> lock(mutex_);
+    const Tensor dout = grad_of(g, 0), y = get(0), gate = get(1);
+    const Launch l(y);
+    auto [dy, dg] = gated_bwd(l, dout, y, gate, ld, task_should_compute_output(1));
+    return {dout, back_to(dg, dt_gate), back_to(dy, dt_y)};
   }
-  static variable_list backward(AutogradContext* ctx, variable_list grads) {
-    const variable_list s = ctx->get_saved_variables();
-    const GatedHeld h = held<GatedHeld>(ctx);
-    const Launch l(s[0]);
-    auto [dy, dg] = gated_bwd(l, grads[0], s[0], s[1], h.ld, h.mod);
-    return {grads[0], back_to(dg, h.gate), back_to(dy, h.y), Tensor()};
-  }
+  std::string name() const override { return "FusedGatedAddBackward"; }
 };
 
 // ------------------------------------------------------------------------------------------------ both at once
-struct BothCall {
-  float eps;
-  bool quant, mod;
-  Op emitted;
-  Tensor sub, x_new, mean, rstd;
+struct Both {
+  Tensor x_new, y, sub, stats;
   Mods mods;      // gate, scale, shift
-};
-struct BothHeld {
-  at::ScalarType x, gate, sub, scale, shift;
-  int64_t ld;
-  bool mod;
+  Op emitted;
 };
 
-Tensor both_fwd(const Launch& l, const Tensor& x_, const Tensor& gate, const Tensor& sub, const Tensor& scale,
-                const Tensor& shift, BothCall& c) {
+Both both_fwd(const Launch& l, const Tensor& x_, const Tensor& gate, const Tensor& sub, const Tensor& scale,
+              const Tensor& shift, float eps, bool quant) {
   const Rows r = rows_of(x_);
   const Tensor x = bf16_contiguous(x_);
-  c.sub = bf16_contiguous(sub);
-  c.mods = mods_of({&gate, &scale, &shift});
-  c.x_new = like(x, l.dev);
-  Tensor y = like(x, l.dev);
-  c.mean = empty({r.n}, F32, l.dev);
-  c.rstd = empty({r.n}, F32, l.dev);
-  if (c.quant) c.emitted = empty_op(r.n, r.d, l.dev);
+  Both c{like(x, l.dev), like(x, l.dev), bf16_contiguous(sub), empty({2, r.n}, F32, l.dev), mods_of({&gate, &scale, &shift}), {}};
+  float* stats = c.stats.data_ptr<float>();
+  if (quant) c.emitted = empty_op(r.n, r.d, l.dev);
   check(anima_adaln_fwd_ex(x.data_ptr(), c.mods.t[0].data_ptr(), c.sub.data_ptr(), c.mods.t[1].data_ptr(),
-                           c.mods.t[2].data_ptr(), c.mods.ld, c.eps, r.n, r.hw, r.d, c.x_new.data_ptr(), y.data_ptr(),
-                           c.mean.data_ptr<float>(), c.rstd.data_ptr<float>(), ptr8(c.emitted.codes), ptr8(c.emitted.scales),
-                           ANIMA_SCALES_TILED, l.stream));
-  return y;
+                           c.mods.t[2].data_ptr(), c.mods.ld, eps, r.n, r.hw, r.d, c.x_new.data_ptr(), c.y.data_ptr(), stats,
+                           stats + r.n, c.emitted.codes, c.emitted.scales, ANIMA_SCALES_TILED, l.stream));
+  return c;
 }
 
-struct GatedAddAdaLN : Function<GatedAddAdaLN> {
-  static variable_list forward(AutogradContext* ctx, const Tensor& x, const Tensor& gate, const Tensor& sub,
-                               const Tensor& scale, const Tensor& shift, BothCall* c) {
-    const Launch l(x);
-    Tensor y = both_fwd(l, x, gate, sub, scale, shift, *c);
-    ctx->save_for_backward({c->sub, c->mods.t[0], c->x_new, c->mods.t[1], c->mean, c->rstd});
-    ctx->set_materialize_grads(false);
-    hold(ctx, BothHeld{x.scalar_type(), gate.scalar_type(), sub.scalar_type(), scale.scalar_type(), shift.scalar_type(),
-                       c->mods.ld, c->mod});
-    return {c->x_new, y};
-  }
-  static variable_list backward(AutogradContext* ctx, variable_list grads) {
-    const BothHeld h = held<BothHeld>(ctx);
-    variable_list out(6);
+struct BothNode : public HostNode {      // saves sub, gate, x_new, scale, statistics
+  int64_t ld;
+  at::ScalarType dt_gate, dt_sub, dt_scale, dt_shift;
+
+  variable_list apply(variable_list&& grads) override {
+    std::lock_guard<std::mutex> lock(mutex_);
+    variable_list out(5);
     const Tensor &d_xnew = grads[0], &d_y = grads[1];
     if (!d_xnew.defined() && !d_y.defined()) return out;
-    const variable_list s = ctx->get_saved_variables();
-    const Tensor &sub = s[0], &gate = s[1], &x_new = s[2], &scale = s[3], &mean = s[4], &rstd = s[5];
+    const Tensor sub = get(0), gate = get(1), x_new = get(2), scale = get(3), stats = get(4);
     const Launch l(x_new);
+    const bool mod = task_should_compute_output(1) || task_should_compute_output(3) || task_should_compute_output(4);
     Tensor dx, dsub, dscale, dshift, dgate;
     if (d_xnew.defined() && d_y.defined()) {      // the usual case: one kernel for both backward ops
       const Rows r = rows_of(x_new);
       const Tensor dy = bf16_contiguous(d_y), dn = bf16_contiguous(d_xnew);
-      const int64_t bytes = h.mod ? check(anima_gated_add_adaln_bwd_workspace_bytes(r.n, r.hw, r.d)) : 0;
+      const int64_t bytes = mod ? check(anima_gated_add_adaln_bwd_workspace_bytes(r.n, r.hw, r.d)) : 0;
       const Tensor ws = scratch(bytes, l.dev);
+      const float* st = stats.data_ptr<float>();
       dx = like(x_new, l.dev);
       dsub = like(x_new, l.dev);
-      if (h.mod) {
+      if (mod) {
         dscale = dense_like(scale, l.dev);
         dshift = dense_like(scale, l.dev);
         dgate = dense_like(gate, l.dev);
       }
       check(anima_adaln_bwd_ex(dy.data_ptr(), dn.data_ptr(), x_new.data_ptr(), scale.data_ptr(), gate.data_ptr(),
-                               sub.data_ptr(), h.ld, mean.data_ptr<float>(), rstd.data_ptr<float>(), r.n, r.hw, r.d,
-                               dx.data_ptr(), dsub.data_ptr(), ptr(dscale), ptr(dshift), ptr(dgate), ptr(ws), bytes,
-                               l.stream));
+                               sub.data_ptr(), ld, st, st + r.n, r.n, r.hw, r.d, dx.data_ptr(), dsub.data_ptr(), ptr(dscale),
+                               ptr(dshift), ptr(dgate), ptr(ws), bytes, l.stream));
     } else {
       dx = d_xnew;
-      if (d_y.defined())
-        std::tie(dx, dscale, dshift) = adaln_bwd(l, d_y, Tensor(), x_new, scale, h.ld, mean, rstd, h.mod);
-      std::tie(dsub, dgate) = gated_bwd(l, dx, sub, gate, h.ld, h.mod);
+      if (d_y.defined()) std::tie(dx, dscale, dshift) = adaln_bwd(l, d_y, Tensor(), x_new, scale, ld, stats, mod);
+      std::tie(dsub, dgate) = gated_bwd(l, dx, sub, gate, ld, mod);
     }
-    out[0] = back_to(dx, h.x);
-    out[1] = back_to(dgate, h.gate);
-    out[2] = back_to(dsub, h.sub);
-    out[3] = back_to(dscale, h.scale);
-    out[4] = back_to(dshift, h.shift);
+    out[0] = dx;
+    out[1] = back_to(dgate, dt_gate);
+    out[2] = back_to(dsub, dt_sub);
+    out[3] = back_to(dscale, dt_scale);
+    out[4] = back_to(dshift, dt_shift);
     return out;
   }
+  std::string name() const override { return "FusedGatedAddAdaLNBackward"; }
 };
 
 // ------------------------------------------------------------------------------------------------ RMSNorm + RoPE
-struct RopeCall {
-  Tensor x, w, cos, sin, rstd;
-  float eps;
-};
+struct RopeNode : public HostNode {      // saves x, rstd
+  Tensor w, cos, sin;
 
-Tensor rope_fwd(const Launch& l, const Tensor& x, const Tensor& weight, RopeCall& c) {
-  TORCH_CHECK_TYPE(x.scalar_type() == BF16, "RMSNorm + RoPE needs bfloat16, got ", x.scalar_type());
-  c.x = x.is_contiguous() ? x : x.detach().contiguous();
-  c.w = weight.detach().to(F32).contiguous();
-  const int64_t heads = x.size(-2), d = x.size(-1), tokens = x.numel() ? x.numel() / (heads * d) : 0;
-  Tensor out = like(x, l.dev);
-  c.rstd = empty({tokens * heads}, F32, l.dev);
-  if (tokens)
-    check(anima_rmsnorm_rope_fwd(c.x.data_ptr(), c.w.data_ptr<float>(), static_cast<float*>(ptr(c.cos)),
-                                 static_cast<float*>(ptr(c.sin)), c.eps, tokens, heads, d, c.cos.defined() ? c.cos.size(0) : 1,
-                                 out.data_ptr(), c.rstd.data_ptr<float>(), l.stream));
-  return out;
-}
-
-struct RopeHeld {
-  Tensor cos, sin;
-};
-struct RmsNormRope : Function<RmsNormRope> {
-  static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& weight, RopeCall* c) {
+  variable_list apply(variable_list&& g) override {
+    std::lock_guard<std::mutex> lock(mutex_);
+    const Tensor dout = bf16_contiguous(grad_of(g, 0)), x = get(0), rstd = get(1);
     const Launch l(x);
-    Tensor out = rope_fwd(l, x, weight, *c);
-    ctx->save_for_backward({c->x, c->w, c->rstd});
-    hold(ctx, RopeHeld{c->cos, c->sin});
-    return out;
-  }
-  static variable_list backward(AutogradContext* ctx, variable_list grads) {
-    const variable_list s = ctx->get_saved_variables();
-    const RopeHeld& h = held<RopeHeld>(ctx);
-    const Tensor &x = s[0], &w = s[1], &rstd = s[2];
-    const Launch l(x);
-    const Tensor dout = bf16_contiguous(grads[0]);
     Tensor dx = like(x, l.dev);
     const int64_t heads = x.size(-2), d = x.size(-1), tokens = x.numel() ? x.numel() / (heads * d) : 0;
     if (tokens)
-      check(anima_rmsnorm_rope_bwd(dout.data_ptr(), x.data_ptr(), w.data_ptr<float>(), static_cast<float*>(ptr(h.cos)),
-                                   static_cast<float*>(ptr(h.sin)), rstd.data_ptr<float>(), tokens, heads, d,
-                                   h.cos.defined() ? h.cos.size(0) : 1, dx.data_ptr(), l.stream));
-    return {dx, Tensor(), Tensor()};
+      check(anima_rmsnorm_rope_bwd(dout.data_ptr(), x.data_ptr(), w.data_ptr<float>(), static_cast<float*>(ptr(cos)),
+                                   static_cast<float*>(ptr(sin)), rstd.data_ptr<float>(), tokens, heads, d,
+                                   cos.defined() ? cos.size(0) : 1, dx.data_ptr(), l.stream));
+    return {dx};
   }
+  std::string name() const override { return "FusedRMSNormRoPEBackward"; }
 };
 
 }  // namespace
@@ -340,47 +274,99 @@ std::tuple<Tensor, Op> adaln(const Tensor& x, const Tensor& scale, const Tensor&
     o = adaln_fwd(l, x, scale, shift, static_cast<float>(eps), quant);
   }
   if (grad) {
-    auto node = std::shared_ptr<AdalnNode>(new AdalnNode(), torch::autograd::deleteNode);
-    node->set_next_edges(torch::autograd::collect_next_edges(x, scale, shift));
-    node->x = {o.x, false};
-    node->scale = {o.mods.t[0], false};
-    node->mean = {o.mean, false};
-    node->rstd = {o.rstd, false};
+    auto node = make_node<AdalnNode>(x, scale, shift);
+    node->save(o.x);
+    node->save(o.mods.t[0]);
+    node->save(o.stats);
     node->ld = o.mods.ld;
     node->dt_x = x.scalar_type();
     node->dt_scale = scale.scalar_type();
     node->dt_shift = shift.scalar_type();
-    torch::autograd::set_history(o.y, node);
+    set_history(o.y, node);
     node->add_input_metadata(x);
     if (x.requires_grad() && !x.is_inference()) remember(x, node);
   }
   return {o.y, o.emitted};
 }
 
-Tensor gated_add(const Tensor& x, const Tensor& gate, const Tensor& y) {
-  if (wants(x) || wants(gate) || wants(y)) return GatedAdd::apply(through_modulation(x), gate, y, wants(gate));
-  const Launch l(x);
-  return gated_fwd(l, x, bf16_contiguous(y), mods_of({&gate}));
+Tensor gated_add(const Tensor& x_, const Tensor& gate, const Tensor& y) {
+  const bool grad = wants(x_) || wants(gate) || wants(y);
+  const Launch l(x_);
+  const Tensor x = grad ? through_modulation(x_) : x_;
+  Tensor out, yc;
+  Mods g;
+  {
+    Below below;
+    yc = bf16_contiguous(y);
+    g = mods_of({&gate});
+    out = gated_fwd(l, x, yc, g);
+  }
+  if (grad) {
+    auto node = make_node<GatedNode>(x, gate, y);
+    node->save(yc);
+    node->save(g.t[0]);
+    node->ld = g.ld;
+    node->dt_gate = gate.scalar_type();
+    node->dt_y = y.scalar_type();
+    set_history(out, node);
+  }
+  return out;
 }
 
-std::tuple<Tensor, Tensor, Op> gated_add_adaln(const Tensor& x, const Tensor& gate, const Tensor& sub, const Tensor& scale,
+std::tuple<Tensor, Tensor, Op> gated_add_adaln(const Tensor& x_, const Tensor& gate, const Tensor& sub, const Tensor& scale,
                                                const Tensor& shift, double eps, bool quant) {
-  const bool mod = wants(gate) || wants(scale) || wants(shift);
-  BothCall c{static_cast<float>(eps), quant, mod};
-  if (mod || wants(x) || wants(sub)) {
-    variable_list r = GatedAddAdaLN::apply(through_modulation(x), gate, sub, scale, shift, &c);
-    return {r[0], r[1], c.emitted};
+  const bool grad = wants(x_) || wants(sub) || wants(gate) || wants(scale) || wants(shift);
+  const Launch l(x_);
+  const Tensor x = grad ? through_modulation(x_) : x_;
+  Both c;
+  {
+    Below below;
+    c = both_fwd(l, x, gate, sub, scale, shift, static_cast<float>(eps), quant);
   }
-  const Launch l(x);
-  Tensor y = both_fwd(l, x, gate, sub, scale, shift, c);
-  return {c.x_new, y, c.emitted};
+  if (grad) {
+    auto node = make_node<BothNode>(x, gate, sub, scale, shift);
+    set_history(c.x_new, node);
+    set_history(c.y, node);
+    node->save(c.sub);
+    node->save(c.mods.t[0]);
+    node->save(c.x_new, true);
+    node->save(c.mods.t[1]);
+    node->save(c.stats);
+    node->ld = c.mods.ld;
+    node->dt_gate = gate.scalar_type();
+    node->dt_sub = sub.scalar_type();
+    node->dt_scale = scale.scalar_type();
+    node->dt_shift = shift.scalar_type();
+  }
+  return {c.x_new, c.y, c.emitted};
 }
 
 Tensor rmsnorm_rope(const Tensor& x, const Tensor& weight, const OptTensor& cos, const OptTensor& sin, double eps) {
-  RopeCall c{Tensor(), Tensor(), cos.value_or(Tensor()), sin.value_or(Tensor()), Tensor(), static_cast<float>(eps)};
-  if (wants(x)) return RmsNormRope::apply(x, weight, &c);
+  TORCH_CHECK_TYPE(x.scalar_type() == BF16, "RMSNorm + RoPE needs bfloat16, got ", x.scalar_type());
   const Launch l(x);
-  return rope_fwd(l, x, weight, c);
+  const int64_t heads = x.size(-2), d = x.size(-1), tokens = x.numel() ? x.numel() / (heads * d) : 0;
+  Tensor out, xc, w, rstd;
+  {
+    Below below;
+    xc = x.is_contiguous() ? x : x.detach().contiguous();
+    w = weight.detach().to(F32).contiguous();
+    out = like(x, l.dev);
+    rstd = empty({tokens * heads}, F32, l.dev);
+    if (tokens)
+      check(anima_rmsnorm_rope_fwd(xc.data_ptr(), w.data_ptr<float>(), static_cast<float*>(ptr(cos)),
+                                   static_cast<float*>(ptr(sin)), static_cast<float>(eps), tokens, heads, d,
+                                   cos ? cos->size(0) : 1, out.data_ptr(), rstd.data_ptr<float>(), l.stream));
+  }
+  if (wants(x)) {
+    auto node = make_node<RopeNode>(x);
+    node->save(xc);
+    node->save(rstd);
+    node->w = w;
+    node->cos = cos.value_or(Tensor());
+    node->sin = sin.value_or(Tensor());
+    set_history(out, node);
+  }
+  return out;
 }
 
 }  // namespace anima_host

@@ -2,7 +2,7 @@
 
 namespace anima_host {
 
-using torch::autograd::Function;
+using torch::autograd::set_history;
 
 bool TLinear::can_fold(int64_t rows, int64_t cols, int64_t batch) const {
   return fold && c.size(0) == 8 && rows > 128 && cols > 128 && rows % 128 == 0 && cols % 8 == 0 && (cols / 8) % 64 == 0 &&
@@ -35,7 +35,7 @@ std::pair<Op, Op> mix_operands(const Launch& l, const Tensor& hidden, const TLin
   if (!col && can_quantise_mix(items, r)) {
     Op o = empty_op(R, r, l.dev);
     check(anima_tlokr_rank_mix_quant(hidden.data_ptr(), t.c.data_ptr(), mask_ptr(t.mask), batch, items / batch, r,
-                                     transpose ? 1 : 0, nullptr, ptr8(o.codes), ptr8(o.scales), nullptr, nullptr,
+                                     transpose ? 1 : 0, nullptr, o.codes, o.scales, nullptr, nullptr,
                                      l.stream));
     return {o, Op{}};
   }
@@ -43,8 +43,8 @@ std::pair<Op, Op> mix_operands(const Launch& l, const Tensor& hidden, const TLin
 }
 
 Tensor gemm_bf16(const Launch& l, const Op& a, const Op& b, double alpha = 1.0) {
-  Tensor c = empty({a.rows(), b.rows()}, BF16, l.dev);
-  gemm(l, a, b, {c.data_ptr(), b.rows(), false}, nullptr, nullptr, 0, alpha);
+  Tensor c = empty({a.rows, b.rows}, BF16, l.dev);
+  gemm(l, a, b, {c.data_ptr(), b.rows, false}, nullptr, nullptr, 0, alpha);
   return c;
 }
 
@@ -53,18 +53,18 @@ Tensor gemm_bf16(const Launch& l, const Op& a, const Op& b, double alpha = 1.0) 
 // the quantisation in its epilogue (hidden never leaves the SM), then ONE GEMM in which those planes times alpha * A
 // are extra K-blocks of the base projection. Other shapes add alpha * delta in the last GEMM's stores.
 void linear_fwd(const Launch& l, const Op& x_row, const Op& gq, int64_t batch, const TLinear& t, void* y) {
-  const int64_t rows = x_row.rows(), n = t.n_out(), vp = t.vp(), r = t.rank();
+  const int64_t rows = x_row.rows, n = t.n_out(), vp = t.vp(), r = t.rank();
   const Tensor b = t.bias && t.bias->defined() ? bf16_contiguous(*t.bias) : Tensor();
   if (t.can_fold(rows, n, batch) && n == 8 * vp) {
     Op planes = empty_op(rows * 8, r, l.dev);
     if (t.fuse_mix) {
-      check(anima_tlokr_hidden_mix_planes(ptr8(gq.codes), ptr8(gq.scales), ptr8(t.bq.codes), ptr8(t.bq.scales),
-                                          t.c.data_ptr(), mask_ptr(t.mask), batch, rows / batch, gq.k(), 0, nullptr,
-                                          ptr8(planes.codes), ptr8(planes.scales), status_word(l.dev), l.stream));
+      check(anima_tlokr_hidden_mix_planes(gq.codes, gq.scales, t.bq.codes, t.bq.scales,
+                                          t.c.data_ptr(), mask_ptr(t.mask), batch, rows / batch, gq.k, 0, nullptr,
+                                          planes.codes, planes.scales, status_word(l.dev), l.stream));
     } else {
       const Tensor hidden = gemm_bf16(l, gq, t.bq);
       check(anima_tlokr_rank_mix_quant_planes(hidden.data_ptr(), t.c.data_ptr(), mask_ptr(t.mask), batch, rows / batch, r,
-                                              0, ptr8(planes.codes), ptr8(planes.scales), nullptr, nullptr, l.stream));
+                                              0, planes.codes, planes.scales, nullptr, nullptr, l.stream));
     }
     gemm_delta(l, x_row, t.w_row, planes, t.a_scaled, y, ptr(b));
     return;
@@ -82,7 +82,7 @@ struct LinearGrads {
 // `g` / `g_col`: operands of the incoming gradient viewed as [rows * 8, vp]; gq / gq_col those of the grouped input.
 LinearGrads linear_bwd(const Launch& l, const Op& gbq, const Op& gbq_col, const Op& gq, const Op& gq_col,
                        at::IntArrayRef lead, const TLinear& t, bool need_x) {
-  const int64_t batch = lead[0], rows = gbq.rows() / 8, K = t.k_in(), vp = t.vp(), r = t.rank(), vq = K / 8;
+  const int64_t batch = lead[0], rows = gbq.rows / 8, K = t.k_in(), vp = t.vp(), r = t.rank(), vq = K / 8;
   LinearGrads g;
   const bool fold = t.can_fold(rows, K, batch);
   if (need_x) {
@@ -107,7 +107,7 @@ LinearGrads linear_bwd(const Launch& l, const Op& gbq, const Op& gbq_col, const 
     // grad_hidden leaves as eight planes + its column form; base dgrad and + grad_hidden @ B are one GEMM
     Op planes = empty_op(rows * 8, r, l.dev), col = empty_op(r, rows * 8, l.dev);
     check(anima_tlokr_rank_mix_quant_planes(g_mixed.data_ptr(), t.c.data_ptr(), mask_ptr(t.mask), batch, rows / batch, r, 1,
-                                            ptr8(planes.codes), ptr8(planes.scales), ptr8(col.codes), ptr8(col.scales),
+                                            planes.codes, planes.scales, col.codes, col.scales,
                                             l.stream));
     gb = gemm_f32(l, col, gq_col);                                     // grad_hidden^T @ grouped [r, vq]
     gemm_delta(l, regroup(l, gbq, rows, 8 * vp), t.w_col, planes, t.bq_col, g.x.data_ptr(), nullptr);
@@ -116,9 +116,9 @@ LinearGrads linear_bwd(const Launch& l, const Op& gbq, const Op& gbq_col, const 
     gb = gemm_f32(l, ghq_col, gq_col);
     if (need_x) gemm(l, ghq, t.bq_col, {g.x.data_ptr(), vq, false}, nullptr, g.x.data_ptr(), vq);
   }
-  g.w1 = cast(gc, t.w1.scalar_type());
-  g.a = cast(ga, t.a.scalar_type());
-  g.b = cast(gb, t.b.scalar_type());
+  g.w1 = cast(gc, t.w1.t.scalar_type());
+  g.a = cast(ga, t.a.t.scalar_type());
+  g.b = cast(gb, t.b.t.scalar_type());
   return g;
 }
 
@@ -126,206 +126,164 @@ struct Needs {
   bool x, factors, bias;
   bool any() const { return x || factors || bias; }
 };
-Needs needs_of(const Tensor& x, const TLinear& t) { return {wants(x), wants(t.w1) || wants(t.a) || wants(t.b), wants(t.bias)}; }
+Needs needs_of(const Tensor& x, const TLinear& t) {
+  return {wants(x), wants(t.w1.t) || wants(t.a.t) || wants(t.b.t), wants(t.bias)};
+}
 
 // Operands of a layer input. With `keep` the grouped view is quantised in both forms by one pass and its row codes
-// serve the base GEMM too; otherwise only the row form exists (`x_row`) and a placeholder stands in.
+// serve the base GEMM too; otherwise only the row form exists (`x_row`).
 struct Input {
   Op x_row, gq, gq_col;
 };
 template <class Quantise>
-Input input_operands(const Launch& l, Op x_row, int64_t rows, int64_t K, bool keep, bool hold_place, Quantise&& q) {
+Input input_operands(const Launch& l, const Op& x_row, int64_t rows, int64_t K, bool keep, Quantise&& q) {
   Input in;
   if (keep) {
     std::tie(in.gq, in.gq_col) = q(rows * 8, K / 8);
     in.x_row = regroup(l, in.gq, rows, K);
   } else {
-    in.x_row = std::move(x_row);
-    in.gq = regroup(l, in.x_row, rows * 8, K / 8);
-    if (hold_place) in.gq_col = placeholder(K / 8, rows * 8, l.dev);
+    in.x_row = x_row;
+    in.gq = regroup(l, x_row, rows * 8, K / 8);
   }
   return in;
 }
-
-void keep_mask(variable_list& v, const TLinear& t) {
-  if (t.mask && t.mask->defined()) v.push_back(*t.mask);
+// what a node saves of it: the grouped operands, or stand-ins for them
+void save_input(HostNode& n, const Launch& l, Input& in, int64_t rows, int64_t K, bool keep) {
+  if (!keep) {
+    in.gq = placeholder(rows * 8, K / 8, l.dev);
+    in.gq_col = placeholder(K / 8, rows * 8, l.dev);
+  }
+  n.save(in.gq);
+  n.save(in.gq_col);
 }
-// The tensors autograd saves are read back through it; the forms and the frozen weight ride along.
-void take_factors(TLinear& t, const variable_list& v, size_t at) {
-  t.w1 = v[at];
-  t.a = v[at + 1];
-  t.b = v[at + 2];
-}
-void take_mask(TLinear& t, const variable_list& v, size_t& at) {
-  if (t.mask && t.mask->defined()) t.mask = v[at++];
-}
-// What a node keeps outside its saved tensors: the parameters and the mask go through save_for_backward.
-TLinear without_saved(TLinear t) {
-  t.w1 = t.a = t.b = Tensor();
-  if (t.mask && t.mask->defined()) t.mask = t.c;          // only marks that there is one
-  return t;
+std::pair<Op, Op> saved_input(HostNode& n, size_t& at, int64_t rows, int64_t K) {
+  Op g, c;
+  g.rows = c.k = rows * 8;
+  g.k = c.rows = K / 8;
+  Op gq = n.get_op(at, g), gq_col = n.get_op(at, c);
+  return {gq, gq_col};
 }
 
 std::vector<int64_t> lead_of(const Tensor& x) { return {x.sizes().begin(), x.sizes().end() - 1}; }
-
+int64_t product(at::IntArrayRef v) { return c10::multiply_integers(v); }
 Tensor grad_bias(const Tensor& gy) { return gy.reshape({-1, gy.size(-1)}).sum(0); }
 
 // ------------------------------------------------------------------------------------------------ one linear
 // ``x W^T + bias + alpha * delta(x)`` as one node: x is quantised once (base GEMM and delta contract the same codes
-// under two scale tilings), so is the incoming gradient; saved are the MXFP8 operands of x in its grouped view and the
-// small factors, the rank-space intermediates are recomputed in backward.
-struct LinearHeld {
+// under two scale tilings), so is the incoming gradient; saved are the MXFP8 operands of x in its grouped view, the
+// rank-space intermediates are recomputed in backward.
+struct TlokrNode : public HostNode {
   TLinear t;
   Needs need;
-};
-struct LinearCall {
-  Op x_row;
-  TLinear t;
-  bool first;
-  Needs need;
-};
 
-Tensor run_linear(const Launch& l, const Tensor& x, LinearCall& c, Input& in) {
-  const int64_t K = c.t.k_in(), rows = x.numel() / K;
-  in = input_operands(l, c.x_row, rows, K, c.need.any() && !c.first, c.need.any(), [&](int64_t r, int64_t k) {
-    return quantize(l, as_matrix(x, k), true, true);
-  });
-  Tensor y = empty(with_last(x.sizes(), c.t.n_out()), BF16, l.dev);
-  linear_fwd(l, in.x_row, in.gq, x.size(0), c.t, y.data_ptr());
-  return y;
-}
-
-struct TlokrLinear : Function<TlokrLinear> {
-  static Tensor forward(AutogradContext* ctx, const Tensor& x, const OptTensor&, const Tensor& w1, const Tensor& a,
-                        const Tensor& b, LinearCall* c) {
-    const Launch l(x);
-    Input in;
-    Tensor y = run_linear(l, x, *c, in);
-    variable_list keep{w1, a, b};
-    push(keep, in.gq);
-    push(keep, in.gq_col);
-    keep_mask(keep, c->t);
-    ctx->save_for_backward(std::move(keep));
-    hold(ctx, LinearHeld{without_saved(c->t), c->need});
-    return y;
-  }
-  static variable_list backward(AutogradContext* ctx, variable_list grads) {
-    LinearHeld h = held<LinearHeld>(ctx);
-    const variable_list saved = ctx->get_saved_variables();   // once: activation checkpointing unpacks on access
-    take_factors(h.t, saved, 0);
-    size_t at = 3;
-    const Op gq = pop(saved, at, true), gq_col = pop(saved, at, true);
-    take_mask(h.t, saved, at);
-    const Tensor& gy = grads[0];
+  variable_list apply(variable_list&& g) override {
+    std::lock_guard<std::mutex> lock(mutex_);
+    const Tensor gy = grad_of(g, 0);
     const Launch l(gy);
-    auto [gbq, gbq_col] = quantize(l, as_matrix(gy, h.t.vp()), true, true);
-    LinearGrads g = linear_bwd(l, gbq, gbq_col, gq, gq_col, lead_of(gy), h.t, h.need.x);
-    variable_list out(6);
-    out[0] = g.x;
-    if (h.need.bias) out[1] = grad_bias(gy);
-    out[2] = g.w1;
-    out[3] = g.a;
-    out[4] = g.b;
-    return out;
+    const auto lead = lead_of(gy);
+    size_t at = 0;
+    const auto [gq, gq_col] = saved_input(*this, at, product(lead), t.k_in());
+    for (const Kept* k : {&t.w1, &t.a, &t.b}) k->get();
+    auto [gbq, gbq_col] = quantize(l, as_matrix(gy, t.vp()), true, true);
+    LinearGrads r = linear_bwd(l, gbq, gbq_col, gq, gq_col, lead, t, need.x);
+    return {r.x, need.bias ? grad_bias(gy) : Tensor(), r.w1, r.a, r.b};
   }
+  std::string name() const override { return "MXTLoKrLinearBackward"; }
 };
 
 // ------------------------------------------------------------------------------------------------ MLP
 // ``layer2(gelu(layer1(x)))``: the activation and its derivative are evaluated inside the quantiser, so neither
 // gelu(h) nor grad * gelu'(h) is written as a bf16 tensor.
-struct MlpHeld {
+struct TlokrMlpNode : public HostNode {
   TLinear t1, t2;
   bool need_x;
-};
-struct MlpCall {
-  Op x_row;
-  TLinear t1, t2;
-  bool first, need_x, back;
-};
 
-Tensor run_mlp(const Launch& l, const Tensor& x, MlpCall& c, Tensor& h, Input& in1, Input& in2) {
-  const int64_t K = c.t1.k_in(), rows = x.numel() / K, hid = c.t1.n_out();
-  const bool keep = c.back && !c.first;
-  in1 = input_operands(l, c.x_row, rows, K, keep, c.back,
-                       [&](int64_t r, int64_t k) { return quantize(l, as_matrix(x, k), true, true); });
-  h = empty(with_last(x.sizes(), hid), BF16, l.dev);
-  linear_fwd(l, in1.x_row, in1.gq, x.size(0), c.t1, h.data_ptr());
-  Op act_row;
-  if (!keep) act_row = quantize_gelu(l, h, Tensor(), rows, hid, true, false).first;
-  in2 = input_operands(l, act_row, rows, hid, keep, c.back,
-                       [&](int64_t r, int64_t k) { return quantize_gelu(l, h, Tensor(), r, k, true, true); });
-  Tensor y = empty(with_last(x.sizes(), c.t2.n_out()), BF16, l.dev);
-  linear_fwd(l, in2.x_row, in2.gq, x.size(0), c.t2, y.data_ptr());
-  return y;
-}
-
-struct TlokrMlp : Function<TlokrMlp> {
-  static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& w1_1, const Tensor& a_1, const Tensor& b_1,
-                        const Tensor& w1_2, const Tensor& a_2, const Tensor& b_2, MlpCall* c) {
-    const Launch l(x);
-    Tensor h;
-    Input in1, in2;
-    Tensor y = run_mlp(l, x, *c, h, in1, in2);
-    variable_list keep{h, w1_1, a_1, b_1, w1_2, a_2, b_2};
-    for (const Op* o : {&in1.gq, &in1.gq_col, &in2.gq, &in2.gq_col}) push(keep, *o);
-    keep_mask(keep, c->t1);
-    keep_mask(keep, c->t2);
-    ctx->save_for_backward(std::move(keep));
-    hold(ctx, MlpHeld{without_saved(c->t1), without_saved(c->t2), c->need_x});
-    return y;
-  }
-  static variable_list backward(AutogradContext* ctx, variable_list grads) {
-    MlpHeld m = held<MlpHeld>(ctx);
-    const variable_list saved = ctx->get_saved_variables();
-    const Tensor& h = saved[0];
-    take_factors(m.t1, saved, 1);
-    take_factors(m.t2, saved, 4);
-    size_t at = 7;
-    const Op gq1 = pop(saved, at, true), gq1_col = pop(saved, at, true), gq2 = pop(saved, at, true),
-             gq2_col = pop(saved, at, true);
-    take_mask(m.t1, saved, at);
-    take_mask(m.t2, saved, at);
-    const Tensor& gy = grads[0];
+  variable_list apply(variable_list&& g) override {
+    std::lock_guard<std::mutex> lock(mutex_);
+    const Tensor gy = grad_of(g, 0);
     const Launch l(gy);
     const auto lead = lead_of(gy);
+    const int64_t rows = product(lead);
+    const Tensor h = get(0);
+    size_t at = 1;
+    const auto [gq1, gq1_col] = saved_input(*this, at, rows, t1.k_in());
+    const auto [gq2, gq2_col] = saved_input(*this, at, rows, t2.k_in());
+    for (const Kept* k : {&t1.w1, &t1.a, &t1.b, &t2.w1, &t2.a, &t2.b}) k->get();
     LinearGrads g2, g1;
     {
-      auto [gbq, gbq_col] = quantize(l, as_matrix(gy, m.t2.vp()), true, true);
-      g2 = linear_bwd(l, gbq, gbq_col, gq2, gq2_col, lead, m.t2, true);
+      auto [gbq, gbq_col] = quantize(l, as_matrix(gy, t2.vp()), true, true);
+      g2 = linear_bwd(l, gbq, gbq_col, gq2, gq2_col, lead, t2, true);
     }
     {
-      const int64_t vp = m.t1.vp();
+      const int64_t vp = t1.vp();
       auto [gbq, gbq_col] = quantize_gelu(l, h, g2.x, h.numel() / vp, vp, true, true);
       g2.x.reset();
-      g1 = linear_bwd(l, gbq, gbq_col, gq1, gq1_col, lead, m.t1, m.need_x);
+      g1 = linear_bwd(l, gbq, gbq_col, gq1, gq1_col, lead, t1, need_x);
     }
-    return {g1.x, g1.w1, g1.a, g1.b, g2.w1, g2.a, g2.b, Tensor()};
+    return {g1.x, g1.w1, g1.a, g1.b, g2.w1, g2.a, g2.b};
   }
+  std::string name() const override { return "MXTLoKrMLPBackward"; }
 };
 
 }  // namespace
 
 Tensor tlokr_linear(const Tensor& x, Op x_row, TLinear t, bool first) {
   const Needs need = needs_of(x, t);
-  LinearCall c{std::move(x_row), std::move(t), first, need};
-  if (need.any()) return TlokrLinear::apply(x, c.t.bias, c.t.w1, c.t.a, c.t.b, &c);
   const Launch l(x);
+  const int64_t K = t.k_in(), rows = x.numel() / K;
+  const bool keep = need.any() && !first;
+  Tensor y;
   Input in;
-  return run_linear(l, x, c, in);
+  {
+    Below below;
+    in = input_operands(l, x_row, rows, K, keep, [&](int64_t, int64_t k) { return quantize(l, as_matrix(x, k), true, true); });
+    y = empty(with_last(x.sizes(), t.n_out()), BF16, l.dev);
+    linear_fwd(l, in.x_row, in.gq, x.size(0), t, y.data_ptr());
+  }
+  if (need.any()) {
+    auto n = make_node<TlokrNode>(x, t.bias, t.w1.t, t.a.t, t.b.t);
+    save_input(*n, l, in, rows, K, keep);
+    n->need = need;
+    n->t = std::move(t);
+    set_history(y, n);
+  }
+  return y;
 }
 
 Tensor tlokr_mlp(const Tensor& x, Op x_row, TLinear t1, TLinear t2, bool first) {
   const Needs n1 = needs_of(x, t1), n2 = needs_of(x, t2);
-  MlpCall c{std::move(x_row), std::move(t1), std::move(t2), first, n1.x, n1.x || n1.factors || n2.factors};
-  if (c.back) return TlokrMlp::apply(x, c.t1.w1, c.t1.a, c.t1.b, c.t2.w1, c.t2.a, c.t2.b, &c);
+  const bool back = n1.x || n1.factors || n2.factors, keep = back && !first;
   const Launch l(x);
-  Tensor h;
+  const int64_t K = t1.k_in(), rows = x.numel() / K, hid = t1.n_out();
+  Tensor y, h;
   Input in1, in2;
-  return run_mlp(l, x, c, h, in1, in2);
+  {
+    Below below;
+    in1 = input_operands(l, x_row, rows, K, keep, [&](int64_t, int64_t k) { return quantize(l, as_matrix(x, k), true, true); });
+    h = empty(with_last(x.sizes(), hid), BF16, l.dev);
+    linear_fwd(l, in1.x_row, in1.gq, x.size(0), t1, h.data_ptr());
+    Op act_row;
+    if (!keep) act_row = quantize_gelu(l, h, Tensor(), rows, hid, true, false).first;
+    in2 = input_operands(l, act_row, rows, hid, keep,
+                         [&](int64_t r, int64_t k) { return quantize_gelu(l, h, Tensor(), r, k, true, true); });
+    y = empty(with_last(x.sizes(), t2.n_out()), BF16, l.dev);
+    linear_fwd(l, in2.x_row, in2.gq, x.size(0), t2, y.data_ptr());
+  }
+  if (back) {
+    auto n = make_node<TlokrMlpNode>(x, t1.w1.t, t1.a.t, t1.b.t, t2.w1.t, t2.a.t, t2.b.t);
+    n->save(h);
+    save_input(*n, l, in1, rows, K, keep);
+    save_input(*n, l, in2, rows, hid, keep);
+    n->need_x = n1.x;
+    n->t1 = std::move(t1);
+    n->t2 = std::move(t2);
+    set_history(y, n);
+  }
+  return y;
 }
 
 Tensor tlokr_forward_only(const Op& x_row, const Op& gq, at::IntArrayRef lead, const TLinear& t) {
-  const Launch l(x_row.codes);
+  const Launch l(x_row.store);
   std::vector<int64_t> shape(lead.begin(), lead.end());
   shape.push_back(t.n_out());
   Tensor y = empty(shape, BF16, l.dev);
@@ -335,7 +293,7 @@ Tensor tlokr_forward_only(const Op& x_row, const Op& gq, at::IntArrayRef lead, c
 
 std::vector<Tensor> tlokr_backward_only(const Op& gbq, const Op& gbq_col, const Op& gq, const Op& gq_col,
                                         at::IntArrayRef lead, const TLinear& t) {
-  const Launch l(gbq.codes);
+  const Launch l(gbq.store);
   LinearGrads g = linear_bwd(l, gbq, gbq_col, gq, gq_col, lead, t, true);
   return {g.x, g.w1, g.a, g.b};
 }

@@ -9,17 +9,17 @@ namespace anima_host {
 struct TLinear {
   Op w_row, w_col;
   OptTensor bias;
-  Tensor w1, a, b;          // parameters: [8, 8], [vp, r], [r, vq]
+  Kept w1, a, b;            // parameters: [8, 8], [vp, r], [r, vq]
   OptTensor mask;           // [batch, r]
   double alpha;
   Tensor c;                 // w1 in bf16
   Op aq, aq_col, bq, bq_col, a_scaled;   // a_scaled: row form of alpha * a (folded delta only)
   bool fold, fuse_mix;      // switches of tlokr.py
 
-  int64_t n_out() const { return w_row.rows(); }
-  int64_t k_in() const { return w_row.k(); }
-  int64_t vp() const { return a.size(0); }
-  int64_t rank() const { return a.size(1); }
+  int64_t n_out() const { return w_row.rows; }
+  int64_t k_in() const { return w_row.k; }
+  int64_t vp() const { return a.t.size(0); }
+  int64_t rank() const { return a.t.size(1); }
   bool can_fold(int64_t rows, int64_t cols, int64_t batch) const;
 };
 

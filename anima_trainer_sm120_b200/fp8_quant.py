@@ -151,8 +151,9 @@ def _wants_grad(*tensors) -> bool:
     return torch.is_grad_enabled() and any(t is not None and t.requires_grad for t in tensors)
 
 
-def _pair(op: ops.MXOperand | None) -> tuple:
-    return (None, None) if op is None else (op.codes, op.scales)
+def _native(op: ops.MXOperand | None) -> tuple:
+    """An operand as the native path takes it: (codes, scales, store)."""
+    return (None, None, None) if op is None else (op.codes, op.scales, op.store)
 
 
 class MXFP8FrozenLinear:
@@ -164,7 +165,7 @@ class MXFP8FrozenLinear:
     @staticmethod
     def apply(x, W_mx: QuantWeight, W_bf16, bias=None):
         x_row, _ = quantize_activation(x, colwise=False)
-        return host().frozen_linear(x, x_row.codes, x_row.scales, *_pair(W_mx.row), *_pair(W_mx.col), W_bf16, bias)
+        return host().frozen_linear(x, *_native(x_row), *_native(W_mx.row), *_native(W_mx.col), W_bf16, bias)
 
 
 def mxfp8_frozen_linear(x, W_mx, W_bf16, bias=None):
@@ -188,7 +189,7 @@ class MXFP8LoKrLinear:
     def apply(x, merged_W, bias=None):
         first = in_first_pass()
         x_row, x_col = quantize_activation(x, colwise=_wants_grad(merged_W) and not first)
-        return host().merged_linear(x, *_pair(x_row), *_pair(x_col), merged_W, bias, first)
+        return host().merged_linear(x, *_native(x_row), *_native(x_col), merged_W, bias, first)
 
 
 def mxfp8_lokr_linear(x, merged_W, bias=None):
@@ -219,7 +220,7 @@ class LoKrLinearFused:
     def apply(x, W, bias, w1, w2, alpha: float):
         first = in_first_pass()
         x_row, x_col = quantize_activation(x, colwise=_wants_grad(w1, w2) and not first)
-        return host().lokr_linear(x, *_pair(x_row), *_pair(x_col), W, bias, w1, w2, float(alpha), first)
+        return host().lokr_linear(x, *_native(x_row), *_native(x_col), W, bias, w1, w2, float(alpha), first)
 
 
 def lokr_linear_fused(x, W, bias, w1, w2, alpha: float = 1.0):

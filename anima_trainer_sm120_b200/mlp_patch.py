@@ -29,7 +29,7 @@ import torch.nn as nn
 
 from . import lokr_patch
 from ._lib import host
-from .fp8_quant import _pair, _wants_grad, in_first_pass, quantize_activation
+from .fp8_quant import _native, _wants_grad, in_first_pass, quantize_activation
 
 _PATCHED: dict[type, object] = {}
 
@@ -39,7 +39,7 @@ class LoKrMLPFused:
     def apply(x, W1, b1, w1a, w2a, alpha1: float, W2, b2, w1b, w2b, alpha2: float):
         first = in_first_pass()           # a checkpointed block's first pass keeps nothing for backward
         x_row, x_col = quantize_activation(x, colwise=_wants_grad(w1a, w2a, w1b, w2b) and not first)
-        return host().lokr_mlp(x, *_pair(x_row), *_pair(x_col), W1, b1, w1a, w2a, float(alpha1), W2, b2, w1b, w2b,
+        return host().lokr_mlp(x, *_native(x_row), *_native(x_col), W1, b1, w1a, w2a, float(alpha1), W2, b2, w1b, w2b,
                                float(alpha2), first)
 
 

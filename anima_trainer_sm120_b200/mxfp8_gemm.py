@@ -27,6 +27,7 @@ import torch
 
 from . import ops
 from ._lib import SCALES_PLAIN, SCALES_TILED, host
+from .fp8_quant import _native
 
 FP8_E4M3_MAX = 448.0
 
@@ -118,7 +119,7 @@ class MXFP8FrozenLinearB200:
         if not wT.is_contiguous():
             raise NotImplementedError("W_bwd must come from quantize_weight_for_dgrad()")
         w_bwd = _as_operand(wT, W_bwd_scales, W_bwd_tiled)
-        return host().frozen_linear(x, x_row.codes, x_row.scales, w.codes, w.scales, w_bwd.codes, w_bwd.scales, None, bias)
+        return host().frozen_linear(x, *_native(x_row), *_native(w), *_native(w_bwd), None, bias)
 
 
 MXFP8FrozenLinearTriton = MXFP8FrozenLinearB200  # name used by anima-trainer call sites

@@ -30,6 +30,7 @@ class MXOperand(NamedTuple):
     codes: torch.Tensor   # uint8 [rows, k]
     scales: torch.Tensor  # uint8, PLAIN [rows, k/32] or TILED (flat, see anima_b200.h)
     layout: int           # SCALES_PLAIN | SCALES_TILED
+    store: torch.Tensor | None = None   # the one allocation both lie in, where the native path made them
 
     @property
     def rows(self) -> int:
@@ -38,6 +39,12 @@ class MXOperand(NamedTuple):
     @property
     def k(self) -> int:
         return self.codes.shape[1]
+
+
+def operand(made: tuple, layout: int = SCALES_TILED) -> MXOperand | None:
+    """The operand of a (codes, scales, store) triple of the native path."""
+    codes, scales, store = made
+    return None if codes is None else MXOperand(codes, scales, layout, store)
 
 
 def scales_bytes(rows: int, k: int, layout: int) -> int:
@@ -86,7 +93,7 @@ def mx_quantize(
     transposed (``[cols, rows]``) — i.e. ``quantize_rowwise(x.t().contiguous())``.
     """
     row, col = _lib.host().mx_quantize(x, rowwise, colwise, layout)
-    return MXOperand(*row, layout) if rowwise else None, MXOperand(*col, layout) if colwise else None
+    return operand(row, layout), operand(col, layout)
 
 
 def mx_quantize_gelu(

@@ -406,13 +406,13 @@ def _tlinear(W_mx, bias, w1, w2_a, w2_b, mask, alpha: float):
 
 
 def _row_operand_unless_kept(x, *trainable):
-    """Row-wise operand of x for a pass that backward will not read, else (None, None): the node then quantises the
+    """Row-wise operand of x for a pass that backward will not read, else nothing: the node then quantises the
     grouped view of x in both forms itself, and its row codes serve the base GEMM too."""
-    from .fp8_quant import _pair, _wants_grad, in_first_pass, quantize_activation
+    from .fp8_quant import _native, _wants_grad, in_first_pass, quantize_activation
     first = in_first_pass()
     if _wants_grad(x, *trainable) and not first:
-        return (None, None), first
-    return _pair(quantize_activation(x, colwise=False)[0]), first
+        return (None, None, None), first
+    return _native(quantize_activation(x, colwise=False)[0]), first
 
 
 class _MXTLoKrLinear:
