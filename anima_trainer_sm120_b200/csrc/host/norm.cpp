@@ -246,18 +246,19 @@ struct BothNode : public HostNode {      // saves sub, gate, x_new, scale, stati
 
 // ------------------------------------------------------------------------------------------------ RMSNorm + RoPE
 struct RopeNode : public HostNode {      // saves x, rstd
-  Tensor w, cos, sin;
+  Kept weight;
+  Tensor cos, sin;
 
   variable_list apply(variable_list&& g) override {
     std::lock_guard<std::mutex> lock(mutex_);
-    const Tensor dout = bf16_contiguous(grad_of(g, 0)), x = get(0), rstd = get(1);
+    const Tensor dout = bf16_contiguous(grad_of(g, 0)), x = get(0), rstd = get(1), w = weight.get();
     const Launch l(x);
     Tensor dx = like(x, l.dev);
     const int64_t heads = x.size(-2), d = x.size(-1), tokens = x.numel() ? x.numel() / (heads * d) : 0;
     if (tokens)
-      check(anima_rmsnorm_rope_bwd(dout.data_ptr(), x.data_ptr(), w.data_ptr<float>(), static_cast<float*>(ptr(cos)),
-                                   static_cast<float*>(ptr(sin)), rstd.data_ptr<float>(), tokens, heads, d,
-                                   cos.defined() ? cos.size(0) : 1, dx.data_ptr(), l.stream));
+      check(anima_rmsnorm_rope_bwd_ex(dout.data_ptr(), x.data_ptr(), w.data_ptr(), w.scalar_type() == BF16,
+                                      static_cast<float*>(ptr(cos)), static_cast<float*>(ptr(sin)), rstd.data_ptr<float>(),
+                                      tokens, heads, d, cos.defined() ? cos.size(0) : 1, dx.data_ptr(), l.stream));
     return {dx};
   }
   std::string name() const override { return "FusedRMSNormRoPEBackward"; }
@@ -349,19 +350,20 @@ Tensor rmsnorm_rope(const Tensor& x, const Tensor& weight, const OptTensor& cos,
   {
     Below below;
     xc = x.is_contiguous() ? x : x.detach().contiguous();
-    w = weight.detach().to(F32).contiguous();
+    w = weight.scalar_type() == BF16 || weight.scalar_type() == F32 ? weight : weight.detach().to(F32);
+    if (!w.is_contiguous() || (reinterpret_cast<uintptr_t>(w.data_ptr()) & 15)) w = w.detach().clone(at::MemoryFormat::Contiguous);
     out = like(x, l.dev);
     rstd = empty({tokens * heads}, F32, l.dev);
     if (tokens)
-      check(anima_rmsnorm_rope_fwd(xc.data_ptr(), w.data_ptr<float>(), static_cast<float*>(ptr(cos)),
-                                   static_cast<float*>(ptr(sin)), static_cast<float>(eps), tokens, heads, d,
-                                   cos ? cos->size(0) : 1, out.data_ptr(), rstd.data_ptr<float>(), l.stream));
+      check(anima_rmsnorm_rope_fwd_ex(xc.data_ptr(), w.data_ptr(), w.scalar_type() == BF16, static_cast<float*>(ptr(cos)),
+                                      static_cast<float*>(ptr(sin)), static_cast<float>(eps), tokens, heads, d,
+                                      cos ? cos->size(0) : 1, out.data_ptr(), rstd.data_ptr<float>(), l.stream));
   }
   if (wants(x)) {
     auto node = make_node<RopeNode>(x);
     node->save(xc);
     node->save(rstd);
-    node->w = w;
+    node->weight = Kept(w);
     node->cos = cos.value_or(Tensor());
     node->sin = sin.value_or(Tensor());
     set_history(out, node);

@@ -419,6 +419,15 @@ int anima_rmsnorm_rope_bwd(const void* dout, const void* x, const float* weight,
                            int64_t tokens, int64_t heads, int64_t head_dim, int64_t seq_len,
                            void* dx, void* stream);
 
+/* The same with the norm weight in bf16 (weight_is_bf16 = 1) or fp32. */
+int anima_rmsnorm_rope_fwd_ex(const void* x, const void* weight, int weight_is_bf16, const float* cos_tab,
+                              const float* sin_tab, float eps, int64_t tokens, int64_t heads,
+                              int64_t head_dim, int64_t seq_len, void* out, float* rstd, void* stream);
+int anima_rmsnorm_rope_bwd_ex(const void* dout, const void* x, const void* weight, int weight_is_bf16,
+                              const float* cos_tab, const float* sin_tab, const float* rstd,
+                              int64_t tokens, int64_t heads, int64_t head_dim, int64_t seq_len, void* dx,
+                              void* stream);
+
 #ifdef __cplusplus
 }
 #endif
