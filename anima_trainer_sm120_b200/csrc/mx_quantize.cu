@@ -17,6 +17,7 @@
 #include <cstdlib>
 #include <mutex>
 
+#include "f32x2.cuh"
 #include "mx_quantize_tile.cuh"
 #include "mx_quantize_tma.cuh"
 
@@ -25,19 +26,29 @@ namespace {
 
 using namespace mxq;
 
+// This thread's chunk of a row-major bf16 matrix, as an offset in elements.
+struct ChunkAt {
+  int64_t off;
+};
+
 struct PlainLoader {
   using Raw = uint4;
+  using Cursor = ChunkAt;
   static constexpr bool kZeroSafe = true;
   static constexpr int kSmemBytes = 0;
   static constexpr bool kIdentity = true, kSecond = false;
   static constexpr int kTmaCtasPerSm = 3;
   __device__ __forceinline__ void prepare(void*) {}
-  __device__ __forceinline__ uint4 second(int64_t, int64_t) const { return make_uint4(0u, 0u, 0u, 0u); }
-  __device__ __forceinline__ uint4 transform(const uint4& raw, const uint4&, int64_t, int64_t) const { return raw; }
+  __device__ __forceinline__ Cursor begin(int64_t r, int64_t c) const { return {r * ld + c}; }
+  __device__ __forceinline__ void next(Cursor& at) const { at.off += 16 * ld; }
+  __device__ __forceinline__ uint4 second(const Cursor&) const { return make_uint4(0u, 0u, 0u, 0u); }
+  __device__ __forceinline__ uint4 transform(const uint4& raw, const uint4&) const { return raw; }
+  __device__ __forceinline__ bool emits() const { return false; }
+  __device__ __forceinline__ void emit(const uint4&, const Cursor&) const {}
   const __nv_bfloat16* x;
   int64_t ld;
-  __device__ __forceinline__ Raw fetch(int64_t r, int64_t c) const { return ldg_stream16(x + r * ld + c); }
-  __device__ __forceinline__ uint4 finish(const Raw& raw, int64_t, int64_t) const { return raw; }
+  __device__ __forceinline__ Raw fetch(const Cursor& at) const { return ldg_stream16(x + at.off); }
+  __device__ __forceinline__ uint4 finish(const Raw& raw, const Cursor&) const { return raw; }
 };
 
 // ---- GELU inside the quantiser ----------------------------------------------------------------
@@ -86,12 +97,18 @@ __device__ __forceinline__ uint32_t u16x2_min(uint32_t a, uint32_t b) {
   asm("min.u16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
   return r;
 }
-// Both table indices of the bf16 pair `w`, one per 16-bit half; false when either value is outside the table.
-__device__ __forceinline__ bool gelu_lut_index2(uint32_t w, uint32_t& idx2) {
+// Both table indices of the bf16 pair `w`, one per 16-bit half (clamped into the table); `out` collects a nonzero bit
+// for a value outside it, so that a chunk's four pairs share one test.
+__device__ __forceinline__ uint32_t gelu_lut_index2(uint32_t w, uint32_t& out) {
   const uint32_t a = w & 0x7fff7fffu;
   const uint32_t c = u16x2_min(u16x2_max(a, kGeluLo2), kGeluHi2);
-  idx2 = (c - kGeluLo2) | ((w >> 4) & 0x08000800u);   // no borrow between the halves: c >= range start in each
-  return c == a;
+  out |= a ^ c;
+  return (c - kGeluLo2) | ((w >> 4) & 0x08000800u);   // no borrow between the halves: c >= range start in each
+}
+__device__ __forceinline__ bool gelu_in_table(uint32_t w) {
+  uint32_t out = 0u;
+  gelu_lut_index2(w, out);
+  return out == 0u;
 }
 // The table is written once per CTA before a barrier; volatile keeps the loads behind that barrier.
 __device__ __forceinline__ uint32_t lds_u16(uint32_t addr) {
@@ -134,33 +151,48 @@ __device__ __noinline__ uint32_t gelu_pair_eager(uint32_t w) {   // a pair with 
   return lo | (hi << 16);
 }
 
+struct GeluAt {      // offsets of the chunk in the inputs (pitch ld) and in act_out (dense)
+  int64_t off, act;
+};
+
 struct GeluLoader {
   using Raw = uint4;
-  static constexpr bool kZeroSafe = false;  // finish may store the activation at (row, col)
+  using Cursor = GeluAt;
+  static constexpr bool kZeroSafe = false;  // finish may store the activation
   static constexpr int kSmemBytes = kGeluLutSize * 2;
   static constexpr bool kIdentity = false, kSecond = false;
   static constexpr int kTmaCtasPerSm = 3;     // 3 x (64 KB of stages + 7.5 KB table)
-  __device__ __forceinline__ uint4 second(int64_t, int64_t) const { return make_uint4(0u, 0u, 0u, 0u); }
-  __device__ __forceinline__ uint4 transform(const uint4& raw, const uint4&, int64_t r, int64_t c) const {
-    return finish(raw, r, c);
-  }
   const __nv_bfloat16* h;
   int64_t ld;
   __nv_bfloat16* act_out;                    // optional: the bf16 activation itself, [rows, cols] contiguous
   int64_t cols;
   uint32_t lut2;                             // shared-memory address of the table in both halves, set by prepare()
   __device__ __forceinline__ void prepare(void* smem) { lut2 = copy_lut(smem, g_gelu_lut); }
-  __device__ __forceinline__ Raw fetch(int64_t r, int64_t c) const { return ldg_stream16(h + r * ld + c); }
-  __device__ __forceinline__ uint32_t pair(uint32_t w) const {
-    uint32_t idx2;
-    if (!gelu_lut_index2(w, idx2)) return gelu_pair_eager(w);
-    const uint32_t addr2 = idx2 * 2u + lut2;
-    return lds_u16(addr2 & 0xffffu) | (lds_u16(addr2 >> 16) << 16);
+  __device__ __forceinline__ Cursor begin(int64_t r, int64_t c) const { return {r * ld + c, r * cols + c}; }
+  __device__ __forceinline__ void next(Cursor& at) const { at.off += 16 * ld; at.act += 16 * cols; }
+  __device__ __forceinline__ Raw fetch(const Cursor& at) const { return ldg_stream16(h + at.off); }
+  __device__ __forceinline__ uint4 second(const Cursor&) const { return make_uint4(0u, 0u, 0u, 0u); }
+  __device__ __forceinline__ bool emits() const { return act_out != nullptr; }
+  __device__ __forceinline__ void emit(const uint4& v, const Cursor& at) const { stg_stream16(act_out + at.act, v); }
+  __device__ __forceinline__ uint4 transform(const uint4& raw, const uint4&) const {
+    const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
+    uint32_t o[4], outside = 0u;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const uint32_t addr2 = gelu_lut_index2(w[k], outside) * 2u + lut2;
+      o[k] = lds_u16(addr2 & 0xffffu) | (lds_u16(addr2 >> 16) << 16);
+    }
+    if (outside) {
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        if (!gelu_in_table(w[k])) o[k] = gelu_pair_eager(w[k]);
+    }
+    return make_uint4(o[0], o[1], o[2], o[3]);
   }
-  __device__ __forceinline__ uint4 finish(const Raw& raw, int64_t r, int64_t c) const {
-    const uint4 out = make_uint4(pair(raw.x), pair(raw.y), pair(raw.z), pair(raw.w));
-    if (act_out) stg_stream16(act_out + r * cols + c, out);
-    return out;
+  __device__ __forceinline__ uint4 finish(const Raw& raw, const Cursor& at) const {
+    const uint4 v = transform(raw, raw);
+    if (emits()) emit(v, at);
+    return v;
   }
 };
 
@@ -172,11 +204,11 @@ __device__ __noinline__ float2 gelu_grad_factor_pair_eager(uint32_t w) {
 // d(pre-activation) = grad_act * gelu'(h), rounded to bf16.
 struct GeluBwdLoader {
   using Raw = uint4;                           // the pre-activation; the incoming gradient is read in finish
+  using Cursor = GeluAt;
   static constexpr bool kZeroSafe = false;     // (keeping both tiles in registers up front spills)
   static constexpr int kSmemBytes = kGeluLutSize * 4;
   static constexpr bool kIdentity = false, kSecond = true;
   static constexpr int kTmaCtasPerSm = 2;     // 2 x (64 KB of stages + 15 KB table)
-  __device__ __forceinline__ uint4 second(int64_t r, int64_t c) const { return ldg_stream16(grad_act + r * ld + c); }
   const __nv_bfloat16* h;
   const __nv_bfloat16* grad_act;
   int64_t ld;
@@ -184,29 +216,34 @@ struct GeluBwdLoader {
   int64_t cols;
   uint32_t lut2;
   __device__ __forceinline__ void prepare(void* smem) { lut2 = copy_lut(smem, g_gelu_grad_lut); }
-  __device__ __forceinline__ Raw fetch(int64_t r, int64_t c) const { return ldg_stream16(h + r * ld + c); }
-  __device__ __forceinline__ float2 factors(uint32_t w) const {
-    uint32_t idx2;
-    if (!gelu_lut_index2(w, idx2)) return gelu_grad_factor_pair_eager(w);
-    const uint32_t addr2 = idx2 * 4u + lut2;
-    return make_float2(lds_f32(addr2 & 0xffffu), lds_f32(addr2 >> 16));
-  }
-  __device__ __forceinline__ uint4 finish(const Raw& raw, int64_t r, int64_t c) const {
-    return transform(raw, ldg_stream16(grad_act + r * ld + c), r, c);
-  }
-  __device__ __forceinline__ uint4 transform(const uint4& raw, const uint4& grad, int64_t r, int64_t c) const {
-    float g[8], o[8];
-    unpack8(grad, g);
-    const uint32_t* w = reinterpret_cast<const uint32_t*>(&raw);
+  __device__ __forceinline__ Cursor begin(int64_t r, int64_t c) const { return {r * ld + c, r * cols + c}; }
+  __device__ __forceinline__ void next(Cursor& at) const { at.off += 16 * ld; at.act += 16 * cols; }
+  __device__ __forceinline__ Raw fetch(const Cursor& at) const { return ldg_stream16(h + at.off); }
+  __device__ __forceinline__ uint4 second(const Cursor& at) const { return ldg_stream16(grad_act + at.off); }
+  __device__ __forceinline__ bool emits() const { return act_out != nullptr; }
+  __device__ __forceinline__ void emit(const uint4& v, const Cursor& at) const { stg_stream16(act_out + at.act, v); }
+  __device__ __forceinline__ uint4 transform(const uint4& raw, const uint4& grad) const {
+    const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w}, g[4] = {grad.x, grad.y, grad.z, grad.w};
+    uint32_t o[4], outside = 0u;
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-      const float2 f = factors(w[k]);
-      o[2 * k] = g[2 * k] * f.x;
-      o[2 * k + 1] = g[2 * k + 1] * f.y;
+      const uint32_t addr2 = gelu_lut_index2(w[k], outside) * 4u + lut2;
+      o[k] = bf16_of_f2(f2_mul(f2_of_bf16(g[k]), f2_make(lds_f32(addr2 & 0xffffu), lds_f32(addr2 >> 16))));
     }
-    const uint4 out = pack8(o);
-    if (act_out) stg_stream16(act_out + r * cols + c, out);
-    return out;
+    if (outside) {
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        if (!gelu_in_table(w[k])) {
+          const float2 f = gelu_grad_factor_pair_eager(w[k]);
+          o[k] = bf16_of_f2(f2_mul(f2_of_bf16(g[k]), f2_make(f.x, f.y)));
+        }
+    }
+    return make_uint4(o[0], o[1], o[2], o[3]);
+  }
+  __device__ __forceinline__ uint4 finish(const Raw& raw, const Cursor& at) const {
+    const uint4 v = transform(raw, second(at));
+    if (emits()) emit(v, at);
+    return v;
   }
 };
 
@@ -422,6 +459,7 @@ template <class Loader>
 int try_quantize_tma(const Loader& load, const void* x, int64_t rows, int64_t cols, int64_t ld, uint8_t* codes_row,
                      uint8_t* scales_row, uint8_t* codes_colT, uint8_t* scales_col, int scale_layout, void* stream) {
   if (rows >= (1ll << 31) || cols >= (1ll << 31)) return 1;
+  if (ceil_div(rows, static_cast<int64_t>(kTile)) * ceil_div(cols, static_cast<int64_t>(kTile)) >= (1ll << 30)) return 1;
   CUtensorMap map;
   if (!make_x_map(&map, x, rows, cols, ld)) return 1;
   const bool row = codes_row != nullptr, col = codes_colT != nullptr;

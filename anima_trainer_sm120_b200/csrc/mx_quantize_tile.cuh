@@ -91,11 +91,114 @@ __device__ __forceinline__ int tiled_offset(int r, int j) {
   return (r & 31) * 16 + (r >> 5) * 4 + j;
 }
 
-// Loader interface (device side), for one chunk of 8 values at (row, col .. col+7), both in range:
-//   using Raw = ...;                                            what the chunk needs from HBM
-//   Raw   fetch(int64_t row, int64_t col) const;                issues the long-latency loads only
-//   uint4 finish(const Raw&, int64_t row, int64_t col) const;   the 8 bf16 values
-//   static constexpr bool kZeroSafe;                            finish(Raw{}) == 0 and reads no memory
+// ---- what both quantiser kernels do with a 128 x 128 tile ---------------------------------------------------------
+// Thread t works on the 8 chunks (8 values, 16 bytes) at tile column 8 * (t & 15), tile rows (t >> 4) + 16 i in the row
+// pass, and on column pair t & 63 of the 32-row group t >> 6 in the column pass. Both passes stay on packed bf16 words
+// (amax, exponent and scaling), addresses advance by constant strides; see mx_row_block for the arithmetic.
+struct RowPass {
+  uint8_t* dst;        // code address of chunk 0
+  int64_t step;        // 16 rows
+  int rows_left;       // rows of the tile inside the matrix, minus this thread's first row; 0 when its columns are outside
+  int sc0;             // scale staging index of chunk 0
+  bool tiled;
+  __device__ __forceinline__ RowPass(const QuantParams& p, int64_t tile_r, int64_t col, int t)
+      : dst(p.codes_row + (tile_r + (t >> 4)) * p.cols + col), step(16 * p.cols), tiled(p.tiled) {
+    const int64_t left = p.rows - tile_r;
+    rows_left = col < p.cols ? static_cast<int>(left < kTile ? left : kTile) - (t >> 4) : 0;
+    sc0 = (t >> 4) * (tiled ? 16 : 4) + ((t & 15) >> 2);
+  }
+  __device__ __forceinline__ bool in(int i) const { return 16 * i < rows_left; }
+  // all lanes of the warp call it; v is zero outside the matrix
+  __device__ __forceinline__ void put(int i, const uint4& v, uint8_t* sc, int t) {
+    uint2 codes;
+    const uint32_t sb = mx_row_block(v, codes);
+    if (in(i)) {
+      *reinterpret_cast<uint2*>(dst) = codes;
+      if ((t & 3) == 0) sc[sc0 + (tiled ? 256 * (i & 1) + 4 * (i >> 1) : 64 * i)] = static_cast<uint8_t>(sb);
+    }
+    dst += step;
+  }
+};
+
+// Column pass: codes of the column pair in w0 / w1 (32 rows each), scale bytes staged. `tile32`: the tile as words.
+__device__ __forceinline__ void col_codes(const QuantParams& p, const uint32_t* tile32, int64_t tile_r, int64_t tile_c, int t,
+                                          uint8_t* sc, uint32_t (&w0)[8], uint32_t (&w1)[8]) {
+  const int cp = t & 63, g = t >> 6;
+  uint32_t cw[32], am = 0u;   // the running maximum starts at 0 and ignores NaN
+#pragma unroll
+  for (int i = 0; i < 32; ++i) {
+    cw[i] = tile32[(32 * g + i) * 64 + cp];
+    am = bf16x2_max(am, cw[i] & 0x7fff7fffu);
+  }
+  const uint32_t sb0 = mx_scale_byte(am & 0xffffu), sb1 = mx_scale_byte(am >> 16);
+  const uint32_t inv2 = (mx_inv_bf16x2(sb0) & 0xffffu) | (mx_inv_bf16x2(sb1) & 0xffff0000u);
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    float a[4], b[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const uint32_t v = bf16x2_mul(cw[4 * q + k], inv2);
+      a[k] = __uint_as_float(v << 16);
+      b[k] = __uint_as_float(v & 0xffff0000u);
+    }
+    w0[q] = e4m3x2(a[0], a[1]) | (e4m3x2(a[2], a[3]) << 16);
+    w1[q] = e4m3x2(b[0], b[1]) | (e4m3x2(b[2], b[3]) << 16);
+  }
+  if (tile_c + 2 * cp < p.cols && tile_r + 32 * g < p.rows) {
+    sc[p.tiled ? tiled_offset(2 * cp, g) : 8 * cp + g] = static_cast<uint8_t>(sb0);
+    if (tile_c + 2 * cp + 1 < p.cols) sc[p.tiled ? tiled_offset(2 * cp + 1, g) : 8 * cp + 4 + g] = static_cast<uint8_t>(sb1);
+  }
+}
+// Transposed codes go through shared memory (the input tile is dead once every thread holds its column pair) so that
+// the global writes are full 128-byte lines: column c of the tile owns 128 bytes = 8 pieces of 16; piece q is stored at
+// q ^ ((c >> 1) & 7) to keep both the per-thread writes and the cooperative reads free of bank conflicts.
+__device__ __forceinline__ void stage_cols(uint4* tile, int t, const uint32_t (&w0)[8], const uint32_t (&w1)[8]) {
+  const int cp = t & 63, g = t >> 6, sw = cp & 7;
+  uint4* c = tile + cp * 16;
+  c[(2 * g) ^ sw] = make_uint4(w0[0], w0[1], w0[2], w0[3]);
+  c[(2 * g + 1) ^ sw] = make_uint4(w0[4], w0[5], w0[6], w0[7]);
+  c[8 + ((2 * g) ^ sw)] = make_uint4(w1[0], w1[1], w1[2], w1[3]);
+  c[8 + ((2 * g + 1) ^ sw)] = make_uint4(w1[4], w1[5], w1[6], w1[7]);
+}
+__device__ __forceinline__ void store_cols(const QuantParams& p, const uint4* tile, int64_t tile_r, int64_t tile_c, int t) {
+  const int c = t >> 3, q = t & 7;      // column c + 32 h, piece q; rows % 32 == 0: a piece is all in or all out
+  uint8_t* dst = p.codes_colT + (tile_c + c) * p.rows + tile_r + q * 16;
+  const uint4* src = tile + c * 8 + (q ^ ((c >> 1) & 7));
+  const int64_t cols_left = p.cols - tile_c - c;
+  if (tile_r + q * 16 < p.rows) {
+#pragma unroll
+    for (int h = 0; h < 4; ++h)
+      if (32 * h < cols_left) stg_stream16(dst + 32 * h * p.rows, src[256 * h]);
+  }
+}
+// Scale bytes of the tile, staged in shared memory: 128 "rows" x 4 blocks of a matrix with `rows` rows and `kb` blocks.
+template <bool CLEAR>
+__device__ __forceinline__ void store_scales(uint8_t* out, uint8_t* sc, bool tiled, int64_t rows, int64_t kb, int64_t tile_row,
+                                             int64_t tile_blk, int t) {
+  if (tiled) {
+    if (t < 128) {
+      uint32_t* src = reinterpret_cast<uint32_t*>(sc) + t;
+      reinterpret_cast<uint32_t*>(out + (tile_row * ceil_div(kb, static_cast<int64_t>(4)) + tile_blk) * 512)[t] = *src;
+      if (CLEAR) *src = 0u;     // each entry is zeroed again by the thread that stored it
+    }
+  } else {
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int idx = t + h * kThreads;
+      const int64_t r = tile_row * kTile + (idx >> 2), k = tile_blk * 4 + (idx & 3);
+      if (r < rows && k < kb) out[r * kb + k] = sc[idx];
+      if (CLEAR) sc[idx] = 0;
+    }
+  }
+}
+
+// Loader interface (device side):
+//   using Raw = ...;                            what one chunk needs from HBM
+//   struct Cursor; Cursor begin(r, c) const;    this thread's chunk at row r, columns c .. c + 7
+//   void next(Cursor&) const;                   16 rows on
+//   Raw   fetch(const Cursor&) const;           issues the long-latency loads only
+//   uint4 finish(const Raw&, const Cursor&) const;   the 8 bf16 values
+//   static constexpr bool kZeroSafe;            finish(Raw{}, ...) == 0 and reads no memory
 //   static constexpr int kSmemBytes; void prepare(void* smem);  per-CTA shared-memory state (a lookup table)
 // All eight fetches of a thread are issued before the first finish, so a loader that computes
 // (merge, GELU) does not serialise its chunks on memory latency.
@@ -110,154 +213,50 @@ __global__ void __launch_bounds__(kThreads, COL ? 3 : 4) mx_quantize_kernel(cons
   const int t = threadIdx.x;
   const int64_t tile_r = static_cast<int64_t>(blockIdx.y) * kTile;
   const int64_t tile_c = static_cast<int64_t>(blockIdx.x) * kTile;
-  const int c16 = t & 15;  // 16-byte chunk (8 elements) within the tile row
-  const int r0 = t >> 4;   // 0..15
-  const int64_t col = tile_c + c16 * 8;
-  const bool col_ok = col < p.cols;  // cols % 32 == 0 or % 8 == 0: a chunk is all in or all out
+  const int64_t col = tile_c + (t & 15) * 8;  // cols % 32 == 0 or % 8 == 0: a chunk is all in or all out
+  RowPass row(p, tile_r, col, t);
 
-  if (ROW) {
-    // Padding entries of a partial tile must be 0 in the tiled layout.
-    reinterpret_cast<uint16_t*>(sc_row)[t] = 0;
-  }
+  // Padding entries of a partial tile must be 0 in the tiled layout.
+  if (ROW) reinterpret_cast<uint16_t*>(sc_row)[t] = 0;
   if (COL) reinterpret_cast<uint16_t*>(sc_col)[t] = 0;
 
   typename Loader::Raw fetched[8];
+  const typename Loader::Cursor first = load.begin(tile_r + (t >> 4), row.rows_left > 0 ? col : 0);
+  {
+    typename Loader::Cursor at = first;
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const int64_t r = tile_r + r0 + 16 * i;
-    fetched[i] = typename Loader::Raw{};
-    if (col_ok && r < p.rows) fetched[i] = load.fetch(r, col);
+    for (int i = 0; i < 8; ++i) {
+      fetched[i] = typename Loader::Raw{};
+      if (row.in(i)) fetched[i] = load.fetch(at);
+      load.next(at);
+    }
   }
   load.prepare(loader_smem);   // after the tile's loads are in flight; visible to all threads after the barrier
   __syncthreads();             // also: zero fill of sc_* visible before the byte stores
 
+  typename Loader::Cursor at = first;
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
-    const int r_in = r0 + 16 * i;
     // kZeroSafe loaders map an all-zero Raw to zeros without touching memory, so out-of-range chunks need no branch
     uint4 v = make_uint4(0u, 0u, 0u, 0u);
-    if (Loader::kZeroSafe || (col_ok && tile_r + r_in < p.rows)) v = load.finish(fetched[i], tile_r + r_in, col);
-    if (COL) tile[r_in * 16 + c16] = v;
-    if (ROW) {
-      float f[8];
-      unpack8(v, f);
-      float amax = 0.f;
-#pragma unroll
-      for (int k = 0; k < 8; ++k) amax = fmaxf(amax, fabsf(f[k]));
-      amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
-      amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
-      amax = fmaxf(amax, kAmaxFloor);
-      const int e = mx_exponent(amax);
-      const float inv = mx_inv_scale(e);
-      uint2 codes;
-      codes.x = e4m3x2(f[0] * inv, f[1] * inv) | (e4m3x2(f[2] * inv, f[3] * inv) << 16);
-      codes.y = e4m3x2(f[4] * inv, f[5] * inv) | (e4m3x2(f[6] * inv, f[7] * inv) << 16);
-      const int64_t r = tile_r + r_in;
-      if (col_ok && r < p.rows) {
-        *reinterpret_cast<uint2*>(p.codes_row + r * p.cols + col) = codes;
-        if ((c16 & 3) == 0) {
-          const int j = c16 >> 2;
-          sc_row[p.tiled ? tiled_offset(r_in, j) : r_in * 4 + j] = static_cast<uint8_t>(e + 127);
-        }
-      }
-    }
+    if (Loader::kZeroSafe || row.in(i)) v = load.finish(fetched[i], at);
+    load.next(at);
+    if (COL) tile[((t >> 4) + 16 * i) * 16 + (t & 15)] = v;
+    if (ROW) row.put(i, v, sc_row, t);
   }
-
   if (COL) {
     __syncthreads();
-    const int cp = t & 63;  // column pair
-    const int g = t >> 6;   // 32-row group within the tile
-    const uint32_t* tile32 = reinterpret_cast<const uint32_t*>(tile);
-    // one pass over the column pair: 32 packed bf16x2 words stay in registers for amax and conversion
-    uint32_t cw[32];
-    // amax of both columns at once on the packed bf16 pairs (|x| by clearing the sign bits, then a packed
-    // max that ignores NaN like fmaxf); the scaling by 2^-e is a packed bf16 multiply, exact for a power of two
-    uint32_t am = 0u;
-#pragma unroll
-    for (int i = 0; i < 32; ++i) {
-      cw[i] = tile32[(32 * g + i) * 64 + cp];
-      am = bf16x2_max(am, cw[i] & 0x7fff7fffu);
-    }
-    const int e0 = mx_exponent(fmaxf(__uint_as_float(am << 16), kAmaxFloor));
-    const int e1 = mx_exponent(fmaxf(__uint_as_float(am & 0xffff0000u), kAmaxFloor));
-    const uint32_t inv2 = (__float_as_uint(mx_inv_scale(e0)) >> 16) | (__float_as_uint(mx_inv_scale(e1)) & 0xffff0000u);
     uint32_t w0[8], w1[8];
-#pragma unroll
-    for (int q = 0; q < 8; ++q) {
-      float a[4], b[4];
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const uint32_t sc = bf16x2_mul(cw[4 * q + k], inv2);
-        a[k] = __uint_as_float(sc << 16);
-        b[k] = __uint_as_float(sc & 0xffff0000u);
-      }
-      w0[q] = e4m3x2(a[0], a[1]) | (e4m3x2(a[2], a[3]) << 16);
-      w1[q] = e4m3x2(b[0], b[1]) | (e4m3x2(b[2], b[3]) << 16);
-    }
-    // Transposed codes go through shared memory (the input tile is dead once every thread holds its
-    // column pair in registers) so that the global writes are full 128-byte lines: column c of the tile
-    // owns 128 bytes = 8 pieces of 16; piece q is stored at q ^ ((c >> 1) & 7) to keep both the
-    // per-thread writes and the cooperative reads free of bank conflicts.
+    col_codes(p, reinterpret_cast<const uint32_t*>(tile), tile_r, tile_c, t, sc_col, w0, w1);
     __syncthreads();
-    {
-      const int c0 = 2 * cp, sw = cp & 7;
-      tile[c0 * 8 + ((2 * g) ^ sw)] = make_uint4(w0[0], w0[1], w0[2], w0[3]);
-      tile[c0 * 8 + ((2 * g + 1) ^ sw)] = make_uint4(w0[4], w0[5], w0[6], w0[7]);
-      tile[(c0 + 1) * 8 + ((2 * g) ^ sw)] = make_uint4(w1[0], w1[1], w1[2], w1[3]);
-      tile[(c0 + 1) * 8 + ((2 * g + 1) ^ sw)] = make_uint4(w1[4], w1[5], w1[6], w1[7]);
-      if (tile_c + c0 < p.cols && tile_r + 32 * g < p.rows) {
-        sc_col[p.tiled ? tiled_offset(c0, g) : c0 * 4 + g] = static_cast<uint8_t>(e0 + 127);
-        if (tile_c + c0 + 1 < p.cols)
-          sc_col[p.tiled ? tiled_offset(c0 + 1, g) : (c0 + 1) * 4 + g] = static_cast<uint8_t>(e1 + 127);
-      }
-    }
+    stage_cols(tile, t, w0, w1);
     __syncthreads();
-#pragma unroll
-    for (int h = 0; h < 4; ++h) {
-      const int idx = t + h * kThreads;  // 1024 pieces: column idx / 8, piece idx % 8
-      const int c = idx >> 3, q = idx & 7;
-      const int64_t col_g = tile_c + c, row_g = tile_r + q * 16;  // rows % 32 == 0: a piece is all in or all out
-      if (col_g < p.cols && row_g < p.rows)
-        stg_stream16(p.codes_colT + col_g * p.rows + row_g, tile[c * 8 + (q ^ ((c >> 1) & 7))]);
-    }
+    store_cols(p, tile, tile_r, tile_c, t);
+  } else {
+    __syncthreads();
   }
-
-  __syncthreads();
-  // Scale bytes of the tile: 128 "rows" x 4 k-blocks, staged in shared memory.
-  if (ROW) {
-    const int64_t kb = p.cols / 32;
-    if (p.tiled) {
-      if (t < 128) {
-        const int64_t chunk = blockIdx.y * ceil_div(kb, 4) + blockIdx.x;
-        reinterpret_cast<uint32_t*>(p.scales_row + chunk * 512)[t] =
-            reinterpret_cast<const uint32_t*>(sc_row)[t];
-      }
-    } else {
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int idx = t + h * kThreads;
-        const int64_t r = tile_r + (idx >> 2), k = tile_c / 32 + (idx & 3);
-        if (r < p.rows && k < kb) p.scales_row[r * kb + k] = sc_row[idx];
-      }
-    }
-  }
-  if (COL) {
-    const int64_t kb = p.rows / 32;
-    if (p.tiled) {
-      if (t < 128) {
-        const int64_t chunk = blockIdx.x * ceil_div(kb, 4) + blockIdx.y;
-        reinterpret_cast<uint32_t*>(p.scales_col + chunk * 512)[t] =
-            reinterpret_cast<const uint32_t*>(sc_col)[t];
-      }
-    } else {
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int idx = t + h * kThreads;
-        const int64_t c = tile_c + (idx >> 2), k = tile_r / 32 + (idx & 3);
-        if (c < p.cols && k < kb) p.scales_col[c * kb + k] = sc_col[idx];
-      }
-    }
-  }
+  if (ROW) store_scales<false>(p.scales_row, sc_row, p.tiled, p.rows, p.cols / 32, blockIdx.y, blockIdx.x, t);
+  if (COL) store_scales<false>(p.scales_col, sc_col, p.tiled, p.cols, p.rows / 32, blockIdx.x, blockIdx.y, t);
 }
 
 }  // namespace mxq

@@ -19,8 +19,9 @@
 //   static constexpr bool kSecond;          there is a second input
 //   static constexpr int kTmaCtasPerSm;     resident CTAs the kernel is compiled for (shared memory: two 32 KB
 //                                           stages plus the table)
-//   uint4 second(int64_t row, int64_t col) const;                         the second input's chunk (a load)
-//   uint4 transform(const uint4& raw, const uint4& second, int64_t row, int64_t col) const;
+//   uint4 second(const Cursor&) const;                       the second input's chunk (a load)
+//   uint4 transform(const uint4& raw, const uint4& second) const;
+//   bool emits() const; void emit(const uint4&, const Cursor&) const;    the transformed values are also wanted in HBM
 #pragma once
 
 #include "mx_quantize_tile.cuh"
@@ -45,8 +46,6 @@ mx_quantize_tma_kernel(const __grid_constant__ CUtensorMap map_x, const QuantPar
   __shared__ __align__(16) uint8_t sc_col[COL ? 512 : 16];
 
   const int t = threadIdx.x;
-  const int c16 = t & 15;  // 16-byte chunk (8 elements) within the tile row
-  const int r0 = t >> 4;   // 0..15
   // dynamic shared memory: the loader's table first (its lookups pack two addresses into 16-bit halves, so it
   // must sit low), then the two stages
   constexpr uint32_t kTableBytes = (Loader::kSmemBytes + 127u) & ~127u;
@@ -54,14 +53,20 @@ mx_quantize_tma_kernel(const __grid_constant__ CUtensorMap map_x, const QuantPar
   uint8_t* const table_ptr = smem_raw + (table0 - smem_u32(smem_raw));
   const uint32_t stage0 = table0 + kTableBytes;
   uint8_t* const stage_ptr0 = table_ptr + kTableBytes;
-  const int64_t tiles_x = ceil_div(p.cols, static_cast<int64_t>(kTile));
-  const int64_t n_tiles = tiles_x * ceil_div(p.rows, static_cast<int64_t>(kTile));
-  const int64_t first = blockIdx.x, step = gridDim.x;
+  // tile counts fit 32 bits (checked by the host): the index divisions stay cheap
+  const uint32_t tiles_x = static_cast<uint32_t>(ceil_div(p.cols, static_cast<int64_t>(kTile)));
+  const uint32_t n_tiles = tiles_x * static_cast<uint32_t>(ceil_div(p.rows, static_cast<int64_t>(kTile)));
+  const uint32_t first = blockIdx.x, step = gridDim.x;
+  auto coords = [&](uint32_t id, uint32_t& ty, uint32_t& tx) {
+    ty = id / tiles_x;
+    tx = id - ty * tiles_x;
+  };
 
   if (ROW) reinterpret_cast<uint16_t*>(sc_row)[t] = 0;  // padding entries of a partial tile must be 0
   if (COL) reinterpret_cast<uint16_t*>(sc_col)[t] = 0;
-  auto issue = [&](int64_t tile_id, int s) {  // one thread: arm the stage's barrier and start the copy
-    const int64_t ty = tile_id / tiles_x, tx = tile_id - ty * tiles_x;
+  auto issue = [&](uint32_t tile_id, int s) {  // one thread: arm the stage's barrier and start the copy
+    uint32_t ty, tx;
+    coords(tile_id, ty, tx);
     mbar_expect_tx(smem_u32(&full_bar[s]), kTmaStageBytes);
     tma_load_2d(stage0 + s * kTmaStageBytes, &map_x, smem_u32(&full_bar[s]), static_cast<int>(tx * kTile),
                 static_cast<int>(ty * kTile));
@@ -76,67 +81,46 @@ mx_quantize_tma_kernel(const __grid_constant__ CUtensorMap map_x, const QuantPar
     if (first + step < n_tiles) issue(first + step, 1);
   }
   load.prepare(table_ptr);  // the table, once per CTA, behind the first copies
-  // chunk i of this thread: tile row r0 + 16 i, columns 8 c16 .. + 7
-  auto chunk_in_range = [&](int64_t tile_id, int i) {
-    const int64_t ty = tile_id / tiles_x, tx = tile_id - ty * tiles_x;
-    return tx * kTile + c16 * 8 < p.cols && ty * kTile + r0 + 16 * i < p.rows;
-  };
   uint4 second[Loader::kSecond ? 8 : 1];
-  auto fetch_second = [&](int64_t tile_id) {
-    const int64_t ty = tile_id / tiles_x, tx = tile_id - ty * tiles_x;
+  auto fetch_second = [&](uint32_t tile_id) {
+    uint32_t ty, tx;
+    coords(tile_id, ty, tx);
+    const int64_t tile_r = static_cast<int64_t>(ty) * kTile, col = static_cast<int64_t>(tx) * kTile + (t & 15) * 8;
+    const RowPass row(p, tile_r, col, t);
+    typename Loader::Cursor at = load.begin(tile_r + (t >> 4), row.rows_left > 0 ? col : 0);
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
       second[i] = make_uint4(0u, 0u, 0u, 0u);
-      if (chunk_in_range(tile_id, i)) second[i] = load.second(ty * kTile + r0 + 16 * i, tx * kTile + c16 * 8);
+      if (row.in(i)) second[i] = load.second(at);
+      load.next(at);
     }
   };
   if (Loader::kSecond && first < n_tiles) fetch_second(first);
   __syncthreads();
 
   int it = 0;
-  for (int64_t tile_id = first; tile_id < n_tiles; tile_id += step, ++it) {
+  for (uint32_t tile_id = first; tile_id < n_tiles; tile_id += step, ++it) {
     const int s = it & 1;
-    const int64_t tile_y = tile_id / tiles_x, tile_x = tile_id - tile_y * tiles_x;
-    const int64_t tile_r = tile_y * kTile, tile_c = tile_x * kTile;
-    const int64_t col = tile_c + c16 * 8;
-    const bool col_ok = col < p.cols;
-    const uint4* tile = reinterpret_cast<const uint4*>(stage_ptr0 + s * kTmaStageBytes);
-    uint4* tile_w = reinterpret_cast<uint4*>(stage_ptr0 + s * kTmaStageBytes);
+    uint32_t tile_y, tile_x;
+    coords(tile_id, tile_y, tile_x);
+    const int64_t tile_r = static_cast<int64_t>(tile_y) * kTile, tile_c = static_cast<int64_t>(tile_x) * kTile;
+    const int64_t col = tile_c + (t & 15) * 8;
+    uint4* tile = reinterpret_cast<uint4*>(stage_ptr0 + s * kTmaStageBytes);
+    RowPass row(p, tile_r, col, t);
 
     if (!mbar_wait(smem_u32(&full_bar[s]), (it >> 1) & 1u, &abort_flag)) break;
 
     if (ROW || !Loader::kIdentity) {
+      uint4* chunk = tile + (t >> 4) * 16 + (t & 15);
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
-        const int r_in = r0 + 16 * i;
-        const int64_t r = tile_r + r_in;
-        uint4 v = tile[r_in * 16 + c16];
+        uint4 v = chunk[256 * i];
         if (!Loader::kIdentity) {
-          v = (col_ok && r < p.rows) ? load.transform(v, second[Loader::kSecond ? i : 0], r, col)
-                                     : make_uint4(0u, 0u, 0u, 0u);
-          if (COL) tile_w[r_in * 16 + c16] = v;
+          v = row.in(i) ? load.transform(v, second[Loader::kSecond ? i : 0]) : make_uint4(0u, 0u, 0u, 0u);
+          if (COL) chunk[256 * i] = v;
+          if (load.emits() && row.in(i)) load.emit(v, load.begin(tile_r + (t >> 4) + 16 * i, col));
         }
-        if (!ROW) continue;
-        float f[8];
-        unpack8(v, f);
-        float amax = 0.f;
-#pragma unroll
-        for (int k = 0; k < 8; ++k) amax = fmaxf(amax, fabsf(f[k]));
-        amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
-        amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
-        amax = fmaxf(amax, kAmaxFloor);
-        const int e = mx_exponent(amax);
-        const float inv = mx_inv_scale(e);
-        uint2 codes;
-        codes.x = e4m3x2(f[0] * inv, f[1] * inv) | (e4m3x2(f[2] * inv, f[3] * inv) << 16);
-        codes.y = e4m3x2(f[4] * inv, f[5] * inv) | (e4m3x2(f[6] * inv, f[7] * inv) << 16);
-        if (col_ok && r < p.rows) {
-          *reinterpret_cast<uint2*>(p.codes_row + r * p.cols + col) = codes;
-          if ((c16 & 3) == 0) {
-            const int j = c16 >> 2;
-            sc_row[p.tiled ? tiled_offset(r_in, j) : r_in * 4 + j] = static_cast<uint8_t>(e + 127);
-          }
-        }
+        if (ROW) row.put(i, v, sc_row, t);
       }
     }
 
@@ -144,103 +128,21 @@ mx_quantize_tma_kernel(const __grid_constant__ CUtensorMap map_x, const QuantPar
 
     if (COL) {
       if (!Loader::kIdentity) __syncthreads();  // the transformed tile is complete
-      const int cp = t & 63;  // column pair
-      const int g = t >> 6;   // 32-row group within the tile
-      const uint32_t* tile32 = reinterpret_cast<const uint32_t*>(tile);
-      uint32_t cw[32];
-      // amax of both columns at once on the packed bf16 pairs (|x| by clearing the sign bits, then a packed
-      // max that ignores NaN like fmaxf); the scaling by 2^-e is a packed bf16 multiply, exact for a power of two
-      uint32_t am = 0u;
-#pragma unroll
-      for (int i = 0; i < 32; ++i) {
-        cw[i] = tile32[(32 * g + i) * 64 + cp];
-        am = bf16x2_max(am, cw[i] & 0x7fff7fffu);
-      }
-      const int e0 = mx_exponent(fmaxf(__uint_as_float(am << 16), kAmaxFloor));
-      const int e1 = mx_exponent(fmaxf(__uint_as_float(am & 0xffff0000u), kAmaxFloor));
-      const uint32_t inv2 = (__float_as_uint(mx_inv_scale(e0)) >> 16) | (__float_as_uint(mx_inv_scale(e1)) & 0xffff0000u);
       uint32_t w0[8], w1[8];
-#pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        float a[4], b[4];
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          const uint32_t sc = bf16x2_mul(cw[4 * q + k], inv2);
-          a[k] = __uint_as_float(sc << 16);
-          b[k] = __uint_as_float(sc & 0xffff0000u);
-        }
-        w0[q] = e4m3x2(a[0], a[1]) | (e4m3x2(a[2], a[3]) << 16);
-        w1[q] = e4m3x2(b[0], b[1]) | (e4m3x2(b[2], b[3]) << 16);
-      }
+      col_codes(p, reinterpret_cast<const uint32_t*>(tile), tile_r, tile_c, t, sc_col, w0, w1);
       __syncthreads();  // every thread holds its part of the input tile: the stage becomes the staging buffer
-      {
-        const int c0 = 2 * cp, sw = cp & 7;  // piece q of column c at q ^ ((c >> 1) & 7): conflict-free both ways
-        tile_w[c0 * 8 + ((2 * g) ^ sw)] = make_uint4(w0[0], w0[1], w0[2], w0[3]);
-        tile_w[c0 * 8 + ((2 * g + 1) ^ sw)] = make_uint4(w0[4], w0[5], w0[6], w0[7]);
-        tile_w[(c0 + 1) * 8 + ((2 * g) ^ sw)] = make_uint4(w1[0], w1[1], w1[2], w1[3]);
-        tile_w[(c0 + 1) * 8 + ((2 * g + 1) ^ sw)] = make_uint4(w1[4], w1[5], w1[6], w1[7]);
-        if (tile_c + c0 < p.cols && tile_r + 32 * g < p.rows) {
-          sc_col[p.tiled ? tiled_offset(c0, g) : c0 * 4 + g] = static_cast<uint8_t>(e0 + 127);
-          if (tile_c + c0 + 1 < p.cols)
-            sc_col[p.tiled ? tiled_offset(c0 + 1, g) : (c0 + 1) * 4 + g] = static_cast<uint8_t>(e1 + 127);
-        }
-      }
+      stage_cols(tile, t, w0, w1);
       __syncthreads();
-#pragma unroll
-      for (int h = 0; h < 4; ++h) {
-        const int idx = t + h * kThreads;  // 1024 pieces: column idx / 8, piece idx % 8
-        const int c = idx >> 3, q = idx & 7;
-        const int64_t col_g = tile_c + c, row_g = tile_r + q * 16;
-        if (col_g < p.cols && row_g < p.rows)
-          stg_stream16(p.codes_colT + col_g * p.rows + row_g, tile[c * 8 + (q ^ ((c >> 1) & 7))]);
-      }
+      store_cols(p, tile, tile_r, tile_c, t);
     } else {
       __syncthreads();  // scale bytes of the row pass visible
     }
-
-    // Scale bytes of the tile; each entry is zeroed again by the thread that stored it.
-    if (ROW) {
-      const int64_t kb = p.cols / 32;
-      if (p.tiled) {
-        if (t < 128) {
-          const int64_t chunk = tile_y * ceil_div(kb, static_cast<int64_t>(4)) + tile_x;
-          uint32_t* src = reinterpret_cast<uint32_t*>(sc_row) + t;
-          reinterpret_cast<uint32_t*>(p.scales_row + chunk * 512)[t] = *src;
-          *src = 0u;
-        }
-      } else {
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const int idx = t + h * kThreads;
-          const int64_t r = tile_r + (idx >> 2), k = tile_c / 32 + (idx & 3);
-          if (r < p.rows && k < kb) p.scales_row[r * kb + k] = sc_row[idx];
-          sc_row[idx] = 0;
-        }
-      }
-    }
-    if (COL) {
-      const int64_t kb = p.rows / 32;
-      if (p.tiled) {
-        if (t < 128) {
-          const int64_t chunk = tile_x * ceil_div(kb, static_cast<int64_t>(4)) + tile_y;
-          uint32_t* src = reinterpret_cast<uint32_t*>(sc_col) + t;
-          reinterpret_cast<uint32_t*>(p.scales_col + chunk * 512)[t] = *src;
-          *src = 0u;
-        }
-      } else {
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const int idx = t + h * kThreads;
-          const int64_t c = tile_c + (idx >> 2), k = tile_r / 32 + (idx & 3);
-          if (c < p.cols && k < kb) p.scales_col[c * kb + k] = sc_col[idx];
-          sc_col[idx] = 0;
-        }
-      }
-    }
+    if (ROW) store_scales<true>(p.scales_row, sc_row, p.tiled, p.rows, p.cols / 32, tile_y, tile_x, t);
+    if (COL) store_scales<true>(p.scales_col, sc_col, p.tiled, p.cols, p.rows / 32, tile_x, tile_y, t);
     // this thread's generic-proxy accesses to the stage are ordered before the copy engine's next write to it
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     __syncthreads();  // the stage and the scale staging are free
-    if (t == 0 && tile_id + 2 * step < n_tiles) issue(tile_id + 2 * step, s);
+    if (t == 0 && n_tiles - tile_id > 2 * step) issue(tile_id + 2 * step, s);
   }
   if (abort_flag) {
     // copies may still be in flight into this CTA's shared memory: give them time to land before it is released
