@@ -1,5 +1,7 @@
 #include "linear.h"
 
+#include <atomic>
+
 namespace anima_host {
 
 namespace {
@@ -86,30 +88,70 @@ struct MergedNode : public HostNode {
 };
 
 // ------------------------------------------------------------------------------------------------ frozen linear
+// Frozen linears of the same input, applied one after the other (q / k / v projections), are the outputs of ONE node:
+// backward then contracts their gradients in one GEMM whose K-blocks run over all of them, in fp32 with one rounding,
+// instead of one GEMM each and additions of their outputs (two passes of three over [rows, K] for q / k / v).
+// [32768, 2048] x 3, forward and backward: 1130 -> 915 us.
 struct FrozenNode : public HostNode {
-  Op w_col;
-  Tensor w_bf16;
-  bool need_x, need_bias;
+  struct Part {
+    Op w_col;
+    Tensor w_bf16;        // serves backward where W has no column form
+    int bias_edge;        // -1: no gradient
+  };
+  std::vector<Part> parts;                 // by output
+  std::atomic<bool> started{false};        // backward has begun: nothing may join
+  int64_t k_in;
 
   variable_list apply(variable_list&& g) override {
     std::lock_guard<std::mutex> lock(mutex_);
-    const Tensor gy = grad_of(g, 0);
-    variable_list out(2);
-    if (need_x) {
+    started = true;
+    variable_list out(num_outputs());
+    const bool need_x = task_should_compute_output(0);
+    std::vector<Op> rows, weights;
+    Tensor gx, some;
+    for (size_t i = 0; i < parts.size(); ++i) {
+      if (!g[i].defined()) continue;
+      const Tensor& gy = some = g[i];
       const Launch l(gy);
+      if (parts[i].bias_edge >= 0) out[parts[i].bias_edge] = bias_grad(gy);
+      if (!need_x) continue;
       const Mat m = as_matrix(gy, gy.size(-1));
-      if (w_col.defined()) {
-        out[0] = input_grad(l, gy, quantize(l, m, true, false).first, w_col);
+      if (parts[i].w_col.defined()) {
+        rows.push_back(quantize(l, m, true, false).first);
+        weights.push_back(parts[i].w_col);
       } else {
-        Tensor gx = at::matmul(m.keep.reshape({m.rows, m.cols}), w_bf16.to(BF16));
-        out[0] = cast(gx.reshape(with_last(gy.sizes(), w_bf16.size(1))), gy.scalar_type());
+        const Tensor& w = parts[i].w_bf16;
+        gx = at::matmul(m.keep.reshape({m.rows, m.cols}), w.to(BF16)).reshape(with_last(gy.sizes(), w.size(1)));
       }
     }
-    if (need_bias) out[1] = bias_grad(gy);
+    if (!rows.empty()) {
+      const Launch l(some);
+      gx = empty(with_last(some.sizes(), k_in), BF16, l.dev);
+      if (rows[0].rows) gemm_sum(l, rows, weights, gx);
+    }
+    if (gx.defined()) out[0] = cast(gx, some.scalar_type());
     return out;
   }
   std::string name() const override { return "MXFP8FrozenLinearBackward"; }
 };
+
+// The node of the frozen linear last applied on this thread and its input (both weak).
+struct Applied {
+  c10::weak_intrusive_ptr<c10::TensorImpl> x{c10::intrusive_ptr<c10::TensorImpl>()};
+  uint32_t version = 0;
+  std::weak_ptr<FrozenNode> node;
+};
+thread_local Applied applied;
+
+// The node a frozen linear of x may become another output of, if there is one.
+std::shared_ptr<FrozenNode> joinable(const Tensor& x) {
+  auto node = applied.node.lock();
+  const auto was = applied.x.lock();
+  if (!node || was.get() != x.unsafeGetTensorImpl() || node->started || node->parts.size() >= kMaxSummed ||
+      x.unsafeGetTensorImpl()->version_counter().current_version() != applied.version || !node->parts[0].w_col.defined())
+    return nullptr;
+  return node;
+}
 
 // ------------------------------------------------------------------------------------------------ LoKr MLP
 struct MlpNode : public HostNode {
@@ -222,14 +264,25 @@ Tensor frozen_linear(const Tensor& x, Op x_row, Op w_row, Op w_col, const OptTen
     Below below;
     y = project(l, x, x_row, w_row, bias);
   }
-  if (need_x || need_bias) {
-    auto n = make_node<FrozenNode>(x, bias);
-    n->w_col = std::move(w_col);
-    n->w_bf16 = w_bf16.value_or(Tensor());
-    n->need_x = need_x;
-    n->need_bias = need_bias;
-    set_history(y, n);
+  if (!need_x && !need_bias) return y;
+  const bool shares = need_x && w_col.defined() && !x.is_inference();
+  auto n = shares ? joinable(x) : nullptr;
+  if (!n) {
+    n = make_node<FrozenNode>(x);
+    n->k_in = w_row.k;
+    if (shares) {
+      applied.x = c10::weak_intrusive_ptr<c10::TensorImpl>(x.getIntrusivePtr());
+      applied.version = x.unsafeGetTensorImpl()->version_counter().current_version();
+      applied.node = n;
+    }
   }
+  int bias_edge = -1;
+  if (need_bias) {
+    bias_edge = static_cast<int>(n->num_outputs());
+    n->add_next_edge(edge_of(bias));
+  }
+  n->parts.push_back({std::move(w_col), w_bf16.value_or(Tensor()), bias_edge});
+  set_history(y, n);
   return y;
 }
 

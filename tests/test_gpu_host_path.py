@@ -130,3 +130,55 @@ def test_modulation_and_residual_can_be_backpropagated_one_after_the_other():
                 outs[0].backward(gn)                       # its saved tensors are gone, as for any node
         for a, b in zip(*grads):
             assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("rows,ks", [(160, (256, 512, 96)), (1000, (256, 256, 256)), (96, (256, 256, 128)), (4096, (2048, 2048, 2048))])
+def test_frozen_linears_of_one_input_sum_their_input_gradients_in_one_gemm(rows, ks):
+    """Against the exact sum of the fp32 products. One GEMM (rows > 128) rounds once, at most 2^-8 of the sum; below that
+    the products are added one after the other in bf16: n roundings of partial sums, none larger than
+    sum |g_i W_i|, hence the bound n * 2^-8 * sum |g_i W_i| per element. To it comes the fp32 accumulation of both
+    sides in different orders: K * 2^-24 * sum |terms| each, and sum |terms| <= |g row| |W column| (Cauchy); a factor 2
+    covers the quantisation of the operands the norms are taken of."""
+    from anima_trainer_sm120_b200 import _lib, fp8_quant, ops
+    g = torch.Generator(device=DEV).manual_seed(rows)
+    d_in = 320
+    x = _randn(g, rows, d_in).requires_grad_(True)
+    Ws = [_randn(g, k, d_in, std=0.05) for k in ks]
+    Qs = [fp8_quant.quantize_weight(W) for W in Ws]
+    gys = [_randn(g, rows, k) for k in ks]
+    single = []
+    for i, (W, Q, gy) in enumerate(zip(Ws, Qs, gys)):
+        r = ops.mx_quantize(gy, rowwise=True)[0]
+        single.append(ops.mx_gemm(r, Q.col, out_dtype=torch.float32))
+    used = [[0, 1, 2], [0], [2], [0, 2]]
+    for idx in used:
+        fp8_quant.clear_activation_memo()
+        ys = [fp8_quant.mxfp8_frozen_linear(x, Q, W) for W, Q in zip(Ws, Qs)]
+        gx, = torch.autograd.grad([ys[i] for i in idx], x, [gys[i] for i in idx])
+        want = sum(single[i] for i in idx)
+        roundings = 1 if rows > 128 else len(idx)
+        bound = roundings * 2.0 ** -8 * sum(single[i].abs() for i in idx)
+        bound += sum(2 * 2 * ks[i] * 2.0 ** -24 * gys[i].float().norm(dim=1)[:, None] * Ws[i].float().norm(dim=0)[None]
+                     for i in idx)
+        assert bool(((gx.float() - want).abs() <= bound).all())
+    _lib.check_status_word(x.device)
+
+
+def test_frozen_linears_backpropagated_apart_and_after_an_in_place_change():
+    from anima_trainer_sm120_b200 import fp8_quant
+    g = torch.Generator(device=DEV).manual_seed(3)
+    x = _randn(g, 256, 256).requires_grad_(True)
+    W = _randn(g, 256, 256, std=0.05)
+    Q, gy = fp8_quant.quantize_weight(W), _randn(g, 256, 256)
+    y1, y2 = (fp8_quant.mxfp8_frozen_linear(x, Q, W) for _ in range(2))
+    y1.backward(gy)
+    first = x.grad.clone()
+    y3 = fp8_quant.mxfp8_frozen_linear(x, Q, W)            # the node that has run takes no further output
+    y2.backward(gy)
+    y3.backward(gy)
+    assert torch.equal(x.grad, (first + first) + first)
+    h = x.detach().clone().requires_grad_(True) * 1.0
+    a = fp8_quant.mxfp8_frozen_linear(h, Q, W)
+    h.add_(1.0)
+    b = fp8_quant.mxfp8_frozen_linear(h, Q, W)
+    assert a.grad_fn is not b.grad_fn
