@@ -48,6 +48,12 @@ static const Tensor& on_cuda(const Tensor& t) {
 Launch::Launch(const Tensor& t)
     : dev(on_cuda(t).device()), guard(dev), stream(c10::cuda::getCurrentCUDAStream(dev.index()).stream()) {}
 
+void admit(const Launch& l, const Tensor& t) {
+  if (!t.defined()) return;
+  TORCH_CHECK(t.device() == l.dev, "tensors on different devices: ", l.dev, " and ", t.device());
+  TORCH_CHECK_NOT_IMPLEMENTED(!t._fw_grad(/*level=*/0).defined(), "forward-mode AD is not implemented for these kernels");
+}
+
 Op op_in(const Tensor& store, int64_t rows, int64_t k) {
   uint8_t* p = static_cast<uint8_t*>(store.data_ptr());
   return {store, Tensor(), p, p + pad256(rows * k), rows, k};

@@ -81,6 +81,18 @@ struct Launch {
   void* stream;
 };
 
+// What these nodes cannot take: tensors of another device, and forward-mode tangents (an autograd function without a
+// rule for them refuses; a node made by hand would drop them without notice).
+void admit(const Launch& l, const Tensor& t);
+inline void admit(const Launch& l, const OptTensor& t) {
+  if (t) admit(l, *t);
+}
+template <class First, class... Rest>
+void admit(const Launch& l, const First& first, const Rest&... rest) {
+  admit(l, first);
+  (admit(l, rest), ...);
+}
+
 int32_t* status_word(const at::Device& dev);      // the GEMM's bounded-wait flag of a device
 Tensor status_word_tensor(int64_t device_index);
 
@@ -173,6 +185,32 @@ std::shared_ptr<N> make_node(const Inputs&... inputs) {
   node->set_next_edges(std::move(edges));
   return node;
 }
+// The node last made for an input on this thread (both weak), for a later call on the same tensor that may become part
+// of it. `get` gives the node while t still is what it saw: same tensor, version, shape and graph edge.
+template <class N>
+struct LastNode {
+  c10::weak_intrusive_ptr<c10::TensorImpl> x{c10::intrusive_ptr<c10::TensorImpl>()};
+  uint32_t version = 0;
+  at::DimVector sizes;
+  std::weak_ptr<N> node;
+
+  void set(const Tensor& t, const std::shared_ptr<N>& n) {      // n's first edge is t's
+    x = c10::weak_intrusive_ptr<c10::TensorImpl>(t.getIntrusivePtr());
+    version = t.unsafeGetTensorImpl()->version_counter().current_version();
+    sizes = t.sizes();
+    node = n;
+  }
+  std::shared_ptr<N> get(const Tensor& t) const {
+    auto n = node.lock();
+    const auto was = x.lock();
+    if (!n || was.get() != t.unsafeGetTensorImpl() ||
+        t.unsafeGetTensorImpl()->version_counter().current_version() != version || t.sizes() != at::IntArrayRef(sizes) ||
+        edge_of(t) != n->next_edge(0))
+      return nullptr;
+    return n;
+  }
+};
+
 // Kernels and allocations of a node run below autograd.
 using Below = at::AutoDispatchBelowADInplaceOrView;
 

@@ -1,7 +1,5 @@
 #include "linear.h"
 
-#include <atomic>
-
 namespace anima_host {
 
 namespace {
@@ -99,8 +97,26 @@ struct FrozenNode : public HostNode {
     int bias_edge;        // -1: no gradient
   };
   std::vector<Part> parts;                 // by output
-  std::atomic<bool> started{false};        // backward has begun: nothing may join
+  bool started = false;                    // backward has begun: nothing may join (under the node's lock)
   int64_t k_in;
+
+  // y becomes another output unless backward has begun. A bias that is itself computed could depend on an earlier
+  // output of this node, a cycle: such a linear keeps a node of its own.
+  bool join(Part part, const OptTensor& bias, const Tensor& y) {
+    std::lock_guard<std::mutex> lock(mutex_);
+    if (started || parts.size() >= kMaxSummed || (wants(bias) && !bias->is_leaf())) return false;
+    add(std::move(part), bias, y);
+    return true;
+  }
+  void add(Part part, const OptTensor& bias, const Tensor& y) {
+    part.bias_edge = -1;
+    if (wants(bias)) {
+      part.bias_edge = static_cast<int>(num_outputs());
+      add_next_edge(edge_of(bias));
+    }
+    parts.push_back(std::move(part));
+    set_history(y, std::static_pointer_cast<FrozenNode>(getptr()));
+  }
 
   variable_list apply(variable_list&& g) override {
     std::lock_guard<std::mutex> lock(mutex_);
@@ -109,7 +125,7 @@ struct FrozenNode : public HostNode {
     const bool need_x = task_should_compute_output(0);
     std::vector<Op> rows, weights;
     Tensor gx, some;
-    for (size_t i = 0; i < parts.size(); ++i) {
+    for (size_t i = 0; i < std::min(parts.size(), g.size()); ++i) {
       if (!g[i].defined()) continue;
       const Tensor& gy = some = g[i];
       const Launch l(gy);
@@ -135,23 +151,7 @@ struct FrozenNode : public HostNode {
   std::string name() const override { return "MXFP8FrozenLinearBackward"; }
 };
 
-// The node of the frozen linear last applied on this thread and its input (both weak).
-struct Applied {
-  c10::weak_intrusive_ptr<c10::TensorImpl> x{c10::intrusive_ptr<c10::TensorImpl>()};
-  uint32_t version = 0;
-  std::weak_ptr<FrozenNode> node;
-};
-thread_local Applied applied;
-
-// The node a frozen linear of x may become another output of, if there is one.
-std::shared_ptr<FrozenNode> joinable(const Tensor& x) {
-  auto node = applied.node.lock();
-  const auto was = applied.x.lock();
-  if (!node || was.get() != x.unsafeGetTensorImpl() || node->started || node->parts.size() >= kMaxSummed ||
-      x.unsafeGetTensorImpl()->version_counter().current_version() != applied.version || !node->parts[0].w_col.defined())
-    return nullptr;
-  return node;
-}
+thread_local LastNode<FrozenNode> applied;
 
 // ------------------------------------------------------------------------------------------------ LoKr MLP
 struct MlpNode : public HostNode {
@@ -188,6 +188,7 @@ Tensor lokr_linear(const Tensor& x, Op x_row, Op x_col, const Tensor& W, const O
                    const Tensor& w2, double alpha, bool first) {
   const bool need_x = wants(x), train = wants(w1) || wants(w2), need_bias = wants(bias);
   const Launch l(x);
+  admit(l, x, W, bias, w1, w2);
   Tensor y;
   Op w_col;
   {
@@ -224,6 +225,7 @@ Tensor lokr_linear(const Tensor& x, Op x_row, Op x_col, const Tensor& W, const O
 Tensor merged_linear(const Tensor& x, Op x_row, Op x_col, const Tensor& merged, const OptTensor& bias, bool first) {
   const bool need_x = wants(x), train = wants(merged), need_bias = wants(bias);
   const Launch l(x);
+  admit(l, x, merged, bias);
   Tensor y;
   Op w_col;
   {
@@ -259,6 +261,7 @@ Tensor frozen_linear(const Tensor& x, Op x_row, Op w_row, Op w_col, const OptTen
   TORCH_CHECK_VALUE(x.size(-1) == w_row.k, "input of width ", x.size(-1), " for a weight with ", w_row.k, " columns");
   const bool need_x = wants(x), need_bias = wants(bias);
   const Launch l(x);
+  admit(l, x, bias, x_row.store, x_row.other, w_row.store, w_row.other, w_col.store, w_col.other);
   Tensor y;
   {
     Below below;
@@ -266,23 +269,13 @@ Tensor frozen_linear(const Tensor& x, Op x_row, Op w_row, Op w_col, const OptTen
   }
   if (!need_x && !need_bias) return y;
   const bool shares = need_x && w_col.defined() && !x.is_inference();
-  auto n = shares ? joinable(x) : nullptr;
-  if (!n) {
-    n = make_node<FrozenNode>(x);
-    n->k_in = w_row.k;
-    if (shares) {
-      applied.x = c10::weak_intrusive_ptr<c10::TensorImpl>(x.getIntrusivePtr());
-      applied.version = x.unsafeGetTensorImpl()->version_counter().current_version();
-      applied.node = n;
-    }
-  }
-  int bias_edge = -1;
-  if (need_bias) {
-    bias_edge = static_cast<int>(n->num_outputs());
-    n->add_next_edge(edge_of(bias));
-  }
-  n->parts.push_back({std::move(w_col), w_bf16.value_or(Tensor()), bias_edge});
-  set_history(y, n);
+  FrozenNode::Part part{std::move(w_col), w_bf16.value_or(Tensor()), -1};
+  if (shares)
+    if (auto n = applied.get(x); n && n->join(part, bias, y)) return y;
+  auto n = make_node<FrozenNode>(x);
+  n->k_in = w_row.k;
+  n->add(std::move(part), bias, y);
+  if (shares) applied.set(x, n);
   return y;
 }
 
@@ -292,6 +285,7 @@ Tensor lokr_mlp(const Tensor& x, Op x_row, Op x_col, const Tensor& W1, const Opt
   const bool train = wants(w1a) || wants(w2a) || wants(w1b) || wants(w2b), need_x = wants(x), back = need_x || train;
   const bool keep = back && !first;
   const Launch l(x);
+  admit(l, x, W1, b1, w1a, w2a, W2, b2, w1b, w2b);
   const int64_t rows = x_row.rows, hid = W1.size(0);
   Tensor y, h;
   Op a_col, W1_col, W2_col;

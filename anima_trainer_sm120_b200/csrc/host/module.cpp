@@ -32,6 +32,7 @@ std::pair<Triple, Triple> py_quantize(const Tensor& x, bool row, bool col, int l
 Tensor py_gemm(const Tensor& ac, const Tensor& as, const Tensor& bc, const Tensor& bs, const OptTensor& bias) {
   const Launch l(ac);
   TORCH_CHECK(bc.device() == l.dev && as.device() == l.dev && bs.device() == l.dev, "tensors on different devices");
+  TORCH_CHECK(!bias || bias->device() == l.dev, "tensors on different devices");
   const Op a = op_of(ac, as), b = op_of(bc, bs);
   TORCH_CHECK_VALUE(!bias || (bias->scalar_type() == BF16 && bias->numel() == b.rows && bias->is_contiguous()),
                     "bias must be contiguous bfloat16 of length N");

@@ -38,7 +38,9 @@ int64_t pitch_of(const Tensor& m) {
 Mods mods_of(std::initializer_list<const Tensor*> ts) {
   Mods m{{}, 0};
   bool in_place = true;
+  const int64_t n = (*ts.begin())->numel();
   for (const Tensor* t : ts) {
+    TORCH_CHECK_VALUE(t->numel() == n, "modulation tensors of different sizes");
     const int64_t ld = pitch_of(*t);
     if (ld < 0 || (ld && m.ld && ld != m.ld)) in_place = false;
     if (ld > 0) m.ld = ld;
@@ -129,27 +131,13 @@ struct AdalnNode : public HostNode {      // saves x, scale, statistics
   std::string name() const override { return "FusedAdaLNBackward"; }
 };
 
-// The x last modulated on this thread and its node (both weak).
-struct Modulated {
-  c10::weak_intrusive_ptr<c10::TensorImpl> x{c10::intrusive_ptr<c10::TensorImpl>()};
-  uint32_t version = 0;
-  std::weak_ptr<torch::autograd::Node> node;
-};
-thread_local Modulated modulated;
+thread_local LastNode<torch::autograd::Node> modulated;
 
-void remember(const Tensor& x, const std::shared_ptr<torch::autograd::Node>& node) {
-  modulated.x = c10::weak_intrusive_ptr<c10::TensorImpl>(x.getIntrusivePtr());
-  modulated.version = x.unsafeGetTensorImpl()->version_counter().current_version();
-  modulated.node = node;
-}
 // x, or its alias whose gradient goes to the modulation's node
 Tensor through_modulation(const Tensor& x) {
   if (!wants(x) || x.is_inference()) return x;
-  const auto node = modulated.node.lock();
-  const auto was = modulated.x.lock();
-  if (!node || was.get() != x.unsafeGetTensorImpl() ||
-      x.unsafeGetTensorImpl()->version_counter().current_version() != modulated.version)
-    return x;
+  const auto node = modulated.get(x);
+  if (!node) return x;
   modulated.node.reset();
   Tensor alias(x.unsafeGetTensorImpl()->shallow_copy_and_detach(x.unsafeGetTensorImpl()->version_counter(), true));
   torch::autograd::impl::set_gradient_edge(alias, torch::autograd::Edge(node, 1));
@@ -269,6 +257,7 @@ struct RopeNode : public HostNode {      // saves x, rstd
 std::tuple<Tensor, Op> adaln(const Tensor& x, const Tensor& scale, const Tensor& shift, double eps, bool quant) {
   const bool grad = wants(x) || wants(scale) || wants(shift);
   const Launch l(x);
+  admit(l, x, scale, shift);
   AdalnOut o;
   {
     at::AutoDispatchBelowADInplaceOrView below;
@@ -285,7 +274,7 @@ std::tuple<Tensor, Op> adaln(const Tensor& x, const Tensor& scale, const Tensor&
     node->dt_shift = shift.scalar_type();
     set_history(o.y, node);
     node->add_input_metadata(x);
-    if (x.requires_grad() && !x.is_inference()) remember(x, node);
+    if (x.requires_grad() && !x.is_inference()) modulated.set(x, node);
   }
   return {o.y, o.emitted};
 }
@@ -293,6 +282,7 @@ std::tuple<Tensor, Op> adaln(const Tensor& x, const Tensor& scale, const Tensor&
 Tensor gated_add(const Tensor& x_, const Tensor& gate, const Tensor& y) {
   const bool grad = wants(x_) || wants(gate) || wants(y);
   const Launch l(x_);
+  admit(l, x_, gate, y);
   const Tensor x = grad ? through_modulation(x_) : x_;
   Tensor out, yc;
   Mods g;
@@ -318,6 +308,7 @@ std::tuple<Tensor, Tensor, Op> gated_add_adaln(const Tensor& x_, const Tensor& g
                                                const Tensor& shift, double eps, bool quant) {
   const bool grad = wants(x_) || wants(sub) || wants(gate) || wants(scale) || wants(shift);
   const Launch l(x_);
+  admit(l, x_, gate, sub, scale, shift);
   const Tensor x = grad ? through_modulation(x_) : x_;
   Both c;
   {
@@ -345,6 +336,7 @@ std::tuple<Tensor, Tensor, Op> gated_add_adaln(const Tensor& x_, const Tensor& g
 Tensor rmsnorm_rope(const Tensor& x, const Tensor& weight, const OptTensor& cos, const OptTensor& sin, double eps) {
   TORCH_CHECK_TYPE(x.scalar_type() == BF16, "RMSNorm + RoPE needs bfloat16, got ", x.scalar_type());
   const Launch l(x);
+  admit(l, x, weight, cos, sin);
   const int64_t heads = x.size(-2), d = x.size(-1), tokens = x.numel() ? x.numel() / (heads * d) : 0;
   Tensor out, xc, w, rstd;
   {

@@ -164,6 +164,20 @@ std::pair<Op, Op> saved_input(HostNode& n, size_t& at, int64_t rows, int64_t K) 
   return {gq, gq_col};
 }
 
+// The kernels index by these shapes: a mismatch must not reach them.
+void check_linear(const Launch& l, const Tensor& x, int64_t k_in, const TLinear& t) {
+  admit(l, t.bias, t.w1.t, t.a.t, t.b.t, t.mask, t.c, t.w_row.store, t.w_row.other, t.w_col.store, t.w_col.other);
+  TORCH_CHECK_NOT_IMPLEMENTED(t.c.dim() == 2 && t.c.size(0) == 8 && t.c.size(1) == 8,
+                              "rank_mix supports an 8x8 factor; got ", t.c.sizes());
+  TORCH_CHECK_VALUE(t.a.t.dim() == 2 && t.b.t.dim() == 2 && t.b.t.size(0) == t.rank() && t.n_out() == 8 * t.vp() &&
+                        t.k_in() == 8 * t.b.t.size(1) && t.w_col.rows == t.k_in() && t.w_col.k == t.n_out(),
+                    "factors ", t.a.t.sizes(), " and ", t.b.t.sizes(), " do not match a weight [", t.n_out(), ", ", t.k_in(), "]");
+  TORCH_CHECK_VALUE(x.dim() >= 2 && k_in == t.k_in(), "input of width ", k_in, " for a weight with ", t.k_in(), " columns");
+  if (t.mask && t.mask->defined())
+    TORCH_CHECK_VALUE(t.mask->dim() == 2 && t.mask->size(0) == x.size(0) && t.mask->size(1) == t.rank(), "mask ",
+                      t.mask->sizes(), " does not match batch ", x.size(0), " and rank ", t.rank());
+}
+
 std::vector<int64_t> lead_of(const Tensor& x) { return {x.sizes().begin(), x.sizes().end() - 1}; }
 int64_t product(at::IntArrayRef v) { return c10::multiply_integers(v); }
 Tensor grad_bias(const Tensor& gy) { return gy.reshape({-1, gy.size(-1)}).sum(0); }
@@ -230,6 +244,8 @@ struct TlokrMlpNode : public HostNode {
 Tensor tlokr_linear(const Tensor& x, Op x_row, TLinear t, bool first) {
   const Needs need = needs_of(x, t);
   const Launch l(x);
+  admit(l, x);
+  check_linear(l, x, x.size(-1), t);
   const int64_t K = t.k_in(), rows = x.numel() / K;
   const bool keep = need.any() && !first;
   Tensor y;
@@ -254,6 +270,9 @@ Tensor tlokr_mlp(const Tensor& x, Op x_row, TLinear t1, TLinear t2, bool first) 
   const Needs n1 = needs_of(x, t1), n2 = needs_of(x, t2);
   const bool back = n1.x || n1.factors || n2.factors, keep = back && !first;
   const Launch l(x);
+  admit(l, x);
+  check_linear(l, x, x.size(-1), t1);
+  check_linear(l, x, t1.n_out(), t2);
   const int64_t K = t1.k_in(), rows = x.numel() / K, hid = t1.n_out();
   Tensor y, h;
   Input in1, in2;

@@ -182,3 +182,61 @@ def test_frozen_linears_backpropagated_apart_and_after_an_in_place_change():
     h.add_(1.0)
     b = fp8_quant.mxfp8_frozen_linear(h, Q, W)
     assert a.grad_fn is not b.grad_fn
+
+
+def test_a_frozen_linear_joins_a_node_only_while_its_input_is_what_that_node_saw():
+    """Same tensor object, but another graph edge, a computed bias (which could depend on the node's own output) or more
+    linears than one launch sums: each gets a node of its own, and the gradients are those of separate tensors."""
+    from anima_trainer_sm120_b200 import fp8_quant
+    g = torch.Generator(device=DEV).manual_seed(4)
+    W = _randn(g, 256, 256, std=0.05)
+    Q, gy = fp8_quant.quantize_weight(W), _randn(g, 256, 256)
+    lin = lambda x, b=None: fp8_quant.mxfp8_frozen_linear(x, Q, W, b)
+    base = _randn(g, 256, 256).requires_grad_(True)
+    x = base * 1.0
+    a = lin(x)
+    x.detach_().requires_grad_(True)               # a leaf now; `a` still belongs to base's graph
+    b = lin(x)
+    assert a.grad_fn is not b.grad_fn
+    ga, = torch.autograd.grad(a, base, gy)
+    gb, = torch.autograd.grad(b, x, gy)
+    assert torch.equal(ga, gb)
+    ys = [lin(base) for _ in range(4)]
+    assert ys[0].grad_fn is ys[2].grad_fn and ys[3].grad_fn is not ys[0].grad_fn
+    y1 = lin(base)
+    y2 = lin(base, y1.mean(0))                     # bias from the first output
+    assert y1.grad_fn is not y2.grad_fn
+    gx, = torch.autograd.grad(y2, base, gy)
+    assert bool(torch.isfinite(gx).all())
+
+
+def test_tensors_of_another_device_tangents_and_wrong_shapes_are_refused_before_a_launch():
+    import torch.autograd.forward_ad as fwAD
+    from anima_trainer_sm120_b200 import adaln_kernel, fp8_quant, tlokr
+    from anima_trainer_sm120_b200.qk_norm_rope import FusedRMSNormRoPE
+    g = torch.Generator(device=DEV).manual_seed(5)
+    W, x = _randn(g, 256, 256, std=0.05), _randn(g, 64, 256)
+    Q, bias = fp8_quant.quantize_weight(W), _randn(g, 256)
+    w1, w2 = _randn(g, 8, 8), _randn(g, 32, 32)
+    x5, mod = _randn(g, 1, 1, 4, 4, 256), _randn(g, 1, 1, 1, 1, 256)
+    heads, w = _randn(g, 1, 16, 2, 128), _randn(g, 128)
+    calls = [(lambda t: fp8_quant.mxfp8_frozen_linear(x, Q, W, t), bias),
+             (lambda t: fp8_quant.lokr_linear_fused(x, W, t, w1, w2, 1.0), bias),
+             (lambda t: fp8_quant.lokr_linear_fused(x, W, None, t, w2, 1.0), w1),
+             (lambda t: adaln_kernel.fused_adaln(x5, t, mod, 1e-6), mod),
+             (lambda t: adaln_kernel.fused_gated_add(x5, t, x5), mod),
+             (lambda t: FusedRMSNormRoPE.apply(heads, t, None, None, 1e-6), w)]
+    for call, t in calls:
+        with pytest.raises(RuntimeError):
+            call(t.cpu())
+        with fwAD.dual_level(), pytest.raises(NotImplementedError):
+            call(fwAD.make_dual(t, torch.ones_like(t)))
+        call(t)
+    big = fp8_quant.quantize_weight(_randn(g, 1024, 512, std=0.05))
+    xt, a, b = _randn(g, 2, 128, 512), _randn(g, 128, 128), _randn(g, 128, 64)
+    for args in [(w1, a, b, torch.ones(1, 128, device=DEV, dtype=BF16)), (w1, a, b, torch.ones(2, 64, device=DEV, dtype=BF16)),
+                 (w1, a[:64], b, None), (w1, a, b[:64], None), (_randn(g, 4, 4), a, b, None)]:
+        with pytest.raises((ValueError, NotImplementedError)):
+            tlokr._MXTLoKrLinear.apply(xt, big, None, *args, 0.5)
+    with pytest.raises(ValueError):
+        adaln_kernel.fused_adaln(x5, mod, _randn(g, 1, 1, 1, 1, 128), 1e-6)
