@@ -12,61 +12,78 @@
 // The wgrad reduction is two-stage (per-CTA partial 8x8 blocks in caller scratch,
 // then a fixed-order sum) and therefore bit-reproducible.
 #include "common.cuh"
+#include "f32x2.cuh"
 #include "mx_quantize_tile.cuh"
 
 namespace anima {
 namespace {
 
-template <bool TRANSPOSE, bool HAS_MASK>
-__global__ void __launch_bounds__(256)
-rank_mix_kernel(const __nv_bfloat16* __restrict__ hidden, const __nv_bfloat16* __restrict__ c,
-                const __nv_bfloat16* __restrict__ mask, int64_t total, int64_t n_per_batch, int r8,
-                __nv_bfloat16* __restrict__ out) {
-  __shared__ float cw[64];  // cw[i*8+j] = weight applied to hidden row j for output row i
-  if (threadIdx.x < 64) {
-    const int i = threadIdx.x >> 3, j = threadIdx.x & 7;
-    cw[threadIdx.x] = __bfloat162float(TRANSPOSE ? c[j * 8 + i] : c[i * 8 + j]);
-  }
-  __syncthreads();
-  const int64_t idx = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
-  if (idx >= total) return;
-  const int64_t row = idx / r8;  // (b, n) flattened
-  const int rc = static_cast<int>(idx - row * r8);
-  const int64_t rank = static_cast<int64_t>(r8) * 8;
-  const __nv_bfloat16* src = hidden + row * 8 * rank + rc * 8;
-
-  uint4 h[8];
-#pragma unroll
-  for (int j = 0; j < 8; ++j) h[j] = ldg_stream16(src + j * rank);
-  float m[8];
-  if (HAS_MASK) {
-    unpack8(*reinterpret_cast<const uint4*>(mask + (row / n_per_batch) * rank + rc * 8), m);
-  }
-  float acc[8][8];
+// The mix of one thread: rows j = 0..7 of an item at 8 ranks -> its 8 mixed rows in bf16. fp32 fma over j ascending from
+// 0, mask, one rounding; the ranks run in pairs (f32x2), which halves the 512 multiply-adds and changes no bit.
+// w[j * 8 + i] = {c, c}, the weight of row j in output row i.
+template <bool HAS_MASK>
+__device__ __forceinline__ void mix8(const uint4 (&h)[8], const f2* w, const uint4& mask, uint4 (&out)[8]) {
+  f2 acc[8][4];
 #pragma unroll
   for (int i = 0; i < 8; ++i)
 #pragma unroll
-    for (int e = 0; e < 8; ++e) acc[i][e] = 0.f;
+    for (int e = 0; e < 4; ++e) acc[i][e] = 0ull;
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
-    float hf[8];
-    unpack8(h[j], hf);
+    const f2 x[4] = {f2_of_bf16(h[j].x), f2_of_bf16(h[j].y), f2_of_bf16(h[j].z), f2_of_bf16(h[j].w)};
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const float w = cw[i * 8 + j];
+    for (int i = 0; i < 8; i += 2) {
+      const ulonglong2 c = *reinterpret_cast<const ulonglong2*>(w + j * 8 + i);
 #pragma unroll
-      for (int e = 0; e < 8; ++e) acc[i][e] = fmaf(hf[e], w, acc[i][e]);
+      for (int e = 0; e < 4; ++e) {
+        acc[i][e] = f2_fma(x[e], c.x, acc[i][e]);
+        acc[i + 1][e] = f2_fma(x[e], c.y, acc[i + 1][e]);
+      }
     }
   }
-  __nv_bfloat16* dst = out + row * 8 * rank + rc * 8;
+  if (HAS_MASK) {
+    const f2 m[4] = {f2_of_bf16(mask.x), f2_of_bf16(mask.y), f2_of_bf16(mask.z), f2_of_bf16(mask.w)};
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    if (HAS_MASK) {
+    for (int i = 0; i < 8; ++i)
 #pragma unroll
-      for (int e = 0; e < 8; ++e) acc[i][e] *= m[e];
-    }
-    stg_stream16(dst + i * rank, pack8(acc[i]));
+      for (int e = 0; e < 4; ++e) acc[i][e] = f2_mul(acc[i][e], m[e]);
   }
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+    out[i] = make_uint4(bf16_of_f2(acc[i][0]), bf16_of_f2(acc[i][1]), bf16_of_f2(acc[i][2]), bf16_of_f2(acc[i][3]));
+}
+template <bool TRANSPOSE>
+__device__ __forceinline__ void stage_weights(const __nv_bfloat16* c, f2* w) {
+  if (threadIdx.x < 64) {
+    const int j = threadIdx.x >> 3, i = threadIdx.x & 7;
+    w[threadIdx.x] = f2_dup(__bfloat162float(TRANSPOSE ? c[j * 8 + i] : c[i * 8 + j]));
+  }
+}
+
+template <bool TRANSPOSE, bool HAS_MASK>
+__global__ void __launch_bounds__(256, 2)
+rank_mix_kernel(const __nv_bfloat16* __restrict__ hidden, const __nv_bfloat16* __restrict__ c,
+                const __nv_bfloat16* __restrict__ mask, int64_t total, int64_t n_per_batch, int r8,
+                __nv_bfloat16* __restrict__ out) {
+  __shared__ __align__(16) f2 w[64];
+  const int64_t idx = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
+  const int64_t row = idx / r8;  // (b, n) flattened
+  const int rc = static_cast<int>(idx - row * r8);
+  const int64_t rank = static_cast<int64_t>(r8) * 8, at = row * 8 * rank + rc * 8;
+
+  uint4 h[8], m = make_uint4(0u, 0u, 0u, 0u);
+  if (idx < total) {       // in flight while the weights are staged
+#pragma unroll
+    for (int j = 0; j < 8; ++j) h[j] = ldg_stream16(hidden + at + j * rank);
+    if (HAS_MASK) m = *reinterpret_cast<const uint4*>(mask + (row / n_per_batch) * rank + rc * 8);
+  }
+  stage_weights<TRANSPOSE>(c, w);
+  __syncthreads();
+  if (idx >= total) return;
+  uint4 y[8];
+  mix8<HAS_MASK>(h, w, m, y);
+#pragma unroll
+  for (int i = 0; i < 8; ++i) stg_stream16(out + at + i * rank, y[i]);
 }
 
 // rank_mix whose output leaves as MXFP8 operands (the factor GEMM that consumes the mixed tensor wants e4m3
@@ -74,12 +91,15 @@ rank_mix_kernel(const __nv_bfloat16* __restrict__ hidden, const __nv_bfloat16* _
 // pair moves). The mix is computed and rounded to bf16 exactly as in rank_mix_kernel, then quantised with the
 // arithmetic of the tile quantiser, so codes and scales equal those of quantising the bf16 tensor.
 //   row form   [R, rank], R = items * 8: a block is 32 consecutive ranks of one row = the 8-rank chunks of four
-//              adjacent lanes (two shuffles);
+//              adjacent lanes;
 //   column form, stored transposed [rank, R]: a block is 32 consecutive rows of one rank = rows i = 0..7 of four
-//              consecutive items, i.e. four threads r8 apart, which exchange their 8-row amax through shared
-//              memory; a thread then writes 8 code bytes (its item's rows) per rank.
+//              consecutive items. A warp holds four items x 64 ranks, so the four threads of a block are lanes 8 apart
+//              and the block's amax is two shuffles; a thread then has 8 code bytes (its item's rows) per rank.
 // The host guarantees rank in {128, 256, 512} (whole 128-column scale chunks, whole item groups per CTA) and
 // items % 16 == 0 (every CTA full, R % 128 == 0: no padding entries in the tiled scale buffers).
+// Bound by instruction issue. us at [8, 4096, 8, 128], scalar arithmetic -> pairs and packed bf16: row 47.1 -> 42.0,
+// column 51.2 -> 42.1, both 71.8 -> 57.3, planes + column 72.7 -> 60.4; rank_mix 33.8 -> 30.8 (all timed with L2
+// rewritten before each launch).
 struct MixCodes {
   uint8_t* codes_row;    // [R, rank] or null
   uint8_t* scales_row;   // tiled
@@ -96,126 +116,97 @@ __global__ void __launch_bounds__(256, 2)
 rank_mix_quant_kernel(const __nv_bfloat16* __restrict__ hidden, const __nv_bfloat16* __restrict__ c,
                       const __nv_bfloat16* __restrict__ mask, int64_t items, int64_t n_per_batch, int r8,
                       __nv_bfloat16* __restrict__ out, const MixCodes q) {
-  __shared__ float cw[64];
-  __shared__ __align__(16) float col_amax[COL ? 2048 : 4];   // [thread][8 ranks]
+  __shared__ __align__(16) f2 w[64];
   __shared__ __align__(16) uint2 stage[COL ? 2048 : 2];      // transposed codes of the CTA: [rank][item] x 8 bytes
-  if (threadIdx.x < 64) {
-    const int i = threadIdx.x >> 3, j = threadIdx.x & 7;
-    cw[threadIdx.x] = __bfloat162float(TRANSPOSE ? c[j * 8 + i] : c[i * 8 + j]);
-  }
-  __syncthreads();
-  const int64_t idx = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;   // < items * r8: every CTA is full
-  const int64_t item = idx / r8;  // (b, n) flattened
-  const int rc = static_cast<int>(idx - item * r8);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, groups = r8 >> 3;
+  const int P = 256 / r8;                                    // items of the CTA, a multiple of 4
+  const int item_local = (warp / groups) * 4 + (lane >> 3), rc = (warp % groups) * 8 + (lane & 7);
+  const int64_t item = static_cast<int64_t>(blockIdx.x) * P + item_local;   // (b, n) flattened; every CTA is full
   const int rank = r8 * 8;
-  const int64_t R = items * 8;
-  const __nv_bfloat16* src = hidden + item * 8 * rank + rc * 8;
+  const int64_t R = items * 8, at = item * 8 * rank + rc * 8;
 
-  uint4 h[8];
+  uint4 h[8], m = make_uint4(0u, 0u, 0u, 0u);
 #pragma unroll
-  for (int j = 0; j < 8; ++j) h[j] = ldg_stream16(src + j * rank);
-  float m[8];
-  if (HAS_MASK) unpack8(*reinterpret_cast<const uint4*>(mask + (item / n_per_batch) * rank + rc * 8), m);
-  float acc[8][8];
+  for (int j = 0; j < 8; ++j) h[j] = ldg_stream16(hidden + at + j * rank);
+  if (HAS_MASK) m = *reinterpret_cast<const uint4*>(mask + (item / n_per_batch) * rank + rc * 8);
+  stage_weights<TRANSPOSE>(c, w);
+  __syncthreads();
+  uint4 y[8];   // the rows as rank_mix would have written them
+  mix8<HAS_MASK>(h, w, m, y);
+  if (out != nullptr) {
 #pragma unroll
-  for (int i = 0; i < 8; ++i)
-#pragma unroll
-    for (int e = 0; e < 8; ++e) acc[i][e] = 0.f;
-#pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    float hf[8];
-    unpack8(h[j], hf);
+    for (int i = 0; i < 8; ++i) stg_stream16(out + at + i * rank, y[i]);
+  }
+  if (ROW) {
+    // row i is a constant step from row i - 1 in the codes and in the tiled scales (plane_rows is a multiple of 128)
+    const int64_t row = q.plane_rows ? item : item * 8;
+    const int64_t code_step = q.plane_rows ? q.plane_rows * rank : rank;
+    const int64_t scale_step = q.plane_rows ? (q.plane_rows >> 7) * (rank >> 7) * 512 : 16;
+    uint8_t* codes_at = q.codes_row + row * rank + rc * 8;
+    uint8_t* scale_at = q.scales_row + ((row >> 7) * (rank >> 7) + (rc >> 4)) * 512 +
+                        mxq::tiled_offset(static_cast<int>(row & 127), (rc >> 2) & 3);
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-      const float w = cw[i * 8 + j];
-#pragma unroll
-      for (int e = 0; e < 8; ++e) acc[i][e] = fmaf(hf[e], w, acc[i][e]);
-    }
-  }
-  float cmax[8];
-#pragma unroll
-  for (int e = 0; e < 8; ++e) cmax[e] = 0.f;
-  uint4 packed[8];   // the rows as rank_mix would have written them (bf16); the column pass re-reads them from here
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    if (HAS_MASK) {
-#pragma unroll
-      for (int e = 0; e < 8; ++e) acc[i][e] *= m[e];
-    }
-    packed[i] = pack8(acc[i]);
-    if (out != nullptr) stg_stream16(out + (item * 8 + i) * rank + rc * 8, packed[i]);
-    float f[8];
-    unpack8(packed[i], f);                         // quantise the rounded values
-    float amax = 0.f;
-#pragma unroll
-    for (int e = 0; e < 8; ++e) {
-      const float a = fabsf(f[e]);
-      amax = fmaxf(amax, a);
-      if (COL) cmax[e] = fmaxf(cmax[e], a);
-    }
-    if (ROW) {
-      amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
-      amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
-      const int ex = mxq::mx_exponent(fmaxf(amax, mxq::kAmaxFloor));
-      const float inv = mxq::mx_inv_scale(ex);
       uint2 codes;
-      codes.x = mxq::e4m3x2(f[0] * inv, f[1] * inv) | (mxq::e4m3x2(f[2] * inv, f[3] * inv) << 16);
-      codes.y = mxq::e4m3x2(f[4] * inv, f[5] * inv) | (mxq::e4m3x2(f[6] * inv, f[7] * inv) << 16);
-      const int64_t row = q.plane_rows ? i * q.plane_rows + item : item * 8 + i;
-      *reinterpret_cast<uint2*>(q.codes_row + row * rank + rc * 8) = codes;
-      if ((rc & 3) == 0) {
-        const int kb = rc >> 2;
-        q.scales_row[((row >> 7) * (rank >> 7) + (kb >> 2)) * 512 + mxq::tiled_offset(static_cast<int>(row & 127), kb & 3)] =
-            static_cast<uint8_t>(ex + 127);
-      }
+      const uint32_t sb = mxq::mx_row_block(y[i], codes);
+      *reinterpret_cast<uint2*>(codes_at) = codes;
+      if ((rc & 3) == 0) *scale_at = static_cast<uint8_t>(sb);
+      codes_at += code_step;
+      scale_at += scale_step;
     }
   }
   if (COL) {
-    float4* mine = reinterpret_cast<float4*>(col_amax + threadIdx.x * 8);
-    mine[0] = make_float4(cmax[0], cmax[1], cmax[2], cmax[3]);
-    mine[1] = make_float4(cmax[4], cmax[5], cmax[6], cmax[7]);
-    __syncthreads();
-    const int item_local = threadIdx.x / r8;
-    const int group0 = (item_local & ~3) * r8 + rc;   // the thread of the group's first item with this rank chunk
+    uint32_t am[4] = {0u, 0u, 0u, 0u};      // largest |x| of each rank, two ranks a word; ignores NaN
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const float4* other = reinterpret_cast<const float4*>(col_amax + (group0 + k * r8) * 8);
-      const float4 lo = other[0], hi = other[1];
-      cmax[0] = fmaxf(cmax[0], lo.x); cmax[1] = fmaxf(cmax[1], lo.y); cmax[2] = fmaxf(cmax[2], lo.z); cmax[3] = fmaxf(cmax[3], lo.w);
-      cmax[4] = fmaxf(cmax[4], hi.x); cmax[5] = fmaxf(cmax[5], hi.y); cmax[6] = fmaxf(cmax[6], hi.z); cmax[7] = fmaxf(cmax[7], hi.w);
+    for (int i = 0; i < 8; ++i) {
+      const uint32_t v[4] = {y[i].x, y[i].y, y[i].z, y[i].w};
+#pragma unroll
+      for (int e = 0; e < 4; ++e) am[e] = mxq::bf16x2_max(am[e], v[e] & 0x7fff7fffu);
+    }
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      am[e] = mxq::bf16x2_max(am[e], __shfl_xor_sync(0xffffffffu, am[e], 8));
+      am[e] = mxq::bf16x2_max(am[e], __shfl_xor_sync(0xffffffffu, am[e], 16));
     }
     const int64_t blk = item >> 2;                    // 32-row block of R
     const int64_t kb4 = R >> 7;                       // scale chunks per 128 ranks
-    // A rank owns P = 256 / r8 pieces of 8 bytes (one per item of the CTA), contiguous in the output. They are
-    // staged in shared memory, piece p of rank chunk rc at p ^ (2 * (rc % (P/2))) (pairs stay together and the
-    // stores of a half-warp spread over the banks), and leave as 16-byte stores in runs of 8 P bytes.
-    const int P = 256 / r8;
-    const int swz = (rc & (P / 2 - 1)) << 1;
+    uint8_t* scale_at = q.scales_col + ((rc >> 4) * kb4 + (blk >> 2)) * 512;
+    // A rank owns P pieces of 8 bytes (one per item of the CTA), contiguous in the output. They are staged in shared
+    // memory, piece p of rank chunk rc at p ^ (2 * (rc % (P/2))) (pairs stay together and the stores of a half-warp
+    // spread over the banks), and leave as 16-byte stores in runs of 8 P bytes.
+    const int piece = item_local ^ ((rc & (P / 2 - 1)) << 1);
 #pragma unroll
-    for (int e = 0; e < 8; ++e) {
-      const int ex = mxq::mx_exponent(fmaxf(cmax[e], mxq::kAmaxFloor));
-      const float inv = mxq::mx_inv_scale(ex);
-      float v[8];   // rank e of rows 0..7: half e % 2 of word e / 2 of each packed row
+    for (int e = 0; e < 4; ++e) {
+      const uint32_t sb0 = mxq::mx_scale_byte(am[e] & 0xffffu), sb1 = mxq::mx_scale_byte(am[e] >> 16);
+      const uint32_t inv2 = (mxq::mx_inv_bf16x2(sb0) & 0xffffu) | (mxq::mx_inv_bf16x2(sb1) & 0xffff0000u);
+      uint32_t lo[2], hi[2];   // codes of ranks 2 e and 2 e + 1, four rows a word
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const uint32_t w = reinterpret_cast<const uint32_t*>(&packed[i])[e >> 1];
-        v[i] = __uint_as_float((e & 1) ? (w & 0xffff0000u) : (w << 16));
+      for (int g = 0; g < 2; ++g) {
+        float a[4], b[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const uint4& r = y[4 * g + k];
+          const uint32_t v = mxq::bf16x2_mul(e == 0 ? r.x : e == 1 ? r.y : e == 2 ? r.z : r.w, inv2);
+          a[k] = __uint_as_float(v << 16);
+          b[k] = __uint_as_float(v & 0xffff0000u);
+        }
+        lo[g] = mxq::e4m3x2(a[0], a[1]) | (mxq::e4m3x2(a[2], a[3]) << 16);
+        hi[g] = mxq::e4m3x2(b[0], b[1]) | (mxq::e4m3x2(b[2], b[3]) << 16);
       }
-      uint2 codes;
-      codes.x = mxq::e4m3x2(v[0] * inv, v[1] * inv) | (mxq::e4m3x2(v[2] * inv, v[3] * inv) << 16);
-      codes.y = mxq::e4m3x2(v[4] * inv, v[5] * inv) | (mxq::e4m3x2(v[6] * inv, v[7] * inv) << 16);
-      const int col = rc * 8 + e;
-      stage[col * P + (item_local ^ swz)] = codes;
-      if ((item_local & 3) == 0)
-        q.scales_col[((col >> 7) * kb4 + (blk >> 2)) * 512 + mxq::tiled_offset(col & 127, static_cast<int>(blk & 3))] =
-            static_cast<uint8_t>(ex + 127);
+      const int col = rc * 8 + 2 * e;
+      stage[col * P + piece] = make_uint2(lo[0], lo[1]);
+      stage[(col + 1) * P + piece] = make_uint2(hi[0], hi[1]);
+      if (lane < 8) {
+        scale_at[mxq::tiled_offset(col & 127, static_cast<int>(blk & 3))] = static_cast<uint8_t>(sb0);
+        scale_at[mxq::tiled_offset((col + 1) & 127, static_cast<int>(blk & 3))] = static_cast<uint8_t>(sb1);
+      }
     }
     __syncthreads();
     const int64_t row0 = static_cast<int64_t>(blockIdx.x) * P * 8;   // first row of R this CTA covers
     const int half = P / 2;                                           // 16-byte units per rank
 #pragma unroll
-    for (int h = 0; h < 4; ++h) {
-      const int u = threadIdx.x + h * 256;          // 1024 units: rank u / half, unit u % half
+    for (int k = 0; k < 4; ++k) {
+      const int u = threadIdx.x + k * 256;          // 1024 units: rank u / half, unit u % half
       const int col = u / half, unit = u - col * half;
       const int s2 = ((col >> 3) & (half - 1)) << 1;
       const uint4 v = *reinterpret_cast<const uint4*>(&stage[col * P + ((2 * unit) ^ s2)]);
