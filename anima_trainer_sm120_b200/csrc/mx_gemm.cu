@@ -9,8 +9,8 @@
 // Two kernel families, both persistent and warp-specialised (warp 0 TMA producer, warp 1 MMA issuer, the
 // other warps epilogue), accumulating in tensor memory (fp32):
 //
-//  * mx_gemm2_kernel<BN> — the main one (M > 128 and N > 128): a cluster of two CTAs owns a 256 x 192 (K < 4096)
-//    or 256 x 256 tile and issues tcgen05.mma.cta_group::2 (M256 x N192|256 x K32); see the comment above it.
+//  * mx_gemm2_kernel<BN> — the main one (M > 128 and N > 128): a cluster of two CTAs owns a 256 x 192 or
+//    256 x 256 tile (see plan_pair) and issues tcgen05.mma.cta_group::2 (M256 x N192|256 x K32); see the comment above it.
 //  * mx_gemm_kernel<BN> — one CTA per 128 x BN tile (BN = 128 or 256) for small or narrow problems:
 //      warp 0  per K-block of 128 one 128x128 A box and one BNx128 B box (128-byte swizzle) plus the
 //              512-byte scale chunks (bulk copies), all completing on the stage's "full" mbarrier;
@@ -665,7 +665,7 @@ static_assert(kEpiHalves == 1 || kEpiHalves == 2, "one or two epilogue warps per
 // 32 KB, i.e. less shared-memory and L2 traffic (and energy) per flop, but the two buffers must share 32 columns
 // of tensor memory and every tile starts only after the epilogue has read those columns of the tile before it
 // (about 2000 idle cycles per tile, measured). The wide form wins once a tile holds enough K-blocks to pay for
-// that gap (K >= 4096 on a power-capped B200), the narrow form below.
+// that gap or saves a round (plan_pair), the narrow form otherwise.
 template <int BN>
 struct Cfg2 {
   static_assert(BN == 192 || BN == 256, "tile widths whose scale columns start at even tensor-memory offsets");
@@ -818,8 +818,8 @@ mx_gemm2_kernel(const __grid_constant__ SegMaps maps, const __grid_constant__ CU
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();  // 0 = leader
   const bool probe = p.clock_probe != nullptr;
-  const long long probe_cycles0 = clock64();
-  const uint64_t probe_ns0 = global_timer_ns();
+  const long long probe_cycles0 = probe ? clock64() : 0;
+  const uint64_t probe_ns0 = probe ? global_timer_ns() : 0;
   const int pair = blockIdx.x >> 1, num_pairs = gridDim.x >> 1;
 
   if (threadIdx.x == 0) {
@@ -1159,7 +1159,8 @@ mx_gemm2_kernel(const __grid_constant__ SegMaps maps, const __grid_constant__ CU
         }
       }
     }
-    if (issuer) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+    // the staging buffers must outlive the stores' reads; their writes are complete when the grid is
+    if (issuer) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
     if (probe && blockIdx.x == 0 && threadIdx.x == 64) p.clock_probe[6] += w_idle;
   }
 
@@ -1296,13 +1297,15 @@ int env_int(const char* name, int fallback) {
 // the whole problem when it has fewer tiles than pairs, may be split along K so that every pair ends at about
 // the same time instead of a few pairs running one more tile while the rest idle: the weight gradient
 // dW[2048, 2048] over K = 32768 is 88 tiles on 74 pairs, i.e. two rounds for 1.19 rounds of work.
-// The choice minimises the modelled finish time (unit: one K-block of a wide tile; a narrow tile costs 128 / width,
-// every item a constant, a split item a larger constant for its fp32 partial store, the finalize pass a
-// constant) over the number of splits; it depends on the shape and the SM count only, so results are
-// reproducible from call to call.
+// The choice minimises the modelled finish time over both tile widths and the number of splits; it depends on the
+// shape and the SM count only, so results are reproducible from call to call. Unit: one K-block of a 192-wide tile,
+// 0.254 us. A K-block of a 256-wide tile costs 1.09 of them, a tile 4 (192) or 7 (256) on top (the pipe waits for the
+// shared accumulator columns), a narrow tile's K-blocks 128 / width, a split item 7 more for its fp32 partial store,
+// the finalize pass 36.
 struct PairPlan {
   int pairs, n_wide, narrow, full_items, tail_tiles, tail_splits, tail_kbs, tail_shift, bn;
   int64_t ws_bytes;
+  double cost;
 };
 
 PairPlan plan_pair_uncached(int64_t M, int64_t N, int64_t K, bool allow_split, int sms, int kBN2) {
@@ -1316,11 +1319,11 @@ PairPlan plan_pair_uncached(int64_t M, int64_t N, int64_t K, bool allow_split, i
   const int n_tiles = pl.n_wide + pl.narrow, tiles = m_tiles * n_tiles;
   const int kb = static_cast<int>(ceil_div(K, BK));
   const int max_pairs = std::max(1, sms / 2);
-  const double kItem = 1.0, kSplitItem = 8.0, kFinalize = 36.0;   // the finalize launch measures 5 - 10 us, a K-block 0.27 us
+  const double kBlock = kBN2 == 256 ? 1.09 : 1.0, kItem = kBN2 == 256 ? 7.0 : 4.0, kSplitItem = kItem + 7.0, kFinalize = 36.0;
   auto tile_cost = [&](int tile, double frac) {
     int mt, nt;
     tile_coords_of(m_tiles, n_tiles, tile, mt, nt);
-    return (nt < pl.n_wide ? 1.0 : 128.0 / kBN2) * kb * frac;
+    return (nt < pl.n_wide ? kBlock : kBlock * 128.0 / kBN2) * kb * frac;
   };
 
   double best = 1e300;
@@ -1344,7 +1347,7 @@ PairPlan plan_pair_uncached(int64_t M, int64_t N, int64_t K, bool allow_split, i
     for (double l : load) finish = std::max(finish, l);
     if (splits > 1) finish += kFinalize;
     if (finish < best - 1e-9) {
-      best = finish;
+      best = pl.cost = finish;
       pl.pairs = pairs;
       pl.full_items = full_items;
       pl.tail_tiles = tail;
@@ -1367,27 +1370,31 @@ PairPlan plan_pair_uncached(int64_t M, int64_t N, int64_t K, bool allow_split, i
   return pl;
 }
 
-// Tile width for a problem: 256 when a tile holds at least 32 K-blocks (its start-up gap is then under a
-// tenth of the tile), else 192. ANIMA_MX_GEMM_BN = 192 / 256 forces one (read per call; for tests and tuning).
-int pair_tile_width(int64_t K) {
-  const int forced = env_int("ANIMA_MX_GEMM_BN", 0);
-  if (forced == 192 || forced == 256) return forced;
-  return K >= 4096 ? 256 : 192;
-}
+// Tile width: 256 when a tile holds at least 32 K-blocks (its start-up gap is then under a tenth of the tile). Below
+// that a tile of either width costs about the same per column, and 256 pays where it needs fewer rounds of tiles: it is
+// taken when the modelled time is at least 15 % shorter. us, 192 against 256: [4096, 2048, 2048] 22.1 / 19.9 (three
+// rounds, two), [2048, 2048, 1024] 12.7 / 10.7 (two, one), [8192, 2048, 1024] 23.2 / 23.5, [4032, 6144, 2048] 44.0 /
+// 44.9, [512, 2048, 1024] 9.0 / 10.1, [4032, 2048, 6144] 46.0 / 39.5.
+constexpr double kWideGain = 0.85;
 
 PairPlan plan_pair(int64_t M, int64_t N, int64_t K, bool allow_split) {
   const int sms = sm_count();
-  const int bn = pair_tile_width(K);
+  const int forced = env_int("ANIMA_MX_GEMM_BN", 0);   // 192 / 256 forces a tile width (read per call; for tests and tuning)
+  const int bn = forced == 192 || forced == 256 ? forced : 0;
   const int narrow = env_int("ANIMA_MX_GEMM_NARROW", 1), tail = env_int("ANIMA_MX_GEMM_TAIL", 1);
   using Key = std::tuple<int64_t, int64_t, int64_t, int, int>;
   static std::mutex mu;
   static std::map<Key, PairPlan> cache;
-  const Key key{M, N, K, sms, (allow_split ? 1 : 0) | (narrow ? 2 : 0) | (tail ? 4 : 0) | (bn == 256 ? 8 : 0)};
+  const Key key{M, N, K, sms, (allow_split ? 1 : 0) | (narrow ? 2 : 0) | (tail ? 4 : 0) | bn << 3};
   std::lock_guard<std::mutex> lock(mu);
   auto it = cache.find(key);
   if (it != cache.end()) return it->second;
   if (cache.size() > 4096) cache.clear();
-  const PairPlan pl = plan_pair_uncached(M, N, K, allow_split, sms, bn);
+  PairPlan pl = plan_pair_uncached(M, N, K, allow_split, sms, bn ? bn : K >= 4096 ? 256 : 192);
+  if (!bn && K < 4096) {
+    const PairPlan wide = plan_pair_uncached(M, N, K, allow_split, sms, 256);
+    if (wide.cost < kWideGain * pl.cost) pl = wide;
+  }
   cache.emplace(key, pl);
   return pl;
 }
