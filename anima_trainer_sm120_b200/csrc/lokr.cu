@@ -114,9 +114,25 @@ __global__ void __launch_bounds__(256) lokr_merge_only_kernel(const MergeLoader<
 constexpr int kMaxFactor = 8;
 constexpr int kKronThreads = 32 * kMaxFactor;
 constexpr int kKronCtasPerSm = 4;
+// A cluster of four CTAs sums its dw1 terms over distributed shared memory and writes one partial of 64 floats: at most
+// one per 128 items, which is what the workspace holds.
+constexpr int kKronCluster = 4;
 
-int64_t kron_blocks(int64_t vp, int64_t vq) {
-  return std::min<int64_t>(ceil_div(vp * (vq / 8), 32), static_cast<int64_t>(kKronCtasPerSm) * sm_count());
+int64_t kron_partials(int64_t vp, int64_t vq) { return ceil_div(vp * (vq / 8), 32 * kKronCluster); }
+int64_t kron_clusters(int64_t vp, int64_t vq) {
+  return std::min<int64_t>(kron_partials(vp, vq),
+                           ceil_div(static_cast<int64_t>(kKronCtasPerSm) * sm_count(), static_cast<int64_t>(kKronCluster)));
+}
+
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ float cluster_peer(const float* own, uint32_t rank) {   // the same variable in CTA `rank`
+  uint32_t addr = static_cast<uint32_t>(__cvta_generic_to_shared(own));
+  float v;
+  asm volatile("mapa.shared::cluster.u32 %0, %0, %1;" : "+r"(addr) : "r"(rank));
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
+  return v;
 }
 
 template <class T>
@@ -131,7 +147,7 @@ __device__ __forceinline__ void load8_f2(const T* src, f2 (&v)[4]) {
 }
 
 template <class G, class F>
-__global__ void __launch_bounds__(kKronThreads, kKronCtasPerSm)
+__global__ void __cluster_dims__(kKronCluster, 1, 1) __launch_bounds__(kKronThreads, kKronCtasPerSm)
 kron_backward_kernel(const G* __restrict__ dw, const F* __restrict__ w1, const F* __restrict__ w2,
                      float alpha, int64_t K, int vp, int vq, int up, int uq, float* __restrict__ dw2,
                      float* __restrict__ partial) {
@@ -186,11 +202,21 @@ kron_backward_kernel(const G* __restrict__ dw, const F* __restrict__ w1, const F
     if (at < static_cast<int64_t>(items) * 8) dw2[at] = alpha * sum;
     __syncthreads();
   }
+  __shared__ float sums[kMaxFactor * kMaxFactor];
 #pragma unroll
   for (int j = 0; j < kMaxFactor; ++j) {
     const float s = warp_sum(t1[j]);
-    if (lane == 0) partial[blockIdx.x * (kMaxFactor * kMaxFactor) + i * kMaxFactor + j] = s;
+    if (lane == 0) sums[i * kMaxFactor + j] = s;
   }
+  __syncthreads();
+  cluster_sync();
+  if (blockIdx.x % kKronCluster == 0 && t < kMaxFactor * kMaxFactor) {
+    float s = sums[t];
+#pragma unroll
+    for (uint32_t r = 1; r < kKronCluster; ++r) s += cluster_peer(sums + t, r);
+    partial[blockIdx.x / kKronCluster * (kMaxFactor * kMaxFactor) + t] = s;
+  }
+  cluster_sync();   // no CTA leaves while its sums may be read
 }
 
 __global__ void kron_backward_finalize_kernel(const float* __restrict__ partial, int blocks, float alpha,
@@ -274,7 +300,7 @@ extern "C" int anima_lokr_merge_quantize(const void* w, const void* w1, const vo
 extern "C" int64_t anima_lokr_kron_backward_workspace_bytes(int64_t N, int64_t K, int64_t up,
                                                             int64_t uq) {
   if (N <= 0 || K <= 0 || up <= 0 || uq <= 0 || N % up || K % uq || (K / uq) % 8) return ANIMA_E_SHAPE;
-  return kron_blocks(N / up, K / uq) * kMaxFactor * kMaxFactor * static_cast<int64_t>(sizeof(float));
+  return kron_partials(N / up, K / uq) * kMaxFactor * kMaxFactor * static_cast<int64_t>(sizeof(float));
 }
 
 extern "C" int anima_lokr_kron_backward(const void* dw, int dw_is_fp32, const void* w1, const void* w2,
@@ -293,7 +319,7 @@ extern "C" int anima_lokr_kron_backward(const void* dw, int dw_is_fp32, const vo
                 "lokr_kron_backward: workspace of %lld bytes required, got %lld", (long long)need,
                 (long long)workspace_bytes);
   const int vp = static_cast<int>(N / up), vq = static_cast<int>(K / uq);
-  const int blocks = static_cast<int>(kron_blocks(vp, vq));
+  const int partials = static_cast<int>(kron_clusters(vp, vq)), blocks = partials * kKronCluster;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   float* ws = static_cast<float*>(workspace);
 #define ANIMA_KRON(G, F)                                                                            \
@@ -307,7 +333,7 @@ extern "C" int anima_lokr_kron_backward(const void* dw, int dw_is_fp32, const vo
   }
 #undef ANIMA_KRON
   ANIMA_CHECK_LAUNCH("lokr_kron_backward");
-  kron_backward_finalize_kernel<<<1, kFinalizeThreads, 0, s>>>(ws, blocks, alpha, (int)up, (int)uq, dw1);
+  kron_backward_finalize_kernel<<<1, kFinalizeThreads, 0, s>>>(ws, partials, alpha, (int)up, (int)uq, dw1);
   ANIMA_CHECK_LAUNCH("lokr_kron_backward finalize");
   return ANIMA_OK;
 }
