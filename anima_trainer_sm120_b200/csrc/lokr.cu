@@ -152,6 +152,10 @@ kron_backward_kernel(const G* __restrict__ dw, const F* __restrict__ w1, const F
                      float alpha, int64_t K, int vp, int vq, int up, int uq, float* __restrict__ dw2,
                      float* __restrict__ partial) {
   __shared__ __align__(16) float acc_s[kMaxFactor][32 * 8];
+  after_previous();
+  dw = after_previous(dw);
+  w1 = after_previous(w1);
+  w2 = after_previous(w2);
   const int t = threadIdx.x, lane = t & 31, i = t >> 5;
   const int vq8 = vq / 8, items = vp * vq8;
   float w1r[kMaxFactor], t1[kMaxFactor];
@@ -221,6 +225,8 @@ kron_backward_kernel(const G* __restrict__ dw, const F* __restrict__ w1, const F
 
 __global__ void kron_backward_finalize_kernel(const float* __restrict__ partial, int blocks, float alpha,
                                               int up, int uq, float* __restrict__ dw1) {
+  after_previous();
+  partial = after_previous(partial);
   const float s = sum_partials_64(partial, blocks);
   const int i = threadIdx.x / kMaxFactor, j = threadIdx.x % kMaxFactor;
   if (threadIdx.x < kMaxFactor * kMaxFactor && i < up && j < uq) dw1[i * uq + j] = alpha * s;
@@ -253,11 +259,11 @@ int launch_merge(const void* w, const void* w1, const void* w2, float alpha, int
   QuantParams p{N, K, codes_row, scales_row, codes_colT, scales_col, scale_layout == ANIMA_SCALES_TILED};
   const dim3 grid(static_cast<unsigned>(ceil_div(K, kTile)), static_cast<unsigned>(ceil_div(N, kTile)));
   if (row && col)
-    mx_quantize_kernel<true, true><<<grid, kThreads, 0, s>>>(p, load);
+    launch_after(mx_quantize_kernel<true, true, MergeLoader<F>>, grid, kThreads, 0, s, p, load);
   else if (row)
-    mx_quantize_kernel<true, false><<<grid, kThreads, 0, s>>>(p, load);
+    launch_after(mx_quantize_kernel<true, false, MergeLoader<F>>, grid, kThreads, 0, s, p, load);
   else
-    mx_quantize_kernel<false, true><<<grid, kThreads, 0, s>>>(p, load);
+    launch_after(mx_quantize_kernel<false, true, MergeLoader<F>>, grid, kThreads, 0, s, p, load);
   return ANIMA_OK;
 }
 
@@ -323,7 +329,7 @@ extern "C" int anima_lokr_kron_backward(const void* dw, int dw_is_fp32, const vo
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   float* ws = static_cast<float*>(workspace);
 #define ANIMA_KRON(G, F)                                                                            \
-  kron_backward_kernel<G, F><<<blocks, kKronThreads, 0, s>>>(                                       \
+  launch_after(kron_backward_kernel<G, F>, blocks, kKronThreads, 0, s,                              \
       static_cast<const G*>(dw), static_cast<const F*>(w1), static_cast<const F*>(w2), alpha, K, vp, \
       vq, (int)up, (int)uq, dw2, ws)
   if (dw_is_fp32) {
@@ -333,7 +339,7 @@ extern "C" int anima_lokr_kron_backward(const void* dw, int dw_is_fp32, const vo
   }
 #undef ANIMA_KRON
   ANIMA_CHECK_LAUNCH("lokr_kron_backward");
-  kron_backward_finalize_kernel<<<1, kFinalizeThreads, 0, s>>>(ws, partials, alpha, (int)up, (int)uq, dw1);
+  launch_after(kron_backward_finalize_kernel, 1, kFinalizeThreads, 0, s, ws, partials, alpha, (int)up, (int)uq, dw1);
   ANIMA_CHECK_LAUNCH("lokr_kron_backward finalize");
   return ANIMA_OK;
 }

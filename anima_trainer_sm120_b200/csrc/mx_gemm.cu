@@ -410,6 +410,7 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  after_previous();
   const uint32_t tmem_base = tmem_base_slot;
 
   const int total_items = p.m_tiles * p.n_tiles * p.splits;
@@ -583,6 +584,7 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
 
 // C = sum over splits (in index order, so the result is reproducible) of partial[s] (+ bias), 4 columns per thread.
 __global__ void __launch_bounds__(256) splitk_finalize_kernel(const GemmParams p) {
+  after_previous();
   const int64_t n4 = p.N / 4, total = static_cast<int64_t>(p.M) * n4, plane = static_cast<int64_t>(p.M) * p.N;
   for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < total;
        i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
@@ -854,6 +856,7 @@ mx_gemm2_kernel(const __grid_constant__ SegMaps maps, const __grid_constant__ CU
   __syncthreads();
   cluster_sync_all();  // both CTAs' barriers are initialised before any remote arrive or TMA completion
   tc_fence_after();
+  after_previous();
   // The kernel owns all 512 columns, so the allocation can only start at column 0; using the constant keeps
   // every tensor-memory address warp-uniform. Anything else is reported through *status and nothing runs.
   const uint32_t tmem_alloc = tmem_base_slot;
@@ -1187,6 +1190,7 @@ mx_gemm2_kernel(const __grid_constant__ SegMaps maps, const __grid_constant__ CU
 // C tile = sum over the K-range partials of a tail tile, in index order (reproducible), then the epilogue
 // (alpha, bias, residual, rounding). One thread per 4 columns of a 256 x pair_bn tile.
 __global__ void __launch_bounds__(256) pair_tail_finalize_kernel(const GemmParams p) {
+  after_previous();
   const int kBN2 = p.pair_bn;
   const int kPerRow = kBN2 / 4, kPerTile = 256 * kPerRow, kTileElems = 256 * kBN2;
   const int64_t total = static_cast<int64_t>(p.tail_tiles) * kPerTile;
@@ -1437,6 +1441,9 @@ int launch_pair(const Segment* segs, int n_segs, GemmParams p, void* workspace, 
                       : launch_pair_width<192>(segs, n_segs, p, pl, workspace, delta, s);
 }
 
+// Launches of at most this many K-blocks a CTA (pair), about 50 us, overlap the kernel ahead of them (see launch_after).
+constexpr int64_t kOverlapBlocks = 192;
+
 template <int kBN2>
 int launch_pair_width(const Segment* segs, int n_segs, GemmParams p, const PairPlan& pl, void* workspace,
                       const DeltaOperands& delta, cudaStream_t s) {
@@ -1498,19 +1505,22 @@ int launch_pair_width(const Segment* segs, int n_segs, GemmParams p, const PairP
   cfg.blockDim = dim3(kThreads2);
   cfg.dynamicSmemBytes = C2::kSmemBytes;
   cfg.stream = s;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;   // see launch_after
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = 2;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  const int64_t k_blocks = static_cast<int64_t>(p.m_tiles) * p.n_tiles * p.k_blocks;
+  cfg.numAttrs = k_blocks <= kOverlapBlocks * pl.pairs ? 2 : 1;
   const cudaError_t rc = cudaLaunchKernelEx(&cfg, mx_gemm2_kernel<kBN2>, maps, mc, mp, mpl, md, mplsf, mdsf, p);
   ANIMA_REQUIRE(rc == cudaSuccess, ANIMA_E_CUDA, "mx_gemm: cluster launch failed: %s", cudaGetErrorString(rc));
   if (pl.ws_bytes) {
     const int64_t threads = static_cast<int64_t>(pl.tail_tiles) * 256 * (kBN2 / 4);
-    pair_tail_finalize_kernel<<<static_cast<unsigned>(std::min<int64_t>(ceil_div(threads, 256), 8LL * sm_count())), 256, 0,
-                                s>>>(p);
+    launch_after(pair_tail_finalize_kernel, static_cast<unsigned>(std::min<int64_t>(ceil_div(threads, 256), 8LL * sm_count())),
+                 256, 0, s, p);
     ANIMA_CHECK_LAUNCH("mx_gemm K-split tail finalize");
   }
   return ANIMA_OK;
@@ -1534,12 +1544,13 @@ int launch(const CUtensorMap& ma, const CUtensorMap& mb, GemmParams p, cudaStrea
   p.n_tiles = static_cast<int>(ceil_div(p.N, BN));
   const int items = p.m_tiles * p.n_tiles * p.splits;
   const int grid = std::min(items, sm_count());
-  mx_gemm_kernel<BN, EPI><<<grid, 64 + 32 * EPI, Cfg<BN>::kSmemBytes, s>>>(ma, mb, p);
+  const bool overlap = static_cast<int64_t>(p.m_tiles) * p.n_tiles * p.k_blocks <= kOverlapBlocks * grid;
+  launch_after(overlap, mx_gemm_kernel<BN, EPI>, grid, 64 + 32 * EPI, Cfg<BN>::kSmemBytes, s, ma, mb, p);
   ANIMA_CHECK_LAUNCH("mx_gemm");
   if (p.splits > 1) {
     const int64_t groups = static_cast<int64_t>(p.M) * (p.N / 4);
-    splitk_finalize_kernel<<<static_cast<unsigned>(std::min<int64_t>(ceil_div(groups, 256), 4LL * sm_count())), 256, 0,
-                             s>>>(p);
+    launch_after(splitk_finalize_kernel, static_cast<unsigned>(std::min<int64_t>(ceil_div(groups, 256), 4LL * sm_count())), 256, 0,
+                 s, p);
     ANIMA_CHECK_LAUNCH("mx_gemm split-K finalize");
   }
   return ANIMA_OK;

@@ -280,6 +280,8 @@ __global__ void mx_dequantize_kernel(const uint8_t* __restrict__ codes,
 
 __global__ void mx_scales_retile_kernel(const uint8_t* __restrict__ plain, int64_t rows, int64_t kb,
                                         uint8_t* __restrict__ tiled) {
+  after_previous();
+  plain = after_previous(plain);
   const int64_t kb4 = ceil_div(kb, 4);
   const int64_t total = ceil_div(rows, 128) * kb4 * 512;
   for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < total;
@@ -301,6 +303,8 @@ __global__ void mx_scales_retile_kernel(const uint8_t* __restrict__ plain, int64
 template <class Idx>
 __global__ void mx_scales_regroup_kernel(const uint8_t* __restrict__ in, Idx kb_in, Idx rows_out, Idx kb_out, Idx total,
                                          uint8_t* __restrict__ out) {
+  after_previous();
+  in = after_previous(in);
   const Idx kb4_out = (kb_out + 3) / 4, kb4_in = (kb_in + 3) / 4;
   for (Idx i = blockIdx.x * static_cast<Idx>(blockDim.x) + threadIdx.x; i < total;
        i += static_cast<Idx>(gridDim.x) * blockDim.x) {
@@ -324,6 +328,8 @@ __global__ void mx_scales_regroup_kernel(const uint8_t* __restrict__ in, Idx kb_
 // accesses). rows_out % 128 may be anything: padded rows are written as zero.
 __global__ void mx_scales_regroup_words_kernel(const uint32_t* __restrict__ in, uint32_t kb4_in, uint32_t rows_out,
                                                uint32_t kb4_out, uint32_t total_words, uint32_t* __restrict__ out) {
+  after_previous();
+  in = after_previous(in);
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < total_words; i += gridDim.x * blockDim.x) {
     const uint32_t chunk = i >> 7, w = i & 127;                 // 128 words per chunk; word w = bytes 4w .. 4w+3
     const uint32_t r_in = (w & 3) * 32 + (w >> 2);              // tiled_offset(r, 0) / 4 = (r % 32) * 4 + r / 32
@@ -405,11 +411,11 @@ int launch_quantize(const char* who, const Loader& load, int64_t rows, int64_t c
   const dim3 grid(static_cast<unsigned>(ceil_div(cols, kTile)), static_cast<unsigned>(ceil_div(rows, kTile)));
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (row && col)
-    mx_quantize_kernel<true, true><<<grid, kThreads, 0, s>>>(p, load);
+    launch_after(mx_quantize_kernel<true, true, Loader>, grid, kThreads, 0, s, p, load);
   else if (row)
-    mx_quantize_kernel<true, false><<<grid, kThreads, 0, s>>>(p, load);
+    launch_after(mx_quantize_kernel<true, false, Loader>, grid, kThreads, 0, s, p, load);
   else
-    mx_quantize_kernel<false, true><<<grid, kThreads, 0, s>>>(p, load);
+    launch_after(mx_quantize_kernel<false, true, Loader>, grid, kThreads, 0, s, p, load);
   ANIMA_CHECK_LAUNCH(who);
   return ANIMA_OK;
 }
@@ -448,7 +454,8 @@ int launch_tma(const CUtensorMap& map, const QuantParams& p, const Loader& load,
   });
   ANIMA_REQUIRE(attr_rc == cudaSuccess, ANIMA_E_CUDA, "mx_quantize: cannot reserve %d bytes of shared memory: %s",
                 kBytes, cudaGetErrorString(attr_rc));
-  mx_quantize_tma_kernel<ROW, COL, Loader><<<grid, kThreads, kBytes, s>>>(map, p, load);
+  const bool overlap = ceil_div(p.rows, static_cast<int64_t>(kTile)) * ceil_div(p.cols, static_cast<int64_t>(kTile)) <= 8LL * sm_count();
+  launch_after(overlap, mx_quantize_tma_kernel<ROW, COL, Loader>, grid, kThreads, kBytes, s, map, p, load);
   ANIMA_CHECK_LAUNCH("mx_quantize (TMA)");
   return ANIMA_OK;
 }
@@ -588,8 +595,7 @@ extern "C" int anima_mx_scales_retile(const uint8_t* plain, int64_t rows, int64_
   if (rows == 0 || k == 0) return ANIMA_OK;
   const int64_t total = anima_mx_scales_bytes(rows, k, ANIMA_SCALES_TILED);
   const int blocks = static_cast<int>(std::min<int64_t>(ceil_div(total, 256), sm_count() * 16));
-  mx_scales_retile_kernel<<<blocks, 256, 0, static_cast<cudaStream_t>(stream)>>>(plain, rows, k / 32,
-                                                                                 tiled);
+  launch_after(mx_scales_retile_kernel, blocks, 256, 0, static_cast<cudaStream_t>(stream), plain, rows, k / 32, tiled);
   ANIMA_CHECK_LAUNCH("mx_scales_retile");
   return ANIMA_OK;
 }
@@ -611,21 +617,18 @@ extern "C" int anima_mx_scales_regroup(const uint8_t* tiled_in, int64_t rows_in,
       (reinterpret_cast<uintptr_t>(tiled_out) & 3) == 0) {
     const uint32_t words = static_cast<uint32_t>(total / 4);
     const int wblocks = static_cast<int>(std::min<int64_t>(ceil_div(static_cast<int64_t>(words), 256), sm_count() * 16));
-    mx_scales_regroup_words_kernel<<<wblocks, 256, 0, s>>>(reinterpret_cast<const uint32_t*>(tiled_in),
-                                                           static_cast<uint32_t>(k_in / 128), static_cast<uint32_t>(rows_out),
-                                                           static_cast<uint32_t>(k_out / 128), words,
-                                                           reinterpret_cast<uint32_t*>(tiled_out));
+    launch_after(mx_scales_regroup_words_kernel, wblocks, 256, 0, s, reinterpret_cast<const uint32_t*>(tiled_in),
+                 static_cast<uint32_t>(k_in / 128), static_cast<uint32_t>(rows_out), static_cast<uint32_t>(k_out / 128), words,
+                 reinterpret_cast<uint32_t*>(tiled_out));
     ANIMA_CHECK_LAUNCH("mx_scales_regroup");
     return ANIMA_OK;
   }
   // 32-bit indices when the padded extents of both tilings (and r * kb_out + b for padded r) stay below 2^31
   if (small)
-    mx_scales_regroup_kernel<uint32_t><<<blocks, 256, 0, s>>>(tiled_in, static_cast<uint32_t>(k_in / 32),
-                                                               static_cast<uint32_t>(rows_out),
-                                                               static_cast<uint32_t>(k_out / 32),
-                                                               static_cast<uint32_t>(total), tiled_out);
+    launch_after(mx_scales_regroup_kernel<uint32_t>, blocks, 256, 0, s, tiled_in, static_cast<uint32_t>(k_in / 32),
+                 static_cast<uint32_t>(rows_out), static_cast<uint32_t>(k_out / 32), static_cast<uint32_t>(total), tiled_out);
   else
-    mx_scales_regroup_kernel<int64_t><<<blocks, 256, 0, s>>>(tiled_in, k_in / 32, rows_out, k_out / 32, total, tiled_out);
+    launch_after(mx_scales_regroup_kernel<int64_t>, blocks, 256, 0, s, tiled_in, k_in / 32, rows_out, k_out / 32, total, tiled_out);
   ANIMA_CHECK_LAUNCH("mx_scales_regroup");
   return ANIMA_OK;
 }

@@ -210,6 +210,7 @@ __global__ void __launch_bounds__(kThreads, COL ? 3 : 4) mx_quantize_kernel(cons
   __shared__ __align__(16) uint8_t sc_row[ROW ? 512 : 16];
   __shared__ __align__(16) uint8_t sc_col[COL ? 512 : 16];
 
+  after_previous();
   const int t = threadIdx.x;
   const int64_t tile_r = static_cast<int64_t>(blockIdx.y) * kTile;
   const int64_t tile_c = static_cast<int64_t>(blockIdx.x) * kTile;

@@ -45,6 +45,7 @@ mx_quantize_tma_kernel(const __grid_constant__ CUtensorMap map_x, const QuantPar
   __shared__ __align__(16) uint8_t sc_row[ROW ? 512 : 16];
   __shared__ __align__(16) uint8_t sc_col[COL ? 512 : 16];
 
+  after_previous();
   const int t = threadIdx.x;
   // dynamic shared memory: the loader's table first (its lookups pack two addresses into 16-bit halves, so it
   // must sit low), then the two stages

@@ -109,6 +109,10 @@ __global__ void __launch_bounds__(kThreads, 2)
 rmsnorm_rope_fwd_kernel(const __nv_bfloat16* __restrict__ x, const void* __restrict__ w, const float* __restrict__ cos_tab,
                         const float* __restrict__ sin_tab, float eps, int64_t tokens, int heads, int heads_per_group,
                         int64_t seq_len, __nv_bfloat16* __restrict__ out, float* __restrict__ rstd_out) {
+  after_previous();
+  w = after_previous(w);
+  cos_tab = after_previous(cos_tab);
+  sin_tab = after_previous(sin_tab);
   const int l = threadIdx.x & (kLanesPerToken - 1);
   const int64_t token = static_cast<int64_t>(blockIdx.x) * kTokensPerCta + threadIdx.x / kLanesPerToken;
   if (token >= tokens) return;   // the eight lanes of a token leave together; shuffles below stay inside them
@@ -167,6 +171,10 @@ rmsnorm_rope_bwd_kernel(const __nv_bfloat16* __restrict__ dout, const __nv_bfloa
                         const void* __restrict__ w, const float* __restrict__ cos_tab, const float* __restrict__ sin_tab,
                         const float* __restrict__ rstd_in, int64_t tokens, int heads, int heads_per_group, int64_t seq_len,
                         __nv_bfloat16* __restrict__ dx) {
+  after_previous();
+  w = after_previous(w);
+  cos_tab = after_previous(cos_tab);
+  sin_tab = after_previous(sin_tab);
   const int l = threadIdx.x & (kLanesPerToken - 1);
   const int64_t token = static_cast<int64_t>(blockIdx.x) * kTokensPerCta + threadIdx.x / kLanesPerToken;
   if (token >= tokens) return;
@@ -189,6 +197,7 @@ rmsnorm_rope_bwd_kernel(const __nv_bfloat16* __restrict__ dout, const __nv_bfloa
   };
 #pragma unroll
   for (int i = 0; i < kBwdStages - 1; ++i) start(h0 + i, i);
+  rstd_in = after_previous(rstd_in);
   float rstd_next = rstd_in[token * heads + h0];
   int slot = 0;
 #pragma unroll 1
@@ -268,7 +277,7 @@ extern "C" int anima_rmsnorm_rope_fwd_ex(const void* x, const void* weight, int 
   const auto* xp = static_cast<const __nv_bfloat16*>(x);
   auto* op = static_cast<__nv_bfloat16*>(out);
   constexpr int kSmem = kFwdStages * 2 * kThreads * 16;
-  auto go = [&](auto kernel) { kernel<<<grid, kThreads, kSmem, s>>>(xp, weight, cos_tab, sin_tab, eps, tokens, (int)heads, hpg, seq_len, op, rstd); };
+  auto go = [&](auto kernel) { launch_after(kernel, grid, kThreads, kSmem, s, xp, weight, cos_tab, sin_tab, eps, tokens, (int)heads, hpg, seq_len, op, rstd); };
   if (cos_tab) weight_is_bf16 ? go(rmsnorm_rope_fwd_kernel<true, true>) : go(rmsnorm_rope_fwd_kernel<true, false>);
   else weight_is_bf16 ? go(rmsnorm_rope_fwd_kernel<false, true>) : go(rmsnorm_rope_fwd_kernel<false, false>);
   ANIMA_CHECK_LAUNCH("rmsnorm_rope_fwd");
@@ -300,7 +309,7 @@ extern "C" int anima_rmsnorm_rope_bwd_ex(const void* dout, const void* x, const 
   });
   ANIMA_REQUIRE(rc == cudaSuccess, ANIMA_E_CUDA, "rmsnorm_rope_bwd: cannot reserve %d bytes of shared memory: %s", kSmem,
                 cudaGetErrorString(rc));
-  auto go = [&](auto kernel) { kernel<<<grid, kThreads, kSmem, s>>>(gp, xp, weight, cos_tab, sin_tab, rstd, tokens, (int)heads, hpg, seq_len, dp); };
+  auto go = [&](auto kernel) { launch_after(kernel, grid, kThreads, kSmem, s, gp, xp, weight, cos_tab, sin_tab, rstd, tokens, (int)heads, hpg, seq_len, dp); };
   if (cos_tab) weight_is_bf16 ? go(rmsnorm_rope_bwd_kernel<true, true>) : go(rmsnorm_rope_bwd_kernel<true, false>);
   else weight_is_bf16 ? go(rmsnorm_rope_bwd_kernel<false, true>) : go(rmsnorm_rope_bwd_kernel<false, false>);
   ANIMA_CHECK_LAUNCH("rmsnorm_rope_bwd");

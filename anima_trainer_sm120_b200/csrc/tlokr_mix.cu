@@ -66,6 +66,9 @@ rank_mix_kernel(const __nv_bfloat16* __restrict__ hidden, const __nv_bfloat16* _
                 const __nv_bfloat16* __restrict__ mask, int64_t total, int64_t n_per_batch, int r8,
                 __nv_bfloat16* __restrict__ out) {
   __shared__ __align__(16) f2 w[64];
+  after_previous();
+  c = after_previous(c);
+  mask = after_previous(mask);
   const int64_t idx = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
   const int64_t row = idx / r8;  // (b, n) flattened
   const int rc = static_cast<int>(idx - row * r8);
@@ -118,6 +121,9 @@ rank_mix_quant_kernel(const __nv_bfloat16* __restrict__ hidden, const __nv_bfloa
                       __nv_bfloat16* __restrict__ out, const MixCodes q) {
   __shared__ __align__(16) f2 w[64];
   __shared__ __align__(16) uint2 stage[COL ? 2048 : 2];      // transposed codes of the CTA: [rank][item] x 8 bytes
+  after_previous();
+  c = after_previous(c);
+  mask = after_previous(mask);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, groups = r8 >> 3;
   const int P = 256 / r8;                                    // items of the CTA, a multiple of 4
   const int item_local = (warp / groups) * 4 + (lane >> 3), rc = (warp % groups) * 8 + (lane & 7);
@@ -244,6 +250,8 @@ rank_mix_wgrad_kernel(const __nv_bfloat16* __restrict__ grad, const __nv_bfloat1
                       const __nv_bfloat16* __restrict__ mask, int64_t items, int64_t n_per_batch, int rank,
                       float* __restrict__ partial) {
   __shared__ float red[kWgradWarps][64];
+  after_previous();
+  mask = after_previous(mask);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int g = lane >> 2, t = lane & 3;
   float acc[4] = {0.f, 0.f, 0.f, 0.f};
@@ -287,6 +295,8 @@ rank_mix_wgrad_kernel(const __nv_bfloat16* __restrict__ grad, const __nv_bfloat1
 
 __global__ void __launch_bounds__(kFinalizeThreads)
 rank_mix_wgrad_finalize_kernel(const float* __restrict__ partial, int blocks, float* __restrict__ dc) {
+  after_previous();
+  partial = after_previous(partial);
   const float s = sum_partials_64(partial, blocks);
   if (threadIdx.x < 64) dc[threadIdx.x] = s;
 }
@@ -319,7 +329,7 @@ extern "C" int anima_tlokr_rank_mix(const void* hidden, const void* c, const voi
   const auto* mp = static_cast<const __nv_bfloat16*>(mask);
   auto* op = static_cast<__nv_bfloat16*>(out);
   const int r8 = static_cast<int>(rank / 8);
-#define ANIMA_MIX(T, M) rank_mix_kernel<T, M><<<grid, 256, 0, s>>>(hp, cp, mp, total, n_per_batch, r8, op)
+#define ANIMA_MIX(T, M) launch_after(rank_mix_kernel<T, M>, grid, 256, 0, s, hp, cp, mp, total, n_per_batch, r8, op)
   if (transpose) {
     if (mask) ANIMA_MIX(true, true); else ANIMA_MIX(true, false);
   } else {
@@ -358,7 +368,7 @@ static int rank_mix_quant_impl(const void* hidden, const void* c, const void* ma
   ANIMA_REQUIRE(!planes || (codes_row && items % 128 == 0), ANIMA_E_SHAPE,
                 "tlokr_rank_mix_quant_planes: needs the row form and batch * n = %lld a multiple of 128", (long long)items);
   const MixCodes q{codes_row, scales_row, codes_colT, scales_col, planes ? items : 0};
-#define ANIMA_MIXQ(T, M, R, C) rank_mix_quant_kernel<T, M, R, C><<<grid, 256, 0, s>>>(hp, cp, mp, items, n_per_batch, r8, op, q)
+#define ANIMA_MIXQ(T, M, R, C) launch_after(rank_mix_quant_kernel<T, M, R, C>, grid, 256, 0, s, hp, cp, mp, items, n_per_batch, r8, op, q)
 #define ANIMA_MIXQ_FORMS(T, M)                                     \
   do {                                                             \
     if (codes_row && codes_colT) ANIMA_MIXQ(T, M, true, true);     \
@@ -422,11 +432,11 @@ extern "C" int anima_tlokr_rank_mix_wgrad(const void* grad_mixed, const void* hi
   const auto* mp = static_cast<const __nv_bfloat16*>(mask);
   const int r = static_cast<int>(rank);
   if (mask)
-    rank_mix_wgrad_kernel<true><<<blocks, kWgradThreads, 0, s>>>(gp, hp, mp, items, n_per_batch, r, ws);
+    launch_after(rank_mix_wgrad_kernel<true>, blocks, kWgradThreads, 0, s, gp, hp, mp, items, n_per_batch, r, ws);
   else
-    rank_mix_wgrad_kernel<false><<<blocks, kWgradThreads, 0, s>>>(gp, hp, mp, items, n_per_batch, r, ws);
+    launch_after(rank_mix_wgrad_kernel<false>, blocks, kWgradThreads, 0, s, gp, hp, mp, items, n_per_batch, r, ws);
   ANIMA_CHECK_LAUNCH("tlokr_rank_mix_wgrad");
-  rank_mix_wgrad_finalize_kernel<<<1, kFinalizeThreads, 0, s>>>(ws, blocks, dc);
+  launch_after(rank_mix_wgrad_finalize_kernel, 1, kFinalizeThreads, 0, s, ws, blocks, dc);
   ANIMA_CHECK_LAUNCH("tlokr_rank_mix_wgrad finalize");
   return ANIMA_OK;
 }
