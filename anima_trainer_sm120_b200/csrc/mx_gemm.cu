@@ -37,6 +37,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "f32x2.cuh"
 #include "mx_quantize_tile.cuh"
 #include "tma_util.cuh"
 
@@ -292,72 +293,79 @@ __device__ __forceinline__ void store_chunk(const GemmParams& p, int row, int co
   }
 }
 
-// One 32-column chunk of the mix epilogue for the thread that owns accumulator row (token, j = lane % 8) and
-// produces output row (token, i = lane % 8). The arithmetic and its order are those of the GEMM's bf16 store
-// followed by rank_mix_quant_kernel (fp32 fma over j ascending from 0, mask, bf16 rounding, MX quantisation of
-// the rounded values), so codes and scale are bit-identical to running the two kernels.
-__device__ __forceinline__ void mix_chunk(const uint32_t (&v)[32], const uint32_t (&cw)[8], int lane,
-                                          const __nv_bfloat16* mask_chunk, __nv_bfloat16* hidden_chunk,
-                                          uint4 (&codes)[2], uint32_t& scale_byte) {
-  uint32_t pk[16];  // the chunk rounded to bf16, two columns per word
+// One 32-column chunk of the mix epilogue. A thread enters with accumulator row (token, j = lane % 8) and leaves with
+// columns 4 q .. 4 q + 3 (q = lane % 8) of all eight output rows of its token: three butterfly exchanges transpose the
+// bf16 words inside each group of eight lanes (24 shuffles a chunk; every lane collecting its whole output row took 128
+// and bound the kernel: [8, 4096, 8, 256] 63.5 us, now 56.4), and the multiply-adds run in pairs. Arithmetic and order are those of the GEMM's bf16 store
+// followed by rank_mix_quant_kernel (fp32 fma over j ascending from 0, mask, bf16 rounding, MX quantisation of the rounded
+// values), so codes and scales are bit-identical to running the two kernels.
+// w[j * 8 + i] = {c, c}; codes[i] = four codes of row i; scales[k] = the scale bytes of rows 2 k and 2 k + 1 in its halves.
+__device__ __forceinline__ void mix_chunk(const uint32_t (&v)[32], const f2* w, int lane, const __nv_bfloat16* mask_chunk,
+                                          __nv_bfloat16* hidden_chunk, uint32_t (&codes)[8], uint32_t (&scales)[4]) {
+  uint32_t h[8][2];  // the chunk rounded to bf16, two columns per word; h[q] = columns 4 q .. 4 q + 3
 #pragma unroll
-  for (int k = 0; k < 16; ++k) {
-    const __nv_bfloat162 h = __floats2bfloat162_rn(__uint_as_float(v[2 * k]), __uint_as_float(v[2 * k + 1]));
-    pk[k] = *reinterpret_cast<const uint32_t*>(&h);
-  }
+  for (int k = 0; k < 16; ++k) h[k >> 1][k & 1] = bf16_of_f2(f2_make(__uint_as_float(v[2 * k]), __uint_as_float(v[2 * k + 1])));
   if (hidden_chunk != nullptr) {
 #pragma unroll
     for (int q = 0; q < 4; ++q)
-      stg_stream16(hidden_chunk + 8 * q, make_uint4(pk[4 * q], pk[4 * q + 1], pk[4 * q + 2], pk[4 * q + 3]));
+      stg_stream16(hidden_chunk + 8 * q, make_uint4(h[2 * q][0], h[2 * q][1], h[2 * q + 1][0], h[2 * q + 1][1]));
   }
-  float acc[32];
 #pragma unroll
-  for (int k = 0; k < 32; ++k) acc[k] = 0.f;
-  const int base = lane & 24;
+  for (int b = 4; b > 0; b >>= 1) {       // afterwards h[j] = row j, this lane's four columns
+    const bool up = (lane & b) != 0;
+#pragma unroll
+    for (int n = 0; n < 8; ++n) {
+      if (n & b) continue;
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const uint32_t got = __shfl_xor_sync(0xffffffffu, up ? h[n][e] : h[n | b][e], b);
+        if (up) h[n][e] = got; else h[n | b][e] = got;
+      }
+    }
+  }
+  f2 acc[8][2];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) acc[i][0] = acc[i][1] = 0ull;
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
-    // fma.rn.f32.bf16: bf16 x bf16 + fp32 with one rounding, i.e. fmaf(float(h), float(w), acc) without the two
-    // instructions that widen the halves of the shuffled word (a third of this loop's instruction count)
-    const uint32_t w = cw[j];
+    const f2 x0 = f2_of_bf16(h[j][0]), x1 = f2_of_bf16(h[j][1]);
 #pragma unroll
-    for (int k = 0; k < 16; ++k) {
-      const uint32_t other = __shfl_sync(0xffffffffu, pk[k], base + j);
-      asm("{\n\t.reg .b16 lo, hi, wl, wh;\n\t"
-          "mov.b32 {lo, hi}, %2;\n\t"
-          "mov.b32 {wl, wh}, %3;\n\t"
-          "fma.rn.f32.bf16 %0, lo, wl, %0;\n\t"
-          "fma.rn.f32.bf16 %1, hi, wl, %1;\n\t}"
-          : "+f"(acc[2 * k]), "+f"(acc[2 * k + 1])
-          : "r"(other), "r"(w));
+    for (int i = 0; i < 8; i += 2) {
+      const ulonglong2 c = *reinterpret_cast<const ulonglong2*>(w + j * 8 + i);
+      acc[i][0] = f2_fma(x0, c.x, acc[i][0]);
+      acc[i][1] = f2_fma(x1, c.x, acc[i][1]);
+      acc[i + 1][0] = f2_fma(x0, c.y, acc[i + 1][0]);
+      acc[i + 1][1] = f2_fma(x1, c.y, acc[i + 1][1]);
     }
   }
   if (mask_chunk != nullptr) {
+    const uint2 m = *reinterpret_cast<const uint2*>(mask_chunk + 4 * (lane & 7));
+    const f2 m0 = f2_of_bf16(m.x), m1 = f2_of_bf16(m.y);
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      float m[8];
-      unpack8(*reinterpret_cast<const uint4*>(mask_chunk + 8 * q), m);
-#pragma unroll
-      for (int e = 0; e < 8; ++e) acc[8 * q + e] *= m[e];
+    for (int i = 0; i < 8; ++i) {
+      acc[i][0] = f2_mul(acc[i][0], m0);
+      acc[i][1] = f2_mul(acc[i][1], m1);
     }
   }
-  float f[32];
-  float amax = 0.f;
+  uint32_t y[8][2];
 #pragma unroll
-  for (int k = 0; k < 16; ++k) {
-    const float2 r = __bfloat1622float2(__floats2bfloat162_rn(acc[2 * k], acc[2 * k + 1]));
-    f[2 * k] = r.x;
-    f[2 * k + 1] = r.y;
-    amax = fmaxf(amax, fmaxf(fabsf(r.x), fabsf(r.y)));
+  for (int i = 0; i < 8; ++i) {
+    y[i][0] = bf16_of_f2(acc[i][0]);
+    y[i][1] = bf16_of_f2(acc[i][1]);
   }
-  const int ex = mxq::mx_exponent(fmaxf(amax, mxq::kAmaxFloor));
-  const float inv = mxq::mx_inv_scale(ex);
-  uint32_t w8[8];
 #pragma unroll
-  for (int q = 0; q < 8; ++q)
-    w8[q] = mxq::e4m3x2(f[4 * q] * inv, f[4 * q + 1] * inv) | (mxq::e4m3x2(f[4 * q + 2] * inv, f[4 * q + 3] * inv) << 16);
-  codes[0] = make_uint4(w8[0], w8[1], w8[2], w8[3]);
-  codes[1] = make_uint4(w8[4], w8[5], w8[6], w8[7]);
-  scale_byte = static_cast<uint32_t>(ex + 127);
+  for (int k = 0; k < 4; ++k) {           // largest |y| of rows 2 k and 2 k + 1 over the token's eight lanes; ignores NaN
+    uint32_t a = mxq::bf16x2_max(0u, y[2 * k][0] & 0x7fff7fffu), b = mxq::bf16x2_max(0u, y[2 * k + 1][0] & 0x7fff7fffu);
+    a = mxq::bf16x2_max(a, y[2 * k][1] & 0x7fff7fffu);
+    b = mxq::bf16x2_max(b, y[2 * k + 1][1] & 0x7fff7fffu);
+    uint32_t am = mxq::bf16x2_max(__byte_perm(a, b, 0x5410), __byte_perm(a, b, 0x7632));
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) am = mxq::bf16x2_max(am, __shfl_xor_sync(0xffffffffu, am, o));
+    const uint32_t sb0 = mxq::mx_scale_byte(am & 0xffffu), sb1 = mxq::mx_scale_byte(am >> 16);
+    scales[k] = sb0 | (sb1 << 16);
+    codes[2 * k] = mxq::mx_codes4(y[2 * k][0], y[2 * k][1], mxq::mx_inv_bf16x2(sb0));
+    codes[2 * k + 1] = mxq::mx_codes4(y[2 * k + 1][0], y[2 * k + 1][1], mxq::mx_inv_bf16x2(sb1));
+  }
 }
 
 // EPI = number of epilogue warps: 4 (one per tensor-memory lane quadrant) for the ordinary epilogue; 8 for the mix
@@ -371,6 +379,7 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   extern __shared__ uint8_t smem_raw[];
   __shared__ volatile int abort_flag;
   __shared__ uint32_t tmem_base_slot;
+  __shared__ __align__(16) f2 mix_w[EPI == 8 ? 64 : 2];   // mix epilogue: {c, c} of row j in output row i at [j * 8 + i]
 
   const uint32_t raw_addr = smem_u32(smem_raw);
   const uint32_t base = (raw_addr + 1023u) & ~1023u;  // 128B-swizzled TMA boxes need 1024-byte alignment
@@ -486,14 +495,15 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     const int quad = warp & 3;  // tensor-memory lane quadrant this warp may access
     bool ok = true;
     int it = 0;
-    if (BN == 128 && p.mix_codes != nullptr) {
+    if (EPI == 8) {
       // mix epilogue: see GemmParams. splits == 1 here, so an item is a tile.
-      uint32_t cw[8];   // this row's mix weights as raw bf16 bits (low half)
-      {
-        const int i = lane & 7;
-#pragma unroll
-        for (int j = 0; j < 8; ++j) cw[j] = __bfloat16_as_ushort(p.mix_transpose ? p.mix_c[j * 8 + i] : p.mix_c[i * 8 + j]);
+      if (threadIdx.x < 128) {   // the first two of the eight epilogue warps
+        const int j = (threadIdx.x - 64) >> 3, i = threadIdx.x & 7;
+        mix_w[threadIdx.x - 64] = f2_dup(__bfloat162float(p.mix_transpose ? p.mix_c[j * 8 + i] : p.mix_c[i * 8 + j]));
       }
+      asm volatile("bar.sync 1, 256;" ::: "memory");   // the epilogue warps
+      const int q = lane & 7;
+      const int64_t row_step = p.mix_items * 128;      // plane row i to i + 1
       for (int item = blockIdx.x; item < total_items && ok; item += gridDim.x, ++it) {
         const int mt = item;  // n_tiles == 1
         const int as = it & 1;
@@ -501,7 +511,7 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         tc_fence_after();
         const int64_t row = static_cast<int64_t>(mt) * BM + quad * 32 + lane;   // accumulator row (token * 8 + j)
         const int64_t token = row >> 3;
-        const int64_t prow = static_cast<int64_t>(lane & 7) * p.mix_items + token;   // plane row this thread writes
+        const int64_t prow = q * p.mix_items + token;   // the plane row whose scales this thread writes
         const __nv_bfloat16* mask_row = p.mix_mask ? p.mix_mask + (token / p.mix_n_per_batch) * 128 : nullptr;
         const uint32_t t_row = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + (as ? C::kAcc1Col : 0);
         constexpr int kChunks = 16 / EPI;                 // chunks per warp: 4, or 2 with two warps per quadrant
@@ -517,14 +527,14 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             __syncwarp();
             if (lane == 0) mbar_arrive(acc_free_bar);
           }
-          uint4 codes[2];
-          uint32_t sb;
-          mix_chunk(v, cw, lane, mask_row ? mask_row + c * 32 : nullptr,
-                    p.mix_hidden ? p.mix_hidden + row * 128 + c * 32 : nullptr, codes, sb);
-          uint8_t* dst = p.mix_codes + prow * 128 + c * 32;
-          stg_stream16(dst, codes[0]);
-          stg_stream16(dst + 16, codes[1]);
-          scale_word |= sb << (8 * (c - c0));
+          uint32_t codes[8], scales[4];
+          mix_chunk(v, mix_w, lane, mask_row ? mask_row + c * 32 : nullptr,
+                    p.mix_hidden ? p.mix_hidden + row * 128 + c * 32 : nullptr, codes, scales);
+          uint8_t* dst = p.mix_codes + token * 128 + c * 32 + q * 4;   // eight lanes write the 32 codes of a plane row
+#pragma unroll
+          for (int i = 0; i < 8; ++i, dst += row_step) *reinterpret_cast<uint32_t*>(dst) = codes[i];
+          const uint32_t two = (q & 4) ? ((q & 2) ? scales[3] : scales[2]) : ((q & 2) ? scales[1] : scales[0]);
+          scale_word |= ((q & 1) ? two >> 16 : two & 0xffffu) << (8 * (c - c0));
         }
         // the row's scale bytes are adjacent in the tiled layout (one 128-column chunk per row tile)
         uint8_t* sdst = p.mix_scales + (prow >> 7) * 512 + mxq::tiled_offset(static_cast<int>(prow & 127), c0);
@@ -582,28 +592,36 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   }
 }
 
-// C = sum over splits (in index order, so the result is reproducible) of partial[s] (+ bias), 4 columns per thread.
+// C = sum over splits of partial[s] (+ bias), four columns per group of kFinalSlices threads: a T-LoKr factor gradient is
+// 8192 such groups over up to 74 splits, which one thread each walked in ten dependent rounds of loads. Slice q of a group
+// adds its contiguous share of the splits in ascending order, then the slices are added in ascending order: a fixed
+// association, so the result is reproducible. [256, 128] over K = 262144 (GEMM and finalize): 31.7 -> 26.9 us.
+constexpr int kFinalSlices = 8;
 __global__ void __launch_bounds__(256) splitk_finalize_kernel(const GemmParams p) {
+  __shared__ float4 sums[kFinalSlices][32];
   after_previous();
   const int64_t n4 = p.N / 4, total = static_cast<int64_t>(p.M) * n4, plane = static_cast<int64_t>(p.M) * p.N;
-  for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < total;
-       i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+  const int lane = threadIdx.x & 31, slice = threadIdx.x >> 5;
+  const int per = (p.splits + kFinalSlices - 1) / kFinalSlices, s0 = slice * per, s1 = min(p.splits, s0 + per);
+  for (int64_t base = blockIdx.x * 32ll; base < total; base += gridDim.x * 32ll) {
+    const int64_t i = base + lane;
     const int64_t row = i / n4, col = (i - row * n4) * 4;
-    const float* src = p.partial + row * p.N + col;
-    float4 acc = *reinterpret_cast<const float4*>(src);
-    // The loads of eight splits are issued together and then added in index order: the sum keeps its fixed
-    // association, and a thread no longer waits one memory latency per split (a [256, 128] factor gradient is
-    // summed over up to 74 splits by 8192 threads).
-    int s = 1;
-    for (; s + 8 <= p.splits; s += 8) {
-      float4 v[8];
-#pragma unroll
-      for (int u = 0; u < 8; ++u) v[u] = *reinterpret_cast<const float4*>(src + (s + u) * plane);
-#pragma unroll
-      for (int u = 0; u < 8; ++u) { acc.x += v[u].x; acc.y += v[u].y; acc.z += v[u].z; acc.w += v[u].w; }
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (i < total) {
+      const float* src = p.partial + row * p.N + col + s0 * plane;
+#pragma unroll 8
+      for (int s = s0; s < s1; ++s, src += plane) {
+        const float4 v = *reinterpret_cast<const float4*>(src);
+        acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
+      }
     }
-    for (; s < p.splits; ++s) {
-      const float4 v = *reinterpret_cast<const float4*>(src + s * plane);
+    __syncthreads();          // the sums of the previous group have been read
+    sums[slice][lane] = acc;
+    __syncthreads();
+    if (slice != 0 || i >= total) continue;
+#pragma unroll
+    for (int q = 1; q < kFinalSlices; ++q) {
+      const float4 v = sums[q][lane];
       acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
     }
     acc.x *= p.alpha; acc.y *= p.alpha; acc.z *= p.alpha; acc.w *= p.alpha;
@@ -1549,7 +1567,7 @@ int launch(const CUtensorMap& ma, const CUtensorMap& mb, GemmParams p, cudaStrea
   ANIMA_CHECK_LAUNCH("mx_gemm");
   if (p.splits > 1) {
     const int64_t groups = static_cast<int64_t>(p.M) * (p.N / 4);
-    launch_after(splitk_finalize_kernel, static_cast<unsigned>(std::min<int64_t>(ceil_div(groups, 256), 4LL * sm_count())), 256, 0,
+    launch_after(splitk_finalize_kernel, static_cast<unsigned>(std::min<int64_t>(ceil_div(groups, 32), 8LL * sm_count())), 256, 0,
                  s, p);
     ANIMA_CHECK_LAUNCH("mx_gemm split-K finalize");
   }
