@@ -205,31 +205,6 @@ void gemm(const Launch& l, const Op& a, const Op& b, const GemmOut& out, const v
                          status_word(l.dev), l.stream));
 }
 
-void gemm_sum(const Launch& l, const std::vector<Op>& g, const std::vector<Op>& w, const Tensor& c) {
-  const int n = static_cast<int>(g.size());
-  const int64_t M = g[0].rows, N = w[0].rows;
-  if (n == 1 || M <= 128 || N <= 128) {
-    for (int i = 0; i < n; ++i)
-      gemm(l, g[i], w[i], {c.data_ptr(), N, false}, nullptr, i ? c.data_ptr() : nullptr, N);
-    return;
-  }
-  const uint8_t *ac[kMaxSummed], *as[kMaxSummed], *bc[kMaxSummed], *bs[kMaxSummed];
-  int64_t K[kMaxSummed];
-  TORCH_CHECK(n <= kMaxSummed, "gemm_sum: ", n, " products");
-  for (int i = 0; i < n; ++i) {
-    need_same_k(g[i], w[i]);
-    ac[i] = g[i].codes;
-    as[i] = g[i].scales;
-    bc[i] = w[i].codes;
-    bs[i] = w[i].scales;
-    K[i] = g[i].k;
-  }
-  const int64_t bytes = check(anima_mx_gemm_cat_workspace_bytes(M, N, n, K));
-  Tensor ws;
-  if (bytes) ws = empty({bytes}, U8, l.dev);
-  check(anima_mx_gemm_cat(n, ac, as, bc, bs, K, c.data_ptr(), M, N, N, 0, ptr(ws), bytes, status_word(l.dev), l.stream));
-}
-
 void gemm_delta(const Launch& l, const Op& a, const Op& b, const Op& planes, const Op& d, void* c, const void* bias) {
   need_same_k(a, b);
   const int64_t M = a.rows, N = b.rows, K = a.k;

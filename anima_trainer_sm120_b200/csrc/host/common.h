@@ -119,9 +119,6 @@ struct GemmOut {
 };
 void gemm(const Launch& l, const Op& a, const Op& b, const GemmOut& out, const void* bias = nullptr,
           const void* residual = nullptr, int64_t ldr = 0, double alpha = 1.0);
-// C = sum of the products g[i] . w[i]^T in one GEMM (or, where its kernel does not apply, one after the other)
-void gemm_sum(const Launch& l, const std::vector<Op>& g, const std::vector<Op>& w, const Tensor& c);
-constexpr int kMaxSummed = 3;
 void gemm_delta(const Launch& l, const Op& a, const Op& b, const Op& planes, const Op& d, void* c, const void* bias);
 Tensor gemm_f32(const Launch& l, const Op& a, const Op& b, double alpha = 1.0);        // [M, N] fp32
 // (dw1, dw2) of dW = [N, K] fp32, in the factors' dtype
@@ -185,8 +182,8 @@ std::shared_ptr<N> make_node(const Inputs&... inputs) {
   node->set_next_edges(std::move(edges));
   return node;
 }
-// The node last made for an input on this thread (both weak), for a later call on the same tensor that may become part
-// of it. `get` gives the node while t still is what it saw: same tensor, version, shape and graph edge.
+// The node last made for an input on this thread (both weak), for a later call on the same tensor whose gradient is to
+// pass through it. `get` gives the node while t still is what it saw: same tensor, version, shape and graph edge.
 template <class N>
 struct LastNode {
   c10::weak_intrusive_ptr<c10::TensorImpl> x{c10::intrusive_ptr<c10::TensorImpl>()};

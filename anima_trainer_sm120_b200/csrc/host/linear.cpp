@@ -86,72 +86,30 @@ struct MergedNode : public HostNode {
 };
 
 // ------------------------------------------------------------------------------------------------ frozen linear
-// Frozen linears of the same input, applied one after the other (q / k / v projections), are the outputs of ONE node:
-// backward then contracts their gradients in one GEMM whose K-blocks run over all of them, in fp32 with one rounding,
-// instead of one GEMM each and additions of their outputs (two passes of three over [rows, K] for q / k / v).
-// [32768, 2048] x 3, forward and backward: 1130 -> 915 us.
 struct FrozenNode : public HostNode {
-  struct Part {
-    Op w_col;
-    Tensor w_bf16;        // serves backward where W has no column form
-    int bias_edge;        // -1: no gradient
-  };
-  std::vector<Part> parts;                 // by output
-  bool started = false;                    // backward has begun: nothing may join (under the node's lock)
-  int64_t k_in;
-
-  // y becomes another output unless backward has begun. A bias that is itself computed could depend on an earlier
-  // output of this node, a cycle: such a linear keeps a node of its own.
-  bool join(Part part, const OptTensor& bias, const Tensor& y) {
-    std::lock_guard<std::mutex> lock(mutex_);
-    if (started || parts.size() >= kMaxSummed || (wants(bias) && !bias->is_leaf())) return false;
-    add(std::move(part), bias, y);
-    return true;
-  }
-  void add(Part part, const OptTensor& bias, const Tensor& y) {
-    part.bias_edge = -1;
-    if (wants(bias)) {
-      part.bias_edge = static_cast<int>(num_outputs());
-      add_next_edge(edge_of(bias));
-    }
-    parts.push_back(std::move(part));
-    set_history(y, std::static_pointer_cast<FrozenNode>(getptr()));
-  }
+  Op w_col;
+  Tensor w_bf16;
+  bool need_x, need_bias;
 
   variable_list apply(variable_list&& g) override {
     std::lock_guard<std::mutex> lock(mutex_);
-    started = true;
-    variable_list out(num_outputs());
-    const bool need_x = task_should_compute_output(0);
-    std::vector<Op> rows, weights;
-    Tensor gx, some;
-    for (size_t i = 0; i < std::min(parts.size(), g.size()); ++i) {
-      if (!g[i].defined()) continue;
-      const Tensor& gy = some = g[i];
+    const Tensor gy = grad_of(g, 0);
+    variable_list out(2);
+    if (need_x) {
       const Launch l(gy);
-      if (parts[i].bias_edge >= 0) out[parts[i].bias_edge] = bias_grad(gy);
-      if (!need_x) continue;
       const Mat m = as_matrix(gy, gy.size(-1));
-      if (parts[i].w_col.defined()) {
-        rows.push_back(quantize(l, m, true, false).first);
-        weights.push_back(parts[i].w_col);
+      if (w_col.defined()) {
+        out[0] = input_grad(l, gy, quantize(l, m, true, false).first, w_col);
       } else {
-        const Tensor& w = parts[i].w_bf16;
-        gx = at::matmul(m.keep.reshape({m.rows, m.cols}), w.to(BF16)).reshape(with_last(gy.sizes(), w.size(1)));
+        Tensor gx = at::matmul(m.keep.reshape({m.rows, m.cols}), w_bf16.to(BF16));
+        out[0] = cast(gx.reshape(with_last(gy.sizes(), w_bf16.size(1))), gy.scalar_type());
       }
     }
-    if (!rows.empty()) {
-      const Launch l(some);
-      gx = empty(with_last(some.sizes(), k_in), BF16, l.dev);
-      if (rows[0].rows) gemm_sum(l, rows, weights, gx);
-    }
-    if (gx.defined()) out[0] = cast(gx, some.scalar_type());
+    if (need_bias) out[1] = bias_grad(gy);
     return out;
   }
   std::string name() const override { return "MXFP8FrozenLinearBackward"; }
 };
-
-thread_local LastNode<FrozenNode> applied;
 
 // ------------------------------------------------------------------------------------------------ LoKr MLP
 struct MlpNode : public HostNode {
@@ -267,15 +225,14 @@ Tensor frozen_linear(const Tensor& x, Op x_row, Op w_row, Op w_col, const OptTen
     Below below;
     y = project(l, x, x_row, w_row, bias);
   }
-  if (!need_x && !need_bias) return y;
-  const bool shares = need_x && w_col.defined() && !x.is_inference();
-  FrozenNode::Part part{std::move(w_col), w_bf16.value_or(Tensor()), -1};
-  if (shares)
-    if (auto n = applied.get(x); n && n->join(part, bias, y)) return y;
-  auto n = make_node<FrozenNode>(x);
-  n->k_in = w_row.k;
-  n->add(std::move(part), bias, y);
-  if (shares) applied.set(x, n);
+  if (need_x || need_bias) {
+    auto n = make_node<FrozenNode>(x, bias);
+    n->w_col = std::move(w_col);
+    n->w_bf16 = w_bf16.value_or(Tensor());
+    n->need_x = need_x;
+    n->need_bias = need_bias;
+    set_history(y, n);
+  }
   return y;
 }
 

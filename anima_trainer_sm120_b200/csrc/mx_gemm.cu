@@ -115,12 +115,6 @@ __device__ __forceinline__ uint32_t make_idesc(uint32_t sf_id) {
          (sf_id << 29) | (sf_id << 4);
 }
 
-constexpr int kMaxSegments = 3;   // q, k and v of one input
-// Operand tensor maps of the pair kernel, one set per segment of the contraction.
-struct SegMaps {
-  CUtensorMap a[kMaxSegments], b[kMaxSegments], sfa[kMaxSegments], sfb[kMaxSegments];
-};
-
 struct GemmParams {
   const uint8_t* a_scales;
   const uint8_t* b_scales;
@@ -168,9 +162,6 @@ struct GemmParams {
   // columns inside one block is one more pipeline stage (A slot: 128 rows of plane i; B slot: the factor rows of
   // the run, half per CTA) and one group of MMAs of that width into the run's accumulator columns.
   int delta, delta_block;
-  // Concatenated contraction (anima_mx_gemm_cat): segment i of the K-blocks, [seg_end[i - 1], seg_end[i]), has operands
-  // of its own (tensor maps SegMaps::*[i]); every other launch has one segment.
-  int segs, seg_end[kMaxSegments];
   // Measurement aid (anima_mx_gemm_set_clock_probe): if not null, CTA 0 of a pair-kernel launch adds the SM
   // cycles and the nanoseconds it ran, so that the clock the GPU actually held under this kernel's power
   // draw can be read back (the driver's sampled clocks mostly see the idle gaps between launches), and the
@@ -811,7 +802,9 @@ __device__ __forceinline__ void tc2_kblock(uint32_t d_tmem, uint32_t a_lo, uint3
 
 template <int BN>
 __global__ void __launch_bounds__(kThreads2, 1)
-mx_gemm2_kernel(const __grid_constant__ SegMaps maps, const __grid_constant__ CUtensorMap map_c, const __grid_constant__ CUtensorMap map_part,
+mx_gemm2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
+                const __grid_constant__ CUtensorMap map_sfa, const __grid_constant__ CUtensorMap map_sfb,
+                const __grid_constant__ CUtensorMap map_c, const __grid_constant__ CUtensorMap map_part,
                 const __grid_constant__ CUtensorMap map_pl, const __grid_constant__ CUtensorMap map_d,
                 const __grid_constant__ CUtensorMap map_plsf, const __grid_constant__ CUtensorMap map_dsf,
                 const GemmParams p) {
@@ -855,12 +848,10 @@ mx_gemm2_kernel(const __grid_constant__ SegMaps maps, const __grid_constant__ CU
     mbar_init(ovl_free_bar(0), 8);  // the four warps of the half that owns the shared columns, in both CTAs
     mbar_init(ovl_free_bar(1), 8);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    for (int i = 0; i < p.segs; ++i) {
-      asm volatile("prefetch.tensormap [%0];" ::"l"(&maps.a[i]) : "memory");
-      asm volatile("prefetch.tensormap [%0];" ::"l"(&maps.b[i]) : "memory");
-      asm volatile("prefetch.tensormap [%0];" ::"l"(&maps.sfa[i]) : "memory");
-      asm volatile("prefetch.tensormap [%0];" ::"l"(&maps.sfb[i]) : "memory");
-    }
+    asm volatile("prefetch.tensormap [%0];" ::"l"(&map_a) : "memory");
+    asm volatile("prefetch.tensormap [%0];" ::"l"(&map_b) : "memory");
+    asm volatile("prefetch.tensormap [%0];" ::"l"(&map_sfa) : "memory");
+    asm volatile("prefetch.tensormap [%0];" ::"l"(&map_sfb) : "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"(&map_c) : "memory");
     if (p.tail_splits > 1) asm volatile("prefetch.tensormap [%0];" ::"l"(&map_part) : "memory");
   }
@@ -903,10 +894,7 @@ mx_gemm2_kernel(const __grid_constant__ SegMaps maps, const __grid_constant__ CU
         const int row_a = it.mt * 256 + static_cast<int>(rank) * 128;
         const int row_b = it.nt * BN + static_cast<int>(rank) * (narrow ? 64 : BN / 2);
         const int sfa_rt = it.mt * 2 + static_cast<int>(rank), sfb_rt = (it.nt * BN) >> 7;
-        int seg = 0, seg_base = 0;
-        while (it.kb0 >= p.seg_end[seg]) seg_base = p.seg_end[seg++];
         for (int kb = it.kb0; kb < it.kb1; ++kb) {
-          if (kb == p.seg_end[seg]) seg_base = p.seg_end[seg++];
           // (try_wait itself blocks for a while before it gives up, so the wait is timed around both)
           const long long t0 = probe ? clock64() : 0;
           if (!mbar_try_wait(empty_bar(s), ph ^ 1u)) ok = mbar_wait(empty_bar(s), ph ^ 1u, &abort_flag);
@@ -916,11 +904,10 @@ mx_gemm2_kernel(const __grid_constant__ SegMaps maps, const __grid_constant__ CU
           if (elect_one()) {
             if (rank == 0) mbar_expect_tx(full_bar(s), C::kTxBytes);
             const uint32_t leader_full = leader_full0 + 8 * s;
-            const int k = kb - seg_base;
-            tma2_load_2d(a_smem(s), &maps.a[seg], leader_full, k * BK, row_a);
-            tma2_load_2d(b_smem(s), &maps.b[seg], leader_full, k * BK, row_b);  // 96-row box; rows past N read as 0
-            tma2_load_3d(sfa_smem(s), &maps.sfa[seg], leader_full, 0, k, sfa_rt);
-            tma2_load_3d(sfb_smem(s), &maps.sfb[seg], leader_full, 0, k, sfb_rt);  // the two 128-column chunks it spans
+            tma2_load_2d(a_smem(s), &map_a, leader_full, kb * BK, row_a);
+            tma2_load_2d(b_smem(s), &map_b, leader_full, kb * BK, row_b);  // 96-row box; rows past N read as 0
+            tma2_load_3d(sfa_smem(s), &map_sfa, leader_full, 0, kb, sfa_rt);
+            tma2_load_3d(sfb_smem(s), &map_sfb, leader_full, 0, kb, sfb_rt);  // the two 128-column chunks it spans
           }
           __syncwarp();
           if (++s == kStages2) { s = 0; ph ^= 1u; }
@@ -1431,39 +1418,25 @@ struct DeltaOperands {
   int64_t block;
 };
 
-// Operands of one segment of the contraction (one segment: the ordinary product).
-struct Segment {
-  const uint8_t *a_codes, *a_scales, *b_codes, *b_scales;
-  int64_t K;
-};
-
 template <int BN>
-int launch_pair_width(const Segment* segs, int n_segs, GemmParams p, const PairPlan& pl, void* workspace,
+int launch_pair_width(const uint8_t* a_codes, const uint8_t* b_codes, GemmParams p, const PairPlan& pl, void* workspace,
                       const DeltaOperands& delta, cudaStream_t s);
 
-// Contraction length the plan is made for: K, or for several segments their K-blocks.
-int64_t planned_k(const Segment* segs, int n_segs) {
-  if (n_segs == 1) return segs[0].K;
-  int64_t kb = 0;
-  for (int i = 0; i < n_segs; ++i) kb += ceil_div(segs[i].K, BK);
-  return kb * BK;
-}
-
-int launch_pair(const Segment* segs, int n_segs, GemmParams p, void* workspace, int64_t workspace_bytes,
+int launch_pair(const uint8_t* a_codes, const uint8_t* b_codes, GemmParams p, void* workspace, int64_t workspace_bytes,
                 const DeltaOperands& delta, cudaStream_t s) {
-  const PairPlan pl = plan_pair(p.M, p.N, planned_k(segs, n_segs), workspace != nullptr);
+  const PairPlan pl = plan_pair(p.M, p.N, p.K, workspace != nullptr);
   ANIMA_REQUIRE(workspace_bytes >= pl.ws_bytes, ANIMA_E_WORKSPACE,
                 "mx_gemm: workspace of %lld bytes is too small (need %lld)", (long long)workspace_bytes,
                 (long long)pl.ws_bytes);
-  return pl.bn == 256 ? launch_pair_width<256>(segs, n_segs, p, pl, workspace, delta, s)
-                      : launch_pair_width<192>(segs, n_segs, p, pl, workspace, delta, s);
+  return pl.bn == 256 ? launch_pair_width<256>(a_codes, b_codes, p, pl, workspace, delta, s)
+                      : launch_pair_width<192>(a_codes, b_codes, p, pl, workspace, delta, s);
 }
 
 // Launches of at most this many K-blocks a CTA (pair), about 50 us, overlap the kernel ahead of them (see launch_after).
 constexpr int64_t kOverlapBlocks = 192;
 
 template <int kBN2>
-int launch_pair_width(const Segment* segs, int n_segs, GemmParams p, const PairPlan& pl, void* workspace,
+int launch_pair_width(const uint8_t* a_codes, const uint8_t* b_codes, GemmParams p, const PairPlan& pl, void* workspace,
                       const DeltaOperands& delta, cudaStream_t s) {
   using C2 = Cfg2<kBN2>;
   static PerDeviceOnce once;
@@ -1489,25 +1462,14 @@ int launch_pair_width(const Segment* segs, int n_segs, GemmParams p, const PairP
   }
   const int sf_bufs = env_int("ANIMA_MX_GEMM_SFBUFS", C2::kMaxSfBufs);
   p.sf_bufs = (sf_bufs == 1 || sf_bufs == 2) ? sf_bufs : C2::kMaxSfBufs;
-  SegMaps maps;
-  CUtensorMap mc, mp;
-  p.segs = n_segs;
-  p.k_blocks = 0;
-  bool encoded = make_c_map(&mc, p);
-  for (int i = 0; i < n_segs; ++i) {
-    const Segment& g = segs[i];
-    const int64_t kb = ceil_div(g.K, BK);
-    p.seg_end[i] = p.k_blocks += static_cast<int>(kb);
-    encoded = encoded && make_map(&maps.a[i], g.a_codes, p.M, g.K, 128) && make_map(&maps.b[i], g.b_codes, p.N, g.K, kBN2 / 2) &&
-              make_sf_map(&maps.sfa[i], g.a_scales, p.sfa_rt, kb, 1) &&
-              make_sf_map(&maps.sfb[i], g.b_scales, p.sfb_rt, kb, kSfbChunks2);
-  }
-  if (pl.ws_bytes)
-    encoded = encoded && make_part_map(&mp, p.pair_partial, static_cast<int64_t>(pl.tail_tiles) * pl.tail_splits, kBN2);
-  else
-    mp = mc;
-  ANIMA_REQUIRE(encoded, ANIMA_E_CUDA, "mx_gemm: cuTensorMapEncodeTiled failed (driver entry point missing or bad operand)");
-  CUtensorMap mpl = maps.a[0], md = maps.b[0], mplsf = maps.sfa[0], mdsf = maps.sfb[0];   // placeholders when there is no delta
+  CUtensorMap ma, mb, msa, msb, mc, mp;
+  ANIMA_REQUIRE(make_map(&ma, a_codes, p.M, p.K, 128) && make_map(&mb, b_codes, p.N, p.K, kBN2 / 2) &&
+                    make_sf_map(&msa, p.a_scales, p.sfa_rt, p.k_blocks, 1) &&
+                    make_sf_map(&msb, p.b_scales, p.sfb_rt, p.k_blocks, kSfbChunks2) && make_c_map(&mc, p) &&
+                    (pl.ws_bytes ? make_part_map(&mp, p.pair_partial, static_cast<int64_t>(pl.tail_tiles) * pl.tail_splits, kBN2)
+                                 : make_c_map(&mp, p)),
+                ANIMA_E_CUDA, "mx_gemm: cuTensorMapEncodeTiled failed (driver entry point missing or bad operand)");
+  CUtensorMap mpl = ma, md = mb, mplsf = msa, mdsf = msb;   // placeholders when there is no delta
   p.delta = delta.planes_codes ? 1 : 0;
   p.delta_block = static_cast<int>(delta.block);
   if (p.delta) {
@@ -1533,7 +1495,7 @@ int launch_pair_width(const Segment* segs, int n_segs, GemmParams p, const PairP
   cfg.attrs = attr;
   const int64_t k_blocks = static_cast<int64_t>(p.m_tiles) * p.n_tiles * p.k_blocks;
   cfg.numAttrs = k_blocks <= kOverlapBlocks * pl.pairs ? 2 : 1;
-  const cudaError_t rc = cudaLaunchKernelEx(&cfg, mx_gemm2_kernel<kBN2>, maps, mc, mp, mpl, md, mplsf, mdsf, p);
+  const cudaError_t rc = cudaLaunchKernelEx(&cfg, mx_gemm2_kernel<kBN2>, ma, mb, msa, msb, mc, mp, mpl, md, mplsf, mdsf, p);
   ANIMA_REQUIRE(rc == cudaSuccess, ANIMA_E_CUDA, "mx_gemm: cluster launch failed: %s", cudaGetErrorString(rc));
   if (pl.ws_bytes) {
     const int64_t threads = static_cast<int64_t>(pl.tail_tiles) * 256 * (kBN2 / 4);
@@ -1645,10 +1607,7 @@ static int mx_gemm_impl(const uint8_t* a_codes, const uint8_t* a_scales, const u
   p.alpha = alpha;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   ANIMA_REQUIRE(!workspace || aligned16(workspace), ANIMA_E_ALIGN, "mx_gemm: workspace must be 16-byte aligned");
-  if (use_pair(M, N)) {
-    const Segment whole{a_codes, a_scales, b_codes, b_scales, K};
-    return launch_pair(&whole, 1, p, workspace, workspace_bytes, delta, s);
-  }
+  if (use_pair(M, N)) return launch_pair(a_codes, b_codes, p, workspace, workspace_bytes, delta, s);
   ANIMA_REQUIRE(!delta.planes_codes, ANIMA_E_UNSUPPORTED,
                 "mx_gemm_delta: M=%lld N=%lld runs on the one-CTA kernel, which has no delta K-blocks", (long long)M,
                 (long long)N);
@@ -1693,54 +1652,6 @@ extern "C" int anima_mx_gemm_ex(const uint8_t* a_codes, const uint8_t* a_scales,
                                 void* workspace, int64_t workspace_bytes, int32_t* status, void* stream) {
   return mx_gemm_impl(a_codes, a_scales, b_codes, b_scales, c, M, N, K, ldc, bias, residual, ldr, alpha, out_dtype,
                       workspace, workspace_bytes, status, stream);
-}
-
-extern "C" int64_t anima_mx_gemm_cat_workspace_bytes(int64_t M, int64_t N, int segments, const int64_t* K) {
-  if (M <= 128 || N <= 128 || segments < 1 || segments > kMaxSegments || !K) return ANIMA_E_UNSUPPORTED;
-  if (M >= (1ll << 31) - 256 || N >= (1ll << 31) - 256) return ANIMA_E_TOO_LARGE;
-  Segment g[kMaxSegments] = {};
-  for (int i = 0; i < segments; ++i) {
-    if (K[i] <= 0 || K[i] >= (1ll << 28)) return ANIMA_E_TOO_LARGE;
-    g[i].K = K[i];
-  }
-  return plan_pair(M, N, planned_k(g, segments), true).ws_bytes;
-}
-
-extern "C" int anima_mx_gemm_cat(int segments, const uint8_t* const* a_codes, const uint8_t* const* a_scales,
-                                 const uint8_t* const* b_codes, const uint8_t* const* b_scales, const int64_t* K, void* c,
-                                 int64_t M, int64_t N, int64_t ldc, int out_dtype, void* workspace, int64_t workspace_bytes,
-                                 int32_t* status, void* stream) {
-  ANIMA_REQUIRE(segments >= 1 && segments <= kMaxSegments, ANIMA_E_ARG, "mx_gemm_cat: 1 to %d segments, got %d", kMaxSegments,
-                segments);
-  ANIMA_REQUIRE(a_codes && a_scales && b_codes && b_scales && K && c, ANIMA_E_ARG, "mx_gemm_cat: null pointer");
-  ANIMA_REQUIRE(M > 128 && N > 128, ANIMA_E_UNSUPPORTED, "mx_gemm_cat: needs M > 128 and N > 128 (M=%lld N=%lld)", (long long)M,
-                (long long)N);
-  ANIMA_REQUIRE(M < (1ll << 31) - 256 && N < (1ll << 31) - 256, ANIMA_E_TOO_LARGE, "mx_gemm_cat: a dimension exceeds 2^31");
-  ANIMA_REQUIRE(out_dtype == 0 || out_dtype == 1, ANIMA_E_ARG, "mx_gemm_cat: out_dtype must be 0 (bf16) or 1 (fp32)");
-  ANIMA_REQUIRE(N % 8 == 0 && ldc >= N && (ldc * (out_dtype ? 4 : 2)) % 16 == 0, ANIMA_E_SHAPE,
-                "mx_gemm_cat: N must be a multiple of 8 and the row pitch of C a multiple of 16 bytes");
-  ANIMA_REQUIRE(aligned16(c) && (!workspace || aligned16(workspace)), ANIMA_E_ALIGN, "mx_gemm_cat: buffers must be 16-byte aligned");
-  Segment g[kMaxSegments];
-  for (int i = 0; i < segments; ++i) {
-    g[i] = {a_codes[i], a_scales[i], b_codes[i], b_scales[i], K[i]};
-    ANIMA_REQUIRE(g[i].a_codes && g[i].a_scales && g[i].b_codes && g[i].b_scales, ANIMA_E_ARG, "mx_gemm_cat: null operand");
-    ANIMA_REQUIRE(K[i] > 0 && K[i] % 32 == 0 && K[i] < (1ll << 28), ANIMA_E_SHAPE, "mx_gemm_cat: K=%lld must be a multiple of 32",
-                  (long long)K[i]);
-    ANIMA_REQUIRE(aligned16(g[i].a_codes) && aligned16(g[i].a_scales) && aligned16(g[i].b_codes) && aligned16(g[i].b_scales),
-                  ANIMA_E_ALIGN, "mx_gemm_cat: all buffers must be 16-byte aligned");
-  }
-  GemmParams p{};
-  p.c = c;
-  p.status = status;
-  p.M = static_cast<int>(M);
-  p.N = static_cast<int>(N);
-  p.ldc = ldc;
-  p.out_fp32 = out_dtype;
-  p.sfa_rt = static_cast<int>(ceil_div(M, 128));
-  p.sfb_rt = static_cast<int>(ceil_div(N, 128));
-  p.splits = 1;
-  p.alpha = 1.f;
-  return launch_pair(g, segments, p, workspace, workspace_bytes, DeltaOperands{}, static_cast<cudaStream_t>(stream));
 }
 
 extern "C" int anima_mx_gemm_pair_plan(int64_t M, int64_t N, int64_t K, int with_workspace, int32_t* out9) {

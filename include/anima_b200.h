@@ -183,16 +183,6 @@ int anima_mx_gemm_delta(const uint8_t* a_codes, const uint8_t* a_scales,
                         const uint8_t* d_codes, const uint8_t* d_scales,
                         void* workspace, int64_t workspace_bytes, int32_t* status, void* stream);
 
-/* C[M,N] = sum over segments i of A_i[M,K_i] . B_i[N,K_i]^T, accumulated in fp32 and rounded once: one GEMM whose
- * contraction is the concatenation of the segments' (1 to 3; K_i a multiple of 32). It is the gradient of an input that
- * several linears share (q / k / v projections), which would otherwise be several GEMMs and additions of their outputs.
- * Needs M > 128 and N > 128; workspace as for anima_mx_gemm_ex (optional). */
-int64_t anima_mx_gemm_cat_workspace_bytes(int64_t M, int64_t N, int segments, const int64_t* K);
-int anima_mx_gemm_cat(int segments, const uint8_t* const* a_codes, const uint8_t* const* a_scales,
-                      const uint8_t* const* b_codes, const uint8_t* const* b_scales, const int64_t* K,
-                      void* c, int64_t M, int64_t N, int64_t ldc, int out_dtype, void* workspace,
-                      int64_t workspace_bytes, int32_t* status, void* stream);
-
 /* The work list the CTA-pair kernel uses for a problem on the current device (no reference counterpart; for
  * tests and tuning, nothing is launched): out9 = { CTA pairs launched, wide tile columns, 1 if a narrow
  * last column (<= 128 outputs, computed with N = 128 instructions) follows them, whole-tile items dealt
