@@ -218,6 +218,9 @@ Tensor merged_linear(const Tensor& x, Op x_row, Op x_col, const Tensor& merged, 
 Tensor frozen_linear(const Tensor& x, Op x_row, Op w_row, Op w_col, const OptTensor& w_bf16, const OptTensor& bias) {
   TORCH_CHECK_VALUE(x.size(-1) == w_row.k, "input of width ", x.size(-1), " for a weight with ", w_row.k, " columns");
   const bool need_x = wants(x), need_bias = wants(bias);
+  TORCH_CHECK_VALUE(!need_x || !w_col.defined() || (w_col.rows == w_row.k && w_col.k == w_row.rows),
+                    "the backward operand [", w_col.rows, ", ", w_col.k, "] is not the transpose of the weight [", w_row.rows, ", ",
+                    w_row.k, "]");
   const Launch l(x);
   admit(l, x, bias, x_row.store, x_row.other, w_row.store, w_row.other, w_col.store, w_col.other);
   Tensor y;
