@@ -121,6 +121,11 @@ Tensor bf16_contiguous(const Tensor& t) {
   return d.is_contiguous() ? d : d.detach().contiguous();
 }
 
+void check_bias(const OptTensor& bias, int64_t n) {
+  TORCH_CHECK_VALUE(!bias || !bias->defined() || bias->numel() == n, "bias must be of length N = ", n, ", got ", bias->numel(),
+                    " elements");
+}
+
 static void need_blocks(int64_t rows, int64_t cols, bool row, bool col) {
   TORCH_CHECK_VALUE(!row || cols % 32 == 0, "rowwise quantisation needs cols % 32 == 0, got ", cols);
   TORCH_CHECK_VALUE(!col || rows % 32 == 0, "columnwise quantisation needs rows % 32 == 0, got ", rows);

@@ -103,6 +103,10 @@ Op placeholder(int64_t rows, int64_t k, const at::Device& dev);
 
 Mat as_matrix(const Tensor& x, int64_t cols);     // any shape whose elements in order are [-1, cols]; cast to bf16
 Tensor bf16_contiguous(const Tensor& t);          // detached
+// A bias of n outputs as the GEMM's epilogue reads it (undefined: none). The kernels index it by n: check_bias, before
+// anything is launched, refuses any other length.
+void check_bias(const OptTensor& bias, int64_t n);
+inline Tensor bias_rows(const OptTensor& bias) { return bias && bias->defined() ? bf16_contiguous(*bias) : Tensor(); }
 
 std::pair<Op, Op> quantize(const Launch& l, const Mat& x, bool row, bool col, int layout = ANIMA_SCALES_TILED);
 // gelu(h) or grad * gelu'(h); h and grad viewed as [rows, cols]

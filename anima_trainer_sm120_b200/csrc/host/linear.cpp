@@ -9,8 +9,7 @@ using torch::autograd::set_history;
 // [*lead, N] in bf16, then in the dtype of the input
 Tensor project(const Launch& l, const Tensor& x, const Op& x_row, const Op& w_row, const OptTensor& bias) {
   const int64_t n = w_row.rows;
-  const Tensor b = bias && bias->defined() ? bf16_contiguous(*bias) : Tensor();
-  TORCH_CHECK_VALUE(!b.defined() || b.numel() == n, "bias must be of length N");
+  const Tensor b = bias_rows(bias);
   Tensor y = empty(with_last(x.sizes(), n), BF16, l.dev);
   if (x_row.rows) gemm(l, x_row, w_row, {y.data_ptr(), n, false}, ptr(b));
   return cast(y, x.scalar_type());
@@ -145,6 +144,7 @@ struct MlpNode : public HostNode {
 Tensor lokr_linear(const Tensor& x, Op x_row, Op x_col, const Tensor& W, const OptTensor& bias, const Tensor& w1,
                    const Tensor& w2, double alpha, bool first) {
   const bool need_x = wants(x), train = wants(w1) || wants(w2), need_bias = wants(bias);
+  check_bias(bias, W.size(0));
   const Launch l(x);
   admit(l, x, W, bias, w1, w2);
   Tensor y;
@@ -182,6 +182,7 @@ Tensor lokr_linear(const Tensor& x, Op x_row, Op x_col, const Tensor& W, const O
 
 Tensor merged_linear(const Tensor& x, Op x_row, Op x_col, const Tensor& merged, const OptTensor& bias, bool first) {
   const bool need_x = wants(x), train = wants(merged), need_bias = wants(bias);
+  check_bias(bias, merged.size(0));
   const Launch l(x);
   admit(l, x, merged, bias);
   Tensor y;
@@ -221,6 +222,7 @@ Tensor frozen_linear(const Tensor& x, Op x_row, Op w_row, Op w_col, const OptTen
   TORCH_CHECK_VALUE(!need_x || !w_col.defined() || (w_col.rows == w_row.k && w_col.k == w_row.rows),
                     "the backward operand [", w_col.rows, ", ", w_col.k, "] is not the transpose of the weight [", w_row.rows, ", ",
                     w_row.k, "]");
+  check_bias(bias, w_row.rows);
   const Launch l(x);
   admit(l, x, bias, x_row.store, x_row.other, w_row.store, w_row.other, w_col.store, w_col.other);
   Tensor y;
@@ -244,6 +246,8 @@ Tensor lokr_mlp(const Tensor& x, Op x_row, Op x_col, const Tensor& W1, const Opt
                 const Tensor& w2b, double alpha2, bool first) {
   const bool train = wants(w1a) || wants(w2a) || wants(w1b) || wants(w2b), need_x = wants(x), back = need_x || train;
   const bool keep = back && !first;
+  check_bias(b1, W1.size(0));
+  check_bias(b2, W2.size(0));
   const Launch l(x);
   admit(l, x, W1, b1, w1a, w2a, W2, b2, w1b, w2b);
   const int64_t rows = x_row.rows, hid = W1.size(0);
@@ -253,7 +257,7 @@ Tensor lokr_mlp(const Tensor& x, Op x_row, Op x_col, const Tensor& W1, const Opt
     Below below;
     Op W1_row, W2_row, a_row;
     std::tie(W1_row, W1_col) = merge_quantize(l, W1, w1a, w2a, alpha1, true, keep && need_x);
-    const Tensor b = b1 && b1->defined() ? bf16_contiguous(*b1) : Tensor();
+    const Tensor b = bias_rows(b1);
     h = empty({rows, hid}, BF16, l.dev);
     if (rows) gemm(l, x_row, W1_row, {h.data_ptr(), hid, false}, ptr(b));
     std::tie(a_row, a_col) = quantize_gelu(l, h, Tensor(), rows, hid, true, keep && train);

@@ -55,7 +55,7 @@ Tensor gemm_bf16(const Launch& l, const Op& a, const Op& b, double alpha = 1.0) 
 // are extra K-blocks of the base projection. Other shapes add alpha * delta in the last GEMM's stores.
 void linear_fwd(const Launch& l, const Op& x_row, const Op& gq, int64_t batch, const TLinear& t, void* y) {
   const int64_t rows = x_row.rows, n = t.n_out(), vp = t.vp(), r = t.rank();
-  const Tensor b = t.bias && t.bias->defined() ? bf16_contiguous(*t.bias) : Tensor();
+  const Tensor b = bias_rows(t.bias);
   if (t.can_fold(rows, n, batch) && n == 8 * vp) {
     Op planes = empty_op(rows * 8, r, l.dev);
     if (t.fuse_mix) {
@@ -244,6 +244,7 @@ struct TlokrMlpNode : public HostNode {
 
 Tensor tlokr_linear(const Tensor& x, Op x_row, TLinear t, bool first) {
   const Needs need = needs_of(x, t);
+  check_bias(t.bias, t.n_out());
   const Launch l(x);
   admit(l, x);
   check_linear(l, x, x.size(-1), t);
@@ -270,6 +271,8 @@ Tensor tlokr_linear(const Tensor& x, Op x_row, TLinear t, bool first) {
 Tensor tlokr_mlp(const Tensor& x, Op x_row, TLinear t1, TLinear t2, bool first) {
   const Needs n1 = needs_of(x, t1), n2 = needs_of(x, t2);
   const bool back = n1.x || n1.factors || n2.factors, keep = back && !first;
+  check_bias(t1.bias, t1.n_out());
+  check_bias(t2.bias, t2.n_out());
   const Launch l(x);
   admit(l, x);
   check_linear(l, x, x.size(-1), t1);
@@ -303,6 +306,7 @@ Tensor tlokr_mlp(const Tensor& x, Op x_row, TLinear t1, TLinear t2, bool first) 
 }
 
 Tensor tlokr_forward_only(const Op& x_row, const Op& gq, at::IntArrayRef lead, const TLinear& t) {
+  check_bias(t.bias, t.n_out());
   const Launch l(x_row.store);
   std::vector<int64_t> shape(lead.begin(), lead.end());
   shape.push_back(t.n_out());
