@@ -104,6 +104,9 @@ Op HostNode::get_op(size_t& at, const Op& shape) {
   if (!shape.rows) return {};
   const Tensor first = get(at++);
   if (shape.other.defined()) return op_of(first, get(at++));
+  TORCH_CHECK(first.is_contiguous() && first.numel() >= store_bytes(shape.rows, shape.k),
+              "a saved operand [", shape.rows, ", ", shape.k, "] has no memory behind it: backward through a pass made under "
+              "first_pass(), whose saved tensors only a checkpoint's recomputation fills in");
   return op_in(first, shape.rows, shape.k);
 }
 

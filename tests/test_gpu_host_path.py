@@ -51,6 +51,17 @@ def _tlokr(rows):
     return (lambda x, w1, a, b: tlokr._MXTLoKrLinear.apply(x, W, None, w1, a, b, mask, 0.5)), ts, (2, rows, 1024)
 
 
+def _tlokr_mlp(rows):
+    from anima_trainer_sm120_b200 import tlokr
+    from anima_trainer_sm120_b200.fp8_quant import quantize_weight
+    g = torch.Generator(device=DEV).manual_seed(rows)
+    W1, W2 = quantize_weight(_randn(g, 1024, 512, std=0.05)), quantize_weight(_randn(g, 512, 1024, std=0.05))
+    f = lambda *s: _randn(g, *s, std=0.1, dtype=torch.float32)
+    ts = [_randn(g, 2, rows, 512), f(8, 8), f(128, 128), f(128, 64), f(8, 8), f(64, 128), f(128, 128)]
+    return (lambda x, c1, a1, b1, c2, a2, b2: tlokr._MXTLoKrMLP.apply(x, W1, None, c1, a1, b1, None, 0.5, W2, None, c2, a2, b2,
+                                                                      None, 0.5)), ts, (2, rows, 512)
+
+
 @pytest.mark.parametrize("make,rows", [(_lokr, 32), (_lokr, 160), (_merged, 96), (_mlp, 64), (_tlokr, 48), (_tlokr, 128)])
 def test_every_gradient_subset_and_the_checkpointed_pass_give_the_same_bits(make, rows):
     from anima_trainer_sm120_b200 import fp8_quant
@@ -85,6 +96,20 @@ def test_every_gradient_subset_and_the_checkpointed_pass_give_the_same_bits(make
 
     y3, again = go(everything, checkpointed)
     assert torch.equal(y3, y) and all(torch.equal(a, b) for a, b in zip(again, grads))
+
+
+@pytest.mark.parametrize("make,rows", [(_lokr, 32), (_merged, 96), (_mlp, 64), (_tlokr, 128), (_tlokr_mlp, 128)])
+def test_backward_through_a_first_pass_without_a_checkpoint_is_refused(make, rows):
+    """Its operands are stand-ins without memory; the refusal comes before the first launch of the node."""
+    from anima_trainer_sm120_b200 import fp8_quant
+    fn, ts, out_shape = make(rows)
+    leaves = [t.clone().requires_grad_() for t in ts]
+    fp8_quant.clear_activation_memo()
+    with fp8_quant.first_pass():
+        y = fn(*leaves)
+    with pytest.raises(RuntimeError, match="first_pass"):
+        y.backward(torch.ones(out_shape, device=DEV, dtype=BF16))
+    assert all(t.grad is None for t in leaves)
 
 
 def _block_inputs(B, hw, D, mod_grad, chunked):
