@@ -491,39 +491,43 @@ void launch_finalize(const float* partial, int64_t bt, int chunks, int nout, int
 
 // ------------------------------------------------------------------ gated residual
 // A thread owns one 16-byte column chunk and walks rows: the gate is read once, and no index is divided per chunk.
-// cw = chunks of a row a CTA covers side by side, threads / cw rows at a time; blockIdx.z = column tile of rows
-// wider than a CTA.
+// cw = chunks of a row a CTA covers side by side, threads / cw rows at a time; rows wider than a CTA have `tiles` column
+// tiles, the inner part of blockIdx.x. blockIdx.y = sample, in steps of gridDim.y where there are more than a grid has.
 constexpr int kGatedThreadsPerSm = 1024;   // backward: 64 registers, two groups of rows in flight per scheduler
 template <int U>
 __global__ void __launch_bounds__(kThreads)
 gated_add_fwd_kernel(const bf16_t* __restrict__ x, const bf16_t* __restrict__ gate, const bf16_t* __restrict__ y, int64_t hw,
-                     int64_t ld_mod, int64_t d, int cw, int64_t rows_per_cta, bf16_t* __restrict__ out) {
+                     int64_t ld_mod, int64_t d, int cw, int64_t rows_per_cta, int64_t samples, unsigned tiles,
+                     bf16_t* __restrict__ out) {
   const int ty = threadIdx.x / cw, tx = threadIdx.x - ty * cw, ny = kThreads / cw;
-  const int64_t bt = blockIdx.y, c = (static_cast<int64_t>(blockIdx.z) * cw + tx) * 8;
+  const unsigned part = blockIdx.x / tiles, tile = blockIdx.x - part * tiles;
+  const int64_t c = (static_cast<int64_t>(tile) * cw + tx) * 8;
   if (ty >= ny || c >= d) return;
-  const int64_t begin = blockIdx.x * rows_per_cta, end = min(hw, begin + rows_per_cta);
-  const uint4 g = *reinterpret_cast<const uint4*>(gate + bt * ld_mod + c);
-  const int64_t base = bt * hw * d + c;
-  for (int64_t r = begin + ty; r < end; r += static_cast<int64_t>(ny) * U) {
-    uint4 xa[U], ya[U];
+  const int64_t begin = part * rows_per_cta, end = min(hw, begin + rows_per_cta);
+  for (int64_t bt = blockIdx.y; bt < samples; bt += gridDim.y) {
+    const uint4 g = *reinterpret_cast<const uint4*>(gate + bt * ld_mod + c);
+    const int64_t base = bt * hw * d + c;
+    for (int64_t r = begin + ty; r < end; r += static_cast<int64_t>(ny) * U) {
+      uint4 xa[U], ya[U];
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const int64_t row = r + static_cast<int64_t>(u) * ny;
-      if (row < end) {
-        xa[u] = ldg_stream16(x + base + row * d);
-        ya[u] = ldg_stream16(y + base + row * d);
+      for (int u = 0; u < U; ++u) {
+        const int64_t row = r + static_cast<int64_t>(u) * ny;
+        if (row < end) {
+          xa[u] = ldg_stream16(x + base + row * d);
+          ya[u] = ldg_stream16(y + base + row * d);
+        }
       }
-    }
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const int64_t row = r + static_cast<int64_t>(u) * ny;
-      if (row < end) {
-        uint4 o;
-        o.x = bf16_of_f2(f2_fma_bf16(g.x, ya[u].x, f2_of_bf16(xa[u].x)));
-        o.y = bf16_of_f2(f2_fma_bf16(g.y, ya[u].y, f2_of_bf16(xa[u].y)));
-        o.z = bf16_of_f2(f2_fma_bf16(g.z, ya[u].z, f2_of_bf16(xa[u].z)));
-        o.w = bf16_of_f2(f2_fma_bf16(g.w, ya[u].w, f2_of_bf16(xa[u].w)));
-        stg_stream16(out + base + row * d, o);
+      for (int u = 0; u < U; ++u) {
+        const int64_t row = r + static_cast<int64_t>(u) * ny;
+        if (row < end) {
+          uint4 o;
+          o.x = bf16_of_f2(f2_fma_bf16(g.x, ya[u].x, f2_of_bf16(xa[u].x)));
+          o.y = bf16_of_f2(f2_fma_bf16(g.y, ya[u].y, f2_of_bf16(xa[u].y)));
+          o.z = bf16_of_f2(f2_fma_bf16(g.z, ya[u].z, f2_of_bf16(xa[u].z)));
+          o.w = bf16_of_f2(f2_fma_bf16(g.w, ya[u].w, f2_of_bf16(xa[u].w)));
+          stg_stream16(out + base + row * d, o);
+        }
       }
     }
   }
@@ -742,16 +746,15 @@ int gated_forward(const void* x, const void* gate, int64_t ld_gate, const void* 
   ANIMA_REQUIRE(all_aligned({x, gate, y, o}), ANIMA_E_ALIGN, "gated_add_fwd: tensors must be 16-byte aligned");
   if (rows == 0) return ANIMA_OK;
   const int64_t bt = rows / hw, d8 = d / 8;
-  ANIMA_REQUIRE(bt <= 65535, ANIMA_E_TOO_LARGE, "gated_add_fwd: rows/hw=%lld exceeds 65535", (long long)bt);
   constexpr int U = 4;
   const int cw = static_cast<int>(std::min<int64_t>(d8, kThreads)), ny = kThreads / cw;
   const int64_t tiles = ceil_div(d8, cw);
-  ANIMA_REQUIRE(tiles <= 65535, ANIMA_E_TOO_LARGE, "gated_add_fwd: d=%lld is too wide", (long long)d);
   // about eight CTAs a SM; a CTA takes at least one unrolled step of rows
   const int64_t want = std::max<int64_t>(1, 8LL * sm_count() / std::max<int64_t>(1, bt * tiles));
   const int64_t rpc = ceil_div(ceil_div(hw, want), static_cast<int64_t>(ny) * U) * ny * U;
-  gated_add_fwd_kernel<U><<<dim3(static_cast<unsigned>(ceil_div(hw, rpc)), static_cast<unsigned>(bt), static_cast<unsigned>(tiles)),
-                            kThreads, 0, static_cast<cudaStream_t>(stream)>>>(in(x), in(gate), in(y), hw, ld_gate, d, cw, rpc, out(o));
+  const dim3 grid(static_cast<unsigned>(ceil_div(hw, rpc) * tiles), static_cast<unsigned>(std::min<int64_t>(bt, 65535)));
+  gated_add_fwd_kernel<U><<<grid, kThreads, 0, static_cast<cudaStream_t>(stream)>>>(
+      in(x), in(gate), in(y), hw, ld_gate, d, cw, rpc, bt, static_cast<unsigned>(tiles), out(o));
   ANIMA_CHECK_LAUNCH("gated_add_fwd");
   return ANIMA_OK;
 }

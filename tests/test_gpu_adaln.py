@@ -129,6 +129,18 @@ def test_gated_add_elementwise_outputs_bit_exact():
     _close(d_g, dg_o.to(BF16))
 
 
+@pytest.mark.parametrize("BT,HW,D", [(65535, 1, 8), (65536, 2, 8), (131073, 1, 16), (2, 3, 2056), (1, 70, 4104)])
+def test_gated_add_takes_any_number_of_samples_and_any_width(BT, HW, D):
+    ops = _ops()
+    g = torch.Generator(device="cuda").manual_seed(BT)
+    x, y = (torch.randn(BT * HW, D, device="cuda", generator=g).to(BF16) for _ in range(2))
+    gate = torch.randn(BT, D, device="cuda", generator=g).to(BF16)
+    want = torch.addcmul(x.float(), gate.float().repeat_interleave(HW, 0), y.float()).to(BF16)
+    got = ops.gated_add_fwd(x, gate, y, HW)
+    # the fp32 product of two bf16 is exact, so one fma or a product and a sum round alike
+    assert torch.equal(got, want)
+
+
 def test_reductions_are_bit_reproducible():
     ops = _ops()
     x, s, b, gate, y2, dy = (t.cuda() for t in _case(8, 512, 2048, seed=7))
