@@ -68,6 +68,7 @@ PROTOTYPES: dict[str, tuple[object, list[object]]] = {
     "anima_gated_add_bwd_workspace_bytes": (I64, [I64, I64, I64]),
     "anima_gated_add_bwd": (c_int, [P, P, P, I64, I64, I64, P, P, P, I64, P]),
     "anima_adaln_fwd_ex": (c_int, [P, P, P, P, P, I64, c_float, I64, I64, I64, P, P, P, P, P, P, c_int, P]),
+    "anima_adaln_bwd_ex_workspace_bytes": (I64, [I64, I64, I64, c_int]),
     "anima_adaln_bwd_ex": (c_int, [P, P, P, P, P, P, I64, P, P, I64, I64, I64, P, P, P, P, P, P, I64, P]),
     "anima_gated_add_fwd_ex": (c_int, [P, P, I64, P, I64, I64, I64, P, P]),
     "anima_gated_add_bwd_ex": (c_int, [P, P, P, I64, I64, I64, I64, P, P, P, I64, P]),

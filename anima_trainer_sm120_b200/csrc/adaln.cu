@@ -203,9 +203,15 @@ struct RowSplit {
   int rows_per_chunk;  // multiple of kRowsPerIter
 };
 
-RowSplit make_split(int64_t bt, int64_t hw, int64_t d, int threads_per_sm = 512) {
+// `sums` = column sums carried (2 dscale, dshift; 3 with dgate; 1 dgate alone). Two splits: the least one, two CTAs a SM,
+// and the full one, which keeps 512 threads a SM (1024 for dgate alone: fewer registers) also where rows are narrow. Every
+// CTA writes partial sums, so the full split needs up to eight times the workspace. The entries of a fixed workspace contract
+// use the least split; the _ex entries the full one where the caller's workspace holds it.
+constexpr int kGatedThreadsPerSm = 1024;   // gated_add_bwd: 64 registers, two groups of rows in flight per scheduler
+RowSplit make_split(int64_t bt, int64_t hw, int64_t d, int sums, bool full) {
   const int threads = static_cast<int>(std::min<int64_t>(kMaxBwdThreads, ceil_div(ceil_div(d, 8), 32) * 32));
-  const int64_t target = static_cast<int64_t>(sm_count()) * std::max(2, threads_per_sm / threads);
+  const int per_sm = full ? std::max(2, (sums == 1 ? kGatedThreadsPerSm : 512) / threads) : 2;
+  const int64_t target = static_cast<int64_t>(sm_count()) * per_sm;
   int64_t chunks = std::max<int64_t>(1, ceil_div(target, std::max<int64_t>(bt, 1)));
   int64_t rpc = ceil_div(ceil_div(hw, chunks), kRowsPerIter) * kRowsPerIter;
   chunks = ceil_div(hw, rpc);
@@ -493,7 +499,6 @@ void launch_finalize(const float* partial, int64_t bt, int chunks, int nout, int
 // A thread owns one 16-byte column chunk and walks rows: the gate is read once, and no index is divided per chunk.
 // cw = chunks of a row a CTA covers side by side, threads / cw rows at a time; rows wider than a CTA have `tiles` column
 // tiles, the inner part of blockIdx.x. blockIdx.y = sample, in steps of gridDim.y where there are more than a grid has.
-constexpr int kGatedThreadsPerSm = 1024;   // backward: 64 registers, two groups of rows in flight per scheduler
 template <int U>
 __global__ void __launch_bounds__(kThreads)
 gated_add_fwd_kernel(const bf16_t* __restrict__ x, const bf16_t* __restrict__ gate, const bf16_t* __restrict__ y, int64_t hw,
@@ -693,10 +698,10 @@ int launch_adaln_bwd(dim3 grid, int threads, const BwdArgs& a, cudaStream_t s) {
   return ANIMA_OK;
 }
 
-int64_t partial_bytes(int64_t rows, int64_t hw, int64_t d, int nout) {
+int64_t partial_bytes(int64_t rows, int64_t hw, int64_t d, int sums, bool full) {
   if (rows < 0 || hw <= 0 || d <= 0 || rows % hw) return ANIMA_E_SHAPE;
-  const int64_t chunks = make_split(rows / hw, hw, d, nout == 1 ? kGatedThreadsPerSm : 512).chunks;
-  return (rows / hw) * chunks * nout * d * static_cast<int64_t>(sizeof(float));
+  const int64_t chunks = make_split(rows / hw, hw, d, sums, full).chunks;
+  return (rows / hw) * chunks * sums * d * static_cast<int64_t>(sizeof(float));
 }
 
 // All AdaLN backward forms (see BwdMode); null dscale, dshift and dgate: no partial sums, no workspace.
@@ -712,11 +717,11 @@ int backward(const char* who, BwdMode mode, BwdArgs a, int64_t rows, void* dscal
   if (rows == 0) return ANIMA_OK;
   const int64_t bt = rows / a.hw;
   if (int rc = check_batch(who, bt)) return rc;
-  const RowSplit sp = make_split(bt, a.hw, a.d);
   const bool mod = dscale || dshift || dgate;
   const int nout = mode == kGated ? 3 : 2;
+  const RowSplit sp = make_split(bt, a.hw, a.d, nout, !mod || workspace_bytes >= partial_bytes(rows, a.hw, a.d, nout, true));
   if (mod) {
-    const int64_t need = partial_bytes(rows, a.hw, a.d, nout);
+    const int64_t need = partial_bytes(rows, a.hw, a.d, nout, false);
     ANIMA_REQUIRE(workspace && aligned16(workspace) && workspace_bytes >= need, ANIMA_E_WORKSPACE,
                   "%s: workspace of %lld bytes (16-byte aligned) required, got %lld", who, (long long)need,
                   (long long)workspace_bytes);
@@ -736,6 +741,13 @@ int backward(const char* who, BwdMode mode, BwdArgs a, int64_t rows, void* dscal
     ANIMA_CHECK_LAUNCH("adaln_bwd finalize");
   }
   return ANIMA_OK;
+}
+
+// What an entry of a fixed workspace contract may use of its workspace: the least split's bytes, however large it is, so
+// that its sums do not depend on the size.
+int64_t at_most_least(int64_t workspace_bytes, int64_t rows, int64_t hw, int64_t d, int sums) {
+  const int64_t least = partial_bytes(rows, hw, d, sums, false);
+  return least >= 0 ? std::min(workspace_bytes, least) : workspace_bytes;
 }
 
 int gated_forward(const void* x, const void* gate, int64_t ld_gate, const void* y, int64_t rows, int64_t hw, int64_t d,
@@ -768,7 +780,7 @@ int gated_backward(const void* dout, const void* y, const void* gate, int64_t ld
   if (rows == 0) return ANIMA_OK;
   const int64_t bt = rows / hw;
   if (int rc = check_batch("gated_add_bwd", bt)) return rc;
-  const RowSplit sp = make_split(bt, hw, d, kGatedThreadsPerSm);
+  const RowSplit sp = make_split(bt, hw, d, 1, !dgate || workspace_bytes >= partial_bytes(rows, hw, d, 1, true));
   const dim3 grid(sp.chunks, static_cast<unsigned>(bt));
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   float* ws = static_cast<float*>(workspace);
@@ -777,7 +789,7 @@ int gated_backward(const void* dout, const void* y, const void* gate, int64_t ld
     ANIMA_CHECK_LAUNCH("gated_add_bwd");
     return ANIMA_OK;
   }
-  const int64_t need = partial_bytes(rows, hw, d, 1);
+  const int64_t need = partial_bytes(rows, hw, d, 1, false);
   ANIMA_REQUIRE(workspace && aligned16(workspace) && workspace_bytes >= need, ANIMA_E_WORKSPACE,
                 "gated_add_bwd: workspace of %lld bytes (16-byte aligned) required, got %lld",
                 (long long)need, (long long)workspace_bytes);
@@ -793,7 +805,12 @@ int gated_backward(const void* dout, const void* y, const void* gate, int64_t ld
 
 using namespace anima;
 
-// The entries with every option: pitch of the modulation rows, null outputs for gradients nobody wants.
+// The entries with every option: pitch of the modulation rows, null outputs for gradients nobody wants, full row split.
+extern "C" int64_t anima_adaln_bwd_ex_workspace_bytes(int64_t rows, int64_t hw, int64_t d, int sums) {
+  if (sums < 1 || sums > 3) return ANIMA_E_ARG;
+  return partial_bytes(rows, hw, d, sums, true);
+}
+
 extern "C" int anima_adaln_fwd_ex(const void* x, const void* gate, const void* sub, const void* scale, const void* shift,
                                   int64_t ld_mod, float eps, int64_t rows, int64_t hw, int64_t d, void* x_new, void* y,
                                   float* mean, float* rstd, uint8_t* codes_row, uint8_t* scales_row, int scale_layout,
@@ -857,7 +874,7 @@ extern "C" int anima_gated_add_adaln_fwd_quant(const void* x, const void* gate, 
 }
 
 extern "C" int64_t anima_adaln_bwd_workspace_bytes(int64_t rows, int64_t hw, int64_t d) {
-  return partial_bytes(rows, hw, d, 2);
+  return partial_bytes(rows, hw, d, 2, false);
 }
 
 extern "C" int anima_adaln_bwd(const void* dy, const void* x, const void* scale, const float* mean,
@@ -866,11 +883,11 @@ extern "C" int anima_adaln_bwd(const void* dy, const void* x, const void* scale,
                                void* stream) {
   ANIMA_REQUIRE(dscale && dshift, ANIMA_E_ARG, "adaln_bwd: null pointer");
   return anima_adaln_bwd_ex(dy, nullptr, x, scale, nullptr, nullptr, d, mean, rstd, rows, hw, d, dx, nullptr, dscale, dshift,
-                            nullptr, workspace, workspace_bytes, stream);
+                            nullptr, workspace, at_most_least(workspace_bytes, rows, hw, d, 2), stream);
 }
 
 extern "C" int64_t anima_gated_add_adaln_bwd_workspace_bytes(int64_t rows, int64_t hw, int64_t d) {
-  return partial_bytes(rows, hw, d, 3);
+  return partial_bytes(rows, hw, d, 3, false);
 }
 
 extern "C" int anima_gated_add_adaln_bwd(const void* d_y, const void* d_xnew, const void* x_new, const void* scale,
@@ -880,7 +897,7 @@ extern "C" int anima_gated_add_adaln_bwd(const void* d_y, const void* d_xnew, co
                                          void* stream) {
   ANIMA_REQUIRE(sub && dscale && dshift && dgate, ANIMA_E_ARG, "gated_add_adaln_bwd: null pointer");
   return anima_adaln_bwd_ex(d_y, d_xnew, x_new, scale, gate, sub, d, mean, rstd, rows, hw, d, dx, dsub, dscale, dshift,
-                            dgate, workspace, workspace_bytes, stream);
+                            dgate, workspace, at_most_least(workspace_bytes, rows, hw, d, 3), stream);
 }
 
 extern "C" int anima_gated_add_fwd(const void* x, const void* gate, const void* y, int64_t rows,
@@ -889,14 +906,15 @@ extern "C" int anima_gated_add_fwd(const void* x, const void* gate, const void* 
 }
 
 extern "C" int64_t anima_gated_add_bwd_workspace_bytes(int64_t rows, int64_t hw, int64_t d) {
-  return partial_bytes(rows, hw, d, 1);
+  return partial_bytes(rows, hw, d, 1, false);
 }
 
 extern "C" int anima_gated_add_bwd(const void* dout, const void* y, const void* gate, int64_t rows,
                                    int64_t hw, int64_t d, void* dy, void* dgate, void* workspace,
                                    int64_t workspace_bytes, void* stream) {
   ANIMA_REQUIRE(y && dgate, ANIMA_E_ARG, "gated_add_bwd: null pointer");
-  return gated_backward(dout, y, gate, d, rows, hw, d, dy, dgate, workspace, workspace_bytes, stream);
+  return gated_backward(dout, y, gate, d, rows, hw, d, dy, dgate, workspace, at_most_least(workspace_bytes, rows, hw, d, 1),
+                        stream);
 }
 
 // ------------------------------------------------------------------ adaln_bwd without caller scratch

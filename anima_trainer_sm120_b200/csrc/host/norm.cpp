@@ -75,7 +75,7 @@ std::tuple<Tensor, Tensor, Tensor> adaln_bwd(const Launch& l, const Tensor& dy_,
   const Tensor dy = bf16_contiguous(dy_), d_res = d_res_.defined() ? bf16_contiguous(d_res_) : Tensor();
   const float* stats = stats_.data_ptr<float>();
   Tensor dx = like(x, l.dev), ds, db;
-  const int64_t bytes = mod ? check(anima_adaln_bwd_workspace_bytes(r.n, r.hw, r.d)) : 0;
+  const int64_t bytes = mod ? check(anima_adaln_bwd_ex_workspace_bytes(r.n, r.hw, r.d, 2)) : 0;
   const Tensor ws = scratch(bytes, l.dev);
   if (mod) {
     ds = dense_like(scale, l.dev);
@@ -90,7 +90,7 @@ std::pair<Tensor, Tensor> gated_bwd(const Launch& l, const Tensor& dout_, const 
                                     bool mod) {
   const Rows r = rows_of(y);
   const Tensor dout = bf16_contiguous(dout_);
-  const int64_t bytes = mod ? check(anima_gated_add_bwd_workspace_bytes(r.n, r.hw, r.d)) : 0;
+  const int64_t bytes = mod ? check(anima_adaln_bwd_ex_workspace_bytes(r.n, r.hw, r.d, 1)) : 0;
   const Tensor ws = scratch(bytes, l.dev);
   Tensor dy = like(y, l.dev), dg;
   if (mod) dg = dense_like(gate, l.dev);
@@ -204,7 +204,7 @@ struct BothNode : public HostNode {      // saves sub, gate, x_new, scale, stati
     if (d_xnew.defined() && d_y.defined()) {      // the usual case: one kernel for both backward ops
       const Rows r = rows_of(x_new);
       const Tensor dy = bf16_contiguous(d_y), dn = bf16_contiguous(d_xnew);
-      const int64_t bytes = mod ? check(anima_gated_add_adaln_bwd_workspace_bytes(r.n, r.hw, r.d)) : 0;
+      const int64_t bytes = mod ? check(anima_adaln_bwd_ex_workspace_bytes(r.n, r.hw, r.d, 3)) : 0;
       const Tensor ws = scratch(bytes, l.dev);
       const float* st = stats.data_ptr<float>();
       dx = like(x_new, l.dev);

@@ -349,12 +349,12 @@ def gated_add_adaln_bwd(d_y: torch.Tensor, d_xnew: torch.Tensor, x_new: torch.Te
     if rows == 0:
         return dx, dsub, dscale, dshift, dgate
     lib = _lib.load()
-    nbytes = check(lib.anima_gated_add_adaln_bwd_workspace_bytes(rows, hw, d))
+    nbytes = check(lib.anima_adaln_bwd_ex_workspace_bytes(rows, hw, d, 3))
     ws = _lib.workspace(nbytes, dev, "gated_adaln_bwd")
     with torch.cuda.device(dev):
-        check(lib.anima_gated_add_adaln_bwd(ptr(d_y), ptr(d_xnew), ptr(x_new), ptr(scale), ptr(mean), ptr(rstd),
-                                            ptr(sub), ptr(gate), rows, hw, d, ptr(dx), ptr(dsub), ptr(dscale),
-                                            ptr(dshift), ptr(dgate), ptr(ws), ws.numel(), _lib.stream_ptr(dev)))
+        check(lib.anima_adaln_bwd_ex(ptr(d_y), ptr(d_xnew), ptr(x_new), ptr(scale), ptr(gate), ptr(sub), d, ptr(mean),
+                                     ptr(rstd), rows, hw, d, ptr(dx), ptr(dsub), ptr(dscale), ptr(dshift), ptr(dgate),
+                                     ptr(ws), ws.numel(), _lib.stream_ptr(dev)))
     return dx, dsub, dscale, dshift, dgate
 
 
@@ -363,14 +363,15 @@ def adaln_bwd(dy: torch.Tensor, x: torch.Tensor, scale: torch.Tensor, mean: torc
     dev = _lib.require_cuda(dy, x, scale, mean, rstd)
     rows, d = x.shape
     lib = _lib.load()
-    nbytes = check(lib.anima_adaln_bwd_workspace_bytes(rows, hw, d))
+    nbytes = check(lib.anima_adaln_bwd_ex_workspace_bytes(rows, hw, d, 2))
     ws = _lib.workspace(nbytes, dev, "adaln")
     dx = torch.empty_like(x)
     dscale = torch.empty_like(scale)
     dshift = torch.empty_like(scale)
     with torch.cuda.device(dev):
-        check(lib.anima_adaln_bwd(ptr(dy), ptr(x), ptr(scale), ptr(mean), ptr(rstd), rows, hw, d, ptr(dx),
-                                  ptr(dscale), ptr(dshift), ptr(ws), ws.numel(), _lib.stream_ptr(dev)))
+        check(lib.anima_adaln_bwd_ex(ptr(dy), None, ptr(x), ptr(scale), None, None, d, ptr(mean), ptr(rstd), rows, hw, d,
+                                     ptr(dx), None, ptr(dscale), ptr(dshift), None, ptr(ws), ws.numel(),
+                                     _lib.stream_ptr(dev)))
     return dx, dscale, dshift
 
 
@@ -389,13 +390,13 @@ def gated_add_bwd(dout: torch.Tensor, y: torch.Tensor, gate: torch.Tensor, hw: i
     dev = _lib.require_cuda(dout, y, gate)
     rows, d = y.shape
     lib = _lib.load()
-    nbytes = check(lib.anima_gated_add_bwd_workspace_bytes(rows, hw, d))
+    nbytes = check(lib.anima_adaln_bwd_ex_workspace_bytes(rows, hw, d, 1))
     ws = _lib.workspace(nbytes, dev, "gated")
     dy = torch.empty_like(y)
     dgate = torch.empty_like(gate)
     with torch.cuda.device(dev):
-        check(lib.anima_gated_add_bwd(ptr(dout), ptr(y), ptr(gate), rows, hw, d, ptr(dy), ptr(dgate),
-                                      ptr(ws), ws.numel(), _lib.stream_ptr(dev)))
+        check(lib.anima_gated_add_bwd_ex(ptr(dout), ptr(y), ptr(gate), d, rows, hw, d, ptr(dy), ptr(dgate), ptr(ws),
+                                         ws.numel(), _lib.stream_ptr(dev)))
     return dy, dgate
 
 

@@ -330,8 +330,11 @@ int anima_gated_add_adaln_bwd(const void* d_y, const void* d_xnew, const void* x
  *            sub != NULL (needs d_res): also dsub and dgate of the gated residual that made x.
  *            dscale, dshift and dgate may be NULL: not computed, and with all of them NULL no workspace is used.
  *   gated_add_bwd_ex   dgate may be NULL (then y may be, and no workspace is used).
- * Workspaces: anima_adaln_bwd_workspace_bytes (no sub), anima_gated_add_adaln_bwd_workspace_bytes (sub),
- * anima_gated_add_bwd_workspace_bytes. */
+ * Workspaces: at least anima_adaln_bwd_workspace_bytes (no sub), anima_gated_add_adaln_bwd_workspace_bytes (sub),
+ * anima_gated_add_bwd_workspace_bytes. With anima_adaln_bwd_ex_workspace_bytes (sums = 2, 3 and 1 for these three) or more,
+ * narrow rows are cut into more pieces: faster, another association of the column sums. The entries above use the least
+ * cut whatever they are given. */
+int64_t anima_adaln_bwd_ex_workspace_bytes(int64_t rows, int64_t hw, int64_t d, int sums);
 int anima_adaln_fwd_ex(const void* x, const void* gate, const void* sub, const void* scale, const void* shift,
                        int64_t ld_mod, float eps, int64_t rows, int64_t hw, int64_t d, void* x_new, void* y,
                        float* mean, float* rstd, uint8_t* codes_row, uint8_t* scales_row, int scale_layout,

@@ -36,6 +36,12 @@ def test_abi_version_and_sizes(lib):
     assert lib.anima_mx_scales_bytes(8, 33, _lib.SCALES_PLAIN) == -3
     assert lib.anima_lokr_kron_backward_workspace_bytes(8192, 2048, 8, 8) == (1024 * 32 // 128) * 64 * 4
     assert lib.anima_adaln_bwd_workspace_bytes(100, 7, 64) == -3       # rows not a multiple of hw
+    # column sums: one chunk of a sample a CTA, two CTAs on each of 148 SMs, 4 rows the least; more only for the _ex entries
+    assert lib.anima_adaln_bwd_workspace_bytes(520 * 64, 64, 1024) == 520 * 2 * 1024 * 4
+    assert lib.anima_gated_add_adaln_bwd_workspace_bytes(2300 * 8, 8, 256) == 2300 * 3 * 256 * 4
+    assert lib.anima_gated_add_bwd_workspace_bytes(1200, 1200, 2048) == 150 * 2048 * 4
+    assert lib.anima_adaln_bwd_ex_workspace_bytes(520 * 64, 64, 1024, 2) == 2 * 520 * 2 * 1024 * 4
+    assert lib.anima_adaln_bwd_ex_workspace_bytes(100, 7, 64, 2) == -3 and lib.anima_adaln_bwd_ex_workspace_bytes(8, 4, 64, 4) == -1
     assert lib.anima_tlokr_rank_mix_wgrad_workspace_bytes(2, 3, 12) == -3  # rank % 8
 
 

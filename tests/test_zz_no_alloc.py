@@ -63,3 +63,21 @@ def test_noalloc_entry_refuses_shapes_beyond_the_built_in_array(lib):
     rc = lib.anima_adaln_bwd_noalloc(dy.data_ptr(), x.data_ptr(), scale.data_ptr(), mean.data_ptr(), mean.data_ptr(),
                                      10, 4, 64, x.data_ptr(), scale.data_ptr(), scale.data_ptr(), None)
     assert rc == -3                                       # rows not a multiple of hw
+
+
+@pytest.mark.parametrize("bt,hw,d", [(520, 64, 1024), (2300, 8, 256), (1100, 20, 512)])
+def test_noalloc_entry_takes_many_samples_of_narrow_rows(lib, bt, hw, d):
+    """They fit the built-in array at one chunk a sample, not at the finer cut of the _ex entries."""
+    from anima_trainer_sm120_b200 import ops
+    assert lib.anima_adaln_bwd_workspace_bytes(bt * hw, hw, d) <= 8 << 20 < lib.anima_adaln_bwd_ex_workspace_bytes(bt * hw, hw, d, 2)
+    x, dy, scale, shift = _inputs(bt, hw, d, bt)
+    _, mean, rstd = ops.adaln_fwd(x, scale, shift, 1e-6, hw)
+    rc, dx, dscale, dshift = _call_noalloc(lib, dy, x, scale, mean, rstd, hw)
+    assert rc == 0, lib.anima_last_error()
+    full = ops.adaln_bwd(dy, x, scale, mean, rstd, hw)
+    assert torch.equal(dx, full[0])
+    # the same fp32 terms in another order, hw of them, then one rounding to bf16 each
+    xh = ((x.float() - mean[:, None]) * rstd[:, None]).view(bt, hw, d)
+    for got, want, terms in ((dscale, full[1], dy.float().view(bt, hw, d) * xh), (dshift, full[2], dy.float().view(bt, hw, d))):
+        bound = 2 * hw * 2.0 ** -24 * terms.abs().sum(1) + 2.0 ** -7 * want.float().abs()
+        assert bool(((got.float() - want.float()).abs() <= bound).all())
