@@ -36,6 +36,7 @@ I64 = c_int64
 PROTOTYPES: dict[str, tuple[object, list[object]]] = {
     "anima_abi_version": (c_int, []),
     "anima_last_error": (c_char_p, []),
+    "anima_kernel_launches": (I64, []),
     "anima_mx_quantize": (c_int, [P, I64, I64, I64, P, P, P, P, c_int, P]),
     "anima_mx_quantize_status": (c_int, []),
     "anima_mx_exponent_probe": (c_int, [P, I64, P, P, P]),

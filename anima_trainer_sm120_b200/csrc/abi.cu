@@ -1,4 +1,5 @@
 // Library-wide plumbing of the C ABI: version, per-thread error text, device facts.
+#include <atomic>
 #include <mutex>
 
 #include "common.cuh"
@@ -7,7 +8,10 @@ namespace anima {
 
 namespace {
 thread_local char g_error[512] = "";
+std::atomic<int64_t> g_launches{0};
 }
+
+void count_launch() { g_launches.fetch_add(1, std::memory_order_relaxed); }
 
 void set_error(const char* fmt, ...) {
   va_list ap;
@@ -34,3 +38,5 @@ int sm_count() {
 
 extern "C" int anima_abi_version(void) { return ANIMA_ABI_VERSION; }
 extern "C" const char* anima_last_error(void) { return anima::g_error; }
+
+extern "C" int64_t anima_kernel_launches(void) { return anima::g_launches.load(std::memory_order_relaxed); }

@@ -22,6 +22,7 @@ namespace anima {
 
 // ---- host-side error reporting -------------------------------------------------
 void set_error(const char* fmt, ...);
+void count_launch();   // one more kernel of this library started (anima_kernel_launches)
 
 #define ANIMA_REQUIRE(cond, code, ...)            \
   do {                                            \
@@ -31,6 +32,7 @@ void set_error(const char* fmt, ...);
     }                                             \
   } while (0)
 
+// after every launch, once
 #define ANIMA_CHECK_LAUNCH(what)                                                   \
   do {                                                                             \
     cudaError_t e__ = cudaGetLastError();                                          \
@@ -38,6 +40,7 @@ void set_error(const char* fmt, ...);
       ::anima::set_error("%s: launch failed: %s", what, cudaGetErrorString(e__));  \
       return ANIMA_E_CUDA;                                                         \
     }                                                                              \
+    ::anima::count_launch();                                                       \
   } while (0)
 
 static inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }

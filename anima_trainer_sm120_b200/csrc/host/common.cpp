@@ -1,6 +1,8 @@
 // Allocation and launch helpers of the native host path (see common.h).
 #include "common.h"
 
+#include <ATen/cuda/CUDAEvent.h>
+
 #include <atomic>
 #include <mutex>
 
@@ -197,6 +199,50 @@ std::pair<Op, Op> merge_quantize(const Launch& l, const Tensor& W, const Tensor&
   return {r, c};
 }
 
+namespace {
+std::atomic<bool> timing{false};
+std::mutex timed_mu;
+struct Timed {
+  at::cuda::CUDAEvent begin{cudaEventDefault}, end{cudaEventDefault};
+  double flops;
+};
+std::vector<std::unique_ptr<Timed>> timed;
+
+class GemmTimer {      // brackets the launches of its scope
+ public:
+  explicit GemmTimer(double flops) {
+    if (!timing.load(std::memory_order_relaxed)) return;
+    t_ = std::make_unique<Timed>();
+    t_->flops = flops;
+    t_->begin.record();
+  }
+  ~GemmTimer() {
+    if (!t_) return;
+    t_->end.record();
+    std::lock_guard<std::mutex> lock(timed_mu);
+    timed.push_back(std::move(t_));
+  }
+
+ private:
+  std::unique_ptr<Timed> t_;
+};
+}  // namespace
+
+void time_gemms(bool on) {
+  std::lock_guard<std::mutex> lock(timed_mu);
+  if (on) timed.clear();
+  timing.store(on);
+}
+std::vector<std::pair<double, double>> gemm_times() {
+  std::lock_guard<std::mutex> lock(timed_mu);
+  std::vector<std::pair<double, double>> out;
+  for (auto& t : timed) {
+    t->end.synchronize();
+    out.emplace_back(t->begin.elapsed_time(t->end), t->flops);
+  }
+  return out;
+}
+
 static void need_same_k(const Op& a, const Op& b) {
   TORCH_CHECK_VALUE(a.k == b.k, "contraction sizes differ: A has K=", a.k, ", B has K=", b.k);
 }
@@ -208,6 +254,7 @@ void gemm(const Launch& l, const Op& a, const Op& b, const GemmOut& out, const v
   const int64_t bytes = check(anima_mx_gemm_workspace_bytes(M, N, K));
   Tensor ws;
   if (bytes) ws = empty({bytes}, U8, l.dev);
+  const GemmTimer timer(2.0 * M * N * K);
   check(anima_mx_gemm_ex(a.codes, a.scales, b.codes, b.scales, out.c, M, N, K, out.ldc, bias,
                          residual, ldr, static_cast<float>(alpha), out.fp32 ? 1 : 0, ptr(ws), bytes,
                          status_word(l.dev), l.stream));
@@ -219,6 +266,7 @@ void gemm_delta(const Launch& l, const Op& a, const Op& b, const Op& planes, con
   const int64_t bytes = check(anima_mx_gemm_workspace_bytes(M, N, K));
   Tensor ws;
   if (bytes) ws = empty({bytes}, U8, l.dev);
+  const GemmTimer timer(2.0 * M * N * K + 256.0 * M * N);
   check(anima_mx_gemm_delta(a.codes, a.scales, b.codes, b.scales, c, M, N, K, N, bias, 0,
                             planes.codes, planes.scales, d.codes, d.scales, ptr(ws), bytes,
                             status_word(l.dev), l.stream));

@@ -116,6 +116,11 @@ Op regroup(const Launch& l, const Op& a, int64_t rows, int64_t k);
 std::pair<Op, Op> merge_quantize(const Launch& l, const Tensor& W, const Tensor& w1, const Tensor& w2, double alpha,
                                  bool row, bool col);
 
+// Measurement aid: while on, every GEMM of this path is bracketed by timed events on its stream (which also keeps it from
+// overlapping its neighbours; not for captures). gemm_times: (ms, flops) of each since it was switched on, oldest first.
+void time_gemms(bool on);
+std::vector<std::pair<double, double>> gemm_times();
+
 struct GemmOut {
   void* c;
   int64_t ldc;

@@ -110,6 +110,8 @@ PYBIND11_MODULE(_host, m) {
   m.doc() = "native autograd nodes and launch sequences above libanima_b200.so";
   py::class_<TLinear>(m, "TLinear");
   ANIMA_DEF("status_word", status_word_tensor);
+  ANIMA_DEF("time_gemms", time_gemms);
+  ANIMA_DEF("gemm_times", gemm_times);
   ANIMA_DEF("mx_quantize", py_quantize);
   ANIMA_DEF("mx_gemm", py_gemm);
   ANIMA_DEF("scales_retile", py_retile);

@@ -1497,6 +1497,7 @@ int launch_pair_width(const uint8_t* a_codes, const uint8_t* b_codes, GemmParams
   cfg.numAttrs = k_blocks <= kOverlapBlocks * pl.pairs ? 2 : 1;
   const cudaError_t rc = cudaLaunchKernelEx(&cfg, mx_gemm2_kernel<kBN2>, ma, mb, msa, msb, mc, mp, mpl, md, mplsf, mdsf, p);
   ANIMA_REQUIRE(rc == cudaSuccess, ANIMA_E_CUDA, "mx_gemm: cluster launch failed: %s", cudaGetErrorString(rc));
+  count_launch();
   if (pl.ws_bytes) {
     const int64_t threads = static_cast<int64_t>(pl.tail_tiles) * 256 * (kBN2 / 4);
     launch_after(pair_tail_finalize_kernel, static_cast<unsigned>(std::min<int64_t>(ceil_div(threads, 256), 8LL * sm_count())),

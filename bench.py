@@ -16,7 +16,8 @@ exchange of the data-parallel step; every rank works on its own batch shard: wea
            resident in HBM; the quantise / merge / Kronecker kernels are inside the timed region.
 `e2e`    = the same metric with every step's x and dy copied from pinned host memory and the adapter
            gradients plus a checksum of y copied back (weights stay resident, as in training).
-`roofline` is for the dominant kernel (the tcgen05 GEMM), timed with CUDA events inside the step; its peak is
+`roofline` is for the dominant kernel (the tcgen05 GEMM), every launch of it bracketed by CUDA events in a few steps
+           of the same kind after the timed region (the events would keep launches from overlapping); its peak is
            2 x the measured bf16 GEMM figure of MEASURED_PEAKS.json: the burst one when the sampled SM clock
            held within 5 % of its maximum or the timed region is shorter than a second, else the sustained one
            (both fractions are printed).
@@ -195,7 +196,7 @@ class Shape:
         self.x_host = x.to(torch.bfloat16).pin_memory() if host else x.to(torch.bfloat16)
         dy = (torch.randn(M_ROWS, n, generator=g) * 0.01).to(torch.bfloat16)
         self.dy_host = dy.pin_memory() if host else dy
-        self.x = self.x_host.to(dev)
+        self.x = self.x_host.to(dev).requires_grad_(True)      # an activation: the layer below wants its gradient
         self.dy = self.dy_host.to(dev)
         self.W = (torch.randn(n, k, generator=g) * 0.02).to(torch.bfloat16).to(dev)
         self.w1 = (torch.randn(FACTOR, FACTOR, generator=g) * 0.1).to(dev).requires_grad_(True)
@@ -245,7 +246,7 @@ def train_steps_per_s(dev, world: int, steps: int = 6, warmup: int = 2, checkpoi
 def run_gpu_arm(args) -> None:
     import torch.distributed as dist
 
-    from anima_trainer_sm120_b200 import _lib, ops
+    from anima_trainer_sm120_b200 import _lib
     from anima_trainer_sm120_b200.fp8_quant import clear_activation_memo, lokr_linear_fused
 
     world = int(os.environ.get("WORLD_SIZE", "1"))
@@ -266,34 +267,6 @@ def run_gpu_arm(args) -> None:
     grad_host = torch.empty(n_grad, dtype=torch.float32).pin_memory()
     chk_host = torch.empty(len(shapes), dtype=torch.float32).pin_memory()
     chk_dev = torch.zeros(len(shapes), dtype=torch.float32, device=dev)
-    gemm_events: list[tuple[torch.cuda.Event, torch.cuda.Event, float]] = []
-    launches = [0]
-
-    # time every tcgen05 GEMM launch with events on the launching stream
-    real_gemm = ops.mx_gemm
-
-    def timed_gemm(a, b, **kw):
-        e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-        e0.record()
-        out = real_gemm(a, b, **kw)
-        e1.record()
-        gemm_events.append((e0, e1, 2.0 * a.rows * b.rows * a.k))
-        # a shape whose last round of tiles is split along K is followed by its finalize kernel
-        if kw.get("split_k", True) and _lib.load().anima_mx_gemm_workspace_bytes(a.rows, b.rows, a.k) > 0:
-            launches[0] += 1
-        return out
-
-    def count(fn, n):
-        def wrapped(*a, **kw):
-            launches[0] += n
-            return fn(*a, **kw)
-        return wrapped
-
-    ops.mx_gemm = count(timed_gemm, 1)
-    ops.mx_quantize = count(ops.mx_quantize, 1)
-    ops.lokr_merge_quantize = count(ops.lokr_merge_quantize, 1)
-    ops.lokr_kron_backward = count(ops.lokr_kron_backward, 2)
-
     # e2e leg: every step's inputs come from pinned host memory. Two device slots per shape let the
     # copy of the NEXT step's inputs (copy stream) run under the current step's kernels; the timed
     # region waits for every copy it issued.
@@ -301,12 +274,12 @@ def run_gpu_arm(args) -> None:
 
     class Slot:
         def __init__(self, s):
-            self.x, self.dy = torch.empty_like(s.x), torch.empty_like(s.dy)
+            self.x, self.dy = torch.empty_like(s.x).requires_grad_(True), torch.empty_like(s.dy)
             self.ready, self.free = torch.cuda.Event(), torch.cuda.Event()
             self.free.record()
 
     def prefetch(s, slot):
-        with torch.cuda.stream(copy_stream):
+        with torch.cuda.stream(copy_stream), torch.no_grad():
             copy_stream.wait_event(slot.free)              # the kernels that read this slot are done
             slot.x.copy_(s.x_host, non_blocking=True)
             slot.dy.copy_(s.dy_host, non_blocking=True)
@@ -326,7 +299,7 @@ def run_gpu_arm(args) -> None:
                 slot = s.slots[s.cur]
                 torch.cuda.current_stream().wait_event(slot.ready)
                 x, dy = slot.x, slot.dy
-            s.w1.grad = s.w2.grad = None
+            s.w1.grad = s.w2.grad = x.grad = None
             clear_activation_memo()     # x is the same tensor object every step: quantise it again, as training does
             y = lokr_linear_fused(x, s.W, None, s.w1, s.w2, 1.0)
             y.backward(dy)
@@ -338,7 +311,7 @@ def run_gpu_arm(args) -> None:
                 flat_grad[off:off + p.numel()].copy_(p.grad.reshape(-1))
                 off += p.numel()
             if e2e:
-                chk_dev[i] = y[::4096, ::512].float().sum()
+                chk_dev[i] = y.detach()[::4096, ::512].float().sum()
         if world > 1:
             dist.all_reduce(flat_grad)
             flat_grad.mul_(1.0 / world)
@@ -350,16 +323,16 @@ def run_gpu_arm(args) -> None:
     def timed(e2e: bool, steps: int, warmup: int):
         for _ in range(warmup):
             step(e2e)
-        gemm_events.clear()
-        launches[0] = 0
         torch.cuda.synchronize()
         if world > 1:
             dist.barrier()
         torch.cuda.synchronize()
         e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        launches.append(_lib.load().anima_kernel_launches())
         e0.record()
         for _ in range(steps):
             step(e2e)
+        launches.append(_lib.load().anima_kernel_launches())
         if e2e:
             torch.cuda.current_stream().wait_stream(copy_stream)   # count every copy issued inside the region
         e1.record()
@@ -380,15 +353,25 @@ def run_gpu_arm(args) -> None:
     # sampled clocks mostly see the gaps between launches of a region this short
     probe = torch.zeros(8, dtype=torch.int64, device=dev)
     _lib.check(_lib.load().anima_mx_gemm_set_clock_probe(probe.data_ptr()))
+    launches = []           # this library's kernels launched before / after each timed region
     ms_total = timed(False, args.steps, max(args.warmup, 3))
     _lib.check(_lib.load().anima_mx_gemm_set_clock_probe(None))
     probe_cycles, probe_ns, probe_n = (int(v) for v in probe.cpu().tolist()[:3])
     clocks = sampler.stop() if rank == 0 else {}
     _lib.check_status_word(dev)
-    n_launch = launches[0]
-    gemm_ms = sum(a.elapsed_time(b) for a, b, _ in gemm_events)
-    gemm_fl = sum(f for _, _, f in gemm_events)
-    n_gemm = len(gemm_events)
+    n_launch = launches[1] - launches[0]
+    timed_steps = 4
+    _lib.host().time_gemms(True)
+    for _ in range(timed_steps):
+        step(False)
+    _lib.host().time_gemms(False)
+    gemms = _lib.host().gemm_times()
+    n_gemm = len(gemms) // timed_steps                            # a step
+    gemm_ms = sum(ms for ms, _ in gemms) / timed_steps
+    gemm_fl = sum(f for _, f in gemms) / timed_steps
+    if gemm_fl != gemm_flops_per_step() or n_launch < args.steps * n_gemm:
+        raise RuntimeError(f"the step ran {gemm_fl:.6g} GEMM flops in {n_gemm} GEMMs ({n_launch} kernels in {args.steps} steps); "
+                           f"the metric counts {gemm_flops_per_step():.6g}")
     prime_e2e()
     ms_e2e = timed(True, args.steps, 1)
     _lib.check_status_word(dev)
@@ -399,7 +382,6 @@ def run_gpu_arm(args) -> None:
     h2d = sum(s.x_host.numel() * 2 + s.dy_host.numel() * 2 for s in shapes)
     train = None
     if not args.no_train_step:
-        ops.mx_gemm = real_gemm                      # no per-launch events inside the training step
         for s in shapes:
             s.__dict__.clear()
         torch.cuda.empty_cache()
@@ -454,7 +436,7 @@ def run_gpu_arm(args) -> None:
         near_max = bool(sm and sm_max and sm >= 0.95 * sm_max)
         use_burst = near_max or ms_total < 1000.0
         peak = 2.0 * (burst if use_burst else sustained)
-        achieved = gemm_fl / (gemm_ms * 1e-3) / 1e12 if gemm_ms > 0 else 0.0
+        achieved = gemm_fl / (gemm_ms * 1e-3) / 1e12
         sm_count = torch.cuda.get_device_properties(dev).multi_processor_count
         ms_step = ms_total / args.steps
         fl = gemm_flops_per_step() * world
@@ -488,8 +470,8 @@ def run_gpu_arm(args) -> None:
                                                   "included) GEMM launches; util = achieved / (SMs x 8192 MAC/clk x "
                                                   "that clock): the kernel runs under the power cap, below the "
                                                   "clock nvidia-smi samples between launches"),
-                         "launches": n_gemm, "avg_launch_ms": gemm_ms / max(n_gemm, 1),
-                         "gemm_share_of_step": gemm_ms / ms_total},
+                         "launches": n_gemm * args.steps, "avg_launch_ms": gemm_ms / n_gemm,
+                         "gemm_share_of_step": gemm_ms / ms_step},
             "clocks": clocks,
         }
         if cpu is not None:

@@ -51,6 +51,8 @@ enum { ANIMA_SCALES_PLAIN = 0, ANIMA_SCALES_TILED = 1 };
 
 int anima_abi_version(void);
 const char* anima_last_error(void);
+/* Kernels of this library launched by this process so far (a captured launch counts once, its replays do not). */
+int64_t anima_kernel_launches(void);
 
 /* ---------------------------------------------------------------- MXFP8 quantise
  * ref: mxfp8_gemm.py:68-183 (quantize_rowwise + _quantize_rowwise_kernel),

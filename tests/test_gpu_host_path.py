@@ -238,6 +238,33 @@ def test_a_frozen_linear_belongs_to_the_graph_its_input_had_when_it_was_applied(
     assert bool(torch.isfinite(gx).all())
 
 
+def test_benchmark_step_runs_the_gemms_its_metric_counts():
+    """The operands of bench.py: forward, input gradient and weight gradient, each seen by the GEMM timer and the launch
+    counter. Without a gradient of x the same step has two GEMMs, so the count is of what ran."""
+    import bench
+    from anima_trainer_sm120_b200 import _lib, fp8_quant
+    rows, bench_rows = 512, bench.M_ROWS
+    try:
+        bench.M_ROWS = rows
+        s = bench.Shape(1024, 512, DEV, seed=0, host=False)
+    finally:
+        bench.M_ROWS = bench_rows
+    lib, host = _lib.load(), _lib.host()
+    for x, products in ((s.x, 3), (s.x.detach(), 2)):
+        fp8_quant.clear_activation_memo()
+        before = lib.anima_kernel_launches()
+        host.time_gemms(True)
+        fp8_quant.lokr_linear_fused(x, s.W, None, s.w1, s.w2, 1.0).backward(s.dy)
+        host.time_gemms(False)
+        times = host.gemm_times()
+        assert [f for _, f in times] == [2.0 * rows * 1024 * 512] * products and all(ms > 0 for ms, _ in times)
+        split = sum(lib.anima_mx_gemm_workspace_bytes(*mnk) > 0
+                    for mnk in [(rows, 1024, 512), (1024, 512, rows), (rows, 512, 1024)][:products])
+        # quantise x, merge, quantise dy, two Kronecker passes, the GEMMs and the finalize passes of split ones
+        assert lib.anima_kernel_launches() - before == 5 + products + split
+    assert s.x.grad is not None
+
+
 def test_tensors_of_another_device_tangents_and_wrong_shapes_are_refused_before_a_launch():
     import torch.autograd.forward_ad as fwAD
     from anima_trainer_sm120_b200 import adaln_kernel, fp8_quant, tlokr
