@@ -18,34 +18,35 @@ Tensor like(const Tensor& x, const at::Device& dev, at::ScalarType dt = BF16) {
 }
 Tensor back_to(const Tensor& t, at::ScalarType dt) { return t.defined() ? cast(t, dt) : t; }
 
-// The (B, T, 1, 1, D) modulation tensors of one call as the kernels take them: bf16 rows with one pitch. Chunks of a
-// wider tensor (what a modulation MLP returns) are used where they lie; anything else is copied dense.
+// The modulation tensors of one call as the kernels take them: bf16 rows of d with one pitch. (B, T, 1, 1, d) tensors, also
+// chunks of a wider tensor (what a modulation MLP returns), are used where they lie; any other shape with as many elements
+// is read in order, as dense rows.
 struct Mods {
   std::vector<Tensor> t;
   int64_t ld;
 };
 // pitch of the samples' rows; 0 = any (one sample), -1 = not usable in place
-int64_t pitch_of(const Tensor& m) {
-  if (m.scalar_type() != BF16 || m.dim() != 5 || m.stride(4) != 1 || m.size(2) * m.size(3) != 1 ||
+int64_t pitch_of(const Tensor& m, int64_t d) {
+  if (m.scalar_type() != BF16 || m.dim() != 5 || m.size(4) != d || m.stride(4) != 1 || m.size(2) * m.size(3) != 1 ||
       (reinterpret_cast<uintptr_t>(m.data_ptr()) & 15))
     return -1;
   const int64_t B = m.size(0), T = m.size(1);
   if (B * T == 1) return 0;
   if (B > 1 && T > 1 && m.stride(0) != T * m.stride(1)) return -1;
   const int64_t ld = T > 1 ? m.stride(1) : m.stride(0);
-  return ld >= m.size(4) && ld % 8 == 0 ? ld : -1;
+  return ld >= d && ld % 8 == 0 ? ld : -1;
 }
-Mods mods_of(std::initializer_list<const Tensor*> ts) {
+Mods mods_of(int64_t d, std::initializer_list<const Tensor*> ts) {
   Mods m{{}, 0};
   bool in_place = true;
   const int64_t n = (*ts.begin())->numel();
   for (const Tensor* t : ts) {
     TORCH_CHECK_VALUE(t->numel() == n, "modulation tensors of different sizes");
-    const int64_t ld = pitch_of(*t);
+    const int64_t ld = pitch_of(*t, d);
     if (ld < 0 || (ld && m.ld && ld != m.ld)) in_place = false;
     if (ld > 0) m.ld = ld;
   }
-  if (!in_place || !m.ld) m.ld = (*ts.begin())->size(-1);
+  if (!in_place || !m.ld) m.ld = d;
   for (const Tensor* t : ts) m.t.push_back(in_place ? *t : bf16_contiguous(*t));
   return m;
 }
@@ -60,7 +61,7 @@ struct AdalnOut {
 };
 AdalnOut adaln_fwd(const Launch& l, const Tensor& x, const Tensor& scale, const Tensor& shift, float eps, bool quant) {
   const Rows r = rows_of(x);
-  AdalnOut o{like(x, l.dev), bf16_contiguous(x), empty({2, r.n}, F32, l.dev), mods_of({&scale, &shift}), {}};
+  AdalnOut o{like(x, l.dev), bf16_contiguous(x), empty({2, r.n}, F32, l.dev), mods_of(r.d, {&scale, &shift}), {}};
   float* stats = o.stats.data_ptr<float>();
   if (quant) o.emitted = empty_op(r.n, r.d, l.dev);
   check(anima_adaln_fwd_ex(o.x.data_ptr(), nullptr, nullptr, o.mods.t[0].data_ptr(), o.mods.t[1].data_ptr(), o.mods.ld, eps, r.n,
@@ -179,7 +180,7 @@ Both both_fwd(const Launch& l, const Tensor& x_, const Tensor& gate, const Tenso
               const Tensor& shift, float eps, bool quant) {
   const Rows r = rows_of(x_);
   const Tensor x = bf16_contiguous(x_);
-  Both c{like(x, l.dev), like(x, l.dev), bf16_contiguous(sub), empty({2, r.n}, F32, l.dev), mods_of({&gate, &scale, &shift}), {}};
+  Both c{like(x, l.dev), like(x, l.dev), bf16_contiguous(sub), empty({2, r.n}, F32, l.dev), mods_of(r.d, {&gate, &scale, &shift}), {}};
   float* stats = c.stats.data_ptr<float>();
   if (quant) c.emitted = empty_op(r.n, r.d, l.dev);
   check(anima_adaln_fwd_ex(x.data_ptr(), c.mods.t[0].data_ptr(), c.sub.data_ptr(), c.mods.t[1].data_ptr(),
@@ -289,7 +290,7 @@ Tensor gated_add(const Tensor& x_, const Tensor& gate, const Tensor& y) {
   {
     Below below;
     yc = bf16_contiguous(y);
-    g = mods_of({&gate});
+    g = mods_of(x.size(-1), {&gate});
     out = gated_fwd(l, x, yc, g);
   }
   if (grad) {

@@ -141,6 +141,24 @@ def test_residual_gradient_through_the_modulation_equals_the_separate_sum(B, hw,
         assert torch.equal(a, b)
 
 
+@pytest.mark.parametrize("shape", [(1, 2, 1, 1, 256), (1, 1, 1, 1, 512), (2, 256), (512,), (4, 1, 1, 1, 128)])
+def test_modulation_of_any_shape_is_read_in_order(shape):
+    """As rows of the activation's width, whatever the shape says; its gradient has that shape."""
+    from anima_trainer_sm120_b200.adaln_kernel import fused_adaln, fused_gated_add, fused_gated_add_adaln
+
+    def go(as_given):
+        x, sub, mods, (gn, gx, gy) = _block_inputs(2, 24, 256, True, False)
+        ms = [m.detach().reshape(as_given).requires_grad_() for m in mods]
+        outs = [fused_adaln(x, ms[1], ms[2], 1e-6), *fused_gated_add_adaln(x, ms[0], sub, ms[3], ms[2], 1e-6),
+                fused_gated_add(x, ms[0], sub)]
+        grads = torch.autograd.grad(outs, [x, sub, *ms], [gn, gx, gy, gx])
+        assert all(g.shape == as_given for g in grads[2:])
+        return [t.detach().reshape(-1) for t in (*outs, *grads)]
+
+    for a, b in zip(go((2, 1, 1, 1, 256)), go(shape)):
+        assert torch.equal(a, b)
+
+
 def test_modulation_and_residual_can_be_backpropagated_one_after_the_other():
     from anima_trainer_sm120_b200.adaln_kernel import fused_adaln, fused_gated_add
     for order in ((0, 1), (1, 0)):
