@@ -48,7 +48,8 @@ struct LokrNode : public HostNode {
     const Launch l(gy);
     size_t at = 0;
     const Op xc = get_op(at, x_col), wc = get_op(at, w_col);
-    auto [g_row, g_col] = quantize(l, as_matrix(gy, gy.size(-1)), need_x, train);
+    Op g_row, g_col;
+    if (need_x || train) std::tie(g_row, g_col) = quantize(l, as_matrix(gy, gy.size(-1)), need_x, train);
     variable_list out(4);
     if (need_x) out[0] = input_grad(l, gy, g_row, wc);
     if (train) std::tie(out[2], out[3]) = kron_backward(l, gemm_f32(l, g_col, xc), w1.get(), w2.get(), alpha);
@@ -70,7 +71,8 @@ struct MergedNode : public HostNode {
     const Launch l(gy);
     size_t at = 0;
     const Op xc = get_op(at, x_col), wc = get_op(at, w_col);
-    auto [g_row, g_col] = quantize(l, as_matrix(gy, gy.size(-1)), need_x, train);
+    Op g_row, g_col;
+    if (need_x || train) std::tie(g_row, g_col) = quantize(l, as_matrix(gy, gy.size(-1)), need_x, train);
     variable_list out(3);
     if (need_x) out[0] = input_grad(l, gy, g_row, wc);
     if (train) {

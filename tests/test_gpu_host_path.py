@@ -159,6 +159,18 @@ def test_modulation_of_any_shape_is_read_in_order(shape):
         assert torch.equal(a, b)
 
 
+def test_gradient_of_the_bias_alone():
+    from anima_trainer_sm120_b200 import fp8_quant
+    g = torch.Generator(device=DEV).manual_seed(7)
+    x, W, gy = _randn(g, 64, 256), _randn(g, 512, 256, std=0.05), _randn(g, 64, 512)
+    Q, w1, w2 = fp8_quant.quantize_weight(W), _randn(g, 8, 8), _randn(g, 64, 32)
+    for call in (lambda b: fp8_quant.lokr_linear_fused(x, W, b, w1, w2, 1.0), lambda b: fp8_quant.mxfp8_lokr_linear(x, W, b),
+                 lambda b: fp8_quant.mxfp8_frozen_linear(x, Q, W, b)):
+        b = torch.zeros(512, device=DEV, dtype=BF16, requires_grad=True)
+        call(b).backward(gy)
+        assert torch.equal(b.grad, gy.sum(0))
+
+
 def test_modulation_and_residual_can_be_backpropagated_one_after_the_other():
     from anima_trainer_sm120_b200.adaln_kernel import fused_adaln, fused_gated_add
     for order in ((0, 1), (1, 0)):
