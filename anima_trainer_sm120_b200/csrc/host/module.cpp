@@ -65,13 +65,13 @@ Tensor py_lokr_mlp(const Tensor& x, O xrc, O xrs, O xr, O xcc, O xcs, O xc, cons
   return lokr_mlp(x, op_of(xrc, xrs, xr), op_of(xcc, xcs, xc), W1, b1, w1a, w2a, alpha1, W2, b2, w1b, w2b, alpha2, first);
 }
 
-TLinear py_tlinear(const Tensor& wrc, const Tensor& wrs, const Tensor& wcc, const Tensor& wcs, O bias, const Tensor& w1,
+TLinear py_tlinear(const Tensor& wrc, const Tensor& wrs, O wcc, O wcs, O bias, const Tensor& w1,
                    const Tensor& a, const Tensor& b, O mask, double alpha, const Tensor& c, const std::vector<Tensor>& forms,
                    bool fold, bool fuse_mix) {
   TORCH_CHECK_VALUE(forms.size() == 8 || forms.size() == 10, "T-LoKr factor forms: 8 or 10 tensors");
   OptTensor m = mask;
   if (m) m = bf16_contiguous(*m);
-  TLinear t{op_of(wrc, wrs), op_of(wcc, wcs), bias, w1, a, b, m, alpha, c, op_of(forms[0], forms[1]),
+  TLinear t{op_of(wrc, wrs), op_of(wcc, wcs, std::nullopt), bias, w1, a, b, m, alpha, c, op_of(forms[0], forms[1]),
             op_of(forms[2], forms[3]), op_of(forms[4], forms[5]), op_of(forms[6], forms[7]), {}, fold, fuse_mix};
   if (forms.size() == 10) t.a_scaled = op_of(forms[8], forms[9]);
   return t;

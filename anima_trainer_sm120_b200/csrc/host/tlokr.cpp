@@ -84,6 +84,7 @@ struct LinearGrads {
 LinearGrads linear_bwd(const Launch& l, const Op& gbq, const Op& gbq_col, const Op& gq, const Op& gq_col,
                        at::IntArrayRef lead, const TLinear& t, bool need_x) {
   const int64_t batch = lead[0], rows = gbq.rows / 8, K = t.k_in(), vp = t.vp(), r = t.rank(), vq = K / 8;
+  TORCH_CHECK_VALUE(!need_x || t.w_col.defined(), "the base weight has no column form: quantise it with its input-gradient operand");
   LinearGrads g;
   const bool fold = t.can_fold(rows, K, batch);
   if (need_x) {
@@ -171,7 +172,8 @@ void check_linear(const Launch& l, const Tensor& x, int64_t k_in, const TLinear&
   TORCH_CHECK_NOT_IMPLEMENTED(t.c.dim() == 2 && t.c.size(0) == 8 && t.c.size(1) == 8,
                               "rank_mix supports an 8x8 factor; got ", t.c.sizes());
   TORCH_CHECK_VALUE(t.a.t.dim() == 2 && t.b.t.dim() == 2 && t.b.t.size(0) == t.rank() && t.n_out() == 8 * t.vp() &&
-                        t.k_in() == 8 * t.b.t.size(1) && t.w_col.rows == t.k_in() && t.w_col.k == t.n_out(),
+                        t.k_in() == 8 * t.b.t.size(1) &&
+                        (!t.w_col.defined() || (t.w_col.rows == t.k_in() && t.w_col.k == t.n_out())),
                     "factors ", t.a.t.sizes(), " and ", t.b.t.sizes(), " do not match a weight [", t.n_out(), ", ", t.k_in(), "]");
   TORCH_CHECK_VALUE(x.dim() >= 2 && k_in == t.k_in(), "input of width ", k_in, " for a weight with ", t.k_in(), " columns");
   if (t.mask && t.mask->defined())

@@ -7,7 +7,7 @@ namespace anima_host {
 
 // One adapted linear: the frozen quantised base, the factors, their MXFP8 / bf16 forms, the rank mask.
 struct TLinear {
-  Op w_row, w_col;
+  Op w_row, w_col;          // w_col may be missing where no input gradient is made
   OptTensor bias;
   Kept w1, a, b;            // parameters: [8, 8], [vp, r], [r, vq]
   OptTensor mask;           // [batch, r]

@@ -401,8 +401,9 @@ def _tlinear(W_mx, bias, w1, w2_a, w2_b, mask, alpha: float):
     if FOLD_DELTA and w2_a.shape[1] == 128:              # alpha * A, the factor a folded delta multiplies by
         op = _scaled_row_form(w2_a, alpha)
         forms += (op.codes, op.scales)
-    return host().tlinear(W_mx.row.codes, W_mx.row.scales, W_mx.col.codes, W_mx.col.scales, bias, w1, w2_a, w2_b, mask,
-                          float(alpha), c, forms, FOLD_DELTA, FUSE_HIDDEN_MIX)
+    col = (None, None) if W_mx.col is None else (W_mx.col.codes, W_mx.col.scales)
+    return host().tlinear(W_mx.row.codes, W_mx.row.scales, *col, bias, w1, w2_a, w2_b, mask, float(alpha), c, forms,
+                          FOLD_DELTA, FUSE_HIDDEN_MIX)
 
 
 def _row_operand_unless_kept(x, *trainable):

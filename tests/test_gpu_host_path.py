@@ -171,6 +171,24 @@ def test_gradient_of_the_bias_alone():
         assert torch.equal(b.grad, gy.sum(0))
 
 
+def test_tlokr_forward_of_a_base_weight_without_its_column_form():
+    """quantize_weight(..., with_dgrad=False): enough for a pass that makes no input gradient."""
+    from anima_trainer_sm120_b200 import tlokr
+    from anima_trainer_sm120_b200.fp8_quant import quantize_weight
+    g = torch.Generator(device=DEV).manual_seed(8)
+    W = _randn(g, 1024, 512, std=0.05)
+    f = lambda *s: _randn(g, *s, std=0.1, dtype=torch.float32).requires_grad_()
+    x, factors, gy = _randn(g, 2, 96, 512), [f(8, 8), f(128, 128), f(128, 64)], _randn(g, 2, 96, 1024)
+    results = []
+    for with_dgrad in (True, False):
+        y = tlokr._MXTLoKrLinear.apply(x, quantize_weight(W, with_dgrad=with_dgrad), None, *factors, None, 0.5)
+        results.append([y.detach(), *torch.autograd.grad(y, factors, gy)])
+    assert all(torch.equal(a, b) for a, b in zip(*results))
+    y = tlokr._MXTLoKrLinear.apply(x.clone().requires_grad_(), quantize_weight(W, with_dgrad=False), None, *factors, None, 0.5)
+    with pytest.raises(ValueError, match="column form"):
+        y.backward(gy)
+
+
 def test_modulation_and_residual_can_be_backpropagated_one_after_the_other():
     from anima_trainer_sm120_b200.adaln_kernel import fused_adaln, fused_gated_add
     for order in ((0, 1), (1, 0)):
