@@ -97,8 +97,8 @@ Op placeholder(int64_t rows, int64_t k, const at::Device& dev) {
 
 const Tensor& Kept::get() const {
   TORCH_CHECK(version == now(),
-              "one of the variables needed for gradient computation has been modified by an inplace operation: a parameter "
-              "of shape ", t.sizes(), " is at version ", now(), "; expected version ", version);
+              "one of the variables needed for gradient computation has been modified by an inplace operation: a tensor of "
+              "shape ", t.sizes(), " is at version ", now(), "; expected version ", version);
   return t;
 }
 

@@ -71,7 +71,7 @@ TLinear py_tlinear(const Tensor& wrc, const Tensor& wrs, O wcc, O wcs, O bias, c
   TORCH_CHECK_VALUE(forms.size() == 8 || forms.size() == 10, "T-LoKr factor forms: 8 or 10 tensors");
   OptTensor m = mask;
   if (m) m = bf16_contiguous(*m);
-  TLinear t{op_of(wrc, wrs), op_of(wcc, wcs, std::nullopt), bias, w1, a, b, m, alpha, c, op_of(forms[0], forms[1]),
+  TLinear t{op_of(wrc, wrs), op_of(wcc, wcs, std::nullopt), bias, w1, a, b, m, mask ? Kept(*mask) : Kept(), alpha, c, op_of(forms[0], forms[1]),
             op_of(forms[2], forms[3]), op_of(forms[4], forms[5]), op_of(forms[6], forms[7]), {}, fold, fuse_mix};
   if (forms.size() == 10) t.a_scaled = op_of(forms[8], forms[9]);
   return t;

@@ -200,7 +200,7 @@ struct TlokrNode : public HostNode {
     const auto lead = lead_of(gy);
     size_t at = 0;
     const auto [gq, gq_col] = saved_input(*this, at, product(lead), t.k_in());
-    for (const Kept* k : {&t.w1, &t.a, &t.b}) k->get();
+    t.check_unchanged();
     auto [gbq, gbq_col] = quantize(l, as_matrix(gy, t.vp()), true, true);
     LinearGrads r = linear_bwd(l, gbq, gbq_col, gq, gq_col, lead, t, need.x);
     return {r.x, need.bias ? grad_bias(gy) : Tensor(), r.w1, r.a, r.b};
@@ -225,7 +225,8 @@ struct TlokrMlpNode : public HostNode {
     size_t at = 1;
     const auto [gq1, gq1_col] = saved_input(*this, at, rows, t1.k_in());
     const auto [gq2, gq2_col] = saved_input(*this, at, rows, t2.k_in());
-    for (const Kept* k : {&t1.w1, &t1.a, &t1.b, &t2.w1, &t2.a, &t2.b}) k->get();
+    t1.check_unchanged();
+    t2.check_unchanged();
     LinearGrads g2, g1;
     {
       auto [gbq, gbq_col] = quantize(l, as_matrix(gy, t2.vp()), true, true);

@@ -11,6 +11,7 @@ struct TLinear {
   OptTensor bias;
   Kept w1, a, b;            // parameters: [8, 8], [vp, r], [r, vq]
   OptTensor mask;           // [batch, r]
+  Kept mask_in;             // the mask as it was given; like the parameters it may not change before backward
   double alpha;
   Tensor c;                 // w1 in bf16
   Op aq, aq_col, bq, bq_col, a_scaled;   // a_scaled: row form of alpha * a (folded delta only)
@@ -20,6 +21,9 @@ struct TLinear {
   int64_t k_in() const { return w_row.k; }
   int64_t vp() const { return a.t.size(0); }
   int64_t rank() const { return a.t.size(1); }
+  void check_unchanged() const {
+    for (const Kept* k : {&w1, &a, &b, &mask_in}) k->get();
+  }
   bool can_fold(int64_t rows, int64_t cols, int64_t batch) const;
 };
 

@@ -189,6 +189,22 @@ def test_tlokr_forward_of_a_base_weight_without_its_column_form():
         y.backward(gy)
 
 
+@pytest.mark.parametrize("which", ["w1", "a", "b", "mask"])
+@pytest.mark.parametrize("mask_dtype", [BF16, torch.float32])
+def test_tlokr_tensors_changed_in_place_before_backward_are_noticed(which, mask_dtype):
+    from anima_trainer_sm120_b200 import tlokr
+    from anima_trainer_sm120_b200.fp8_quant import quantize_weight
+    g = torch.Generator(device=DEV).manual_seed(9)
+    f = lambda *s: _randn(g, *s, std=0.1, dtype=torch.float32).requires_grad_()
+    ts = {"w1": f(8, 8), "a": f(128, 128), "b": f(128, 64), "mask": torch.ones(2, 128, device=DEV, dtype=mask_dtype)}
+    x, W = _randn(g, 2, 64, 512).requires_grad_(), quantize_weight(_randn(g, 1024, 512, std=0.05))
+    y = tlokr._MXTLoKrLinear.apply(x, W, None, ts["w1"], ts["a"], ts["b"], ts["mask"], 0.5)
+    with torch.no_grad():
+        ts[which].mul_(0.5)
+    with pytest.raises(RuntimeError, match="modified by an inplace operation"):
+        y.backward(torch.ones_like(y))
+
+
 def test_modulation_and_residual_can_be_backpropagated_one_after_the_other():
     from anima_trainer_sm120_b200.adaln_kernel import fused_adaln, fused_gated_add
     for order in ((0, 1), (1, 0)):
