@@ -88,19 +88,21 @@ struct MergedNode : public HostNode {
 
 // ------------------------------------------------------------------------------------------------ frozen linear
 struct FrozenNode : public HostNode {
-  Op w_col;
+  Op w_col;                // its shape alone where it is a saved tensor
   Tensor w_bf16;
-  bool need_x, need_bias;
+  bool need_x, need_bias, w_saved;
 
   variable_list apply(variable_list&& g) override {
     std::lock_guard<std::mutex> lock(mutex_);
     const Tensor gy = grad_of(g, 0);
     variable_list out(2);
+    size_t at = 0;
+    const Op w = w_saved ? get_op(at, w_col) : w_col;
     if (need_x) {
       const Launch l(gy);
       const Mat m = as_matrix(gy, gy.size(-1));
-      if (w_col.defined()) {
-        out[0] = input_grad(l, gy, quantize(l, m, true, false).first, w_col);
+      if (w.defined()) {
+        out[0] = input_grad(l, gy, quantize(l, m, true, false).first, w);
       } else {
         Tensor gx = at::matmul(m.keep.reshape({m.rows, m.cols}), w_bf16.to(BF16));
         out[0] = cast(gx.reshape(with_last(gy.sizes(), w_bf16.size(1))), gy.scalar_type());
@@ -218,7 +220,8 @@ Tensor merged_linear(const Tensor& x, Op x_row, Op x_col, const Tensor& merged, 
   return y;
 }
 
-Tensor frozen_linear(const Tensor& x, Op x_row, Op w_row, Op w_col, const OptTensor& w_bf16, const OptTensor& bias) {
+Tensor frozen_linear(const Tensor& x, Op x_row, Op w_row, Op w_col, const OptTensor& w_bf16, const OptTensor& bias,
+                     bool save_weight) {
   TORCH_CHECK_VALUE(x.size(-1) == w_row.k, "input of width ", x.size(-1), " for a weight with ", w_row.k, " columns");
   const bool need_x = wants(x), need_bias = wants(bias);
   TORCH_CHECK_VALUE(!need_x || !w_col.defined() || (w_col.rows == w_row.k && w_col.k == w_row.rows),
@@ -234,7 +237,9 @@ Tensor frozen_linear(const Tensor& x, Op x_row, Op w_row, Op w_col, const OptTen
   }
   if (need_x || need_bias) {
     auto n = make_node<FrozenNode>(x, bias);
-    n->w_col = std::move(w_col);
+    n->w_saved = save_weight && w_col.defined();
+    if (n->w_saved) n->save(w_col);
+    n->w_col = n->w_saved ? shape_of(w_col) : std::move(w_col);
     n->w_bf16 = w_bf16.value_or(Tensor());
     n->need_x = need_x;
     n->need_bias = need_bias;

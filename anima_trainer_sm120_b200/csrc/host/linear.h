@@ -11,9 +11,10 @@ Tensor lokr_linear(const Tensor& x, Op x_row, Op x_col, const Tensor& W, const O
                    const Tensor& w2, double alpha, bool first);
 // y = x merged^T + bias with the gradient of merged
 Tensor merged_linear(const Tensor& x, Op x_row, Op x_col, const Tensor& merged, const OptTensor& bias, bool first);
-// y = x W^T + bias, W frozen and quantised; `w_bf16` serves backward when W has no column form
+// y = x W^T + bias, W frozen and quantised; `w_bf16` serves backward when W has no column form. `save_weight`: the column
+// form is a saved tensor (hooks, version check, released by backward) instead of the caller's to keep as it is.
 Tensor frozen_linear(const Tensor& x, Op x_row, Op w_row, Op w_col, const OptTensor& w_bf16,
-                     const OptTensor& bias);
+                     const OptTensor& bias, bool save_weight);
 // layer2(gelu(layer1(x))) with both layers LoKr linears
 Tensor lokr_mlp(const Tensor& x, Op x_row, Op x_col, const Tensor& W1, const OptTensor& b1, const Tensor& w1a,
                 const Tensor& w2a, double alpha1, const Tensor& W2, const OptTensor& b2, const Tensor& w1b,

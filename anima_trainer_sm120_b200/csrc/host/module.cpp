@@ -56,8 +56,9 @@ Tensor py_lokr(const Tensor& x, O xrc, O xrs, O xr, O xcc, O xcs, O xc, const Te
 Tensor py_merged(const Tensor& x, O xrc, O xrs, O xr, O xcc, O xcs, O xc, const Tensor& merged, O bias, bool first) {
   return merged_linear(x, op_of(xrc, xrs, xr), op_of(xcc, xcs, xc), merged, bias, first);
 }
-Tensor py_frozen(const Tensor& x, O xrc, O xrs, O xr, O wrc, O wrs, O wr, O wcc, O wcs, O wc, O w_bf16, O bias) {
-  return frozen_linear(x, op_of(xrc, xrs, xr), op_of(wrc, wrs, wr), op_of(wcc, wcs, wc), w_bf16, bias);
+Tensor py_frozen(const Tensor& x, O xrc, O xrs, O xr, O wrc, O wrs, O wr, O wcc, O wcs, O wc, O w_bf16, O bias,
+                 bool save_weight) {
+  return frozen_linear(x, op_of(xrc, xrs, xr), op_of(wrc, wrs, wr), op_of(wcc, wcs, wc), w_bf16, bias, save_weight);
 }
 Tensor py_lokr_mlp(const Tensor& x, O xrc, O xrs, O xr, O xcc, O xcs, O xc, const Tensor& W1, O b1, const Tensor& w1a,
                    const Tensor& w2a, double alpha1, const Tensor& W2, O b2, const Tensor& w1b, const Tensor& w2b,

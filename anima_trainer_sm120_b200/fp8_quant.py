@@ -165,7 +165,7 @@ class MXFP8FrozenLinear:
     @staticmethod
     def apply(x, W_mx: QuantWeight, W_bf16, bias=None):
         x_row, _ = quantize_activation(x, colwise=False)
-        return host().frozen_linear(x, *_native(x_row), *_native(W_mx.row), *_native(W_mx.col), W_bf16, bias)
+        return host().frozen_linear(x, *_native(x_row), *_native(W_mx.row), *_native(W_mx.col), W_bf16, bias, False)
 
 
 def mxfp8_frozen_linear(x, W_mx, W_bf16, bias=None):

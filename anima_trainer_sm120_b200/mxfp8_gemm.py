@@ -106,7 +106,8 @@ def mxfp8_matmul(A: MXFP8Block, B_data: torch.Tensor, B_scales: torch.Tensor,
 class MXFP8FrozenLinearB200:
     """``y = x @ W.T (+ bias)`` for a frozen, pre-quantised W; forward and dgrad both run
     as MXFP8 tensor-core GEMMs. Signature of ``MXFP8FrozenLinearTriton.apply``; backward
-    reads no activation, so none is saved (the reference saves the quantised one, :384-385)."""
+    reads no activation, so none is saved (the reference saves the quantised one, :384-385); W_bwd is
+    a saved tensor, as there."""
 
     @staticmethod
     def apply(x, W_fwd_data, W_fwd_scales, W_bwd_data, W_bwd_scales, bias=None, W_fwd_tiled=None, W_bwd_tiled=None):
@@ -119,7 +120,7 @@ class MXFP8FrozenLinearB200:
         if not wT.is_contiguous():
             raise NotImplementedError("W_bwd must come from quantize_weight_for_dgrad()")
         w_bwd = _as_operand(wT, W_bwd_scales, W_bwd_tiled)
-        return host().frozen_linear(x, *_native(x_row), *_native(w), *_native(w_bwd), None, bias)
+        return host().frozen_linear(x, *_native(x_row), *_native(w), *_native(w_bwd), None, bias, True)
 
 
 MXFP8FrozenLinearTriton = MXFP8FrozenLinearB200  # name used by anima-trainer call sites

@@ -205,6 +205,25 @@ def test_tlokr_tensors_changed_in_place_before_backward_are_noticed(which, mask_
         y.backward(torch.ones_like(y))
 
 
+def test_backward_weight_of_the_block_level_frozen_linear_is_a_saved_tensor():
+    """W_bwd changed in place, or a second backward through a freed graph, is refused; a retained graph is not."""
+    from anima_trainer_sm120_b200 import mxfp8_gemm
+    g = torch.Generator(device=DEV).manual_seed(10)
+    W, x, gy = _randn(g, 256, 128, std=0.05), _randn(g, 96, 128).requires_grad_(), _randn(g, 96, 256)
+    go = lambda: mxfp8_gemm.mxfp8_frozen_linear_triton(x, mxfp8_gemm.quantize_weight_for_lhs(W), W_bwd)
+    W_bwd = mxfp8_gemm.quantize_weight_for_dgrad(W)
+    y = go()
+    first, = torch.autograd.grad(y, x, gy, retain_graph=True)
+    again, = torch.autograd.grad(y, x, gy)
+    assert torch.equal(first, again)
+    with pytest.raises(RuntimeError, match="second time"):
+        y.backward(gy)
+    y = go()
+    W_bwd.data.zero_()
+    with pytest.raises(RuntimeError, match="modified by an inplace operation"):
+        y.backward(gy)
+
+
 def test_modulation_and_residual_can_be_backpropagated_one_after_the_other():
     from anima_trainer_sm120_b200.adaln_kernel import fused_adaln, fused_gated_add
     for order in ((0, 1), (1, 0)):

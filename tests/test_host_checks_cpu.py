@@ -23,7 +23,7 @@ def _bf16(*shape):
 @pytest.mark.parametrize("rows,k,ok", [(64, 96, True), (128, 96, False), (32, 96, False), (64, 128, False), (96, 64, False)])
 def test_backward_operand_of_a_frozen_linear_must_be_the_transpose_of_the_weight(rows, k, ok):
     x = _bf16(32, 64).requires_grad_(True)                  # weight [96, 64]: its column form is [64, 96]
-    call = lambda t: host().frozen_linear(t, *_op(32, 64), *_op(96, 64), *_op(rows, k), None, None)
+    call = lambda t: host().frozen_linear(t, *_op(32, 64), *_op(96, 64), *_op(rows, k), None, None, False)
     with pytest.raises(RuntimeError if ok else ValueError, match="CUDA" if ok else "transpose"):
         call(x)
     with pytest.raises(RuntimeError, match="CUDA"):         # a pass without an input gradient does not read it
@@ -48,7 +48,7 @@ def test_a_bias_that_is_not_one_value_per_output_is_refused(which, short):
     calls = {
         "lokr": lambda: host().lokr_linear(x, *x_row, *NONE, W, b, w1, w2, 1.0, False),
         "merged": lambda: host().merged_linear(x, *x_row, *NONE, W, b, False),
-        "frozen": lambda: host().frozen_linear(x, *x_row, *_op(n, k), *NONE, None, b),
+        "frozen": lambda: host().frozen_linear(x, *x_row, *_op(n, k), *NONE, None, b, False),
         "mlp": lambda: host().lokr_mlp(x, *x_row, *NONE, W, b_in, w1, w2, 1.0, _bf16(k, n), b_out, w1, w2t, 1.0, False),
         "tlokr": lambda: host().tlokr_linear(x, *x_row, _tlinear(n, k, b), False),
         "tlokr-mlp": lambda: host().tlokr_mlp(x, *x_row, _tlinear(n, k, b_in), _tlinear(k, n, b_out), False),
