@@ -141,6 +141,12 @@ inline std::vector<int64_t> with_last(at::IntArrayRef shape, int64_t last) {
 }
 inline bool wants(const Tensor& t) { return at::GradMode::is_enabled() && t.defined() && t.requires_grad(); }
 inline bool wants(const OptTensor& t) { return t && wants(*t); }
+// An output belongs to the graph as soon as any tensor of the call wants a gradient, also one these nodes have no rule for
+// (a frozen weight left trainable, the bias of a fused MLP, a norm weight): that tensor's gradient is then none.
+template <class... T>
+bool any_wants(const T&... t) {
+  return (wants(t) || ...);
+}
 inline Tensor cast(const Tensor& t, at::ScalarType dt) { return t.scalar_type() == dt ? t : t.to(dt); }
 
 // ------------------------------------------------------------------------------------------------ autograd nodes

@@ -123,6 +123,7 @@ struct MlpNode : public HostNode {
 
   variable_list apply(variable_list&& g) override {
     std::lock_guard<std::mutex> lock(mutex_);
+    if (!need_x && !train) return variable_list(5);
     const Tensor gy = grad_of(g, 0);
     const Launch l(gy);
     const Tensor h = get(0);
@@ -163,7 +164,7 @@ Tensor lokr_linear(const Tensor& x, Op x_row, Op x_col, const Tensor& W, const O
       if (train) x_col = placeholder(W.size(1), x_row.rows, l.dev);
     }
   }
-  if (need_x || train || need_bias) {
+  if (any_wants(x, W, bias, w1, w2)) {
     auto n = make_node<LokrNode>(x, bias, w1, w2);
     if (train) {
       n->w1 = Kept(w1);
@@ -235,7 +236,7 @@ Tensor frozen_linear(const Tensor& x, Op x_row, Op w_row, Op w_col, const OptTen
     Below below;
     y = project(l, x, x_row, w_row, bias);
   }
-  if (need_x || need_bias) {
+  if (any_wants(x, w_bf16, bias)) {
     auto n = make_node<FrozenNode>(x, bias);
     n->w_saved = save_weight && w_col.defined();
     if (n->w_saved) n->save(w_col);
@@ -279,9 +280,9 @@ Tensor lokr_mlp(const Tensor& x, Op x_row, Op x_col, const Tensor& W1, const Opt
       }
     }
   }
-  if (back) {
+  if (any_wants(x, W1, b1, w1a, w2a, W2, b2, w1b, w2b)) {
     auto n = make_node<MlpNode>(x, w1a, w2a, w1b, w2b);
-    n->save(h);
+    if (back) n->save(h);
     for (auto [op, shape] : {std::pair{&x_col, &n->x_col}, {&a_col, &n->a_col}, {&W1_col, &n->W1_col}, {&W2_col, &n->W2_col}}) {
       if (op == &x_col && !train) continue;
       n->save(*op);

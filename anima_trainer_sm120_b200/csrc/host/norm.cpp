@@ -240,6 +240,7 @@ struct RopeNode : public HostNode {      // saves x, rstd
 
   variable_list apply(variable_list&& g) override {
     std::lock_guard<std::mutex> lock(mutex_);
+    if (!task_should_compute_output(0)) return variable_list(1);
     const Tensor dout = bf16_contiguous(grad_of(g, 0)), x = get(0), rstd = get(1), w = weight.get();
     const Launch l(x);
     Tensor dx = like(x, l.dev);
@@ -352,7 +353,7 @@ Tensor rmsnorm_rope(const Tensor& x, const Tensor& weight, const OptTensor& cos,
                                       static_cast<float*>(ptr(sin)), static_cast<float>(eps), tokens, heads, d,
                                       cos ? cos->size(0) : 1, out.data_ptr(), rstd.data_ptr<float>(), l.stream));
   }
-  if (wants(x)) {
+  if (any_wants(x, weight, cos, sin)) {
     auto node = make_node<RopeNode>(x);
     node->save(xc);
     node->save(rstd);

@@ -213,10 +213,11 @@ struct TlokrNode : public HostNode {
 // gelu(h) nor grad * gelu'(h) is written as a bf16 tensor.
 struct TlokrMlpNode : public HostNode {
   TLinear t1, t2;
-  bool need_x;
+  bool need_x, back;
 
   variable_list apply(variable_list&& g) override {
     std::lock_guard<std::mutex> lock(mutex_);
+    if (!back) return variable_list(7);
     const Tensor gy = grad_of(g, 0);
     const Launch l(gy);
     const auto lead = lead_of(gy);
@@ -295,12 +296,15 @@ Tensor tlokr_mlp(const Tensor& x, Op x_row, TLinear t1, TLinear t2, bool first) 
     y = empty(with_last(x.sizes(), t2.n_out()), BF16, l.dev);
     linear_fwd(l, in2.x_row, in2.gq, x.size(0), t2, y.data_ptr());
   }
-  if (back) {
+  if (back || n1.bias || n2.bias) {
     auto n = make_node<TlokrMlpNode>(x, t1.w1.t, t1.a.t, t1.b.t, t2.w1.t, t2.a.t, t2.b.t);
-    n->save(h);
-    save_input(*n, l, in1, rows, K, keep);
-    save_input(*n, l, in2, rows, hid, keep);
+    if (back) {
+      n->save(h);
+      save_input(*n, l, in1, rows, K, keep);
+      save_input(*n, l, in2, rows, hid, keep);
+    }
     n->need_x = n1.x;
+    n->back = back;
     n->t1 = std::move(t1);
     n->t2 = std::move(t2);
     set_history(y, n);

@@ -224,6 +224,40 @@ def test_backward_weight_of_the_block_level_frozen_linear_is_a_saved_tensor():
         y.backward(gy)
 
 
+@pytest.mark.parametrize("which", ["lokr W", "frozen W", "mlp W1", "mlp b2", "tlokr mlp b1", "norm weight"])
+def test_output_belongs_to_the_graph_of_a_trainable_tensor_without_a_gradient_rule(which):
+    """As for any autograd function: backward runs, that tensor's gradient is none, the others are what they are without it."""
+    from anima_trainer_sm120_b200 import fp8_quant, tlokr
+    from anima_trainer_sm120_b200.fp8_quant import quantize_weight
+    from anima_trainer_sm120_b200.mlp_patch import LoKrMLPFused
+    from anima_trainer_sm120_b200.qk_norm_rope import FusedRMSNormRoPE
+    g = torch.Generator(device=DEV).manual_seed(11)
+    W1, W2, x = _randn(g, 512, 256, std=0.05), _randn(g, 256, 512, std=0.05), _randn(g, 1, 64, 256)
+    w1, w2, w2t, f = _randn(g, 8, 8), _randn(g, 64, 32), _randn(g, 32, 64), lambda *s: _randn(g, *s, std=0.1)
+    a1, b1, a2, b2 = f(64, 128), f(128, 32), f(32, 128), f(128, 64)
+    Q1, Q2, heads = quantize_weight(W1), quantize_weight(W2), _randn(g, 1, 16, 2, 128)
+    call, t, inp = {
+        "lokr W": (lambda x, t: fp8_quant.lokr_linear_fused(x, t, None, w1, w2, 1.0), W1, x),
+        "frozen W": (lambda x, t: fp8_quant.mxfp8_frozen_linear(x, Q1, t), W1, x),
+        "mlp W1": (lambda x, t: LoKrMLPFused.apply(x, t, None, w1, w2, 1.0, W2, None, w1, w2t, 1.0), W1, x),
+        "mlp b2": (lambda x, t: LoKrMLPFused.apply(x, W1, None, w1, w2, 1.0, W2, t, w1, w2t, 1.0), _randn(g, 256), x),
+        "tlokr mlp b1": (lambda x, t: tlokr._MXTLoKrMLP.apply(x, Q1, t, w1, a1, b1, None, 0.5, Q2, None, w1, a2, b2, None, 0.5),
+                         _randn(g, 512), x),
+        "norm weight": (lambda x, t: FusedRMSNormRoPE.apply(x, t, None, None, 1e-6), _randn(g, 128), heads),
+    }[which]
+    grads = []
+    for x_wants in (False, True):
+        for t_wants in (False, True):
+            xi, ti = inp.clone().requires_grad_(x_wants), t.clone().requires_grad_(t_wants)
+            y = call(xi, ti)
+            assert y.requires_grad == (x_wants or t_wants)
+            if y.requires_grad:
+                y.backward(torch.ones_like(y))
+                assert ti.grad is None
+                grads.append(xi.grad)
+    assert grads[0] is None and torch.equal(grads[1], grads[2])
+
+
 def test_modulation_and_residual_can_be_backpropagated_one_after_the_other():
     from anima_trainer_sm120_b200.adaln_kernel import fused_adaln, fused_gated_add
     for order in ((0, 1), (1, 0)):
