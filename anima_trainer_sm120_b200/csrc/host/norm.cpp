@@ -111,7 +111,7 @@ struct AdalnNode : public HostNode {      // saves x, scale, statistics
   variable_list apply(variable_list&& g) override {
     std::lock_guard<std::mutex> lock(mutex_);
     variable_list out(3);
-    if (!g[0].defined()) {      // only the alias was used: nothing of this node's own
+    if (!g[0].defined() && g[1].defined()) {      // only the alias was used: nothing of this node's own
       out[0] = g[1];
       return out;
     }
@@ -119,7 +119,7 @@ struct AdalnNode : public HostNode {      // saves x, scale, statistics
     const Tensor x = get(0), scale = get(1), stats = get(2);
     const Launch l(x);
     const bool mod = task_should_compute_output(1) || task_should_compute_output(2);
-    auto [dx, ds, db] = adaln_bwd(l, g[0], g[1], x, scale, ld, stats, mod);
+    auto [dx, ds, db] = adaln_bwd(l, grad_of(g, 0), g[1], x, scale, ld, stats, mod);
     out[0] = back_to(dx, dt_x);
     out[1] = back_to(ds, dt_scale);
     out[2] = back_to(db, dt_shift);
@@ -196,8 +196,7 @@ struct BothNode : public HostNode {      // saves sub, gate, x_new, scale, stati
   variable_list apply(variable_list&& grads) override {
     std::lock_guard<std::mutex> lock(mutex_);
     variable_list out(5);
-    const Tensor &d_xnew = grads[0], &d_y = grads[1];
-    if (!d_xnew.defined() && !d_y.defined()) return out;
+    const Tensor &d_y = grads[1], d_xnew = grads[0].defined() || d_y.defined() ? grads[0] : grad_of(grads, 0);
     const Tensor sub = get(0), gate = get(1), x_new = get(2), scale = get(3), stats = get(4);
     const Launch l(x_new);
     const bool mod = task_should_compute_output(1) || task_should_compute_output(3) || task_should_compute_output(4);
@@ -220,7 +219,12 @@ struct BothNode : public HostNode {      // saves sub, gate, x_new, scale, stati
                                ptr(dshift), ptr(dgate), ptr(ws), bytes, l.stream));
     } else {
       dx = d_xnew;
-      if (d_y.defined()) std::tie(dx, dscale, dshift) = adaln_bwd(l, d_y, Tensor(), x_new, scale, ld, stats, mod);
+      if (d_y.defined()) {
+        std::tie(dx, dscale, dshift) = adaln_bwd(l, d_y, Tensor(), x_new, scale, ld, stats, mod);
+      } else if (mod) {          // no gradient reached y: zeros, as for any output of a node that runs
+        dscale = at::zeros_like(scale, at::MemoryFormat::Contiguous);
+        dshift = at::zeros_like(scale, at::MemoryFormat::Contiguous);
+      }
       std::tie(dsub, dgate) = gated_bwd(l, dx, sub, gate, ld, mod);
     }
     out[0] = dx;

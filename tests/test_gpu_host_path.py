@@ -258,6 +258,37 @@ def test_output_belongs_to_the_graph_of_a_trainable_tensor_without_a_gradient_ru
     assert grads[0] is None and torch.equal(grads[1], grads[2])
 
 
+class _NoGradient(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, t):
+        return t.clone()
+
+    @staticmethod
+    def backward(ctx, g):
+        return None
+
+
+@pytest.mark.parametrize("used", ["x_new", "y", "neither"])
+def test_outputs_without_an_incoming_gradient_count_as_zero(used):
+    from anima_trainer_sm120_b200.adaln_kernel import fused_adaln, fused_gated_add_adaln
+    results = []
+    for explicit in (True, False):
+        x, sub, (g0, sc, sh, _), (_, gx, gy) = _block_inputs(2, 24, 256, True, False)
+        x_new, y = fused_gated_add_adaln(x, g0, sub, sc, sh, 1e-6)
+        zero = torch.zeros_like(gx)
+        if explicit:
+            outs, gs = [x_new, y], [gx if used == "x_new" else zero, gy if used == "y" else zero]
+        elif used == "neither":
+            outs, gs = [_NoGradient.apply(y)], [gy]
+        else:
+            outs, gs = [x_new if used == "x_new" else y], [gx if used == "x_new" else gy]
+        results.append(torch.autograd.grad(outs, [x, sub, g0, sc, sh], gs))
+    assert all(torch.equal(a, b) for a, b in zip(*results))
+    x, _, (_, sc, sh, _), (gn, _, _) = _block_inputs(2, 24, 256, True, False)
+    for t in torch.autograd.grad(_NoGradient.apply(fused_adaln(x, sc, sh, 1e-6)), [x, sc, sh], gn):
+        assert t.count_nonzero() == 0
+
+
 def test_modulation_and_residual_can_be_backpropagated_one_after_the_other():
     from anima_trainer_sm120_b200.adaln_kernel import fused_adaln, fused_gated_add
     for order in ((0, 1), (1, 0)):
