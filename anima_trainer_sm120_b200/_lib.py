@@ -80,6 +80,7 @@ PROTOTYPES: dict[str, tuple[object, list[object]]] = {
     "anima_tlokr_rank_mix_wgrad_workspace_bytes": (I64, [I64, I64, I64]),
     "anima_tlokr_rank_mix_wgrad": (c_int, [P, P, P, I64, I64, I64, P, P, I64, P]),
     "anima_rmsnorm_rope_fwd_ex": (c_int, [P, P, c_int, P, P, c_float, I64, I64, I64, I64, P, P, P]),
+    "anima_rmsnorm_rope_fwd_keep": (c_int, [P, P, c_int, P, P, c_float, I64, I64, I64, I64, P, P, P, P]),
     "anima_rmsnorm_rope_bwd_ex": (c_int, [P, P, P, c_int, P, P, P, I64, I64, I64, I64, P, P]),
     "anima_rmsnorm_rope_fwd": (c_int, [P, P, P, P, c_float, I64, I64, I64, I64, P, P, P]),
     "anima_rmsnorm_rope_bwd": (c_int, [P, P, P, P, P, P, I64, I64, I64, I64, P, P]),

@@ -238,19 +238,24 @@ struct BothNode : public HostNode {      // saves sub, gate, x_new, scale, stati
 };
 
 // ------------------------------------------------------------------------------------------------ RMSNorm + RoPE
-struct RopeNode : public HostNode {      // saves x, rstd
+// Saves x and rstd. A bf16 norm weight is copied by the forward kernel, behind rstd: it may change before backward (as when
+// the node converted it). An fp32 one is read in place and may not.
+struct RopeNode : public HostNode {
   Kept weight;
+  int64_t copy_at = -1;         // place of that copy in rstd
   Tensor cos, sin;
 
   variable_list apply(variable_list&& g) override {
     std::lock_guard<std::mutex> lock(mutex_);
     if (!task_should_compute_output(0)) return variable_list(1);
-    const Tensor dout = bf16_contiguous(grad_of(g, 0)), x = get(0), rstd = get(1), w = weight.get();
+    const Tensor dout = bf16_contiguous(grad_of(g, 0)), x = get(0), rstd = get(1);
+    const bool copied = copy_at >= 0;
+    const void* w = copied ? rstd.data_ptr<float>() + copy_at : weight.get().data_ptr();
     const Launch l(x);
     Tensor dx = like(x, l.dev);
     const int64_t heads = x.size(-2), d = x.size(-1), tokens = x.numel() ? x.numel() / (heads * d) : 0;
     if (tokens)
-      check(anima_rmsnorm_rope_bwd_ex(dout.data_ptr(), x.data_ptr(), w.data_ptr(), w.scalar_type() == BF16,
+      check(anima_rmsnorm_rope_bwd_ex(dout.data_ptr(), x.data_ptr(), w, copied,
                                       static_cast<float*>(ptr(cos)), static_cast<float*>(ptr(sin)), rstd.data_ptr<float>(),
                                       tokens, heads, d, cos.defined() ? cos.size(0) : 1, dx.data_ptr(), l.stream));
     return {dx};
@@ -344,6 +349,9 @@ Tensor rmsnorm_rope(const Tensor& x, const Tensor& weight, const OptTensor& cos,
   const Launch l(x);
   admit(l, x, weight, cos, sin);
   const int64_t heads = x.size(-2), d = x.size(-1), tokens = x.numel() ? x.numel() / (heads * d) : 0;
+  const bool grad = any_wants(x, weight, cos, sin), copied = grad && weight.scalar_type() == BF16;
+  TORCH_CHECK_VALUE(weight.numel() >= d, "norm weight of ", weight.numel(), " elements for heads of ", d);
+  const int64_t copy_at = (tokens * heads + 3) / 4 * 4;
   Tensor out, xc, w, rstd;
   {
     Below below;
@@ -351,17 +359,19 @@ Tensor rmsnorm_rope(const Tensor& x, const Tensor& weight, const OptTensor& cos,
     w = weight.scalar_type() == BF16 || weight.scalar_type() == F32 ? weight : weight.detach().to(F32);
     if (!w.is_contiguous() || (reinterpret_cast<uintptr_t>(w.data_ptr()) & 15)) w = w.detach().clone(at::MemoryFormat::Contiguous);
     out = like(x, l.dev);
-    rstd = empty({tokens * heads}, F32, l.dev);
+    rstd = empty({copied ? copy_at + d / 2 : tokens * heads}, F32, l.dev);
     if (tokens)
-      check(anima_rmsnorm_rope_fwd_ex(xc.data_ptr(), w.data_ptr(), w.scalar_type() == BF16, static_cast<float*>(ptr(cos)),
-                                      static_cast<float*>(ptr(sin)), static_cast<float>(eps), tokens, heads, d,
-                                      cos ? cos->size(0) : 1, out.data_ptr(), rstd.data_ptr<float>(), l.stream));
+      check(anima_rmsnorm_rope_fwd_keep(xc.data_ptr(), w.data_ptr(), w.scalar_type() == BF16, static_cast<float*>(ptr(cos)),
+                                        static_cast<float*>(ptr(sin)), static_cast<float>(eps), tokens, heads, d,
+                                        cos ? cos->size(0) : 1, out.data_ptr(), rstd.data_ptr<float>(),
+                                        copied ? rstd.data_ptr<float>() + copy_at : nullptr, l.stream));
   }
-  if (any_wants(x, weight, cos, sin)) {
+  if (grad) {
     auto node = make_node<RopeNode>(x);
     node->save(xc);
     node->save(rstd);
-    node->weight = Kept(w);
+    if (copied) node->copy_at = copy_at;
+    else node->weight = Kept(w);
     node->cos = cos.value_or(Tensor());
     node->sin = sin.value_or(Tensor());
     set_history(out, node);

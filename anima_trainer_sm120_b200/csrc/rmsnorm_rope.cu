@@ -108,9 +108,12 @@ template <bool ROPE, bool WBF16>
 __global__ void __launch_bounds__(kThreads, 2)
 rmsnorm_rope_fwd_kernel(const __nv_bfloat16* __restrict__ x, const void* __restrict__ w, const float* __restrict__ cos_tab,
                         const float* __restrict__ sin_tab, float eps, int64_t tokens, int heads, int heads_per_group,
-                        int64_t seq_len, __nv_bfloat16* __restrict__ out, float* __restrict__ rstd_out) {
+                        int64_t seq_len, __nv_bfloat16* __restrict__ out, float* __restrict__ rstd_out,
+                        uint4* __restrict__ w_copy) {
   after_previous();
   w = after_previous(w);
+  if (w_copy != nullptr && blockIdx.x + blockIdx.y == 0 && threadIdx.x < kHeadDim * (WBF16 ? 2 : 4) / 16)
+    w_copy[threadIdx.x] = static_cast<const uint4*>(w)[threadIdx.x];
   cos_tab = after_previous(cos_tab);
   sin_tab = after_previous(sin_tab);
   const int l = threadIdx.x & (kLanesPerToken - 1);
@@ -262,12 +265,12 @@ int check(const char* who, int64_t tokens, int64_t heads, int64_t head_dim, int6
 
 using namespace anima;
 
-extern "C" int anima_rmsnorm_rope_fwd_ex(const void* x, const void* weight, int weight_is_bf16, const float* cos_tab,
-                                         const float* sin_tab, float eps, int64_t tokens, int64_t heads, int64_t head_dim,
-                                         int64_t seq_len, void* out, float* rstd, void* stream) {
+extern "C" int anima_rmsnorm_rope_fwd_keep(const void* x, const void* weight, int weight_is_bf16, const float* cos_tab,
+                                           const float* sin_tab, float eps, int64_t tokens, int64_t heads, int64_t head_dim,
+                                           int64_t seq_len, void* out, float* rstd, void* weight_copy, void* stream) {
   ANIMA_REQUIRE(x && weight && out && rstd, ANIMA_E_ARG, "rmsnorm_rope_fwd: null pointer");
   if (int rc = check("rmsnorm_rope_fwd", tokens, heads, head_dim, seq_len, cos_tab, sin_tab)) return rc;
-  ANIMA_REQUIRE(aligned16(x) && aligned16(out) && aligned16(weight) && (!cos_tab || (aligned16(cos_tab) && aligned16(sin_tab))), ANIMA_E_ALIGN,
+  ANIMA_REQUIRE(aligned16(x) && aligned16(out) && aligned16(weight) && aligned16(weight_copy) && (!cos_tab || (aligned16(cos_tab) && aligned16(sin_tab))), ANIMA_E_ALIGN,
                 "rmsnorm_rope_fwd: tensors must be 16-byte aligned");
   if (tokens * heads == 0) return ANIMA_OK;
   const int64_t blocks = ceil_div(tokens, kTokensPerCta);
@@ -277,11 +280,18 @@ extern "C" int anima_rmsnorm_rope_fwd_ex(const void* x, const void* weight, int 
   const auto* xp = static_cast<const __nv_bfloat16*>(x);
   auto* op = static_cast<__nv_bfloat16*>(out);
   constexpr int kSmem = kFwdStages * 2 * kThreads * 16;
-  auto go = [&](auto kernel) { launch_after(kernel, grid, kThreads, kSmem, s, xp, weight, cos_tab, sin_tab, eps, tokens, (int)heads, hpg, seq_len, op, rstd); };
+  auto go = [&](auto kernel) { launch_after(kernel, grid, kThreads, kSmem, s, xp, weight, cos_tab, sin_tab, eps, tokens, (int)heads, hpg, seq_len, op, rstd, static_cast<uint4*>(weight_copy)); };
   if (cos_tab) weight_is_bf16 ? go(rmsnorm_rope_fwd_kernel<true, true>) : go(rmsnorm_rope_fwd_kernel<true, false>);
   else weight_is_bf16 ? go(rmsnorm_rope_fwd_kernel<false, true>) : go(rmsnorm_rope_fwd_kernel<false, false>);
   ANIMA_CHECK_LAUNCH("rmsnorm_rope_fwd");
   return ANIMA_OK;
+}
+
+extern "C" int anima_rmsnorm_rope_fwd_ex(const void* x, const void* weight, int weight_is_bf16, const float* cos_tab,
+                                         const float* sin_tab, float eps, int64_t tokens, int64_t heads, int64_t head_dim,
+                                         int64_t seq_len, void* out, float* rstd, void* stream) {
+  return anima_rmsnorm_rope_fwd_keep(x, weight, weight_is_bf16, cos_tab, sin_tab, eps, tokens, heads, head_dim, seq_len, out,
+                                     rstd, nullptr, stream);
 }
 
 extern "C" int anima_rmsnorm_rope_bwd_ex(const void* dout, const void* x, const void* weight, int weight_is_bf16,

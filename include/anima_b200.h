@@ -428,6 +428,12 @@ int anima_rmsnorm_rope_bwd(const void* dout, const void* x, const float* weight,
 int anima_rmsnorm_rope_fwd_ex(const void* x, const void* weight, int weight_is_bf16, const float* cos_tab,
                               const float* sin_tab, float eps, int64_t tokens, int64_t heads,
                               int64_t head_dim, int64_t seq_len, void* out, float* rstd, void* stream);
+/* And the weight as this launch read it, copied to weight_copy (its type, 16-byte aligned; NULL: not): what backward is to
+ * use where the caller's weight may change before it. */
+int anima_rmsnorm_rope_fwd_keep(const void* x, const void* weight, int weight_is_bf16, const float* cos_tab,
+                                const float* sin_tab, float eps, int64_t tokens, int64_t heads,
+                                int64_t head_dim, int64_t seq_len, void* out, float* rstd, void* weight_copy,
+                                void* stream);
 int anima_rmsnorm_rope_bwd_ex(const void* dout, const void* x, const void* weight, int weight_is_bf16,
                               const float* cos_tab, const float* sin_tab, const float* rstd,
                               int64_t tokens, int64_t heads, int64_t head_dim, int64_t seq_len, void* dx,

@@ -258,6 +258,24 @@ def test_output_belongs_to_the_graph_of_a_trainable_tensor_without_a_gradient_ru
     assert grads[0] is None and torch.equal(grads[1], grads[2])
 
 
+@pytest.mark.parametrize("dtype", [BF16, torch.float32])
+@pytest.mark.parametrize("tokens,heads", [(1, 1), (5, 3), (40, 16)])
+def test_norm_weight_changed_before_backward(dtype, tokens, heads):
+    """A bf16 weight is used as forward read it; an fp32 one is a kept tensor, whose change is refused."""
+    from anima_trainer_sm120_b200.qk_norm_rope import FusedRMSNormRoPE
+    g = torch.Generator(device=DEV).manual_seed(tokens)
+    x, gy = _randn(g, 1, tokens, heads, 128).requires_grad_(), _randn(g, 1, tokens, heads, 128)
+    w = (1 + _randn(g, 128, std=0.1, dtype=torch.float32)).to(dtype)
+    want, = torch.autograd.grad(FusedRMSNormRoPE.apply(x, w, None, None, 1e-6), x, gy)
+    y = FusedRMSNormRoPE.apply(x, w, None, None, 1e-6)
+    w.mul_(3)
+    if dtype == BF16:
+        assert torch.equal(torch.autograd.grad(y, x, gy)[0], want)
+    else:
+        with pytest.raises(RuntimeError, match="modified by an inplace operation"):
+            y.backward(gy)
+
+
 class _NoGradient(torch.autograd.Function):
     @staticmethod
     def forward(ctx, t):
