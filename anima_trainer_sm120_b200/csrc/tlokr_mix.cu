@@ -355,8 +355,8 @@ static int rank_mix_quant_impl(const void* hidden, const void* c, const void* ma
   ANIMA_REQUIRE(items % 16 == 0, ANIMA_E_SHAPE, "tlokr_rank_mix_quant: batch * n = %lld must be a multiple of 16",
                 (long long)items);
   ANIMA_REQUIRE(aligned16(hidden) && aligned16(out) && (!mask || aligned16(mask)) &&
-                    (reinterpret_cast<uintptr_t>(codes_row) & 7) == 0 && (reinterpret_cast<uintptr_t>(codes_colT) & 7) == 0,
-                ANIMA_E_ALIGN, "tlokr_rank_mix_quant: misaligned tensor");
+                    (reinterpret_cast<uintptr_t>(codes_row) & 7) == 0 && aligned16(codes_colT),
+                ANIMA_E_ALIGN, "tlokr_rank_mix_quant: misaligned tensor (column codes are stored 16 bytes at a time)");
   if (items == 0) return ANIMA_OK;
   const int r8 = static_cast<int>(rank / 8);
   const unsigned grid = static_cast<unsigned>(items * r8 / 256);

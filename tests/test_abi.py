@@ -70,6 +70,9 @@ def test_argument_errors_are_reported_not_executed(lib):
     assert lib.anima_gated_add_bwd(p16, p16, p16, 8, 4, 64, p16, p16, p16, 16, None) == -6
     # kron factor larger than 8x8
     assert lib.anima_lokr_kron_backward(p16, 0, p16, p16, 0, 1.0, 256, 256, 16, 16, p16, p16, p16, 1 << 20, None) == -5
+    # rank mix: column codes leave in 16-byte stores, row codes in 8-byte ones (checked before the size of an empty batch)
+    assert lib.anima_tlokr_rank_mix_quant(p16, p16, None, 0, 16, 128, 0, None, None, None, p16 + 8, p16, None) == -2
+    assert lib.anima_tlokr_rank_mix_quant(p16, p16, None, 0, 16, 128, 0, None, p16 + 8, p16, p16, p16, None) == 0
     # empty inputs are a no-op success
     assert lib.anima_mx_quantize(p16, 0, 32, 32, p16, p16, None, None, 0, None) == 0
     assert lib.anima_gated_add_fwd(p16, p16, p16, 0, 4, 64, p16, None) == 0
