@@ -472,7 +472,14 @@ int try_quantize_tma(const Loader& load, const void* x, int64_t rows, int64_t co
   const bool row = codes_row != nullptr, col = codes_colT != nullptr;
   QuantParams p{rows, cols, codes_row, scales_row, codes_colT, scales_col, scale_layout == ANIMA_SCALES_TILED};
   const int64_t tiles = ceil_div(rows, static_cast<int64_t>(kTile)) * ceil_div(cols, static_cast<int64_t>(kTile));
-  const unsigned grid = static_cast<unsigned>(std::min<int64_t>(tiles, static_cast<int64_t>(Loader::kTmaCtasPerSm) * sm_count()));
+  // Resident CTAs a SM. Plain row + column quantisation of a tensor well beyond L2 is bound by HBM with as many bytes
+  // written as read; a third CTA then only mixes the two directions more (4.8 TB/s instead of 5.6). Where most of the output
+  // stays in L2 it hides latency and shortens the last round, and the forms that look up GELU need it for their arithmetic.
+  // us with 3 / 2: [32768, 8192] 227.8 / 194.5, [32768, 6144] 169.0 / 144.5, [32768, 2048] 54.0 / 51.7 (4096 tiles);
+  // [24576, 2048] 40.7 / 41.2 (3072 tiles), [16384, 2048] 28.8 / 29.0, [8192, 2048] 15.4 / 20.7. The line is at 3552 tiles.
+  const bool streams = Loader::kIdentity && row && col && tiles >= 24LL * sm_count();
+  const int64_t resident = streams ? std::min(2, Loader::kTmaCtasPerSm) : Loader::kTmaCtasPerSm;
+  const unsigned grid = static_cast<unsigned>(std::min<int64_t>(tiles, resident * sm_count()));
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (row && col) return launch_tma<true, true>(map, p, load, grid, s);
   if (row) return launch_tma<true, false>(map, p, load, grid, s);

@@ -149,6 +149,16 @@ def test_full_size_properties():
     assert bool((err <= step).all())
 
 
+@pytest.mark.parametrize("rows,cols", [(28288, 2048), (28416, 2048), (28448, 2048), (28416, 2016)])
+def test_both_forms_equal_each_form_alone_around_the_resident_cta_rule(rows, cols):
+    """3536, 3552, 3568 tiles of 128 x 128 (24 a SM is 3552), and a ragged last column tile."""
+    ops = _ops()
+    x = _activations(rows, cols, seed=rows).cuda()
+    row, col = ops.mx_quantize(x, rowwise=True, colwise=True)
+    for got, want in ((row, ops.mx_quantize(x, rowwise=True)[0]), (col, ops.mx_quantize(x, rowwise=False, colwise=True)[1])):
+        assert torch.equal(got.codes, want.codes) and torch.equal(got.scales, want.scales)
+
+
 def test_exponent_rule_against_the_references_expression_on_this_gpu(capsys):
     """The reference computes the block exponent as ceil(log2(amax) - log2(448)) in fp32 with the GPU's approximate
     log2 (mxfp8_gemm.py:118-120); the library uses the exact integer rule. Evaluate both on the device for EVERY
