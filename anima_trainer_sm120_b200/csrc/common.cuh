@@ -77,8 +77,8 @@ cudaError_t per_device_once(PerDeviceOnce& st, F&& f) {
 // touches no global memory; EVERY kernel started this way calls it in every CTA, which makes its own completion imply
 // the completion of all work before it on the stream.
 // It saves about 1 us a launch, so it is for short kernels: `overlap` (default: at most eight CTAs a SM). With it on every
-// launch [32768, 2048] x 3 frozen linears took 949 us instead of 930, the AdaLN sequence at [8, 4096, 2048] 580 instead
-// of 571 (early CTAs of the next kernel disturb the last waves of a large one); quantise + GEMM of 1000 rows 41.4 -> 37.8,
+// launch the AdaLN sequence at [8, 4096, 2048] took 580 us instead of 571 (early CTAs of the next kernel disturb the last
+// waves of a large one; K = 2048 GEMMs of 32768 rows lost 2 % the same way); quantise + GEMM of 1000 rows 41.4 -> 37.8,
 // q / k / v of 4096 rows 75.8 -> 70.3, RMSNorm + RoPE of q and k 232 -> 224.
 __device__ __forceinline__ void after_previous() {
   asm volatile("griddepcontrol.wait;" ::: "memory");

@@ -586,7 +586,8 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
 // C = sum over splits of partial[s] (+ bias), four columns per group of kFinalSlices threads: a T-LoKr factor gradient is
 // 8192 such groups over up to 74 splits, which one thread each walked in ten dependent rounds of loads. Slice q of a group
 // adds its contiguous share of the splits in ascending order, then the slices are added in ascending order: a fixed
-// association, so the result is reproducible. [256, 128] over K = 262144 (GEMM and finalize): 31.7 -> 26.9 us.
+// association, so the result is reproducible. GEMM and finalize over K = 262144, each launch after an L2 rewrite, us: [256, 128]
+// 32.3 -> 28.7, [128, 256] 39.4 -> 33.3, [1024, 128] 65.5 either way (on a GPU hot from minutes of GEMMs 34 / 40 / 75).
 constexpr int kFinalSlices = 8;
 __global__ void __launch_bounds__(256) splitk_finalize_kernel(const GemmParams p) {
   __shared__ float4 sums[kFinalSlices][32];

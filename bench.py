@@ -361,10 +361,14 @@ def run_gpu_arm(args) -> None:
     _lib.check_status_word(dev)
     n_launch = launches[1] - launches[0]
     timed_steps = 4
+    probe.zero_()                                                 # the clock of these launches, for their utilisation
+    _lib.check(_lib.load().anima_mx_gemm_set_clock_probe(probe.data_ptr()))
     _lib.host().time_gemms(True)
     for _ in range(timed_steps):
         step(False)
     _lib.host().time_gemms(False)
+    _lib.check(_lib.load().anima_mx_gemm_set_clock_probe(None))
+    gemm_cycles, gemm_ns = (int(v) for v in probe.cpu().tolist()[:2])
     gemms = _lib.host().gemm_times()
     n_gemm = len(gemms) // timed_steps                            # a step
     gemm_ms = sum(ms for ms, _ in gemms) / timed_steps
@@ -464,11 +468,11 @@ def run_gpu_arm(args) -> None:
                          "frac_of_nominal_4500": achieved / 4500.0,
                          "sm_mhz_in_kernel": round(1000.0 * probe_cycles / probe_ns, 1) if probe_ns else None,
                          "tensor_pipe_util_at_that_clock": (
-                             achieved * 1e12 / (sm_count * 16384.0 * (probe_cycles / probe_ns) * 1e9)
-                             if probe_ns else None),
+                             achieved * 1e12 / (sm_count * 16384.0 * (gemm_cycles / gemm_ns) * 1e9)
+                             if gemm_ns else None),
                          "in_kernel_clock_note": ("SM cycles / ns summed by CTA 0 over the timed region's (warm-up "
                                                   "included) GEMM launches; util = achieved / (SMs x 8192 MAC/clk x "
-                                                  "that clock): the kernel runs under the power cap, below the "
+                                                  "the clock of the event-timed launches): the kernel runs under the power cap, below the "
                                                   "clock nvidia-smi samples between launches"),
                          "launches": n_gemm * args.steps, "avg_launch_ms": gemm_ms / n_gemm,
                          "gemm_share_of_step": gemm_ms / ms_step},
