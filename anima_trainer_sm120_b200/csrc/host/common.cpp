@@ -240,6 +240,7 @@ std::vector<std::pair<double, double>> gemm_times() {
     t->end.synchronize();
     out.emplace_back(t->begin.elapsed_time(t->end), t->flops);
   }
+  timed.clear();
   return out;
 }
 

@@ -117,7 +117,8 @@ std::pair<Op, Op> merge_quantize(const Launch& l, const Tensor& W, const Tensor&
                                  bool row, bool col);
 
 // Measurement aid: while on, every GEMM of this path is bracketed by timed events on its stream (which also keeps it from
-// overlapping its neighbours; not for captures). gemm_times: (ms, flops) of each since it was switched on, oldest first.
+// overlapping its neighbours; not for captures). gemm_times: (ms, flops) of each since it was switched on, oldest first, which
+// are then forgotten.
 void time_gemms(bool on);
 std::vector<std::pair<double, double>> gemm_times();
 
