@@ -20,7 +20,7 @@ Tensor back_to(const Tensor& t, at::ScalarType dt) { return t.defined() ? cast(t
 
 // The modulation tensors of one call as the kernels take them: bf16 rows of d with one pitch. (B, T, 1, 1, d) tensors, also
 // chunks of a wider tensor (what a modulation MLP returns), are used where they lie; any other shape with as many elements
-// is read in order, as dense rows.
+// is read in order, as dense rows. Backward asks again for what it unpacks: a saved-tensor hook may hand a chunk back dense.
 struct Mods {
   std::vector<Tensor> t;
   int64_t ld;
@@ -104,7 +104,6 @@ std::pair<Tensor, Tensor> gated_bwd(const Launch& l, const Tensor& dout_, const 
 // modulation (every sublayer does) takes its x from there, so its gradient arrives here and dx = that + dx_ln is one
 // kernel instead of two and an addition (3 passes over a gradient). Values are those of the separate addition.
 struct AdalnNode : public HostNode {      // saves x, scale, statistics
-  int64_t ld;
   at::ScalarType dt_x, dt_scale, dt_shift;
   bool used = false;
 
@@ -118,8 +117,9 @@ struct AdalnNode : public HostNode {      // saves x, scale, statistics
     used = true;
     const Tensor x = get(0), scale = get(1), stats = get(2);
     const Launch l(x);
+    const Mods m = mods_of(x.size(-1), {&scale});
     const bool mod = task_should_compute_output(1) || task_should_compute_output(2);
-    auto [dx, ds, db] = adaln_bwd(l, grad_of(g, 0), g[1], x, scale, ld, stats, mod);
+    auto [dx, ds, db] = adaln_bwd(l, grad_of(g, 0), g[1], x, m.t[0], m.ld, stats, mod);
     out[0] = back_to(dx, dt_x);
     out[1] = back_to(ds, dt_scale);
     out[2] = back_to(db, dt_shift);
@@ -156,14 +156,14 @@ Tensor gated_fwd(const Launch& l, const Tensor& x_, const Tensor& y, const Mods&
 }
 
 struct GatedNode : public HostNode {      // saves y, gate
-  int64_t ld;
   at::ScalarType dt_gate, dt_y;
 
   variable_list apply(variable_list&& g) override {
     std::lock_guard<std::mutex> lock(mutex_);
     const Tensor dout = grad_of(g, 0), y = get(0), gate = get(1);
     const Launch l(y);
-    auto [dy, dg] = gated_bwd(l, dout, y, gate, ld, task_should_compute_output(1));
+    const Mods m = mods_of(y.size(-1), {&gate});
+    auto [dy, dg] = gated_bwd(l, dout, y, m.t[0], m.ld, task_should_compute_output(1));
     return {dout, back_to(dg, dt_gate), back_to(dy, dt_y)};
   }
   std::string name() const override { return "FusedGatedAddBackward"; }
@@ -190,15 +190,17 @@ Both both_fwd(const Launch& l, const Tensor& x_, const Tensor& gate, const Tenso
 }
 
 struct BothNode : public HostNode {      // saves sub, gate, x_new, scale, statistics
-  int64_t ld;
   at::ScalarType dt_gate, dt_sub, dt_scale, dt_shift;
 
   variable_list apply(variable_list&& grads) override {
     std::lock_guard<std::mutex> lock(mutex_);
     variable_list out(5);
     const Tensor &d_y = grads[1], d_xnew = grads[0].defined() || d_y.defined() ? grads[0] : grad_of(grads, 0);
-    const Tensor sub = get(0), gate = get(1), x_new = get(2), scale = get(3), stats = get(4);
+    const Tensor sub = get(0), x_new = get(2), stats = get(4), saved_gate = get(1), saved_scale = get(3);
     const Launch l(x_new);
+    const Mods m = mods_of(x_new.size(-1), {&saved_gate, &saved_scale});
+    const Tensor &gate = m.t[0], &scale = m.t[1];
+    const int64_t ld = m.ld;
     const bool mod = task_should_compute_output(1) || task_should_compute_output(3) || task_should_compute_output(4);
     Tensor dx, dsub, dscale, dshift, dgate;
     if (d_xnew.defined() && d_y.defined()) {      // the usual case: one kernel for both backward ops
@@ -279,7 +281,6 @@ std::tuple<Tensor, Op> adaln(const Tensor& x, const Tensor& scale, const Tensor&
     node->save(o.x);
     node->save(o.mods.t[0]);
     node->save(o.stats);
-    node->ld = o.mods.ld;
     node->dt_x = x.scalar_type();
     node->dt_scale = scale.scalar_type();
     node->dt_shift = shift.scalar_type();
@@ -307,7 +308,6 @@ Tensor gated_add(const Tensor& x_, const Tensor& gate, const Tensor& y) {
     auto node = make_node<GatedNode>(x, gate, y);
     node->save(yc);
     node->save(g.t[0]);
-    node->ld = g.ld;
     node->dt_gate = gate.scalar_type();
     node->dt_y = y.scalar_type();
     set_history(out, node);
@@ -335,7 +335,6 @@ std::tuple<Tensor, Tensor, Op> gated_add_adaln(const Tensor& x_, const Tensor& g
     node->save(c.x_new, true);
     node->save(c.mods.t[1]);
     node->save(c.stats);
-    node->ld = c.mods.ld;
     node->dt_gate = gate.scalar_type();
     node->dt_sub = sub.scalar_type();
     node->dt_scale = scale.scalar_type();

@@ -3,6 +3,8 @@ gradients, the no-grad forward and the checkpointed form must give the bits of t
 same operands), so the comparisons are exact."""
 from __future__ import annotations
 
+import contextlib
+
 import pytest
 import torch
 from torch.utils.checkpoint import checkpoint
@@ -274,6 +276,35 @@ def test_norm_weight_changed_before_backward(dtype, tokens, heads):
     else:
         with pytest.raises(RuntimeError, match="modified by an inplace operation"):
             y.backward(gy)
+
+
+@pytest.mark.parametrize("chunked", [False, True])
+def test_saved_tensors_moved_by_hooks_give_the_same_gradients(chunked):
+    """save_on_cpu hands every saved tensor back dense: also the chunks of one modulation tensor, whose rows had a pitch."""
+    from anima_trainer_sm120_b200.adaln_kernel import fused_adaln, fused_gated_add, fused_gated_add_adaln
+    results = []
+    for moved in (False, True):
+        x, sub, (g0, sc, sh, sc1), (gn, gx, gy) = _block_inputs(3, 40, 256, True, chunked)
+        with torch.autograd.graph.save_on_cpu() if moved else contextlib.nullcontext():
+            outs = [fused_adaln(x, sc, sh, 1e-6), *fused_gated_add_adaln(x, g0, sub, sc1, sh, 1e-6),
+                    fused_gated_add(x.detach(), g0, sub)]
+        results.append(torch.autograd.grad(outs, [x, sub, g0, sc, sh, sc1], [gn, gx, gy, gx]))
+    assert all(torch.equal(a, b) for a, b in zip(*results))
+
+
+@pytest.mark.parametrize("make,rows", [(_lokr, 160), (_merged, 96), (_mlp, 64), (_tlokr, 128), (_tlokr_mlp, 128)])
+def test_saved_operands_moved_by_hooks_give_the_same_gradients(make, rows):
+    from anima_trainer_sm120_b200 import fp8_quant
+    fn, ts, out_shape = make(rows)
+    gy = _randn(torch.Generator(device=DEV).manual_seed(1), *out_shape)
+    results = []
+    for moved in (False, True):
+        fp8_quant.clear_activation_memo()
+        leaves = [t.clone().requires_grad_() for t in ts]
+        with torch.autograd.graph.save_on_cpu() if moved else contextlib.nullcontext():
+            y = fn(*leaves)
+        results.append(torch.autograd.grad(y, leaves, gy))
+    assert all(torch.equal(a, b) for a, b in zip(*results))
 
 
 class _NoGradient(torch.autograd.Function):
